@@ -228,7 +228,7 @@ struct Handle {
   // batched Cholesky workspace (dense blocks X, Y and line-search trials)
   DBuf<MatDesc<double>> d_descs;
   DBuf<int> d_info;
-  DBuf<unsigned> coop_bar;  // grid-barrier state of the single-launch Schur Cholesky
+  DBuf<unsigned> flow_flags;  // tile flags of the Cholesky launches
   DBuf<double> d_dmin, d_dmax;
   size_t desc_cap = 0;
   DBuf<double> trials;
@@ -501,18 +501,21 @@ struct Handle {
     double* sdmin = d_stats.p;
     double* sdmax = d_stats.p + n;
     int* sinfo = reinterpret_cast<int*>(d_stats.p + 2 * n);
-    if (nmax >= 192 && zero_upper)
-      potrf_batched<double, 64>(d_descs.p, (int)n, nmax, sinfo, sdmin, sdmax, st, zero_upper);
-    else if (nmax >= 192)
-      potrf_batched<double, 48>(d_descs.p, (int)n, nmax, sinfo, sdmin, sdmax, st, zero_upper);
-    else
-      potrf_batched<double, 32>(d_descs.p, (int)n, nmax, sinfo, sdmin, sdmax, st, zero_upper);
+    potrf_flow(d_descs.p, (int)n, nmax, sinfo, sdmin, sdmax, flow_flags_for((int)n, nmax), sms, st,
+               zero_upper);
     d2h(hp + dbytes, d_stats.p, sbytes);
     sync();
     const double* hs = reinterpret_cast<const double*>(hp + dbytes);
     std::memcpy(dmin.data(), hs, n * sizeof(double));
     std::memcpy(dmax.data(), hs + n, n * sizeof(double));
     std::memcpy(info.data(), hs + 2 * n, n * sizeof(int));
+    for (int v : info)
+      if (v < 0) throw CudaError("Cholesky: a wait for a tile gave up");
+  }
+  unsigned* flow_flags_for(int nmat, int nmax) {  // potrf_flow's flag words
+    const size_t need = potrf_flow_flag_words(nmat, nmax);
+    if (flow_flags.n < need) flow_flags.alloc(2 * need);
+    return flow_flags.p;
   }
 
   // ------------------------------------------------------------ create ----
@@ -1335,15 +1338,9 @@ struct Handle {
     int att = 0;
     while (true) {
       copy_reg(m, S.p, Sf.p, att == 0 ? 0.0 : reg, st);
-      if (potrf_single_pays<double, 64>(m)) {
-        if (coop_bar.n < 4) coop_bar.alloc(4);
-        potrf_single<double, 64>(Sf.p, m, m, d_info.p, d_dmin.p, d_dmax.p,
-                                 reinterpret_cast<CoopBar*>(coop_bar.p), true, st);
-      } else {
-        ensure_descs(1);
-        h2d(d_descs.p, &md, sizeof(md));
-        potrf_batched<double, 64>(d_descs.p, 1, m, d_info.p, d_dmin.p, d_dmax.p, st);
-      }
+      ensure_descs(1);
+      h2d(d_descs.p, &md, sizeof(md));
+      potrf_flow(d_descs.p, 1, m, d_info.p, d_dmin.p, d_dmax.p, flow_flags_for(1, m), sms, st);
       info.resize(1);
       dmn.resize(1);
       dmx.resize(1);
@@ -1351,7 +1348,7 @@ struct Handle {
       d2h(dmn.data(), d_dmin.p, sizeof(double));
       d2h(dmx.data(), d_dmax.p, sizeof(double));
       sync();
-      if (info[0] < 0) throw CudaError("Schur Cholesky: a grid barrier timed out");
+      if (info[0] < 0) throw CudaError("Schur Cholesky: a wait for a tile gave up");
       if (info[0] == 0 || att >= 6) break;
       ++att;
       reg = (att == 1) ? kSqrtEps : reg * 10.0;

@@ -22,38 +22,23 @@ template <class T, int NB>
 void potrf_batched(const MatDesc<T>* d_mats, int nmat, int nmax, int* info, T* dmin, T* dmax,
                    cudaStream_t st, bool zero_upper = true);
 
-// Grid-barrier state of one potrf_single call site (device memory, 16 bytes).
-struct CoopBar {
-  unsigned count, gen, err, fail;
-};
-
-// Lower Cholesky in place of one n×n matrix (leading dimension ld) in a single
-// cooperative launch, for orders above the whole-panel shared-memory size.
-// info[0] = 0 on success, the 1-based failing pivot, or −1 when a grid
-// barrier timed out (the call site's `bar` must not be shared by concurrent
-// calls).  dmin/dmax: min/max |L_ii|.
-template <class T, int NB>
-void potrf_single(T* a, int n, int ld, int* info, T* dmin, T* dmax, CoopBar* bar, bool zero_upper,
-                  cudaStream_t st);
-
-// Whether potrf_single is the faster path for one matrix of order n: FP64
-// orders above the whole-panel shared-memory size (measured on the B200 with
-// identical factors: 0.88 vs 0.93 ms at n = 1000, 1.78 vs 1.99 ms at 2000,
-// 3.09 vs 3.26 ms at 3000; below that size, and in FP32, the batched path is
-// as fast or faster).
-template <class T, int NB>
-inline bool potrf_single_pays(int n) {
-  return sizeof(T) == 8 && sizeof(T) * (size_t)(n | 1) * NB > 224 * 1024;
-}
+// The same for FP64 matrices in one launch (potrf_flow.cu): a CTA per matrix
+// runs the pivot chain, sms/nmat − 1 others its remaining tiles, ordered by tile
+// flags.  `flags` (potrf_flow_flag_words(nmat, nmax) words) must not be shared by
+// concurrent calls.  info[b] = −1 when a wait for a tile gave up (about a second).
+size_t potrf_flow_flag_words(int nmat, int nmax);
+void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, double* dmin,
+                double* dmax, unsigned* flags, int sms, cudaStream_t st, bool zero_upper = true);
 
 // W_b = L_b^{-1} for lower-triangular L_b (W zero-initialised by the caller).
 template <class T, int NB>
 void trinv_batched(const MatDesc<T>* d_L, const MatDesc<T>* d_W, int nmat, int nmax,
                    cudaStream_t st);
 
-// Inverses of the NB×NB diagonal tiles of a lower factor L (n×n): Dinv[s] (NB×NB, col-major).
-template <class T, int NB>
-void factor_diag_inverses(const T* L, long long ld, int n, T* Dinv, cudaStream_t st);
+// Inverses of the 64×64 diagonal tiles of a lower factor L (n×n): Dinv[s]
+// (64×64, column-major), and into the diagonal tiles of Linv (n×n) unless null.
+void factor_diag_inverses(const double* L, long long ld, int n, double* Dinv, double* Linv,
+                          cudaStream_t st);
 
 // rhs ← (L Lᵀ)^{-1} rhs by blocked forward/backward substitution (work: n).
 template <class T, int NB>

@@ -286,7 +286,7 @@ struct NormalHandle {
   std::vector<int> cone_dim;
   DBuf<long long> d_off;
   DBuf<int> d_dim, d_row, d_ok, d_info;
-  DBuf<unsigned> coop_bar;  // grid-barrier state of the single-launch Cholesky
+  DBuf<unsigned> flow_flags;  // tile flags of the Cholesky launch
   DBuf<double> B, Bh, coef, weights, D, Dinv, Dis, w, lam, eta, eta2, s, z, v, out;
   DBuf<double> Q, F, Finv_diag, partial, rhs, t, red, work, u, gemv_part;
   DBuf<double> dmin, dmax;
@@ -573,7 +573,7 @@ struct NormalHandle {
       SDPX_CUDA(cudaEventRecord(ev[2], st));
       d2h(&info, d_info.p, sizeof(int));
       sync();
-      if (info < 0) throw CudaError("normal-matrix Cholesky: a grid barrier timed out");
+      if (info < 0) throw CudaError("normal-matrix Cholesky: a wait for a tile gave up");
       float a = 0.f, f = 0.f;
       SDPX_CUDA(cudaEventElapsedTime(&a, ev[0], ev[1]));
       SDPX_CUDA(cudaEventElapsedTime(&f, ev[1], ev[2]));
@@ -587,24 +587,19 @@ struct NormalHandle {
     assemble_ms = asm_ms;
     factor_ms = fac_ms;
     if (info != 0) return 1;
-    if (m > 0) factor_diag_inverses<double, 64>(F.p, m, m, Finv_diag.p, st);
+    if (m > 0) factor_diag_inverses(F.p, m, m, Finv_diag.p, nullptr, st);
     sync();
     have_factor = true;
     return 0;
   }
 
-  // Cholesky of the reduced matrix F in place: one cooperative launch above the
-  // whole-panel size, the batched panels below it (identical factors).
+  // Cholesky of the reduced matrix F in place.
   void factor_F() {
-    if (potrf_single_pays<double, 64>(m)) {
-      if (coop_bar.n < 4) coop_bar.alloc(4);
-      potrf_single<double, 64>(F.p, m, m, d_info.p, dmin.p, dmax.p,
-                               reinterpret_cast<CoopBar*>(coop_bar.p), true, st);
-      return;
-    }
     MatDesc<double> md{F.p, m, m};
     h2d(descs.p, &md, sizeof(md));
-    potrf_batched<double, 64>(descs.p, 1, m, d_info.p, dmin.p, dmax.p, st);
+    const size_t need = potrf_flow_flag_words(1, m);
+    if (flow_flags.n < need) flow_flags.alloc(need);
+    potrf_flow(descs.p, 1, m, d_info.p, dmin.p, dmax.p, flow_flags.p, sms, st);
   }
 
   // One assembly + Cholesky attempt with LP weights already on the device
@@ -629,9 +624,9 @@ struct NormalHandle {
     int info = 1;
     d2h(&info, d_info.p, sizeof(int));
     sync();
-    if (info < 0) throw CudaError("normal-matrix Cholesky: a grid barrier timed out");
+    if (info < 0) throw CudaError("normal-matrix Cholesky: a wait for a tile gave up");
     if (info != 0) return 1;
-    factor_diag_inverses<double, 64>(F.p, m, m, Finv_diag.p, st);
+    factor_diag_inverses(F.p, m, m, Finv_diag.p, nullptr, st);
     if (split) make_inverse();
     have_factor = true;
     return 0;
