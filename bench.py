@@ -1015,11 +1015,11 @@ def run_ours(args, world, rank, local):
                               f"(the reference arm times that complete solve)")}
         line = {
             "metric": metric_name(wl),
-            "path": "mixed precision (split-BF16 Schur, FP32 factor, FP64 refinement, FP64 tail)",
+            "path": "mixed precision (split-BF16 Schur, FP64 factor and refinement, FP64 tail)",
             "value": ms_per_step / 1000.0, "unit": "s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": False,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "f64 in/out; Schur assembly mode per precision_trace, FP32 factor, FP64 refinement",
+            "dtype": "f64 in/out; Schur assembly mode per precision_trace, FP64 factor and refinement",
             "data": "synthetic",
             "config": workload_config(wl),
             "status": last.status.value, "iterations": last.iterations,

@@ -43,7 +43,7 @@ typedef struct {
 
 /* Precision modes of the Newton system. */
 #define SDPX_B200_FP64 0  /* plain FP64 Schur assembly and Cholesky                */
-#define SDPX_B200_MIXED 1 /* split-BF16 Schur assembly, FP32 Cholesky, FP64 refine  */
+#define SDPX_B200_MIXED 1 /* split-BF16 Schur assembly, FP64 Cholesky, FP64 refine  */
 
 int sdpx_b200_abi_version(void);
 /* Message of the last failed sdpx_b200_create on this thread. */
@@ -57,7 +57,7 @@ void sdpx_b200_destroy(sdpx_b200_handle* h);
 const char* sdpx_b200_last_error(const sdpx_b200_handle* h);
 int sdpx_b200_set_precision(sdpx_b200_handle* h, int mode);
 /* Current precision mode (mixed mode switches itself to FP64 when the guard
- * fails), number of such switches, and the last FP32-factor condition estimate. */
+ * fails), number of such switches, and the last mixed-mode factor condition estimate. */
 int sdpx_b200_get_precision(sdpx_b200_handle* h, int* mode, int* fallbacks, double* cond_estimate);
 
 /* Ruiz + per-variable + objective scaling of the resident data in place
@@ -115,7 +115,7 @@ int sdpx_b200_solve(sdpx_b200_handle* h);
 int sdpx_b200_direction_residual(sdpx_b200_handle* h, double* residual, double* rnorm);
 /* Residual-driven refinement with rollback (`_refine_native_direction!`,
  * src/kkt.jl:3891-3963).  policy: 0 fixed, 1 adaptive/auto; tol ≤ 0 selects
- * 64·eps.  In mixed mode the correction solves use the FP32 factor and the
+ * 64·eps.  In mixed mode the correction solves use the factor of the split S and the
  * residual is the FP64 Newton residual. */
 int sdpx_b200_refine(sdpx_b200_handle* h, int policy, double tol, int cap, int fixed_steps,
                      int* steps, double* residual);
@@ -174,7 +174,7 @@ int sdpx_b200_original_residuals(sdpx_b200_handle* h, const double* x, const dou
  * update, objectives, the cold start and the equilibration carry the B, b, y
  * terms of src/step.jl:25-72, src/kkt.jl:3689-3708 and
  * src/solver/interior_point.jl:699-1311 once they are set.  In the mixed
- * precision mode B̃ comes from the FP32 factor and Q is factored in FP64 with
+ * precision mode B̃ comes from the factor of the split S and Q is factored in FP64 with
  * up to 8 diagonal regularisations (src/kernels/mixed_precision_kkt.jl:481-520,
  * 1045-1082); the guard refines against the FP64 KKT operator with the B terms. */
 

@@ -215,7 +215,7 @@ struct Handle {
   DBuf<double> seg_part;           // seg_dot partials
   int seg_parts = 8;
   double last_bpr = 0.0;
-  int mixed_predicted_steps = 32;  // from the last FP32 factor's condition estimate
+  int mixed_predicted_steps = 32;  // from the last mixed factor's condition estimate
   long long mixed_guard_steps = 0;
   long long operator_applications = 0;  // matrix-free FP64 Newton operator (mixed mode)
   long long schur_builds = 0;
@@ -1305,6 +1305,39 @@ struct Handle {
   }
 
   // ------------------------------------------------------- factorisation --
+  // Sf ← Cholesky of S, with ≤ 6 regularised retries; returns the retries.
+  int factor_S(int* ok, double* lo, double* hi) {
+    MatDesc<double> md{Sf.p, m, m};
+    double reg = 0.0;
+    int att = 0, info = 0;
+    ensure_descs(1);
+    while (true) {
+      copy_reg(m, S.p, Sf.p, att == 0 ? 0.0 : reg, st);
+      h2d(d_descs.p, &md, sizeof(md));
+      potrf_flow(d_descs.p, 1, m, d_info.p, d_dmin.p, d_dmax.p, flow_flags_for(1, m), sms, st);
+      d2h(&info, d_info.p, sizeof(int));
+      d2h(lo, d_dmin.p, sizeof(double));
+      d2h(hi, d_dmax.p, sizeof(double));
+      sync();
+      if (info < 0) throw CudaError("Schur Cholesky: a wait for a tile gave up");
+      if (info == 0 || att >= 6) break;
+      ++att;
+      reg = (att == 1) ? kSqrtEps : reg * 10.0;
+    }
+    *ok = info == 0 ? 1 : 0;
+    return att;
+  }
+  // Solves with the factor are applied 3-5 times per iteration (predictor,
+  // corrector, refinement corrections; more in mixed mode), so L is inverted once
+  // (recursive doubling on the DMMA tiles) and each solve is two GEMVs instead of
+  // 2·ceil(m/64) dependent substitution launches; the FP64 refinement follows.
+  void invert_factor() {
+    if (Linv.n < (size_t)m * m) {
+      Linv.alloc((size_t)m * m);
+      tmp_mm.alloc((size_t)m * m);
+    }
+    trinv_recursive_f64(Sf.p, m, Linv.p, Dinv.p, tmp_mm.p, st);
+  }
   void factorize(int* ok, int* attempts, double* quality) {
     PhaseScope ps(this, 2);
     if (precision == SDPX_B200_MIXED && mixed) {
@@ -1324,50 +1357,17 @@ struct Handle {
         }
       }
       if (*ok && mixed_predicted_steps <= 32) return;
-      // Static rejection: the FP32 factor of the split-assembled S is not
+      // Static rejection: the factor of the split-assembled S is not
       // predicted to converge in ≤ 32 refinements (or failed) — FP64 from here.
       precision = SDPX_B200_FP64;
       ++mixed_fallbacks;
       schur_build_fp64(identity_metric ? 1 : 0);
     }
-    MatDesc<double> md{Sf.p, m, m};
-    std::vector<MatDesc<double>> one{md};
-    std::vector<int> info;
-    std::vector<double> dmn, dmx;
-    double reg = 0.0;
-    int att = 0;
-    while (true) {
-      copy_reg(m, S.p, Sf.p, att == 0 ? 0.0 : reg, st);
-      ensure_descs(1);
-      h2d(d_descs.p, &md, sizeof(md));
-      potrf_flow(d_descs.p, 1, m, d_info.p, d_dmin.p, d_dmax.p, flow_flags_for(1, m), sms, st);
-      info.resize(1);
-      dmn.resize(1);
-      dmx.resize(1);
-      d2h(info.data(), d_info.p, sizeof(int));
-      d2h(dmn.data(), d_dmin.p, sizeof(double));
-      d2h(dmx.data(), d_dmax.p, sizeof(double));
-      sync();
-      if (info[0] < 0) throw CudaError("Schur Cholesky: a wait for a tile gave up");
-      if (info[0] == 0 || att >= 6) break;
-      ++att;
-      reg = (att == 1) ? kSqrtEps : reg * 10.0;
-    }
-    *attempts = att;
-    *ok = info[0] == 0 ? 1 : 0;
-    double hi = dmx[0], lo = dmn[0];
+    double lo = 0.0, hi = 0.0;
+    *attempts = factor_S(ok, &lo, &hi);
     *quality = (*ok && hi > 0 && std::isfinite(hi)) ? std::min(1.0, std::max(0.0, lo / hi)) : 0.0;
     if (*ok) {
-      // Solves with the FP64 factor are applied 3-5 times per iteration
-      // (predictor, corrector, refinement corrections), so L is inverted once
-      // (recursive doubling on the DMMA tiles) and each solve is two GEMVs
-      // instead of 2·ceil(m/64) dependent substitution launches; the FP64
-      // refinement against S follows as before.
-      if (Linv.n < (size_t)m * m) {
-        Linv.alloc((size_t)m * m);
-        tmp_mm.alloc((size_t)m * m);
-      }
-      trinv_recursive_f64(Sf.p, m, Linv.p, Dinv.p, tmp_mm.p, st);
+      invert_factor();
       if (n_eq) {
         bool rank_deficient = false;
         if (!factor_equality(&rank_deficient)) {
@@ -1384,10 +1384,6 @@ struct Handle {
 
   // ------------------------------------------------------------- solves ----
   void solve_into(double* vec) {  // vec ← S⁻¹ vec with the current factor
-    if (precision == SDPX_B200_MIXED && mixed) {
-      mixed_solve(vec);
-      return;
-    }
     gemv_n(Linv.p, m, m, vec, work_m2.p, gemv_part.p, gemv_chunks, st);
     gemv_t(Linv.p, m, m, work_m2.p, 1.0, nullptr, 0.0, vec, st);
   }
@@ -2593,7 +2589,6 @@ struct Handle {
   void mixed_check_err();
   void schur_split_bf16(bool identity);
   void mixed_factorize(int* ok, int* attempts, double* quality);
-  void mixed_solve(double* vec);
   void mixed_residual();
 
   // ------------------------------------------- equality rows (n > 0) ------
@@ -2601,7 +2596,7 @@ struct Handle {
   // y.  p = b − Bᵀx, ρ_p = p − Bᵀdx.  The equality factor is either the
   // Cholesky of Q = B̂ᵀB̂ (eq_kind 1) or the column-pivoted QR of B̂ (eq_kind
   // 2, kept for the rest of the solve once used), B̂ = L_S⁻¹B·D with D the
-  // column scales.  In mixed mode L_S is the FP32 factor and Q's Cholesky takes
+  // column scales.  In mixed mode L_S is the split S's factor and Q's Cholesky takes
   // regularisation retries instead of the rank test.
   int n_eq = 0;
   DBuf<double> Beq, Beq0, beq;

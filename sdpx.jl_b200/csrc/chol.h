@@ -14,18 +14,14 @@ struct MatDesc {
 };
 
 // Lower Cholesky in place of every matrix in d_mats (device array of nmat
-// descriptors, largest order nmax).  info[b] = 0 on success, else the 1-based
-// index of the first non-positive pivot.  dmin/dmax receive min/max |L_ii|.
-// The strict upper triangle is zeroed unless zero_upper is false (positive-
-// definiteness tests that only read info/dmin/dmax).
-template <class T, int NB>
-void potrf_batched(const MatDesc<T>* d_mats, int nmat, int nmax, int* info, T* dmin, T* dmax,
-                   cudaStream_t st, bool zero_upper = true);
-
-// The same for FP64 matrices in one launch (potrf_flow.cu): a CTA per matrix
+// descriptors, largest order nmax), one launch (potrf_flow.cu): a CTA per matrix
 // runs the pivot chain, sms/nmat − 1 others its remaining tiles, ordered by tile
-// flags.  `flags` (potrf_flow_flag_words(nmat, nmax) words) must not be shared by
-// concurrent calls.  info[b] = −1 when a wait for a tile gave up (about a second).
+// flags.  info[b] = 0 on success, else the 1-based index of the first non-positive
+// pivot (the no-throw contract of SDPX's `kchol!`, src/kernels/generic.jl:133-155),
+// or −1 when a wait for a tile gave up (about a second).  dmin/dmax receive min/max
+// |L_ii|.  The strict upper triangle is zeroed unless zero_upper is false (positive-
+// definiteness tests that only read info/dmin/dmax).  `flags`
+// (potrf_flow_flag_words(nmat, nmax) words) must not be shared by concurrent calls.
 size_t potrf_flow_flag_words(int nmat, int nmax);
 void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, double* dmin,
                 double* dmax, unsigned* flags, int sms, cudaStream_t st, bool zero_upper = true);

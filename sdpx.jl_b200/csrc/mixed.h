@@ -1,5 +1,5 @@
-// Mixed-precision workspace of the B200 core: FP32 factor of the Schur
-// complement and buffers of the split-BF16 Schur assembly.
+// Mixed-precision workspace of the B200 core: the buffers of the split-BF16
+// Schur assembly.
 #pragma once
 #include <vector>
 
@@ -25,18 +25,6 @@ struct MixedWorkspace {
   void* Lpl[3] = {nullptr, nullptr, nullptr};
   float* partial = nullptr;
   int* err = nullptr;
-  double* L64 = nullptr;    // FP32 factor promoted to FP64
-  double* Linv = nullptr;   // explicit inverse of the factor (preconditioner apply)
-  double* Dinv64 = nullptr;
-  double* tmp64 = nullptr;
-  float* Sf = nullptr;      // m×m FP32 factor
-  float* Dinv = nullptr;    // FP32 inverses of the 64×64 diagonal tiles
-  float* v32 = nullptr;     // m
-  float* w32 = nullptr;     // m
-  int* info = nullptr;
-  float* dmin = nullptr;
-  float* dmax = nullptr;
-  void* desc = nullptr;
   double cond_estimate = 1.0;
   // The device blocks behind the pointers above come from the process-wide
   // cache of idle device blocks, so a handle created and destroyed per solve
@@ -52,10 +40,5 @@ struct MixedWorkspace {
     ptr = static_cast<P*>(static_cast<void*>(blocks[n_blocks++].p));
   }
 };
-
-// FP64 ↔ FP32 conversions and the regularised FP32 copy of the lower S.
-void copy_reg_f32(int m, const double* S, float* Sf, double reg, cudaStream_t st);
-void f64_to_f32(long long n, const double* a, float* b, cudaStream_t st);
-void f32_to_f64(long long n, const float* a, double* b, cudaStream_t st);
 
 }  // namespace sdpx

@@ -32,7 +32,7 @@ def solve(prob: SDPProblem, *, tolerance: float = 1e-8, precision: str = "fp64",
 
     `precision="fp64"` is the plain FP64 device path; `precision="mixed"`
     assembles the Schur complement with split-BF16 tensor-core products, factors
-    it in FP32 and refines the Newton system in FP64, switching to the FP64 path
+    it and refines the Newton system in FP64, switching to the FP64 path
     when the condition estimate or the stagnation detector calls for it.
     `certificate=True` attaches the device-computed cold-path certificate
     (`result.certificate`) before the device data is released.  The loop runs

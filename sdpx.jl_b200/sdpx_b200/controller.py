@@ -64,7 +64,7 @@ class SolverOptions:
     equality_solver: str = "auto"
     verbosity: int = 0
     # B200 precision mode: "fp64" (plain FP64 device path) or "mixed"
-    # (split-BF16 Schur assembly + FP32 factor + FP64 refinement, FP64 switch).
+    # (split-BF16 Schur assembly + its FP64 factor + FP64 refinement, FP64 switch).
     precision: str = "fp64"
     mixed_condition_limit: float = 1e8
 
