@@ -29,6 +29,7 @@
 #include "dbuf.h"
 #include "equality.h"
 #include "sparse_schur.h"
+#include "step_bound.h"
 #include "dd_kernels.h"
 #include "mixed.h"
 #include "ozaki.h"
@@ -105,7 +106,7 @@ struct Handle {
 
   // iterate and workspaces
   DBuf<double> x, dx, d, v, r, rho, work_m, work_m2, xbest, keptx, dxbest;
-  DBuf<double> X, Y, P, R, Z, dX, dY, LX, MY, W, T1, T2, Xbest, Ybest, tmpK, tmpK2;
+  DBuf<double> X, Y, P, R, Z, dX, dY, LX, MY, W, WY, T1, T2, Xbest, Ybest, tmpK, tmpK2;
   DBuf<double> gemv_part;
   int gemv_chunks = 8;
   // Lower-triangle copy of 𝒜 for the memory-bound operator passes (𝒜v and
@@ -171,7 +172,7 @@ struct Handle {
     amul(dx.p, adx.p);
     adx_ver = dx_ver;
   }
-  DBuf<double> S, Sf, Dinv;
+  DBuf<double> S, Sf;
   DBuf<double> Linv, tmp_mm;       // explicit inverse of the FP64 factor, its scratch
   // FP64 Gram engine of the Schur SYRK: 0 = FP64 DMMA tiles, 1 = exact int8
   // digit products (48-bit digits, int32 accumulation, FP64 level sums).
@@ -621,7 +622,7 @@ struct Handle {
     // Workspaces.
     for (auto* b : {&x, &dx, &d, &v, &r, &rho, &work_m, &work_m2, &xbest, &keptx, &dxbest})
       b->alloc(m), b->zero(st);
-    for (auto* b : {&X, &Y, &P, &R, &Z, &dX, &dY, &LX, &MY, &W, &T1, &T2, &Xbest, &Ybest, &tmpK2})
+    for (auto* b : {&X, &Y, &P, &R, &Z, &dX, &dY, &LX, &MY, &W, &WY, &T1, &T2, &Xbest, &Ybest, &tmpK2})
       b->alloc(K), b->zero(st);
     oz_err.alloc(1);
     oz_err.zero(st);
@@ -662,7 +663,6 @@ struct Handle {
     Pc.alloc((size_t)K * m);
     S.alloc((size_t)m * m);
     Sf.alloc((size_t)m * m);
-    Dinv.alloc((size_t)ceil_div(m, 64) * 64 * 64);
     syrk = plan_syrk_f64(m, K, sms);
     partial.alloc(syrk.partial_doubles);
     red.alloc(64);
@@ -678,7 +678,10 @@ struct Handle {
     // Gershgorin scratch
     std::vector<long long> coff(dense.size());
     long long tot = 0;
-    for (size_t b = 0; b < dense.size(); ++b) coff[b] = tot, tot += dense[b].k;
+    for (size_t b = 0; b < dense.size(); ++b) {
+      coff[b] = tot, tot += dense[b].k;
+      if (step_bound_fits(dense[b].k)) sb_blocks.push_back((int)b);
+    }
     g_cand.alloc(tot);
     g_cand_off.alloc(dense.size());
     if (!dense.empty()) h2d(g_cand_off.p, coff.data(), coff.size() * sizeof(long long));
@@ -872,6 +875,7 @@ struct Handle {
 
   // -------------------------------------------------------- iterate I/O --
   void set_iterate(const double* hx, const double* hX, const double* hY) {
+    iterate_changed();
     if (hx) h2d(x.p, hx, m * sizeof(double));
     if (hX) {
       h2d(tmpK.p, hX, Ku * sizeof(double));
@@ -889,6 +893,7 @@ struct Handle {
     sync();
   }
   void fixed_start(double wp, double wd) {
+    iterate_changed();
     x.zero(st);
     if (n_eq) yv.zero(st);
     X.zero(st);
@@ -906,12 +911,16 @@ struct Handle {
   }
 
   // ------------------------------------------------------ block factors --
+  // Whether LX, MY, W and WY belong to the current X and Y (iterate_changed).
+  bool block_factors_current = false;
+  void iterate_changed() { block_factors_current = false; }
   bool factor_blocks() {
+    block_factors_current = false;
     // LX = chol(X), MY = chol(Y) for every dense block (batched), 1×1 by sqrt.
     std::vector<MatDesc<double>> mats;
-    for (auto& b : dense) {
-      d2d(LX.p + b.off, X.p + b.off, sizeof(double) * b.k * b.k);
-      d2d(MY.p + b.off, Y.p + b.off, sizeof(double) * b.k * b.k);
+    if (od) {  // the dense blocks come first in the stacked layout
+      d2d(LX.p, X.p, sizeof(double) * od);
+      d2d(MY.p, Y.p, sizeof(double) * od);
     }
     for (auto& b : dense) mats.push_back({LX.p + b.off, b.k, b.k});
     for (auto& b : dense) mats.push_back({MY.p + b.off, b.k, b.k});
@@ -938,19 +947,24 @@ struct Handle {
     }
     diag_factor_ok = fail_h == 0;
     if (ok && !dense.empty()) {
-      // W = L_X^{-1} for the Schur products and the block solves.
-      W.zero(st);
-      std::vector<MatDesc<double>> Ls, Ws;
-      for (auto& b : dense) {
-        Ls.push_back({LX.p + b.off, b.k, b.k});
-        Ws.push_back({W.p + b.off, b.k, b.k});
-      }
-      ensure_descs(2 * nb);
-      h2d(d_descs.p, Ls.data(), nb * sizeof(MatDesc<double>));
-      h2d(d_descs.p + nb, Ws.data(), nb * sizeof(MatDesc<double>));
-      trinv_batched<double, 32>(d_descs.p, d_descs.p + nb, (int)nb, kmax, st);
-      sync();
+      // W = L_X⁻¹ for the Schur products, the block solves and the step bounds, WY =
+      // L_Y⁻¹ for the step bounds (their strict upper triangles stay zero).
+      TrinvList q;
+      for (int side = 0; side < 2; ++side)
+        for (auto& blk : dense) {
+          if (q.count == kTrinvMax) {
+            trinv(q, st);
+            q.count = 0;
+          }
+          q.n[q.count] = blk.k;
+          q.L[q.count] = (side ? MY.p : LX.p) + blk.off;
+          q.W[q.count] = (side ? WY.p : W.p) + blk.off;
+          q.tmp[q.count] = (side ? T2.p : T1.p) + blk.off;
+          ++q.count;
+        }
+      trinv(q, st);
     }
+    block_factors_current = ok;
     return ok;
   }
 
@@ -1334,9 +1348,16 @@ struct Handle {
   void invert_factor() {
     if (Linv.n < (size_t)m * m) {
       Linv.alloc((size_t)m * m);
+      Linv.zero(st);
       tmp_mm.alloc((size_t)m * m);
     }
-    trinv_recursive_f64(Sf.p, m, Linv.p, Dinv.p, tmp_mm.p, st);
+    TrinvList q;
+    q.count = 1;
+    q.n[0] = m;
+    q.L[0] = Sf.p;
+    q.W[0] = Linv.p;
+    q.tmp[0] = tmp_mm.p;
+    trinv(q, st);
   }
   void factorize(int* ok, int* attempts, double* quality) {
     PhaseScope ps(this, 2);
@@ -1843,14 +1864,61 @@ struct Handle {
     potrf_host_list(mats, info, dmn, dmx, false);
   }
 
+  // The bounds of the dense blocks that step_bounds takes, from λ_min of
+  // L⁻¹·dM·L⁻ᵀ (both sides, one launch): queued into sb_out, [X blocks | Y blocks]
+  // of the block list sb_blocks.  Scratch: T1, T2, Z, tmpK2.
+  std::vector<int> sb_blocks;
+  DBuf<StepBoundDesc> sb_desc;
+  DBuf<double> sb_out;
+  void queue_step_bounds() {
+    const int n = (int)sb_blocks.size();
+    const double *Ws[2] = {W.p, WY.p}, *dMs[2] = {dX.p, dY.p};
+    double *Ts[2] = {T1.p, T2.p}, *Gs[2] = {Z.p, tmpK2.p};
+    int kb = 0;
+    for (int b : sb_blocks) kb = std::max(kb, dense[b].k);
+    if (sb_desc.n < 2 * (size_t)n) {
+      std::vector<StepBoundDesc> d;
+      for (int side = 0; side < 2; ++side)
+        for (int b : sb_blocks) d.push_back({Gs[side] + dense[b].off, dense[b].k});
+      sb_desc.alloc(d.size());
+      sb_out.alloc(d.size());
+      h2d(sb_desc.p, d.data(), d.size() * sizeof(StepBoundDesc));
+      sync();
+    }
+    for (int pass = 0; pass < 2; ++pass) {  // T = W·dM, then G = T·Wᵀ
+      GemmGroups g;
+      auto flush = [&]() {
+        gemm_f64_grouped(g, false, pass == 0, st);
+        g.n = 0;
+      };
+      for (int side = 0; side < 2; ++side)
+        for (int b : sb_blocks) {
+          if (g.n == kGemmGroups) flush();
+          const DenseBlk& B = dense[b];
+          g.A[g.n] = blk_as_A(pass == 0 ? Ws[side] : Ts[side], B.off, B.k);
+          g.B[g.n] = pass == 0 ? blk_as_B(dMs[side], B.off, B.k) : blk_as_A(Ws[side], B.off, B.k);
+          g.C[g.n] = blk_out(pass == 0 ? Ts[side] : Gs[side], B.off, B.k);
+          g.alpha[g.n] = 1.0;
+          g.beta[g.n] = 0.0;
+          g.mode[g.n] = pass == 0 ? KR_A_LOWER : KR_B_UPPER;
+          ++g.n;
+        }
+      flush();
+    }
+    step_bounds(sb_desc.p, 2 * n, kb, sb_out.p, st);
+  }
+
   // Fraction-to-boundary bounds of both sides (src/kernels/generic.jl:350-422):
-  // closed forms for 1×1 and 2×2 blocks, otherwise a full-step Cholesky test
-  // followed by 64 bisection steps.  Every (side, block) bisection advances in
-  // the same rounds: each round factors, in one batch, the complete 4-level
-  // subtree of midpoints of every unfinished interval, and the sequential
-  // bisection path is replayed through it — the result equals the sequential one.
+  // closed forms for 1×1 and 2×2 blocks.  Larger blocks: with `eigen` (the affine
+  // predictor's bounds, which only steer σ) the eigenvalue bound wherever the block
+  // factors are at hand and the order fits, in place of up to 13 rounds of
+  // Cholesky trials; otherwise a full-step Cholesky test followed by 64 bisection
+  // steps.  Every (side, block) bisection advances in the same rounds: each round
+  // factors, in one batch, the complete subtree of the next midpoints of every
+  // unfinished interval, and the sequential bisection path is replayed through it —
+  // the result equals the sequential one.
   long long ftb_rounds = 0, ftb_trials = 0;  // batched trial rounds / trials of the bisections
-  void ftb_bounds(double* boundX, double* boundY) {
+  void ftb_bounds(double* boundX, double* boundY, bool eigen = false) {
     double b2[2] = {1.0, 1.0};
     const double* Ms[2] = {X.p, Y.p};
     const double* dMs[2] = {dX.p, dY.p};
@@ -1860,9 +1928,18 @@ struct Handle {
       }
       for (auto& s2 : fetch_k2(Ms[side], dMs[side])) b2[side] = std::min(b2[side], ftb2(s2));
     }
-    if (nd) {
-      d2h(h_red + 8, red.p + 8, 2 * sizeof(double));
+    eigen = eigen && block_factors_current && !sb_blocks.empty();
+    if (nd) d2h(h_red + 8, red.p + 8, 2 * sizeof(double));
+    if (eigen) {
+      queue_step_bounds();
+      const size_t n = sb_blocks.size();
+      double* hb = reinterpret_cast<double*>(pinned(2 * n * sizeof(double)));
+      d2h(hb, sb_out.p, 2 * n * sizeof(double));
       sync();
+      for (size_t q = 0; q < 2 * n; ++q) b2[q / n] = std::min(b2[q / n], hb[q]);
+    }
+    if (nd) {
+      if (!eigen) sync();
       b2[0] = std::min(b2[0], h_red[8]);
       b2[1] = std::min(b2[1], h_red[9]);
     }
@@ -1876,7 +1953,7 @@ struct Handle {
     std::vector<Bis> probs;
     for (int side = 0; side < 2; ++side)
       for (size_t b = 0; b < dense.size(); ++b)
-        if (dense[b].k > 2) {
+        if (dense[b].k > 2 && !(eigen && step_bound_fits(dense[b].k))) {
           Bis q;
           q.side = side;
           q.b = (int)b;
@@ -1965,19 +2042,18 @@ struct Handle {
     double tX = 1.0, tY = 1.0;
     if (adaptive) {
       double bX, bY;
-      ftb_bounds(&bX, &bY);
+      ftb_bounds(&bX, &bY, true);
       tX = bX < 1 ? bX : 1.0;
       tY = bY < 1 ? bY : 1.0;
     }
-    std::vector<double> c12(2 * (size_t)L);
     seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, nullptr, 0.0, Y.p, nullptr, 0.0, seg_part.p,
             work_L.p, st);
     seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, dX.p, tX, Y.p, dY.p, tY, seg_part.p,
             work_L.p + L, st);
-    d2h(c12.data(), work_L.p, 2 * L * sizeof(double));  // both in one read-back
+    double* c1 = reinterpret_cast<double*>(pinned(2 * (size_t)L * sizeof(double)));
+    d2h(c1, work_L.p, 2 * L * sizeof(double));  // both in one read-back
     sync();
-    const double* c1 = c12.data();
-    const double* c2 = c12.data() + L;
+    const double* c2 = c1 + L;
     double s1 = 0, s2 = 0;
     for (int l = 0; l < L; ++l) s1 += c1[l], s2 += c2[l];
     out[0] = s1;
@@ -2062,6 +2138,7 @@ struct Handle {
   // -------------------------------------------------------------- update --
   void update(double tX, double tY, double* compl_total, int* finite, double* block_dots) {
     PhaseScope ps(this, 6);
+    iterate_changed();
     combine(K, X.p, tX, dX.p, st);
     combine(K, Y.p, tY, dY.p, st);
     combine(m, x.p, tX, dx.p, st);
@@ -2140,6 +2217,7 @@ struct Handle {
 
   // ---------------------------------------------------------- cold start --
   void cold_start_iterate() {
+    iterate_changed();
     d2d(x.p, keptx.p, m * sizeof(double));
     amul(x.p, tmpK.p);
     axpbypcz(K, 1.0, tmpK.p, -1.0, Cst.p, 0.0, nullptr, X.p, st);
@@ -2237,6 +2315,7 @@ struct Handle {
     *ok_out = ok ? 1 : 0;
   }
   void apply_block_shifts(double* M, const std::vector<double>& shifts) {
+    iterate_changed();
     if (!dense.empty()) {
       std::vector<double> sh(dense.size());
       for (size_t b = 0; b < dense.size(); ++b) sh[b] = shifts[dense[b].user];
@@ -2828,6 +2907,7 @@ int sdpx_b200_block_dots(sdpx_b200_handle* h, double* d, double* tx, double* ty)
 }
 int sdpx_b200_scale_iterate(sdpx_b200_handle* h, int which, double f) {
   GUARD(h, {
+    h->h.iterate_changed();
     sdpx::scale(h->h.K, which == 0 ? h->h.X.p : h->h.Y.p, f, h->h.st);
     h->h.sync();
   });
@@ -2845,6 +2925,7 @@ int sdpx_b200_restore_best(sdpx_b200_handle* h) {
   GUARD(h, {
     auto& H = h->h;
     H.d2d(H.x.p, H.xbest.p, H.m * sizeof(double));
+    H.iterate_changed();
     H.d2d(H.X.p, H.Xbest.p, H.K * sizeof(double));
     H.d2d(H.Y.p, H.Ybest.p, H.K * sizeof(double));
     if (H.n_eq) H.d2d(H.yv.p, H.ybest.p, H.n_eq * sizeof(double));

@@ -26,24 +26,27 @@ size_t potrf_flow_flag_words(int nmat, int nmax);
 void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, double* dmin,
                 double* dmax, unsigned* flags, int sms, cudaStream_t st, bool zero_upper = true);
 
-// W_b = L_b^{-1} for lower-triangular L_b (W zero-initialised by the caller).
-template <class T, int NB>
-void trinv_batched(const MatDesc<T>* d_L, const MatDesc<T>* d_W, int nmat, int nmax,
-                   cudaStream_t st);
-
 // Inverses of the 64×64 diagonal tiles of a lower factor L (n×n): Dinv[s]
-// (64×64, column-major), and into the diagonal tiles of Linv (n×n) unless null.
-void factor_diag_inverses(const double* L, long long ld, int n, double* Dinv, double* Linv,
-                          cudaStream_t st);
+// (64×64, column-major).
+void factor_diag_inverses(const double* L, long long ld, int n, double* Dinv, cudaStream_t st);
 
 // rhs ← (L Lᵀ)^{-1} rhs by blocked forward/backward substitution (work: n).
 template <class T, int NB>
 void cholesky_solve(const T* L, long long ld, int n, const T* Dinv, T* rhs, T* work,
                     cudaStream_t st);
 
-// Linv = L⁻¹ (n×n, column-major, ld n) by recursive doubling over 64×64 tiles.
-// Dinv: ceil(n/64)·64·64 scratch, tmp: n·n scratch.
-void trinv_recursive_f64(const double* L, int n, double* Linv, double* Dinv, double* tmp,
-                         cudaStream_t st);
+// Lower factors to invert together: W_b = L_b⁻¹ (n_b×n_b, column-major, ld n_b), tmp_b
+// n_b×n_b scratch.  The strict upper triangle of W must be zero on entry and is not
+// written.
+constexpr int kTrinvMax = 16;
+struct TrinvList {
+  int count = 0;
+  int n[kTrinvMax];
+  const double* L[kTrinvMax];
+  double *W[kTrinvMax], *tmp[kTrinvMax];
+};
+void invert_diag_tiles(const TrinvList& q, cudaStream_t st);  // the 64×64 diagonal tiles alone
+// By recursive doubling over 64×64 tiles, every step one launch for the whole list.
+void trinv(const TrinvList& q, cudaStream_t st);
 
 }  // namespace sdpx

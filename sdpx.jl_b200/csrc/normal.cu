@@ -304,15 +304,21 @@ struct NormalHandle {
   DBuf<int> serr;
   // Explicit inverse of the reduced factor for the refined (mixed) solves:
   // each solve is two GEMVs over L⁻¹ instead of 2·⌈m/64⌉ dependent launches.
-  DBuf<double> Linv, Ltmp, Ldinv;
+  DBuf<double> Linv, Ltmp;
   bool have_inverse = false;
   void make_inverse() {
     if (Linv.n < (size_t)m * m) {
       Linv.alloc((size_t)m * m);
+      Linv.zero(st);
       Ltmp.alloc((size_t)m * m);
-      Ldinv.alloc((size_t)ceil_div(std::max(m, 1), 64) * 64 * 64);
     }
-    trinv_recursive_f64(F.p, m, Linv.p, Ldinv.p, Ltmp.p, st);
+    TrinvList q;
+    q.count = 1;
+    q.n[0] = m;
+    q.L[0] = F.p;
+    q.W[0] = Linv.p;
+    q.tmp[0] = Ltmp.p;
+    trinv(q, st);
     have_inverse = true;
   }
   // v ← Q⁻¹v = L⁻ᵀ(L⁻¹v) with the explicit inverse (work: m).
@@ -587,7 +593,7 @@ struct NormalHandle {
     assemble_ms = asm_ms;
     factor_ms = fac_ms;
     if (info != 0) return 1;
-    if (m > 0) factor_diag_inverses(F.p, m, m, Finv_diag.p, nullptr, st);
+    if (m > 0) factor_diag_inverses(F.p, m, m, Finv_diag.p, st);
     sync();
     have_factor = true;
     return 0;
@@ -626,7 +632,7 @@ struct NormalHandle {
     sync();
     if (info < 0) throw CudaError("normal-matrix Cholesky: a wait for a tile gave up");
     if (info != 0) return 1;
-    factor_diag_inverses(F.p, m, m, Finv_diag.p, nullptr, st);
+    factor_diag_inverses(F.p, m, m, Finv_diag.p, st);
     if (split) make_inverse();
     have_factor = true;
     return 0;

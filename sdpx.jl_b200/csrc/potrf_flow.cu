@@ -604,16 +604,11 @@ __global__ void __launch_bounds__(FT + FIO, 1)
   }
 }
 
-// W_s = (tile s of L)⁻¹ into Dinv (64×64 column-major, zero-padded) and, when
-// Linv is given, into its diagonal tiles: the strips solve X·Lᵀ = I, so
-// X = L⁻ᵀ and W = Xᵀ.  49 → 6 µs a call against one thread per column, whose chain was
-// 64 rows of up to 63 dependent products and a division each.
-__global__ void __launch_bounds__(FT) k_tile_inverse(const double* L, long long ld, int n, double* Dinv,
-                                                     double* Linv) {
-  extern __shared__ __align__(16) double fsm[];
-  double *D = fsm, *X = fsm + kTile;
-  __shared__ double inv[FB];
-  const int s0 = blockIdx.x * FB, w = min(FB, n - s0);
+// Tile s of L (lower, w of its rows in range) inverted: X = L⁻ᵀ in shared X, from the
+// strips' solves of X·Lᵀ = I, so that W = Xᵀ.  49 → 6 µs a call against one thread per
+// column, whose chain was 64 rows of up to 63 dependent products and a division each.
+__device__ __forceinline__ void invert_tile(const double* L, long long ld, int s0, int w, double* D, double* X,
+                                            double* inv) {
   for (int e = threadIdx.x; e < FB * FB; e += FT) {
     const int r = e & 63, c = e >> 6;
     D[c * FLD + r] = (r < w && c <= r) ? L[(size_t)(s0 + c) * ld + s0 + r] : (r == c ? 1.0 : 0.0);
@@ -624,13 +619,32 @@ __global__ void __launch_bounds__(FT) k_tile_inverse(const double* L, long long 
   __syncthreads();
   solve_strip(X, D, inv);
   __syncthreads();
+}
+
+// Dinv[s] = (tile s of L)⁻¹, 64×64 column-major, zeros above the diagonal and outside.
+__global__ void __launch_bounds__(FT) k_tile_inverse(const double* L, long long ld, int n, double* Dinv) {
+  extern __shared__ __align__(16) double fsm[];
+  __shared__ double inv[FB];
+  const int s0 = blockIdx.x * FB, w = min(FB, n - s0);
+  invert_tile(L, ld, s0, w, fsm, fsm + kTile, inv);
   double* out = Dinv + (size_t)blockIdx.x * FB * FB;
   for (int e = threadIdx.x; e < FB * FB; e += FT) {
     const int c = e & 63, r = e >> 6;  // W[c][r] = X[r][c]
-    const bool in = r <= c && c < w;
-    const double v = in ? X[c * FLD + r] : 0.0;
-    out[e] = v;
-    if (Linv && in) Linv[(size_t)(s0 + r) * n + s0 + c] = v;
+    out[e] = r <= c && c < w ? fsm[kTile + c * FLD + r] : 0.0;
+  }
+}
+
+// The diagonal tiles of W_b = L_b⁻¹ (lower parts).
+__global__ void __launch_bounds__(FT) k_tile_inverse_list(const __grid_constant__ TrinvList q) {
+  extern __shared__ __align__(16) double fsm[];
+  __shared__ double inv[FB];
+  const int n = q.n[blockIdx.y], s0 = blockIdx.x * FB, w = min(FB, n - s0);
+  if (w <= 0) return;
+  invert_tile(q.L[blockIdx.y], n, s0, w, fsm, fsm + kTile, inv);
+  double* W = q.W[blockIdx.y];
+  for (int e = threadIdx.x; e < FB * FB; e += FT) {
+    const int c = e & 63, r = e >> 6;
+    if (r <= c && c < w) W[(size_t)(s0 + r) * n + s0 + c] = fsm[kTile + c * FLD + r];
   }
 }
 
@@ -672,11 +686,20 @@ void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, do
   SDPX_LAUNCH_CHECK();
 }
 
-void factor_diag_inverses(const double* L, long long ld, int n, double* Dinv, double* Linv,
-                          cudaStream_t st) {
+void factor_diag_inverses(const double* L, long long ld, int n, double* Dinv, cudaStream_t st) {
   const size_t smem = sizeof(double) * 2 * kTile;
   ensure_smem(k_tile_inverse, smem);
-  k_tile_inverse<<<ceil_div(n, FB), FT, smem, st>>>(L, ld, n, Dinv, Linv);
+  k_tile_inverse<<<ceil_div(n, FB), FT, smem, st>>>(L, ld, n, Dinv);
+  SDPX_LAUNCH_CHECK();
+}
+
+void invert_diag_tiles(const TrinvList& q, cudaStream_t st) {
+  int nmax = 0;
+  for (int b = 0; b < q.count; ++b) nmax = std::max(nmax, q.n[b]);
+  if (nmax == 0) return;
+  const size_t smem = sizeof(double) * 2 * kTile;
+  ensure_smem(k_tile_inverse_list, smem);
+  k_tile_inverse_list<<<dim3(ceil_div(nmax, FB), q.count), FT, smem, st>>>(q);
   SDPX_LAUNCH_CHECK();
 }
 

@@ -1,0 +1,18 @@
+// Fraction-to-boundary bounds from the smallest eigenvalue (step_bound.cu).
+#pragma once
+#include "common.cuh"
+
+namespace sdpx {
+
+struct StepBoundDesc {
+  const double* G;  // L⁻¹·dM·L⁻ᵀ, column-major k×k (symmetric up to rounding)
+  int k;
+};
+
+// Whether an order fits the kernel (its rows in the shared memory of one cluster).
+bool step_bound_fits(int k);
+// out[q] = min(1, −1/λ_min(G_q)) (1 when λ_min ≥ −1, 0 when G is not finite) for the
+// n matrices of the device list; kmax: the largest order, step_bound_fits(kmax).
+void step_bounds(const StepBoundDesc* d_list, int n, int kmax, double* out, cudaStream_t st);
+
+}  // namespace sdpx
