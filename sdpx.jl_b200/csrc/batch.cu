@@ -74,49 +74,44 @@ __global__ void __launch_bounds__(kThreads)
   const double* X = pool.X + I.kk_off;
   const double* Y = pool.Y + I.kk_off;
   const double* C = pool.C + I.kk_off;
-  const double* x = pool.x + I.m_off;
+  __shared__ double xs[kMaxM];
+  cta_load_vec(xs, pool.x + I.m_off, m);
   double pmax = 0.0;
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j < m; ++j) s += x[j] * A[(long long)j * kk + e];
+  cta_amul(A, xs, m, (int)kk, [&](int e, double s) {
     const double v = s - X[e] - C[e];
     P[e] = v;
     pmax = fmax(pmax, abs_nan_inf(v));
-    Xs[e] = X[e];
-    Ys[e] = Y[e];
-  }
+  });
+  cta_load_tile(Xs, X, k);
+  cta_load_tile(Ys, Y, k);
   pmax = cta_max(pmax, red);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double dmax = 0.0;
-  for (int j = warp; j < m; j += nw) {  // d_j = c_j − ⟨A_j, Y⟩, one warp per j
-    double s = 0.0;
-    for (long long e = lane; e < kk; e += 32) s += A[(long long)j * kk + e] * Y[e];
-    s = warp_sum(s);
+  cta_atmul(A, Y, m, (int)kk, [&](int j, double s) {  // d_j = c_j − ⟨A_j, Y⟩
     const double dv = pool.c[I.m_off + j] - s;
     if (lane == 0) pool.d[I.m_off + j] = dv;
     dmax = fmax(dmax, abs_nan_inf(dv));
-  }
+  });
   dmax = cta_max(dmax, red);
   double* R = pool.R + I.kk_off;
   const double mu = in[kMu];
   const bool add_mu = in[kUseAffine] == 0.0;
-  cta_gemm_dmma(Xs, false, Ys, R, k);  // R = X·Y (global), then −XY (+μI)
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    const int r = (int)(e % k), c = (int)(e / k);
-    double s = -R[e];
-    if (add_mu && r == c) s += mu;
-    R[e] = s;
-  }
-  __syncthreads();
+  const int nb = (k + 7) / 8;
+  cta_tile_gemm<false, kFull>(Xs, Ys, nb, [&](int r, int c, double v) {  // R = −XY (+μI)
+    if (r < k && c < k) R[r + c * k] = (add_mu && r == c) ? mu - v : -v;
+  });
   if (threadIdx.x == 0) {
     out[oPres] = pmax;
     out[oDres] = dmax;
     out[oOk] = 1.0;
   }
   if (in[kFactor] == 0.0) return;
+  __syncthreads();
+  __shared__ double invx[64], invy[64];
+  __shared__ int sfail;
   double xmn = 0, xmx = 0, ymn = 0, ymx = 0;
-  const bool okx = cta_chol(Xs, k, sflag, &xmn, &xmx);
-  const bool oky = okx && cta_chol(Ys, k, sflag, &ymn, &ymx);
+  const bool okx = cta_tile_chol(Xs, k, invx, &sfail, &xmn, &xmx, red);
+  const bool oky = okx && cta_tile_chol(Ys, k, invy, &sfail, &ymn, &ymx, red);
   if (threadIdx.x == 0) {
     auto q = [](double mn, double mx) {
       return (mx > 0 && isfinite(mx)) ? fmin(1.0, fmax(0.0, mn / mx)) : 0.0;
@@ -128,20 +123,14 @@ __global__ void __launch_bounds__(kThreads)
   if (!(okx && oky)) return;
   double* LX = pool.LX + I.kk_off;
   double* LY = pool.LY + I.kk_off;
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    const int r = (int)(e % k), c = (int)(e / k);
-    LX[e] = r >= c ? Xs[e] : 0.0;
-    LY[e] = r >= c ? Ys[e] : 0.0;
-  }
+  cta_each(Xs, k, [&](int r, int c, double v) { LX[r + c * k] = r >= c ? v : 0.0; });
+  cta_each(Ys, k, [&](int r, int c, double v) { LY[r + c * k] = r >= c ? v : 0.0; });
   __syncthreads();
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    const int r = (int)(e % k), c = (int)(e / k);
-    Ys[e] = r >= c ? Xs[e] : 0.0;  // lower L_X
-  }
-  __syncthreads();
-  cta_trinv(Ys, Xs, k);
+  cta_tile_inverse_t(Ys, Xs, invx, nb);  // Ys = L_X⁻ᵀ
   double* W = pool.W + I.kk_off;
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) W[e] = Xs[e];
+  const int nw8 = kThreads / 32;
+  for (int c = warp; c < k; c += nw8)
+    for (int r = lane; r < k; r += 32) W[r + c * k] = r >= c ? Ys[r * FLD + c] : 0.0;
 }
 
 // B2a: the Schur panel P̂_j = W·A_j·L_Y (W = L_X⁻¹, both lower) for the
@@ -322,74 +311,108 @@ __global__ void __launch_bounds__(Cfg::NT)
   }
 }
 
-// Blocked lower Cholesky of the m×m column-major M in place (global memory,
-// one CTA): 16-column panels factored column by column (pivot, scale, rank-1
-// update inside the panel), then the trailing block updated by the panel as a
-// rank-16 SYRK on DMMA m8n8k4 fragments (8×8 lower tiles, one per warp in
-// turn).  False at the first pivot that is not > 0.
-__device__ bool cta_chol_blocked(double* M, int m, double* sflag) {
-  constexpr int NB = 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  for (int jb = 0; jb < m; jb += NB) {
-    const int je = min(m, jb + NB);
-    for (int j = jb; j < je; ++j) {
-      if (threadIdx.x == 0) {
-        const double d = M[j + (long long)j * m];
-        sflag[0] = d;
-        sflag[1] = d > 0.0 ? sqrt(d) : 0.0;
-      }
+// Copies of the h×w tile of the m×m column-major M at (r0, c0) (this CTA's own data).
+__device__ __forceinline__ void cta_tile_in(double* T, const double* M, int m, int r0, int c0, int h, int w,
+                                            bool identity) {
+  const int r = threadIdx.x & 63, cb = threadIdx.x >> 6;
+  const double* p = M + r0 + r + (long long)c0 * m;
+  double v[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int c = cb + 4 * u;
+    v[u] = (r < h && c < w) ? p[(long long)c * m] : (identity && r == c ? 1.0 : 0.0);
+  }
+#pragma unroll
+  for (int u = 0; u < 16; ++u) T[(cb + 4 * u) * FLD + r] = v[u];
+}
+__device__ __forceinline__ void cta_tile_out(const double* T, double* M, int m, int r0, int c0, int h, int w,
+                                             bool lower) {
+  const int r = threadIdx.x & 63, cb = threadIdx.x >> 6;
+  double* p = M + r0 + r + (long long)c0 * m;
+#pragma unroll 4
+  for (int u = 0; u < 16; ++u) {
+    const int c = cb + 4 * u;
+    if (r < h && c < w && (!lower || r >= c)) p[(long long)c * m] = T[c * FLD + r];
+  }
+}
+
+// Lower Cholesky of the m×m column-major M in place (global memory, L2; one CTA), 64
+// columns at a time: the diagonal tile in shared memory (tile64), the rows below
+// solved tile by tile, then the trailing tiles updated on DMMA fragments.  T0, T1:
+// tiles.  False at the first pivot that is not > 0.  (Column by column from global
+// memory the 512-instance phase took 0.54 ms.)
+__device__ bool cta_chol_tiles(double* M, int m, double* T0, double* T1, double* inv, int* sfail,
+                               double* dmin, double* dmax, double* red) {
+  using namespace tile64;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nt = (m + 63) / 64;
+  double lo = INFINITY, hi = 0.0;
+  for (int j = 0; j < nt; ++j) {
+    const int c0 = 64 * j, w = min(64, m - c0);
+    cta_tile_in(T0, M, m, c0, c0, w, w, true);
+    double mn, mx;
+    if (!cta_tile_chol(T0, w, inv, sfail, &mn, &mx, red)) return false;
+    lo = fmin(lo, mn);
+    hi = fmax(hi, mx);
+    cta_tile_out(T0, M, m, c0, c0, w, w, true);
+    for (int i = j + 1; i < nt; ++i) {
+      const int r0 = 64 * i, h = min(64, m - r0);
       __syncthreads();
-      if (!(sflag[0] > 0.0)) return false;
-      const double ljj = sflag[1];
-      const double inv = 1.0 / ljj;
-      for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) M[i + (long long)j * m] *= inv;
-      if (threadIdx.x == 0) M[j + (long long)j * m] = ljj;
+      cta_tile_in(T1, M, m, r0, c0, h, 64, false);
       __syncthreads();
-      const int nc = je - j - 1, rows = m - j - 1;  // panel columns right of j, all rows below j
-      for (long long e = threadIdx.x; e < (long long)nc * rows; e += blockDim.x) {
-        const int ii = j + 1 + (int)(e % rows), ll = j + 1 + (int)(e / rows);
-        if (ii >= ll)
-          M[ii + (long long)ll * m] -= M[ii + (long long)j * m] * M[ll + (long long)j * m];
-      }
+      solve_strip(T1, T0, inv);
       __syncthreads();
+      cta_tile_out(T1, M, m, r0, c0, h, 64, false);
     }
-    // trailing block rows, cols ≥ je:  M −= L_panel · L_panelᵀ (lower 8×8 tiles)
-    const int n = m - je;
-    if (n <= 0) break;
-    const int nb8 = (n + 7) / 8;
-    const int ntile = nb8 * (nb8 + 1) / 2;
-    for (int tile = warp; tile < ntile; tile += nw) {
-      int ti = (int)((sqrt(8.0 * tile + 1.0) - 1.0) * 0.5);
-      while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-      while (ti * (ti + 1) / 2 > tile) --ti;
-      const int tj = tile - ti * (ti + 1) / 2;
-      const int r = je + ti * 8 + g, cB = je + tj * 8 + g;
-      double c0 = 0.0, c1 = 0.0;
-      for (int kk = jb; kk < je; kk += 4) {
-        const int p = kk + t;
-        const bool okp = p < je;
-        const double a = (okp && r < m) ? M[r + (long long)p * m] : 0.0;
-        const double b = (okp && cB < m) ? M[cB + (long long)p * m] : 0.0;
-        dmma_8x8x4(c0, c1, a, b);
+    // M(i, q) −= L(i, j)·L(q, j)ᵀ; with one row tile below, T1 already holds it
+    for (int q = j + 1; q < nt; ++q)
+      for (int i = q; i < nt; ++i) {
+        const int q0 = 64 * q, r0 = 64 * i, hq = min(64, m - q0), h = min(64, m - r0);
+        __syncthreads();
+        if (nt > j + 2) {
+          if (i == q) cta_tile_in(T0, M, m, q0, c0, hq, 64, false);
+          else cta_tile_in(T1, M, m, r0, c0, h, 64, false);
+          __syncthreads();
+        }
+        const double* B = nt > j + 2 ? T0 : T1;
+        const double* A = i == q ? B : T1;
+        if (8 * warp < h) {
+          double acc[8][2] = {};
+#pragma unroll 2
+          for (int kk = 0; kk < 64; kk += 4) {
+            const double av = A[(kk + t) * FLD + 8 * warp + g];
+#pragma unroll
+            for (int f = 0; f < 8; ++f) mma8(acc[f][0], acc[f][1], av, B[(kk + t) * FLD + 8 * f + g]);
+          }
+          const int r = 8 * warp + g;
+#pragma unroll
+          for (int f = 0; f < 8; ++f)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int c = 8 * f + 2 * t + e;
+              if (r < h && c < hq && (i != q || r >= c))
+                M[r0 + r + (long long)(q0 + c) * m] -= acc[f][e];
+            }
+        }
       }
-      const int cc = je + tj * 8 + 2 * t;
-      if (r < m) {
-        if (cc < m && r >= cc) M[r + (long long)cc * m] -= c0;
-        if (cc + 1 < m && r >= cc + 1) M[r + (long long)(cc + 1) * m] -= c1;
-      }
-    }
     __syncthreads();
   }
+  *dmin = lo;
+  *dmax = hi;
   return true;
 }
+
+constexpr size_t kFactorSmem = sizeof(double) * 2 * 64 * FLD;
 
 // B3: Cholesky of S with ≤ 6 regularisation retries, S_ii += δ·max(|S_ii|, 1)
 // with δ = √eps then ×10 (src/kkt.jl:1419-1445); quality = min/max |L_jj|.
 __global__ void __launch_bounds__(kThreads)
     k_b_factor(Pool pool, const int* act, const double* par, double* res) {
   INST_PROLOGUE
-  __shared__ double sflag[4];
+  extern __shared__ __align__(16) double sm[];
+  __shared__ double inv[64], red[32];
+  __shared__ int sfail;
+  double mn = 0.0, mx = 0.0;
   const double* S = pool.S + I.mm_off;
   double* L = pool.LS + I.mm_off;
   const long long mm = (long long)m * m;
@@ -404,7 +427,7 @@ __global__ void __launch_bounds__(kThreads)
       L[e] = v;
     }
     __syncthreads();
-    ok = cta_chol_blocked(L, m, sflag);
+    ok = cta_chol_tiles(L, m, sm, sm + 64 * FLD, inv, &sfail, &mn, &mx, red);
     __syncthreads();
     if (ok || attempts >= 6) break;
     ++attempts;
@@ -413,36 +436,88 @@ __global__ void __launch_bounds__(kThreads)
   if (threadIdx.x == 0) {
     out[oOk] = ok ? 1.0 : 0.0;
     out[oReg] = attempts;
-    double q = 0.0;
-    if (ok) {
-      double mn = fabs(L[0]), mx = mn;
-      for (int j = 1; j < m; ++j) {
-        mn = fmin(mn, fabs(L[j + (long long)j * m]));
-        mx = fmax(mx, fabs(L[j + (long long)j * m]));
-      }
-      q = (mx > 0 && isfinite(mx)) ? fmin(1.0, fmax(0.0, mn / mx)) : 0.0;
-    }
-    out[oQual] = q;
+    out[oQual] = ok && mx > 0 && isfinite(mx) ? fmin(1.0, fmax(0.0, mn / mx)) : 0.0;
   }
 }
 
-// v ← S⁻¹v with the lower factor L (m×m, global), v in shared memory.
-__device__ void cta_cholsolve(const double* L, int m, double* v, double* red) {
-  for (int j = 0; j < m; ++j) {  // forward: L y = v, column-oriented
-    __syncthreads();
-    const double yj = v[j] / L[j + (long long)j * m];
-    __syncthreads();
-    if (threadIdx.x == 0) v[j] = yj;
-    for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) v[i] -= L[i + (long long)j * m] * yj;
-  }
-  for (int j = m - 1; j >= 0; --j) {  // backward: Lᵀ z = y, one dot per row
-    __syncthreads();
-    double s = 0.0;
-    for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) s += L[i + (long long)j * m] * v[i];
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) v[j] = (v[j] - s) / L[j + (long long)j * m];
-  }
+// v ← S⁻¹v with the lower factor L (m×m column-major, global), v in shared memory, 32
+// columns at a time: the diagonal block by one warp (a shuffle, a product and an fma a
+// column) while the others fetch the next one, the rest by all.  D: two 32×33
+// blocks.  (One column at a time, two CTA barriers and a division each, the
+// 512-instance phase took 0.26 ms.)
+__device__ void cta_cholsolve(const double* L, int m, double* v, double* D) {
+  constexpr int NB = 32, LD = NB + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = kThreads / 32;
+  const int nblk = (m + NB - 1) / NB;
+  auto fetch = [&](int b, double* T, int first) {  // T[c·LD + r] = L(r, c) of block b
+    const int s = b * NB;
+    for (int c = warp - first; c < NB; c += nw - first)
+      if (c >= 0)
+        T[c * LD + lane] = (s + lane < m && s + c < m && lane >= c) ? L[s + lane + (long long)(s + c) * m]
+                                                                    : (lane == c ? 1.0 : 0.0);
+  };
+  fetch(0, D, 0);
   __syncthreads();
+  for (int b = 0; b < nblk; ++b) {  // forward: L y = v
+    const int s = b * NB, w = min(NB, m - s);
+    const double* T = D + (b & 1) * NB * LD;
+    if (warp == 0) {
+      double x = lane < w ? v[s + lane] : 0.0;
+      const double inv = 1.0 / T[lane * LD + lane];
+#pragma unroll 8
+      for (int c = 0; c < NB; ++c) {
+        const double y = __shfl_sync(0xffffffffu, x * inv, c);
+        if (lane == c) x = y;
+        else if (lane > c) x -= T[c * LD + lane] * y;
+      }
+      if (lane < w) v[s + lane] = x;
+    } else if (b + 1 < nblk) {
+      fetch(b + 1, D + ((b + 1) & 1) * NB * LD, 1);
+    }
+    __syncthreads();
+    for (int i = s + NB + threadIdx.x; i < m; i += kThreads) {
+      const double* l = L + i + (long long)s * m;
+      double a[NB], x = v[i];
+#pragma unroll
+      for (int c = 0; c < NB; ++c) a[c] = l[(long long)c * m];
+#pragma unroll
+      for (int c = 0; c < NB; ++c) x -= a[c] * v[s + c];
+      v[i] = x;
+    }
+    __syncthreads();
+  }
+  for (int b = nblk - 1; b >= 0; --b) {  // backward: Lᵀ z = y (D holds the last block)
+    const int s = b * NB, w = min(NB, m - s);
+    const double* T = D + (b & 1) * NB * LD;
+    // v_b −= L(below, b)ᵀ·z(below): four columns a warp
+    double acc[4] = {};
+    for (int i = s + NB + lane; i < m; i += 32) {
+      const double z = v[i];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u] += L[i + (long long)(s + 4 * warp + u) * m] * z;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[u] = warp_sum(acc[u]);
+    if (s + NB < m && lane < 4) {
+      const double a = lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3];
+      v[s + 4 * warp + lane] -= a;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      double x = lane < w ? v[s + lane] : 0.0;
+      const double inv = 1.0 / T[lane * LD + lane];
+#pragma unroll 8
+      for (int c = NB - 1; c >= 0; --c) {
+        const double z = __shfl_sync(0xffffffffu, x * inv, c);
+        if (lane == c) x = z;
+        else if (lane < c) x -= T[lane * LD + c] * z;
+      }
+      if (lane < w) v[s + lane] = x;
+    } else if (b > 0) {
+      fetch(b - 1, D + ((b - 1) & 1) * NB * LD, 1);
+    }
+    __syncthreads();
+  }
 }
 
 // B4: right-hand side r = −(d + ⟨A_j, X⁻¹(PY − R)⟩) (`rhs_from_R`); kMode 1
@@ -455,40 +530,46 @@ __global__ void __launch_bounds__(kThreads)
   double* M2 = M1 + pool.kq;
   double* M3 = M2 + pool.kq;
   double* R = pool.R + I.kk_off;
-  const double* X = pool.X + I.kk_off;
   const double* Y = pool.Y + I.kk_off;
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    M1[e] = X[e];
-    M2[e] = Y[e];
-  }
-  __syncthreads();
+  const int nb = (k + 7) / 8;
   if (in[kMode] == 1.0) {  // R = target·I − X·Y − dX·dY
-    cta_gemm_dmma(M1, false, M2, M3, k);                                    // X·Y
-    cta_gemm_dmma(pool.dX + I.kk_off, false, pool.dY + I.kk_off, M1, k);  // dX·dY
-    for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-      const int r = (int)(e % k), c = (int)(e / k);
-      double v = -M3[e] - M1[e];
-      if (r == c) v += in[kTarget];
-      R[e] = v;
-    }
+    cta_load_tile(M1, pool.X + I.kk_off, k);
+    cta_load_tile(M2, Y, k);
     __syncthreads();
+    cta_tile_gemm<false, kFull>(M1, M2, nb, [&](int r, int c, double v) { M3[c * FLD + r] = -v; });
+    __syncthreads();
+    cta_load_tile(M1, pool.dX + I.kk_off, k);
+    cta_load_tile(M2, pool.dY + I.kk_off, k);
+    __syncthreads();
+    const double target = in[kTarget];
+    cta_tile_gemm<false, kFull>(M1, M2, nb, [&](int r, int c, double v) {
+      double u = M3[c * FLD + r] - v;
+      if (r == c) u += target;
+      if (r < k && c < k) R[r + c * k] = u;
+      M3[c * FLD + r] = u;
+    });
+    __syncthreads();
+  } else {
+    cta_load_tile(M3, R, k);
   }
-  // Z = P·Y − R, then X⁻¹Z = Wᵀ·W·Z
-  const double* P = pool.P + I.kk_off;
-  cta_gemm_dmma(P, false, M2, M3, k);  // P·Y
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) M1[e] = M3[e] - R[e];
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) M3[e] = pool.W[I.kk_off + e];
+  // PY − R, then X⁻¹(PY − R) = Wᵀ·W·(PY − R)
+  cta_load_tile(M1, pool.P + I.kk_off, k);
+  cta_load_tile(M2, Y, k);
   __syncthreads();
-  cta_gemm_dmma(M3, false, M1, M2, k);  // W·(PY − R)
-  cta_gemm_dmma(M3, true, M2, M1, k);   // X⁻¹(PY − R) = Wᵀ·W·(PY − R)
-  const double* A = pool.A + I.a_off;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int j = warp; j < m; j += nw) {
-    double s = 0.0;
-    for (long long e = lane; e < kk; e += 32) s += A[(long long)j * kk + e] * M1[e];
-    s = warp_sum(s);
+  cta_tile_gemm<false, kFull>(M1, M2, nb,
+                              [&](int r, int c, double v) { M3[c * FLD + r] = v - M3[c * FLD + r]; });
+  __syncthreads();
+  cta_load_tile(M1, pool.W + I.kk_off, k);
+  __syncthreads();
+  double* Z = pool.Z + I.kk_off;
+  cta_tile_cholsolve(M1, M3, M2, nb, [&](int r, int c, double v) {
+    if (r < k && c < k) Z[r + c * k] = v;
+  });
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  cta_atmul(pool.A + I.a_off, Z, m, (int)kk, [&](int j, double s) {
     if (lane == 0) pool.r[I.m_off + j] = -(pool.d[I.m_off + j] + s);
-  }
+  });
 }
 
 // B5: kMode 0: dx = S⁻¹r; kMode 1 (a refinement correction): dxb = dx,
@@ -496,12 +577,11 @@ __global__ void __launch_bounds__(kThreads)
 __global__ void __launch_bounds__(kThreads)
     k_b_solve(Pool pool, const int* act, const double* par, double* res) {
   INST_PROLOGUE
-  __shared__ double v[kMaxM];
-  __shared__ double red[32];
+  __shared__ double v[kMaxM], D[2 * 32 * 33];
   const bool corr = in[kMode] == 1.0;
   const double* src = corr ? pool.rho + I.m_off : pool.r + I.m_off;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) v[i] = src[i];
-  cta_cholsolve(pool.LS + I.mm_off, m, v, red);
+  cta_load_vec(v, src, m);
+  cta_cholsolve(pool.LS + I.mm_off, m, v, D);
   double* dx = pool.dx + I.m_off;
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
     if (corr) {
@@ -522,31 +602,26 @@ __global__ void __launch_bounds__(kThreads)
   double* M2 = M1 + pool.kq;
   double* M3 = M2 + pool.kq;
   const double* A = pool.A + I.a_off;
-  const double* dx = pool.dx + I.m_off;
+  __shared__ double dxs[kMaxM];
+  cta_load_vec(dxs, pool.dx + I.m_off, m);
   double* dX = pool.dX + I.kk_off;
   const double* P = pool.P + I.kk_off;
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j < m; ++j) s += dx[j] * A[(long long)j * kk + e];
-    const double v = s + P[e];
-    dX[e] = v;
-    M1[e] = v;
-    M2[e] = pool.Y[I.kk_off + e];
-    M3[e] = pool.W[I.kk_off + e];
-  }
+  cta_amul(A, dxs, m, (int)kk, [&](int e, double s) { dX[e] = s + P[e]; });
+  cta_load_tile(M2, pool.Y + I.kk_off, k);
   __syncthreads();
-  const double* R = pool.R + I.kk_off;
-  double* Z = pool.Z + I.kk_off;
-  cta_gemm_dmma(M1, false, M2, Z, k);  // dX·Y (global scratch)
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) M1[e] = R[e] - Z[e];
+  cta_load_tile(M1, dX, k);
+  cta_load_tile(M3, pool.R + I.kk_off, k);
   __syncthreads();
-  cta_gemm_dmma(M3, false, M1, M2, k);
-  cta_gemm_dmma(M3, true, M2, M1, k);
+  const int nb = (k + 7) / 8;
+  cta_tile_gemm<false, kFull>(M1, M2, nb,
+                              [&](int r, int c, double v) { M3[c * FLD + r] -= v; });  // R − dX·Y
+  __syncthreads();
+  cta_load_tile(M1, pool.W + I.kk_off, k);
+  __syncthreads();
+  cta_tile_cholsolve(M1, M3, M2, nb, [&](int r, int c, double v) { M3[c * FLD + r] = v; });
+  __syncthreads();
   double* dY = pool.dY + I.kk_off;
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    const int r = (int)(e % k), c = (int)(e / k);
-    dY[e] = 0.5 * (M1[e] + M1[c + r * k]);
-  }
+  cta_each(M3, k, [&](int r, int c, double v) { dY[r + c * k] = 0.5 * (v + M3[r * FLD + c]); });
 }
 
 // B7: affine diagnostics: with kMode 1 the fraction-to-boundary bounds of X
@@ -558,7 +633,8 @@ __global__ void __launch_bounds__(kThreads)
   extern __shared__ __align__(16) double sm[];
   __shared__ double red[32];
   __shared__ int flags[kTrialWarps];
-  __shared__ double small[4 * kMaxK];
+  __shared__ LambdaScratch ls[2];
+  __shared__ double inv[64], bounds[2];
   double tX = 1.0, tY = 1.0;
   if (in[kMode] == 1.0) {
     double bX, bY;
@@ -566,9 +642,10 @@ __global__ void __launch_bounds__(kThreads)
       double* S0 = sm;
       double* S1 = S0 + pool.kq;
       double* S2 = S1 + pool.kq;
-      bX = cta_ftb_eig(nullptr, pool.W + I.kk_off, pool.dX + I.kk_off, k, S0, S1, S2, small, red);
-      __syncthreads();
-      bY = cta_ftb_eig(pool.LY + I.kk_off, nullptr, pool.dY + I.kk_off, k, S0, S1, S2, small, red);
+      cta_ftb_eig(pool.W + I.kk_off, pool.LY + I.kk_off, pool.dX + I.kk_off, pool.dY + I.kk_off, k, S0, S1,
+                  S2, ls, inv, bounds);
+      bX = bounds[0];
+      bY = bounds[1];
     } else {
       bX = cta_ftb_tree(pool.X + I.kk_off, pool.dX + I.kk_off, k, sm, pool.kp, flags);
       bY = cta_ftb_tree(pool.Y + I.kk_off, pool.dY + I.kk_off, k, sm, pool.kp, flags);
@@ -721,12 +798,10 @@ __global__ void k_b_elementwise(Pool pool, const int* act, const double* par, do
   double* X = pool.X + I.kk_off;
   double* Y = pool.Y + I.kk_off;
   if (mode == 5) {
-    const double* A = pool.A + I.a_off;
-    for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-      double s = 0.0;
-      for (int j = 0; j < m; ++j) s += pool.x[I.m_off + j] * A[(long long)j * kk + e];
-      X[e] = s - pool.C[I.kk_off + e];
-    }
+    __shared__ double xs[kMaxM];
+    cta_load_vec(xs, pool.x + I.m_off, m);
+    cta_amul(pool.A + I.a_off, xs, m, (int)kk,
+             [&](int e, double s) { X[e] = s - pool.C[I.kk_off + e]; });
     return;
   }
   for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
@@ -762,21 +837,16 @@ __global__ void __launch_bounds__(kThreads)
   INST_PROLOGUE
   __shared__ double red[32];
   const double* A = pool.A + I.a_off;
+  __shared__ double xs[kMaxM];
+  cta_load_vec(xs, pool.x + I.m_off, m);
   double pm = 0.0;
-  for (long long e = threadIdx.x; e < kk; e += blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j < m; ++j) s += pool.x[I.m_off + j] * A[(long long)j * kk + e];
+  cta_amul(A, xs, m, (int)kk, [&](int e, double s) {
     pm = fmax(pm, abs_nan_inf(s - pool.X[I.kk_off + e] - pool.C[I.kk_off + e]));
-  }
+  });
   pm = cta_max(pm, red);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   double dm = 0.0;
-  for (int j = warp; j < m; j += nw) {
-    double s = 0.0;
-    for (long long e = lane; e < kk; e += 32) s += A[(long long)j * kk + e] * pool.Y[I.kk_off + e];
-    s = warp_sum(s);
-    dm = fmax(dm, abs_nan_inf(pool.c[I.m_off + j] - s));
-  }
+  cta_atmul(A, pool.Y + I.kk_off, m, (int)kk,
+            [&](int j, double s) { dm = fmax(dm, abs_nan_inf(pool.c[I.m_off + j] - s)); });
   dm = cta_max(dm, red);
   if (threadIdx.x == 0) {
     out[oPres] = pm;
@@ -1050,11 +1120,15 @@ struct Engine {
   Pinned h_stage[2];          // upload staging (create only)
   cudaEvent_t ev_stage[2] = {nullptr, nullptr};
   Pool pool{};
-  int schur_threads = 256, schur_tile = 32;
+  // Schur launch shape: the DMMA products, work items of a size picked per call
+  // (grain < 0).  Timed over sizes 4..64 and 32 or 400 instances they were 1.3 to 4
+  // times as fast as the best scalar shape everywhere (0.075 against 0.128 ms for 32
+  // instances of order 4..12, 2.8 against 7.6 ms for 400 of order 32..64).
+  int schur_threads = 128, schur_tile = 64;
   // Affine fraction-to-boundary bounds: 0 the bisection of Cholesky trials
   // (eight at a time), 1 the eigenvalue bound −1/λ_min(L⁻¹·dM·L⁻ᵀ).
   int bound_mode = 1;
-  double grain = 4.0e6;
+  double grain = -1.0;
   std::vector<Run> runs;
   std::string err;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -1165,11 +1239,13 @@ struct Engine {
     pool.W = W.p, pool.dX = dX.p, pool.dY = dY.p, pool.Z = Z.p, pool.Xb = Xb.p, pool.Yb = Yb.p;
     pool.x = x.p, pool.dx = dx.p, pool.d = d.p, pool.r = r.p, pool.rho = rho.p;
     pool.xb = xb.p, pool.dxb = dxb.p, pool.S = S.p, pool.LS = LS.p;
-    pool.kq = (long long)kmax * kmax;
+    pool.kq = (long long)((kmax + 7) & ~7) * FLD;  // a k×k tile64 tile (≥ kmax²)
     pool.kp = (long long)kmax * (kmax + 1) / 2;
     for (PhaseKernel kf : {k_b_residuals, k_b_rhs, k_b_dirblocks})
       SDPX_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem_bytes(3)));
+    SDPX_CUDA(cudaFuncSetAttribute(k_b_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kFactorSmem));
     for (PhaseKernel kf : {k_b_affine, k_b_linesearch})
       SDPX_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)std::max(smem_trials(), smem_bytes(3))));
@@ -1315,6 +1391,11 @@ struct Engine {
     // Per instance the tile that pads least: 32 for T·P̂ when k ≤ 32 (one k×k
     // tile per constraint) and for the SYRK when m ≤ 64, else 64.
     std::vector<int4> tp64, tp32, sy64, sy32;
+    if (g < 0) {  // about 16 items a SM, of at least 2.5e5 flops (a launch's tail) …
+      double total = 0;  // … and at most 1e6 (the finest of the timed grains, the fastest)
+      for (int q = 0; q < n; ++q) total += cost(q);
+      g = std::min(1.0e6, std::max(2.5e5, total / (148.0 * 16.0)));
+    }
     auto split = [&](std::vector<int4>& w, int q, int units, double flops) {
       int parts = g > 0 ? (int)std::ceil(flops / g) : 1;
       parts = std::max(1, std::min(parts, units));
@@ -1645,7 +1726,7 @@ struct Engine {
         schur(ok1, schur_threads, schur_tile, grain);
       }
       const auto tf0 = std::chrono::steady_clock::now();
-      out = phase(K_factor, ok1, 0, true);
+      out = phase(K_factor, ok1, dd ? 0 : kFactorSmem, true);
       t_factor += std::chrono::duration<double>(std::chrono::steady_clock::now() - tf0).count();
       std::vector<int> ok2;
       for (size_t q = 0; q < ok1.size(); ++q) {

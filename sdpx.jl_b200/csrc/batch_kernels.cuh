@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "lambda_bound.cuh"
+#include "tile64.cuh"
 
 namespace sdpx {
 namespace batch {
@@ -56,6 +58,82 @@ __device__ __forceinline__ double abs_nan_inf(double v) {
 // ------------------------------------------------------------ reductions --
 __device__ inline double cta_sum(double v, double* red) { return block_sum(v, red); }
 __device__ inline double cta_max(double v, double* red) { return block_max(v, red); }
+
+// ------------------------------------------------ passes over the constraints
+// One CTA reads its instance's 𝒜 (up to 6.5 MB) in every phase, so what counts is
+// how many loads each thread has in flight: with one at a time the 512-instance
+// residual phase took 1.5 ms, where its bytes take 0.09 ms.  Both passes issue
+// 16 loads a thread before their first use; sums keep the order j = 0, 1, … .
+
+// f(e, Σ_j x[j]·A[j·kk + e]) for the elements e of this thread (x in shared memory).
+template <class F>
+__device__ __forceinline__ void cta_amul(const double* A, const double* x, int m, int kk, F f) {
+  constexpr int EV = 4, JU = 4;
+  const int nt = blockDim.x;
+  for (int e0 = threadIdx.x; e0 < kk; e0 += EV * nt) {
+    double s[EV] = {};
+    const double* a = A + e0;
+    int j = 0;
+    for (; j + JU <= m; j += JU, a += (long long)JU * kk) {
+      double v[JU][EV];
+#pragma unroll
+      for (int u = 0; u < JU; ++u)
+#pragma unroll
+        for (int q = 0; q < EV; ++q) v[u][q] = e0 + q * nt < kk ? a[u * kk + q * nt] : 0.0;
+#pragma unroll
+      for (int u = 0; u < JU; ++u)
+#pragma unroll
+        for (int q = 0; q < EV; ++q) s[q] += x[j + u] * v[u][q];
+    }
+    for (; j < m; ++j, a += kk)
+#pragma unroll
+      for (int q = 0; q < EV; ++q)
+        if (e0 + q * nt < kk) s[q] += x[j] * a[q * nt];
+#pragma unroll
+    for (int q = 0; q < EV; ++q)
+      if (e0 + q * nt < kk) f(e0 + q * nt, s[q]);
+  }
+}
+
+// f(j, ⟨A_j, y⟩) for every j, four constraints a warp at a time (y's elements are read
+// once for the four); f runs in all lanes.
+template <class F>
+__device__ __forceinline__ void cta_atmul(const double* A, const double* y, int m, int kk, F f) {
+  constexpr int JW = 4, U = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int j0 = warp * JW; j0 < m; j0 += nw * JW) {
+    const double* a[JW];
+#pragma unroll
+    for (int w = 0; w < JW; ++w) a[w] = A + (long long)min(j0 + w, m - 1) * kk;
+    double s[JW] = {};
+    for (int e0 = lane; e0 < kk; e0 += 32 * U) {
+      double v[U][JW], yv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool in = e0 + 32 * u < kk;
+        yv[u] = in ? y[e0 + 32 * u] : 0.0;
+#pragma unroll
+        for (int w = 0; w < JW; ++w) v[u][w] = in ? a[w][e0 + 32 * u] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (e0 + 32 * u < kk)
+#pragma unroll
+          for (int w = 0; w < JW; ++w) s[w] += v[u][w] * yv[u];
+    }
+#pragma unroll
+    for (int w = 0; w < JW; ++w) {
+      const double t = warp_sum(s[w]);
+      if (j0 + w < m) f(j0 + w, t);
+    }
+  }
+}
+
+// The vector x (m) in shared memory (ends with a CTA barrier).
+__device__ __forceinline__ void cta_load_vec(double* xs, const double* x, int m) {
+  for (int i = threadIdx.x; i < m; i += blockDim.x) xs[i] = x[i];
+  __syncthreads();
+}
 
 // ------------------------------------------------------ small factorisations
 // In-place lower Cholesky of the k×k column-major M (shared memory), the
@@ -102,46 +180,96 @@ __device__ bool cta_chol(double* M, int k, double* sflag, double* dmin, double* 
   return true;
 }
 
-// C = op(A)·B for k×k column-major operands (shared or global memory) on the
-// FP64 tensor cores: each warp takes 8×8 output tiles in turn and runs the
-// m8n8k4 DMMA over k in steps of 4 (loads past k read 0).  ta: A transposed.
-// C must not alias A or B.  Ends with a CTA barrier.
-__device__ void cta_gemm_dmma(const double* A, bool ta, const double* B, double* C, int k) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int nb = (k + 7) / 8;
-  for (int tile = warp; tile < nb * nb; tile += nw) {
-    const int i0 = (tile % nb) * 8, j0 = (tile / nb) * 8;
-    const int r = i0 + g, cB = j0 + g;
-    double c0 = 0.0, c1 = 0.0;
-    for (int kk = 0; kk < k; kk += 4) {
-      const int p = kk + t;
-      const bool okp = p < k;
-      const double a = (okp && r < k) ? (ta ? A[p + r * k] : A[r + p * k]) : 0.0;
-      const double b = (okp && cB < k) ? B[p + cB * k] : 0.0;
-      dmma_8x8x4(c0, c1, a, b);
-    }
-    const int cc = j0 + 2 * t;
-    if (r < k) {
-      if (cc < k) C[r + cc * k] = c0;
-      if (cc + 1 < k) C[r + (cc + 1) * k] = c1;
-    }
+// ------------------------------------------- k×k matrices in shared tiles
+// The phases keep a k×k matrix (k ≤ 64) as a tile64 tile: column c at c·FLD, padded
+// with the identity to 8·nb rows and columns, nb = ⌈k/8⌉, so the DMMA products need no
+// guards and their fragment reads no bank conflicts.
+using tile64::FLD;
+
+// S ← G (k×k column-major, global); t: its transpose.  All loads are issued before the
+// first shared store (one memory round trip a matrix).
+__device__ __forceinline__ void cta_load_tile(double* S, const double* G, int k, bool t = false) {
+  const int r = threadIdx.x & 63, cb = threadIdx.x >> 6, k8 = (k + 7) & ~7;
+  double v[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int c = cb + 4 * u;
+    v[u] = (r < k && c < k) ? G[r + c * k] : (r == c ? 1.0 : 0.0);
   }
-  __syncthreads();
+  if (r < k8)
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int c = cb + 4 * u;
+      if (c < k8) S[t ? r * FLD + c : c * FLD + r] = v[u];
+    }
+}
+// f(r, c, S(r, c)) over the k×k elements, lanes along the columns.
+template <class F>
+__device__ __forceinline__ void cta_each(const double* S, int k, F f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int c = warp; c < k; c += kThreads / 32)
+    for (int r = lane; r < k; r += 32) f(r, c, S[c * FLD + r]);
 }
 
-// W = L⁻¹ (lower, k×k): one thread per column, forward substitution.
-__device__ void cta_trinv(const double* L, double* W, int k) {
-  for (int e = threadIdx.x; e < k * k; e += blockDim.x) W[e] = 0.0;
-  __syncthreads();
-  for (int c = threadIdx.x; c < k; c += blockDim.x) {
-    W[c + c * k] = 1.0 / L[c + c * k];
-    for (int r = c + 1; r < k; ++r) {
-      double s = 0.0;
-      for (int p = c; p < r; ++p) s += L[r + p * k] * W[p + c * k];
-      W[r + c * k] = -s / L[r + r * k];
+// f(r, c, Σ_p op(A)(r, p)·B(p, c)) over the 8·nb square, for tiles A, B; ta: A
+// transposed.  first(i), last(i): the range of 8-blocks p that block row i needs (a
+// triangular A).  Each warp takes pairs of 8×8 output blocks of a block row in
+// turn, two chains to cover the pipe's latency.
+enum TileTri { kFull, kLower, kUpper };  // op(A)
+template <bool ta, TileTri tri, class F>
+__device__ __forceinline__ void cta_tile_gemm(const double* A, const double* B, int nb, F f) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int pairs = (nb + 1) / 2;
+  for (int u = warp; u < nb * pairs; u += kThreads / 32) {
+    const int i = u % nb, c0 = 16 * (u / nb);
+    const bool two = c0 + 8 < 8 * nb;
+    const int p0 = tri == kUpper ? 2 * i : 0, p1 = tri == kLower ? 2 * i + 2 : 2 * nb;
+    double acc[2][2] = {};
+    for (int p = p0; p < p1; ++p) {
+      const int q = 4 * p + t;
+      const double a = ta ? A[(8 * i + g) * FLD + q] : A[q * FLD + 8 * i + g];
+      tile64::mma8(acc[0][0], acc[0][1], a, B[(c0 + g) * FLD + q]);
+      if (two) tile64::mma8(acc[1][0], acc[1][1], a, B[(c0 + 8 + g) * FLD + q]);
     }
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (v == 0 || two) f(8 * i + g, c0 + 8 * v + 2 * t + e, acc[v][e]);
   }
+}
+
+// X⁻¹·B = Wᵀ·(W·B) for W = L_X⁻¹ in a tile: T (scratch) ← W·B, then f of the product.
+template <class F>
+__device__ __forceinline__ void cta_tile_cholsolve(const double* W, const double* B, double* T, int nb, F f) {
+  cta_tile_gemm<false, kLower>(W, B, nb, [&](int r, int c, double v) { T[c * FLD + r] = v; });
+  __syncthreads();
+  cta_tile_gemm<true, kUpper>(W, T, nb, f);
+}
+
+// Lower Cholesky of the tile M in place (inv: reciprocal pivots).  False at a pivot
+// that is not > 0 (or NaN).  min/max |L_jj| to *dmin/*dmax.  Ends with a CTA barrier.
+__device__ __forceinline__ bool cta_tile_chol(double* M, int k, double* inv, int* sfail, double* dmin,
+                                              double* dmax, double* red) {
+  if (threadIdx.x == 0) *sfail = tile64::kNoFail;
+  __syncthreads();
+  tile64::factor_tile(M, inv, (k + 7) / 8, sfail);
+  __syncthreads();
+  if (*sfail != tile64::kNoFail) return false;
+  const double v = (int)threadIdx.x < k ? M[threadIdx.x * FLD + threadIdx.x] : 0.0;
+  *dmax = cta_max(v, red);
+  *dmin = -cta_max((int)threadIdx.x < k ? -v : -INFINITY, red);
+  return true;
+}
+
+// X ← L⁻ᵀ for the factor in D (inv: reciprocal pivots).  Ends with a CTA barrier.
+__device__ __forceinline__ void cta_tile_inverse_t(double* X, const double* D, const double* inv, int nb) {
+  for (int e = threadIdx.x; e < 64 * 8 * nb; e += kThreads) {
+    const int r = e & 63, c = e >> 6;
+    X[c * FLD + r] = r == c ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  if ((int)(threadIdx.x >> 5) < nb) tile64::solve_strip(X, D, inv, nb);
   __syncthreads();
 }
 
@@ -367,160 +495,70 @@ __device__ double cta_backtrack(const double* X, const double* dX, int k, double
 // tridiagonalisation of G and a Sturm-count multisection of the tridiagonal
 // matrix (one shift per thread per round).
 
-namespace eigdetail {
-// Number of eigenvalues of the symmetric tridiagonal (a, b) below x (the
-// negative pivots of the LDLᵀ recurrence of T − x·I, zero pivots nudged).
-__device__ __forceinline__ int sturm_count(const double* a, const double* b, int n, double x,
-                                           double tiny) {
-  int neg = 0;
-  double q = a[0] - x;
-  if (q == 0.0) q = -tiny;
-  if (q < 0.0) ++neg;
-  for (int i = 1; i < n; ++i) {
-    q = (a[i] - x) - b[i - 1] * b[i - 1] / q;
-    if (q == 0.0) q = -tiny;
-    if (q < 0.0) ++neg;
-  }
-  return neg;
-}
-}  // namespace eigdetail
 
-// λ_min of the symmetric k×k G (shared memory, overwritten); v, w: k doubles
-// each, ab: 2k doubles (shared).  Called by the whole CTA.
-__device__ double cta_lambda_min(double* G, int k, double* v, double* w, double* ab,
-                                 double* red) {
-  // Householder tridiagonalisation: column j's subdiagonal part is reduced
-  // to α·e₁ by H = I − β·v·vᵀ applied on both sides of the trailing block.
-  for (int j = 0; j + 2 < k; ++j) {
-    const int n = k - j - 1, o = j + 1;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const double x = G[(o + i) + j * k];
-      v[i] = x;
-      s += x * x;
-    }
-    s = block_sum(s, red);
-    const double norm = sqrt(s);
-    const double x0 = G[o + j * k];
-    const double alpha = x0 > 0.0 ? -norm : norm;
-    if (norm == 0.0) continue;  // column already reduced (uniform)
-    if (threadIdx.x == 0) v[0] = x0 - alpha;
-    __syncthreads();
-    double vv = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) vv += v[i] * v[i];
-    vv = block_sum(vv, red);
-    if (!(vv > 0.0)) continue;
-    const double beta = 2.0 / vv;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {  // p = β·A·v
-      double t = 0.0;
-      for (int c = 0; c < n; ++c) t += G[(o + i) + (o + c) * k] * v[c];
-      w[i] = beta * t;
-    }
-    __syncthreads();
-    double pv = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) pv += w[i] * v[i];
-    pv = block_sum(pv, red);
-    const double K = 0.5 * beta * pv;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) w[i] -= K * v[i];  // w = p − K·v
-    __syncthreads();
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {  // A −= v·wᵀ + w·vᵀ
-      const int r = e % n, c = e / n;
-      G[(o + r) + (o + c) * k] -= v[r] * w[c] + w[r] * v[c];
-    }
-    if (threadIdx.x == 0) G[o + j * k] = alpha;
-    __syncthreads();
-  }
-  double* a = ab;
-  double* b = ab + k;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) {
-    a[i] = G[i + i * k];
-    if (i + 1 < k) b[i] = G[(i + 1) + i * k];
-  }
-  __syncthreads();
-  // Gershgorin interval, then multisection: each thread counts at one shift
-  double lo = 0.0, hi = 0.0, bmax = 0.0;
-  if (threadIdx.x == 0) {
-    lo = a[0], hi = a[0];
-    for (int i = 0; i < k; ++i) {
-      const double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i + 1 < k ? fabs(b[i]) : 0.0);
-      lo = fmin(lo, a[i] - r);
-      hi = fmax(hi, a[i] + r);
-      if (i + 1 < k) bmax = fmax(bmax, fabs(b[i]));
-    }
-    red[0] = lo;
-    red[1] = hi;
-    red[2] = fmax(bmax, fmax(fabs(lo), fabs(hi)));
-  }
-  __syncthreads();
-  lo = red[0];
-  hi = red[1];
-  const double tiny = 2.2250738585072014e-308 * fmax(1.0, red[2] * red[2]);  // pivot floor
-  __syncthreads();
-  __shared__ int cnt[kThreads];
-  for (int round = 0; round < 12; ++round) {
-    const double step = (hi - lo) / (blockDim.x + 1);
-    if (!(step > 0.0) || hi - lo <= 4.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)))
-      break;
-    const double x = lo + (threadIdx.x + 1) * step;
-    cnt[threadIdx.x] = eigdetail::sturm_count(a, b, k, x, tiny);
-    __syncthreads();
-    // smallest eigenvalue ∈ (last shift with count 0, first shift with count ≥ 1]
-    int first = blockDim.x;
-    for (int t = 0; t < (int)blockDim.x; ++t)
-      if (cnt[t] > 0) {
-        first = t;
-        break;
+// The bounds of both sides: the left half of the CTA takes X along dX, the right half
+// Y along dY.  W = L_X⁻¹ and L_Y as left by the residual phase (global, k×k); S0, S1,
+// S2: tiles.  out[0], out[1] (shared) receive the bounds.
+__device__ __forceinline__ void cta_ftb_eig(const double* W, const double* LY, const double* dX,
+                                            const double* dY, int k, double* S0, double* S1, double* S2,
+                                            LambdaScratch* ls, double* inv, double* out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nb = (k + 7) / 8;
+  // M ← G = W·M·Wᵀ with Wt = Wᵀ in a tile, the strips' products W·M kept in registers.
+  auto congruence = [&](const double* Wt, double* M) {
+    double x[8][2] = {}, y[8][2] = {};
+    if (warp < nb) {
+      for (int p = 0; p < 2 * warp + 2; ++p) {  // W is lower
+        const int q = 4 * p + t;
+        const double a = Wt[(8 * warp + g) * FLD + q];
+#pragma unroll
+        for (int f = 0; f < 8; ++f)
+          if (f < nb) tile64::mma8(x[f][0], x[f][1], a, M[(8 * f + g) * FLD + q]);
       }
-    const double nlo = first == 0 ? lo : lo + first * step;
-    const double nhi = first == (int)blockDim.x ? hi : lo + (first + 1) * step;
-    __syncthreads();
-    lo = nlo;
-    hi = nhi;
-  }
-  return 0.5 * (lo + hi);
-}
-
-// Fraction-to-boundary bound of M along dM from the factor L of M (lower,
-// global): W = L⁻¹ (given, or computed when Winv is null), G = W·dM·Wᵀ.
-// S0, S1, S2: three k×k shared slots; small: 4k + 32 doubles of shared scratch.
-__device__ double cta_ftb_eig(const double* L, const double* Wg, const double* dM, int k,
-                              double* S0, double* S1, double* S2, double* small, double* red) {
-  const int kk = k * k;
-  if (Wg) {
-    for (int e = threadIdx.x; e < kk; e += blockDim.x) S0[e] = Wg[e];
-  } else {
-    for (int e = threadIdx.x; e < kk; e += blockDim.x) {
-      const int r = e % k, c = e / k;
-      S2[e] = r >= c ? L[e] : 0.0;
+#pragma unroll
+      for (int p = 0; p < 16; ++p) {
+        const int src = (lane & 28) | (2 * (p & 1) + (t >> 1)), q = 4 * p + t;
+        const double v0 = __shfl_sync(0xffffffffu, x[p / 2][0], src);
+        const double v1 = __shfl_sync(0xffffffffu, x[p / 2][1], src);
+        const double a = (t & 1) ? v1 : v0;
+#pragma unroll
+        for (int f = p / 2; f < 8; ++f)  // Wᵀ is upper
+          if (f < nb && p < 2 * nb) tile64::mma8(y[f][0], y[f][1], a, Wt[(8 * f + g) * FLD + q]);
+      }
     }
     __syncthreads();
-    cta_trinv(S2, S0, k);
-  }
-  for (int e = threadIdx.x; e < kk; e += blockDim.x) S1[e] = dM[e];
+    if (warp < nb)
+#pragma unroll
+      for (int f = 0; f < 8; ++f)
+        if (f < nb) {
+          M[(8 * f + 2 * t) * FLD + 8 * warp + g] = y[f][0];
+          M[(8 * f + 2 * t + 1) * FLD + 8 * warp + g] = y[f][1];
+        }
+  };
+  cta_load_tile(S0, W, k, true);
+  cta_load_tile(S1, dX, k);
+  cta_load_tile(S2, LY, k);
   __syncthreads();
-  for (int e = threadIdx.x; e < kk; e += blockDim.x) {  // T = W·dM (W lower)
-    const int r = e % k, c = e / k;
-    double s = 0.0;
-    for (int p = 0; p <= r; ++p) s += S0[r + p * k] * S1[p + c * k];
-    S2[e] = s;
+  if (threadIdx.x < 64 && (int)threadIdx.x < 8 * nb) inv[threadIdx.x] = 1.0 / S2[threadIdx.x * FLD + threadIdx.x];
+  congruence(S0, S1);
+  __syncthreads();
+  cta_tile_inverse_t(S0, S2, inv, nb);  // S0 = L_Y⁻ᵀ
+  cta_load_tile(S2, dY, k);
+  __syncthreads();
+  congruence(S0, S2);
+  __syncthreads();
+  for (int e = threadIdx.x; e < 64 * k; e += kThreads) {  // G and Gᵀ differ in rounding only
+    const int r = e & 63, c = e >> 6;
+    if (r < k && r > c) {
+      S1[c * FLD + r] = S1[r * FLD + c] = 0.5 * (S1[c * FLD + r] + S1[r * FLD + c]);
+      S2[c * FLD + r] = S2[r * FLD + c] = 0.5 * (S2[c * FLD + r] + S2[r * FLD + c]);
+    }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < kk; e += blockDim.x) {  // G = T·Wᵀ
-    const int r = e % k, c = e / k;
-    double s = 0.0;
-    for (int p = 0; p <= c; ++p) s += S2[r + p * k] * S0[c + p * k];
-    S1[e] = s;
-  }
+  const int side = warp >> 2;
+  const double b = lambda_bound_64(side ? S2 : S1, k, ls[side], (int)threadIdx.x & 127, 6 + side);
+  if ((threadIdx.x & 127) == 0) out[side] = b;
   __syncthreads();
-  for (int e = threadIdx.x; e < kk; e += blockDim.x) {  // symmetrise into S2
-    const int r = e % k, c = e / k;
-    S2[e] = 0.5 * (S1[e] + S1[c + r * k]);
-  }
-  __syncthreads();
-  const double lmin = cta_lambda_min(S2, k, small, small + k, small + 2 * k, red);
-  if (!(lmin == lmin)) return 0.0;  // non-finite direction: no step
-  if (1.0 + lmin > 0.0) return 1.0;
-  return -1.0 / lmin;
 }
 
 }  // namespace batch

@@ -19,6 +19,7 @@
 //   here               0.021     0.48      1.21 ms
 // and within 4e-15 of −1/λ_min in 64 bits where the bisection is, iterates of κ = 100.
 #include "step_bound.h"
+#include "lambda_bound.cuh"
 
 namespace sdpx {
 namespace {
@@ -53,37 +54,6 @@ __device__ __forceinline__ double bsum(double v, double* red) {
     s += u.x + u.y;
   }
   return s;
-}
-
-// Number of eigenvalues below x of the tridiagonal (d, e2 = squared off-diagonal,
-// all scaled to norm ≤ 1): sign changes of the leading minors of T − x·I by their
-// three-term recurrence, one fma a row in the chain, rescaled every four rows.
-// e2 ≥ 1e-36 keeps two consecutive minors from vanishing together (a change of T
-// of 1e-18 of its norm).
-__device__ __forceinline__ int minors_below(const double* d, const double* e2, int k, double x) {
-  double pp = 1.0, p = d[0] - x;
-  int neg = __double2hiint(p) < 0;
-  int i = 1;
-  for (; i + 3 < k; i += 4) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const double q = fma(d[i + u] - x, p, -e2[i + u - 1] * pp);
-      neg += (unsigned)(__double2hiint(q) ^ __double2hiint(p)) >> 31;
-      pp = p;
-      p = q;
-    }
-    const int ex = max((__double2hiint(p) >> 20) & 2047, (__double2hiint(pp) >> 20) & 2047);
-    const double f = __hiloint2double(min(2046, max(1, 2046 - ex)) << 20, 0);  // ≈ 2^(1023−ex)
-    p *= f;
-    pp *= f;
-  }
-  for (; i < k; ++i) {
-    const double q = fma(d[i] - x, p, -e2[i - 1] * pp);
-    neg += (unsigned)(__double2hiint(q) ^ __double2hiint(p)) >> 31;
-    pp = p;
-    p = q;
-  }
-  return neg;
 }
 
 __host__ __device__ inline size_t bound_smem_doubles(int k, int C) {
@@ -234,9 +204,7 @@ __global__ void __launch_bounds__(BT, 1) k_step_bound(const StepBoundDesc* list,
           h = nh;
           if (h - l <= 2e-16 * fabs(l)) break;
         }
-        // from below, as the bisection's last passing trial is: l ≤ λ_min·f up to its
-        // last ulp, the quotient is rounded once; two ulps cover both
-        b = fmin(1.0, __longlong_as_double(__double_as_longlong(-f / l) - 2));
+        b = bound_from_below(l / f);
       }
       if (threadIdx.x == 0) out[blockIdx.x / C] = b;
     }
