@@ -246,42 +246,91 @@ __global__ void __launch_bounds__(NT) k_b_syrk(Pool pool, const int* act, const 
 // work items {row, first, end} as for the scalar kernels.  Each instance takes
 // the tile that pads least: 32×32 for T·P̂ when k ≤ 32 and for the SYRK when
 // m ≤ 64, else 64×64.
-using DmmaCfgKN = F64Cfg<64, 64, 2, 2, false, true>;  // A MN-contiguous, B K-contiguous
 using DmmaCfgKK = F64Cfg<64, 64, 2, 2, true, true>;   // both K-contiguous
-using DmmaCfgKN32 = F64Cfg<32, 32, 2, 2, false, true>;  // 32×32 tiles for small instances
 using DmmaCfgKK32 = F64Cfg<32, 32, 2, 2, true, true>;
 
-// T and P̂ fused per constraint: work item {row, first j, end j}; T_j = W·A_j
-// goes to this CTA's k×k scratch (pool.T + blockIdx.x·kq, reused for every j,
-// so it stays in L2), then P̂_j = T_j·L_Y.
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::NT)
-    k_b_dmma_tp(Pool pool, const int* act, const int4* work) {
-  extern __shared__ __align__(16) double smem[];
+// P̂_j = W·A_j·L_Y for the constraints of one work item {row, first j, end j}.  W and
+// L_Y stay in shared tiles, the next A_j's are fetched into registers during the
+// products, and a strip's T = W·A_j goes from accumulators to A fragments by shuffle:
+// the products, with the triangles' zero blocks left out, are what is left.  Below
+// order 33 several constraints share the CTA: ws = 8, 4, 2 or 1 warps each for
+// nb = ⌈k/8⌉ > 4, > 2, 2, 1 block rows.  (Through the general 64×64 tile loop, T
+// through L2, the 512-instance launch took 1.16 ms.)
+template <int NB>
+__device__ __forceinline__ void tp_strip(const double* Ws, const double* Ls, const double* As, int s, double* Pj,
+                                         int k) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double x[NB][2] = {}, y[NB][2] = {};
+#pragma unroll 2
+  for (int p = 0; p < 2 * s + 2; ++p) {  // W is lower
+    const int q = 4 * p + t;
+    const double a = Ws[q * FLD + 8 * s + g];
+#pragma unroll
+    for (int f = 0; f < NB; ++f) tile64::mma8(x[f][0], x[f][1], a, As[(8 * f + g) * FLD + q]);
+  }
+#pragma unroll
+  for (int p = 0; p < 2 * NB; ++p) {
+    const int src = (lane & 28) | (2 * (p & 1) + (t >> 1)), q = 4 * p + t;
+    const double v0 = __shfl_sync(0xffffffffu, x[p / 2][0], src);
+    const double v1 = __shfl_sync(0xffffffffu, x[p / 2][1], src);
+    const double a = (t & 1) ? v1 : v0;
+#pragma unroll
+    for (int f = 0; f <= p / 2; ++f) tile64::mma8(y[f][0], y[f][1], a, Ls[(8 * f + g) * FLD + q]);  // L_Y is lower
+  }
+  const int r = 8 * s + g;
+  if (r < k)
+#pragma unroll
+    for (int f = 0; f < NB; ++f)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (8 * f + 2 * t + e < k) Pj[r + (8 * f + 2 * t + e) * k] = y[f][e];
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_b_dmma_tp(Pool pool, const int* act, const int4* work) {
+  extern __shared__ __align__(16) double sm[];
   const int4 wi = work[blockIdx.x];
   const Inst I = pool.inst[act[wi.x]];
-  const int k = I.k;
-  const long long kk = (long long)k * k;
-  double* T = pool.T + (long long)blockIdx.x * pool.kq;
-  const Opnd Aw{pool.W + I.kk_off, k, 1, 0, 1 << 30, k, k};     // (r, p) at r + p·k
-  const Opnd At{T, k, 1, 0, 1 << 30, k, k};                      // (r, q) at r + q·k
-  const Opnd Bl{pool.LY + I.kk_off, 1, k, 0, 1 << 30, k, k};    // (q, c) at q + c·k
-  for (int j = wi.y; j < wi.z; ++j) {
-    const Opnd Bj{pool.A + I.a_off + (long long)j * kk, 1, k, 0, 1 << 30, k, k};  // (p, c)
-    double acc[Cfg::FM][Cfg::FN][2];
-    zero_acc<Cfg>(acc);
-    f64_tile_mainloop<Cfg>(acc, Aw, Bj, 0, 0, 0, k, smem);
-    for_each_acc<Cfg>(acc, [&](int r, int c, double v) {
-      if (r < k && c < k) T[r + (long long)c * k] = v;
-    });
+  const int k = I.k, nb = (k + 7) / 8, kk = k * k;
+  double *Ws = sm, *Ls = Ws + pool.kq, *As = Ls + pool.kq;
+  const int ws = nb > 4 ? 8 : nb > 2 ? 4 : nb;  // warps and 8-column blocks of As per constraint
+  const int per = 8 / ws, warp = threadIdx.x >> 5;
+  cta_load_tile(Ws, pool.W + I.kk_off, k);
+  cta_load_tile(Ls, pool.LY + I.kk_off, k);
+  const double* A = pool.A + I.a_off;
+  double* Ph = pool.Ph + I.a_off;
+  // thread → row r, columns cb + 4·u of As; column 8·ws·v + c is column c of constraint v
+  const int r = threadIdx.x & 63, cb = threadIdx.x >> 6;
+  double v[16];
+  auto fetch = [&](int j0) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int col = cb + 4 * u, j = j0 + col / (8 * ws), c = col % (8 * ws);
+      v[u] = (r < k && c < k && j < wi.z) ? A[(long long)j * kk + r + c * k] : 0.0;
+    }
+  };
+  fetch(wi.y);
+  for (int j0 = wi.y; j0 < wi.z; j0 += per) {
+    __syncthreads();  // the previous products' reads of As are done
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      if (r < 8 * nb) As[(cb + 4 * u) * FLD + r] = v[u];
     __syncthreads();
-    zero_acc<Cfg>(acc);
-    f64_tile_mainloop<Cfg>(acc, At, Bl, 0, 0, 0, k, smem);
-    double* Pj = pool.Ph + I.a_off + (long long)j * kk;
-    for_each_acc<Cfg>(acc, [&](int r, int c, double v) {
-      if (r < k && c < k) Pj[r + (long long)c * k] = v;
-    });
-    __syncthreads();
+    if (j0 + per < wi.z) fetch(j0 + per);
+    const int j = j0 + warp / ws, s = warp % ws;
+    if (j < wi.z && s < nb) {
+      const double* Aj = As + (warp / ws) * 8 * ws * FLD;
+      double* Pj = Ph + (long long)j * kk;
+      switch (nb) {
+        case 1: tp_strip<1>(Ws, Ls, Aj, s, Pj, k); break;
+        case 2: tp_strip<2>(Ws, Ls, Aj, s, Pj, k); break;
+        case 3: tp_strip<3>(Ws, Ls, Aj, s, Pj, k); break;
+        case 4: tp_strip<4>(Ws, Ls, Aj, s, Pj, k); break;
+        case 5: tp_strip<5>(Ws, Ls, Aj, s, Pj, k); break;
+        case 6: tp_strip<6>(Ws, Ls, Aj, s, Pj, k); break;
+        case 7: tp_strip<7>(Ws, Ls, Aj, s, Pj, k); break;
+        default: tp_strip<8>(Ws, Ls, Aj, s, Pj, k); break;
+      }
+    }
   }
 }
 
@@ -708,18 +757,18 @@ __global__ void k_b_rollback(Pool pool, const int* act, const double* par, doubl
 
 // B10: backtracking line search per side: the first t of 1, γ, γ², … for
 // which M + t·dM has a Cholesky factor with min|L_jj| > kRatio·max|L_jj|, or
-// the first t below kMinStep (src/kernels/threaded.jl:1751-1818); eight
-// candidates at a time.
+// the first t below kMinStep (src/kernels/threaded.jl:1751-1818).
 __global__ void __launch_bounds__(kThreads)
     k_b_linesearch(Pool pool, const int* act, const double* par, double* res) {
   INST_PROLOGUE
   extern __shared__ __align__(16) double sm[];
-  __shared__ int flags[kTrialWarps];
+  __shared__ double inv[64], red[32];
+  __shared__ int sfail;
   const double gamma = in[kGamma], min_step = in[kMinStep], ratio = in[kRatio];
   const double tX = cta_backtrack(pool.X + I.kk_off, pool.dX + I.kk_off, k, gamma, min_step,
-                                  ratio, sm, pool.kp, flags);
+                                  ratio, sm, inv, &sfail, red);
   const double tY = cta_backtrack(pool.Y + I.kk_off, pool.dY + I.kk_off, k, gamma, min_step,
-                                  ratio, sm, pool.kp, flags);
+                                  ratio, sm, inv, &sfail, red);
   if (threadIdx.x == 0) {
     out[oTX] = tX;
     out[oTY] = tY;
@@ -1147,6 +1196,7 @@ struct Engine {
     if (st) cudaStreamDestroy(st);
   }
 
+  size_t smem_tp() const { return smem_bytes(2) + sizeof(double) * 64 * FLD; }
   size_t smem_bytes(int mats) const { return (size_t)mats * (size_t)pool.kq * sizeof(double); }
   // Packed lower triangles of X, dX and kTrialWarps trial slots (the step-length phases).
   size_t smem_trials() const {
@@ -1365,15 +1415,13 @@ struct Engine {
 
   // The Schur assembly on the FP64 tensor cores: three grouped DMMA products
   // (T = W·A, P̂ = T·L_Y, S = P̂P̂ᵀ), work items of about `g` flops, largest first.
-  DBuf<double> Tbuf;  // one k×k scratch per fused T·P̂ work item
   bool dmma_attrs = false;
   void schur_dmma(const std::vector<int>& ids, double g) {
     const int n = (int)ids.size();
     if (n == 0) return;
     if (!dmma_attrs) {
-      SDPX_CUDA(cudaFuncSetAttribute(k_b_dmma_tp<DmmaCfgKN>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)DmmaCfgKN::SMEM_BYTES));
+      SDPX_CUDA(cudaFuncSetAttribute(k_b_dmma_tp, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem_tp()));
       SDPX_CUDA(cudaFuncSetAttribute(k_b_dmma_syrk<DmmaCfgKK>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)DmmaCfgKK::SMEM_BYTES));
@@ -1388,9 +1436,8 @@ struct Engine {
       return 4.0 * I.k * I.k * I.k * I.m + (double)I.k * I.k * I.m * I.m;
     };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost(a) > cost(b); });
-    // Per instance the tile that pads least: 32 for T·P̂ when k ≤ 32 (one k×k
-    // tile per constraint) and for the SYRK when m ≤ 64, else 64.
-    std::vector<int4> tp64, tp32, sy64, sy32;
+    // The SYRK's tile per instance: 32 when m ≤ 64 (it pads least), else 64.
+    std::vector<int4> tp, sy64, sy32;
     if (g < 0) {  // about 16 items a SM, of at least 2.5e5 flops (a launch's tail) …
       double total = 0;  // … and at most 1e6 (the finest of the timed grains, the fastest)
       for (int q = 0; q < n; ++q) total += cost(q);
@@ -1406,46 +1453,28 @@ struct Engine {
     for (int q = 0; q < n; ++q) ha[q] = ids[q];
     for (int q : order) {
       const Inst& I = inst[ids[q]];
-      split(I.k <= 32 ? tp32 : tp64, q, I.m, 4.0 * I.k * I.k * I.k * I.m);
+      split(tp, q, I.m, 4.0 * I.k * I.k * I.k * I.m);
       const int T = I.m <= 64 ? 32 : 64;
       const int nt = (I.m + T - 1) / T, tri = nt * (nt + 1) / 2;
       split(T == 32 ? sy32 : sy64, q, tri, (double)I.k * I.k * I.m * I.m);
       schur_flops += 2.0 * I.k * I.k * I.k * I.m + (double)I.k * I.k * I.m * I.m;
     }
-    const size_t ntp = tp64.size() + tp32.size();
-    if (Tbuf.n < ntp * (size_t)pool.kq) {
-      Tbuf.alloc(ntp * (size_t)pool.kq + ntp * (size_t)pool.kq / 4);
-      pool.T = Tbuf.p;
-    }
-    const size_t nw = ntp + sy64.size() + sy32.size();
+    const size_t nw = tp.size() + sy64.size() + sy32.size();
     if (d_work.n < nw) d_work.alloc(nw + nw / 4);
     h_work.ensure(nw * sizeof(int4));
     int4* hw = static_cast<int4*>(h_work.p);
     size_t o = 0;
-    for (auto* w : {&tp64, &tp32, &sy64, &sy32}) {
+    for (auto* w : {&tp, &sy64, &sy32}) {
       std::copy(w->begin(), w->end(), hw + o);
       o += w->size();
     }
     SDPX_CUDA(cudaMemcpyAsync(d_act.p, ha, n * sizeof(int), cudaMemcpyHostToDevice, st));
     SDPX_CUDA(cudaMemcpyAsync(d_work.p, hw, nw * sizeof(int4), cudaMemcpyHostToDevice, st));
     SDPX_CUDA(cudaEventRecord(ev[0], st));
-    // The T·P̂ kernels index their scratch by blockIdx.x: the 32-tile launch
-    // takes the slots after the 64-tile one's.
-    Pool p32 = pool;
-    p32.T = pool.T + (long long)tp64.size() * pool.kq;
     const int4* w = d_work.p;
-    if (!tp64.empty()) {
-      k_b_dmma_tp<DmmaCfgKN><<<(int)tp64.size(), DmmaCfgKN::NT, DmmaCfgKN::SMEM_BYTES, st>>>(
-          pool, d_act.p, w);
-      SDPX_LAUNCH_CHECK();
-    }
-    w += tp64.size();
-    if (!tp32.empty()) {
-      k_b_dmma_tp<DmmaCfgKN32><<<(int)tp32.size(), DmmaCfgKN32::NT, DmmaCfgKN32::SMEM_BYTES,
-                                 st>>>(p32, d_act.p, w);
-      SDPX_LAUNCH_CHECK();
-    }
-    w += tp32.size();
+    k_b_dmma_tp<<<(int)tp.size(), kThreads, smem_tp(), st>>>(pool, d_act.p, w);
+    SDPX_LAUNCH_CHECK();
+    w += tp.size();
     if (!sy64.empty()) {
       k_b_dmma_syrk<DmmaCfgKK><<<(int)sy64.size(), DmmaCfgKK::NT, DmmaCfgKK::SMEM_BYTES, st>>>(
           pool, d_act.p, w);
@@ -1458,8 +1487,7 @@ struct Engine {
       SDPX_LAUNCH_CHECK();
     }
     SDPX_CUDA(cudaEventRecord(ev[1], st));
-    launches += (tp64.empty() ? 0 : 1) + (tp32.empty() ? 0 : 1) + (sy64.empty() ? 0 : 1) +
-                (sy32.empty() ? 0 : 1);
+    launches += 1 + (sy64.empty() ? 0 : 1) + (sy32.empty() ? 0 : 1);
     SDPX_CUDA(cudaEventSynchronize(ev[1]));
     float ms = 0;
     SDPX_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
@@ -1895,7 +1923,7 @@ struct Engine {
         R.d_res = R.sd_res;
       }
       const auto tl1 = std::chrono::steady_clock::now();
-      out = phase(k_b_linesearch, ok3, smem_trials(), [&](int id, double* in) {
+      out = phase(k_b_linesearch, ok3, smem_bytes(1), [&](int id, double* in) {
         const Run& R = runs[id];
         in[kGamma] = R.params.backtracking;
         in[kMinStep] = R.params.minimum_step;

@@ -36,7 +36,6 @@ struct Pool {
   const Inst* inst;
   const double* A;
   double* Ph;
-  double* T;  // k×k scratch per work item of the DMMA Schur path (T_j = W·A_j)
   const double* C;
   const double* c;
   double *X, *Y, *P, *R, *LX, *LY, *W, *dX, *dY, *Z, *Xb, *Yb;
@@ -440,50 +439,37 @@ __device__ double cta_ftb_tree(const double* X, const double* dX, int k, double*
 }
 
 // Backtracking (src/kernels/threaded.jl:1751-1818): the first t of 1, γ, γ², …
-// whose trial passes (Cholesky and, for ratio > 0, the diagonal-ratio margin),
-// or the first t below min_step; kTrialWarps candidates per round, one per
-// warp.  Called by the whole CTA.  γ ∈ (0, 1) reaches min_step > 0 long
-// before the round guard, which bounds the loop for any other input.  sm and
-// flags as for cta_ftb_tree.
-__device__ double cta_backtrack(const double* X, const double* dX, int k, double gamma,
-                                double min_step, double ratio, double* sm, long long kp,
-                                int* flags) {
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* Xp = sm;
-  double* dXp = sm + kp;
-  double* slot = sm + (2 + w) * kp;
-  cta_load_packed(X, dX, k, Xp, dXp);
-  double t_next = 1.0;
-  for (int round = 0; round < 512; ++round) {
-    double cand[kTrialWarps];
-    int nc = 0;
-    double tt = t_next;
+// whose trial X + t·dX passes (Cholesky and, for ratio > 0, the diagonal-ratio
+// margin), or the first t below min_step.  One trial after the other, each by the whole
+// CTA in one tile M: eight at a time, a warp each in packed slots, took 166 KB of
+// shared memory (one CTA an SM) and 5 times as long a trial.  γ ∈ (0, 1) reaches
+// min_step > 0 long before the round guard, which bounds the loop for any other
+// input.
+__device__ double cta_backtrack(const double* X, const double* dX, int k, double gamma, double min_step,
+                                double ratio, double* M, double* inv, int* sfail, double* red) {
+  const int r = threadIdx.x & 63, cb = threadIdx.x >> 6, k8 = (k + 7) & ~7;
+  double x[16], dx[16];
 #pragma unroll
-    for (int j = 0; j < kTrialWarps; ++j) {
-      if (nc > 0 && cand[nc - 1] < min_step) break;
-      cand[j] = tt;
-      nc = j + 1;
-      tt *= gamma;
-    }
-    double mine = 0.0;
-#pragma unroll
-    for (int j = 0; j < kTrialWarps; ++j)
-      if (j == w) mine = cand[j];
-    if (w < nc) {
-      const bool ok = warp_trial(Xp, dXp, mine, k, ratio, slot);
-      if (lane == 0) flags[w] = ok ? 1 : 0;
-    }
-    __syncthreads();
-    int f[kTrialWarps];
-#pragma unroll
-    for (int n = 0; n < kTrialWarps; ++n) f[n] = flags[n];
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kTrialWarps; ++j)
-      if (j < nc && (f[j] || cand[j] < min_step)) return cand[j];
-    t_next = cand[nc - 1] * gamma;
+  for (int u = 0; u < 16; ++u) {
+    const int c = cb + 4 * u;
+    const bool in = r < k && c < k;
+    x[u] = in ? X[r + c * k] : (r == c ? 1.0 : 0.0);
+    dx[u] = in ? dX[r + c * k] : 0.0;
   }
-  return t_next;
+  double t = 1.0;
+  for (int round = 0; round < 4096; ++round) {
+    __syncthreads();
+    if (r < k8)
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (cb + 4 * u < k8) M[(cb + 4 * u) * FLD + r] = x[u] + t * dx[u];
+    double mn, mx;
+    bool ok = cta_tile_chol(M, k, inv, sfail, &mn, &mx, red);
+    if (ok && ratio > 0.0) ok = isfinite(mn) && isfinite(mx) && mx > 0 && mn > ratio * mx;
+    if (ok || t < min_step) return t;
+    t *= gamma;
+  }
+  return t;
 }
 
 // ------------------------------------- fraction to the boundary by eigenvalue
