@@ -1275,10 +1275,10 @@ struct Engine {
       for (int r = 0; r < N; ++r) work_rank[order[r]] = r;
     }
     d_act.alloc(N);
-    d_par.alloc((size_t)N * kNIn);
+    d_par.alloc((size_t)N * kNIn + (N + 1) / 2);  // input rows, then the instance list
     d_res.alloc((size_t)N * oNOut);
     h_act.ensure(N * sizeof(int));
-    h_par.ensure((size_t)N * kNIn * sizeof(double));
+    h_par.ensure(kStage * stage_stride());
     h_res.ensure((size_t)N * oNOut * sizeof(double));
     pool.inst = d_inst.p;
     pool.A = A.p;
@@ -1332,32 +1332,33 @@ struct Engine {
                       bool read) {
     const int n = (int)ids.size();
     if (n == 0) return nullptr;
-    // The staging buffers are reused by every launch: the copies queued from
-    // them by the previous one must have run first.
-    SDPX_CUDA(cudaStreamSynchronize(st));
     // CTAs in decreasing order of the instance's work (largest first, so the
     // last wave of a phase holds small instances); rows map back to `ids`.
     lpt.resize(n);
     std::iota(lpt.begin(), lpt.end(), 0);
     std::stable_sort(lpt.begin(), lpt.end(),
                      [&](int a, int b) { return work_rank[ids[a]] < work_rank[ids[b]]; });
-    int* ha = static_cast<int*>(h_act.p);
-    double* hp = static_cast<double*>(h_par.p);
-    std::memset(hp, 0, (size_t)n * kNIn * sizeof(double));
+    // Input rows and instance list in one copy, from the next of kStage staging slots:
+    // the stream is waited for only when all are in use (each read-back frees them).
+    const size_t pbytes = (size_t)n * kNIn * sizeof(double), bytes = pbytes + n * sizeof(int);
+    if (staged == kStage) sync_stream();
+    char* hs = static_cast<char*>(h_par.p) + (size_t)staged++ * stage_stride();
+    double* hp = reinterpret_cast<double*>(hs);
+    int* ha = reinterpret_cast<int*>(hs + pbytes);
+    std::memset(hp, 0, pbytes);
     for (int q = 0; q < n; ++q) {
       ha[q] = ids[lpt[q]];
       fill(ids[lpt[q]], hp + (size_t)q * kNIn);
     }
-    SDPX_CUDA(cudaMemcpyAsync(d_act.p, ha, n * sizeof(int), cudaMemcpyHostToDevice, st));
-    SDPX_CUDA(cudaMemcpyAsync(d_par.p, hp, (size_t)n * kNIn * sizeof(double),
-                              cudaMemcpyHostToDevice, st));
-    kf<<<n, kThreads, smem, st>>>(pool, d_act.p, d_par.p, d_res.p);
+    SDPX_CUDA(cudaMemcpyAsync(d_par.p, hs, bytes, cudaMemcpyHostToDevice, st));
+    kf<<<n, kThreads, smem, st>>>(pool, reinterpret_cast<const int*>(d_par.p + (size_t)n * kNIn), d_par.p,
+                                  d_res.p);
     SDPX_LAUNCH_CHECK();
     ++launches;
     if (!read) return nullptr;
     SDPX_CUDA(cudaMemcpyAsync(h_res.p, d_res.p, (size_t)n * oNOut * sizeof(double),
                               cudaMemcpyDeviceToHost, st));
-    SDPX_CUDA(cudaStreamSynchronize(st));
+    sync_stream();
     const double* launched = static_cast<const double*>(h_res.p);
     rows.resize((size_t)n * oNOut);
     for (int q = 0; q < n; ++q)
@@ -1366,6 +1367,13 @@ struct Engine {
     return rows.data();
   }
   std::vector<int> lpt, work_rank;  // launch order; rank of each instance by work
+  static constexpr int kStage = 16;
+  int staged = 0;  // staging slots in use
+  size_t stage_stride() const { return ((size_t)N * (kNIn * sizeof(double) + sizeof(int)) + 63) & ~size_t(63); }
+  void sync_stream() {
+    SDPX_CUDA(cudaStreamSynchronize(st));
+    staged = 0;
+  }
   std::vector<double> rows;         // output rows in the caller's order
   const double* phase(PhaseKernel kf, const std::vector<int>& ids, size_t smem, bool read) {
     return phase(kf, ids, smem, [](int, double*) {}, read);

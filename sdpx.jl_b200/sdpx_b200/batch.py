@@ -103,6 +103,7 @@ class BatchSolver:
             raise SDPXB200Error("sdpx_b200_batch_create: " +
                                 self._lib.sdpx_b200_batch_create_error().decode())
         self._h = h
+        self._read_back = None
         self.shape = None
 
     def _call(self, name, *args):
@@ -193,26 +194,34 @@ class BatchSolver:
         res = (SolveResult * n)()
         self._call("sdpx_b200_batch_optimize", C.byref(no), res)
         dp = C.POINTER(C.c_double)
-        mt = sum(p.m for p in self.problems)
-        kt = sum(p.k[0] * p.k[0] for p in self.problems)
-        xs, Xs, Ys = np.zeros(mt), np.zeros(kt), np.zeros(kt)
+        if self._read_back is None:  # X and Y are read back here and copied out per instance
+            kt = sum(p.k[0] * p.k[0] for p in self.problems)
+            self._read_back = np.zeros(kt), np.zeros(kt)
+        xs = np.zeros(sum(p.m for p in self.problems))
+        Xs, Ys = self._read_back
         if solutions:  # one read-back of every instance's x, X, Y
             self._call("sdpx_b200_batch_get_solutions", xs.ctypes.data_as(dp),
                        Xs.ctypes.data_as(dp), Ys.ctypes.data_as(dp))
+        else:
+            Xs[:] = 0.0
+            Ys[:] = 0.0
         out = []
         mo = ko = 0
-        for i, p in enumerate(self.problems):
+        fields = np.frombuffer(res, dtype=np.dtype(SolveResult))  # columns, not field by field
+        cols = [fields[name].tolist() for name in (
+            "status", "p_obj", "d_obj", "p_res", "d_res", "iterations", "restarts",
+            "fp64_iterations", "seconds")]
+        status = {code: Status(name) for code, name in STATUS_NAMES.items()}
+        for p, r, st, po, do, pr, dr, it, rs, nf, sec in zip(self.problems, res, *cols):
             k = p.k[0]
             x, X, Y = xs[mo:mo + p.m], Xs[ko:ko + k * k], Ys[ko:ko + k * k]
             mo += p.m
             ko += k * k
-            r = res[i]
             out.append(SDPResult(
-                status=Status(STATUS_NAMES[r.status]), message=r.message.decode(errors="replace"),
+                status=status[st], message=r.message.decode(errors="replace"),
                 x=x, X=[X.reshape(k, k).T.copy()], y=np.zeros(0), Y=[Y.reshape(k, k).T.copy()],
-                pObj=r.p_obj, dObj=r.d_obj, p_res=r.p_res, d_res=r.d_res,
-                iterations=r.iterations, restarts=r.restarts,
-                precision_trace=["fp64"] * r.fp64_iterations, seconds=r.seconds))
+                pObj=po, dObj=do, p_res=pr, d_res=dr, iterations=it, restarts=rs,
+                precision_trace=["fp64"] * nf, seconds=sec))
         return out
 
     def set_solution(self, i: int, x=None, X=None, Y=None):
