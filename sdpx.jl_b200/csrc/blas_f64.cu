@@ -11,8 +11,9 @@
 namespace sdpx {
 
 // Tile configurations.  128×128 / 8 warps for the large Schur products,
-// 64×64 / 4 warps for per-block k×k products.
-using CfgBigKT = F64Cfg<128, 128, 2, 4, true, true>;    // SYRK: both operands K-contiguous
+// 64×64 / 4 warps for per-block k×k products and the Gram products (…2: rows 16-byte
+// aligned).
+using CfgBigKT = F64Cfg<128, 128, 2, 4, true, true>;    // both operands K-contiguous
 using CfgBigMK = F64Cfg<128, 128, 2, 4, false, true>;   // A MN-contiguous, B K-contiguous
 using CfgSmMK = F64Cfg<64, 64, 2, 2, false, true>;
 using CfgSmKK = F64Cfg<64, 64, 2, 2, true, true>;
@@ -22,6 +23,8 @@ using CfgSmKM = F64Cfg<64, 64, 2, 2, true, false>;
 // products of the Newton step: 400×400 is 49 tiles of 64 but 169 of 32).
 using CfgTnMK = F64Cfg<32, 32, 2, 2, false, true>;
 using CfgTnKK = F64Cfg<32, 32, 2, 2, true, true>;
+using CfgSmKK2 = F64Cfg<64, 64, 2, 2, true, true, 2>;
+using CfgTnKK2 = F64Cfg<32, 32, 2, 2, true, true, 2>;
 using CfgTnMM = F64Cfg<32, 32, 2, 2, false, false>;
 using CfgTnKM = F64Cfg<32, 32, 2, 2, true, false>;
 
@@ -113,7 +116,7 @@ __global__ void k_syrk_reduce(const double* partial, int ntri, int nchunk, int m
   while ((ti + 1) * (ti + 2) / 2 <= tri) ++ti;
   while (ti * (ti + 1) / 2 > tri) --ti;
   const int tj = tri - ti * (ti + 1) / 2;
-  for (int e = threadIdx.x; e < BM * BN; e += blockDim.x) {
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < BM * BN; e += gridDim.y * blockDim.x) {
     int r = e % BM, c = e / BM;
     int gi = ti * BM + r, gj = tj * BN + c;
     if (gi >= m || gj >= m) continue;
@@ -214,56 +217,101 @@ void trmm_right_lower_inplace_f64(const Opnd& T, const Opnd& L, const OutDesc& C
   SDPX_LAUNCH_CHECK();
 }
 
-SyrkPlan plan_syrk_f64(int m, long long K, int sm_count) {
+// Tile order and K split of a lower Gram product by a model of its time in SM cycles.
+// `resident` CTAs of a tile fit an SM; a K step of 16 costs a CTA `latency` alone and
+// `rate` when the others hide it (a step of the 64-tile is 1088 cycles of DMMA issue);
+// `fixed` is a unit's prologue and store.  The partial tiles are written and read again.
+// One CTA of 128×128 an SM left nothing to hide a step's copies and barriers behind:
+// it measured no faster than one of these at any size, at most 28 TFLOP/s.  µs with the
+// reduction, 128 / 64 / 32 (K chunks from this model): 3000×26400 8677 / 7549 / 8569
+// (31.5 TFLOP/s), 1000×30150 1270 / 1085 / 1179, 1500×9000 830 / 764 / 757, 700×4000
+// 103 / 89 / 91, 317×2408 35 / 22 / 21, 61×333 39 / 23 / 13, 5×333 39 / 21 / 11.
+struct SyrkTile {
+  int bm, resident;
+  double latency, rate, fixed;
+};
+constexpr SyrkTile kSyrkTiles[] = {{64, 3, 2000, 1130, 8000}, {32, 7, 800, 325, 5000}};
+// Chunks of 128 rows or more, and of 2048 or less where 16 chunks and 1 GiB of partial
+// tiles allow: a longer running sum rounds more (3000×26400: relative error of the
+// solve 6.0e-16 with chunks of 8800 rows, 4.3e-16 with 2048, no slower).
+constexpr int kMaxChunks = 32, kMinChunkRows = 128, kMaxChunkRows = 2048;
+constexpr long long kPartialDoubles = 1LL << 27;
+
+static SyrkPlan syrk_plan(int m, long long K, int bm, int nchunk) {
   SyrkPlan p;
-  p.bm = CfgBigKT::BM;
-  int nt = ceil_div(m, p.bm);
+  p.bm = bm;
+  const int nt = ceil_div(m, bm);
   p.ntri = nt * (nt + 1) / 2;
-  // Choose the number of K chunks so the unit count fills whole waves of one
-  // CTA per SM, with at least 256 rows of K per chunk.
-  int best_c = 1;
-  double best_eff = 0.0;
-  long long max_c = K / 256;
-  if (max_c < 1) max_c = 1;
-  if (max_c > 16) max_c = 16;
-  for (int c = 1; c <= max_c; ++c) {
-    long long units = (long long)p.ntri * c;
-    double waves = (double)units / sm_count;
-    double eff = waves / std::ceil(waves);
-    // Prefer more work per wave up to ~4 waves; past that, only efficiency counts.
-    double score = eff * std::min(1.0, waves / 4.0);
-    if (score > best_eff + 1e-9) {
-      best_eff = score;
-      best_c = c;
-    }
-  }
-  long long kc = (K + best_c - 1) / best_c;
-  kc = ((kc + 15) / 16) * 16;
+  const long long kc = ((K + nchunk - 1) / nchunk + 15) / 16 * 16;
   p.kchunk = (int)kc;
   p.nchunk = (int)((K + kc - 1) / kc);
-  p.partial_doubles = (size_t)p.nchunk * p.ntri * p.bm * p.bm;
+  p.partial_doubles = (size_t)p.nchunk * p.ntri * bm * bm;
   return p;
+}
+
+static double syrk_cycles(const SyrkPlan& p, const SyrkTile& t, int sms) {
+  const double units = (double)p.ntri * p.nchunk, steps = p.kchunk / 16;
+  const int n = (int)std::ceil(units / sms), full = n / t.resident, rest = n % t.resident;
+  const double round = steps * std::max(t.latency, t.resident * t.rate) + t.fixed;
+  const double last = rest ? steps * std::max(t.latency, rest * t.rate) + t.fixed : 0.0;
+  return full * round + last + (double)p.partial_doubles * 16 * 4.75e-4;  // 4 TB/s at 1.9 GHz
+}
+
+static SyrkPlan best_split(int m, long long K, int sms, const SyrkTile& t, long long max_chunks, double* cycles) {
+  max_chunks = std::max<long long>(1, std::min({max_chunks, K / kMinChunkRows, (long long)kMaxChunks}));
+  const long long tiles = (long long)syrk_plan(m, K, t.bm, 1).partial_doubles;
+  const long long min_chunks = std::max<long long>(
+      1, std::min<long long>({ceil_div(K, kMaxChunkRows), 16, kPartialDoubles / tiles, max_chunks}));
+  SyrkPlan best;
+  for (int c = (int)min_chunks; c <= max_chunks; ++c) {
+    const SyrkPlan p = syrk_plan(m, K, t.bm, c);
+    const double cy = syrk_cycles(p, t, sms);
+    if (c == min_chunks || cy < *cycles) best = p, *cycles = cy;
+  }
+  return best;
+}
+
+SyrkPlan plan_syrk_f64(int m, long long K, int sm_count) {
+  SyrkPlan best;
+  double least = 0.0;
+  for (const SyrkTile& t : kSyrkTiles) {
+    double cycles = 0.0;
+    const SyrkPlan p = best_split(m, K, sm_count, t, kMaxChunks, &cycles);
+    if (&t == kSyrkTiles || cycles < least) best = p, least = cycles;
+  }
+  return best;
+}
+
+template <class Cfg>
+static void launch_syrk(const Opnd& P, const SyrkPlan& plan, double* partial, double* S, long long lds,
+                        int m, double beta, cudaStream_t st) {
+  ensure_smem(k_syrk_splitk<Cfg>, Cfg::SMEM_BYTES);
+  const int units = plan.ntri * plan.nchunk;
+  k_syrk_splitk<Cfg><<<units, Cfg::NT, Cfg::SMEM_BYTES, st>>>(P, plan.ntri, plan.kchunk, partial);
+  const int slices = std::max(1, std::min(Cfg::BM * Cfg::BN / 256, 592 / std::max(1, plan.ntri)));
+  k_syrk_reduce<Cfg::BM, Cfg::BN><<<dim3(plan.ntri, slices), 256, 0, st>>>(partial, plan.ntri, plan.nchunk, m,
+                                                                           S, lds, beta);
+  SDPX_LAUNCH_CHECK_N(2);
 }
 
 void syrk_lower_f64(const Opnd& P, const SyrkPlan& plan, double* partial, double* S, long long lds,
                     int m, double beta, cudaStream_t st) {
-  using Cfg = CfgBigKT;
-  ensure_smem(k_syrk_splitk<Cfg>, Cfg::SMEM_BYTES);
-  int units = plan.ntri * plan.nchunk;
-  k_syrk_splitk<Cfg><<<units, Cfg::NT, Cfg::SMEM_BYTES, st>>>(P, plan.ntri, plan.kchunk, partial);
-  SDPX_LAUNCH_CHECK();
-  k_syrk_reduce<Cfg::BM, Cfg::BN><<<plan.ntri, 256, 0, st>>>(partial, plan.ntri, plan.nchunk, m, S,
-                                                             lds, beta);
-  SDPX_LAUNCH_CHECK();
+  const bool even = P.kstride == 1 && ((P.inner_stride | P.outer_stride) & 1) == 0 &&
+                    (reinterpret_cast<uintptr_t>(P.base) & 15) == 0;
+  if (plan.bm == 32)
+    return even ? launch_syrk<CfgTnKK2>(P, plan, partial, S, lds, m, beta, st)
+                : launch_syrk<CfgTnKK>(P, plan, partial, S, lds, m, beta, st);
+  return even ? launch_syrk<CfgSmKK2>(P, plan, partial, S, lds, m, beta, st)
+              : launch_syrk<CfgSmKK>(P, plan, partial, S, lds, m, beta, st);
 }
 
 // ---------------------------------------------------------------------------
 // Allocation-free variant of the split-K lower Gram product S = PᵀP.
 //
 // The split-K partial tiles live in a fixed file-scope device array instead of
-// caller- or library-allocated memory.  One K chunk of every lower 128×128 tile
-// must fit (ntri·128·128 doubles, ntri = t(t+1)/2, t = ceil(m/128)): the stated
-// limit m ≤ 2048 (t = 16, 2.2 Mi doubles) leaves room for a second chunk.  K is
+// caller- or library-allocated memory.  One K chunk of every lower 64×64 tile
+// must fit (ntri·64·64 doubles, ntri = t(t+1)/2, t = ceil(m/64)): the stated
+// limit m ≤ 2048 (t = 32, 2.1 Mi doubles) leaves room for a second chunk.  K is
 // bounded by the int32 K indexing of the tile loop: chunk starts plus a chunk
 // length must stay below 2³¹, which K ≤ 2³⁰ guarantees.  Every GPU that loads
 // the library holds the array until the process exits, and all calls share it.
@@ -297,7 +345,7 @@ static double* noalloc_scratch_address() {
 size_t gram_noalloc_capacity_doubles() { return kNoAllocScratchDoubles; }
 
 void syrk_lower_f64_noalloc(const double* P, long long K, int m, double* S, cudaStream_t st) {
-  using Cfg = CfgBigKT;
+  using Cfg = CfgSmKK;
   const int nt = ceil_div(m, Cfg::BM);
   const long long ntri = (long long)nt * (nt + 1) / 2;
   const long long tile = (long long)Cfg::BM * Cfg::BN;
@@ -314,14 +362,9 @@ void syrk_lower_f64_noalloc(const double* P, long long K, int m, double* S, cuda
   int dev = 0, sms = 148;
   SDPX_CUDA(cudaGetDevice(&dev));
   SDPX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // As many K chunks as the scratch holds, capped by the normal plan.
-  SyrkPlan plan = plan_syrk_f64(m, K, sms);
-  long long max_chunks = (long long)kNoAllocScratchDoubles / (ntri * tile);
-  int nchunk = (int)std::max<long long>(1, std::min<long long>(plan.nchunk, max_chunks));
-  long long kc = (K + nchunk - 1) / nchunk;
-  kc = ((kc + 15) / 16) * 16;
-  plan.kchunk = (int)kc;
-  plan.nchunk = (int)((K + kc - 1) / kc);
+  // At most as many K chunks as the scratch holds.
+  double cycles = 0.0;
+  const SyrkPlan plan = best_split(m, K, sms, kSyrkTiles[0], (long long)kNoAllocScratchDoubles / (ntri * tile), &cycles);
   Opnd Pd;
   Pd.base = P;
   Pd.kstride = 1;

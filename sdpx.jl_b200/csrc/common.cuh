@@ -105,6 +105,12 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pre
   int n = pred ? 8 : 0;  // zero-fill when out of range
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
 }
+// 16 bytes (both addresses 16-byte aligned), of which the first `bytes` are read and the
+// rest zero-filled.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {

@@ -11,8 +11,11 @@
 
 namespace sdpx {
 
-template <int BM_, int BN_, int WARPS_M_, int WARPS_N_, bool A_KCONTIG_, bool B_KCONTIG_>
+// VEC = 2: both operands K-contiguous with 16-byte aligned rows (even strides, an
+// aligned base), copied two elements at a time.
+template <int BM_, int BN_, int WARPS_M_, int WARPS_N_, bool A_KCONTIG_, bool B_KCONTIG_, int VEC_ = 1>
 struct F64Cfg {
+  static constexpr int VEC = VEC_;
   static constexpr int BM = BM_, BN = BN_, BK = 16, STAGES = 3;
   static constexpr int WARPS_M = WARPS_M_, WARPS_N = WARPS_N_;
   static constexpr int NT = WARPS_M * WARPS_N * 32;
@@ -23,8 +26,9 @@ struct F64Cfg {
   static constexpr int LDB = B_KCONTIG ? (BK + 4) : (BN + 4);
   static constexpr int A_STAGE = A_KCONTIG ? BM * LDA : BK * LDA;
   static constexpr int B_STAGE = B_KCONTIG ? BN * LDB : BK * LDB;
-  static constexpr int A_PER_T = BM * BK / NT;
-  static constexpr int B_PER_T = BN * BK / NT;
+  static constexpr int A_PER_T = BM * BK / NT / VEC;
+  static constexpr int B_PER_T = BN * BK / NT / VEC;
+  static_assert(VEC == 1 || (A_KCONTIG && B_KCONTIG), "pairs run along K");
   static constexpr size_t SMEM_BYTES = sizeof(double) * STAGES * (A_STAGE + B_STAGE);
   static_assert(BM * BK % NT == 0 && BN * BK % NT == 0, "tile/thread mismatch");
   static_assert(WTM % 8 == 0 && WTN % 8 == 0, "warp tile must be a multiple of 8");
@@ -39,12 +43,12 @@ struct StagePlan {
   int sidx[PER_T];       // shared-memory index inside a stage
 };
 
-template <int TILE_MN, int PER_T, int NT, int LD, bool KCONTIG>
+template <int TILE_MN, int PER_T, int NT, int LD, bool KCONTIG, int VEC>
 __device__ __forceinline__ void make_plan(StagePlan<PER_T>& p, const Opnd& o, int mn0) {
   constexpr int BK = 16;
 #pragma unroll
   for (int j = 0; j < PER_T; ++j) {
-    int idx = threadIdx.x + j * NT;
+    int idx = (threadIdx.x + j * NT) * VEC;
     int mm, kk;
     if (KCONTIG) {
       mm = idx / BK;
@@ -61,7 +65,7 @@ __device__ __forceinline__ void make_plan(StagePlan<PER_T>& p, const Opnd& o, in
   }
 }
 
-template <int PER_T>
+template <int VEC, int PER_T>
 __device__ __forceinline__ void issue_stage(double* s, const StagePlan<PER_T>& p, const Opnd& o,
                                             int k0, int k_end) {
 #pragma unroll
@@ -69,7 +73,8 @@ __device__ __forceinline__ void issue_stage(double* s, const StagePlan<PER_T>& p
     int k = k0 + p.kk[j];
     bool ok = (p.off[j] >= 0) && (k < k_end);
     const double* src = ok ? (o.base + p.off[j] + (long long)k * o.kstride) : o.base;
-    cp_async8(s + p.sidx[j], src, ok);
+    if (VEC == 2) cp_async16(s + p.sidx[j], src, !ok ? 0 : k + 1 < k_end ? 16 : 8);
+    else cp_async8(s + p.sidx[j], src, ok);
   }
 }
 
@@ -82,8 +87,8 @@ __device__ void f64_tile_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2], const Opnd
   double* sB = smem + ST * Cfg::A_STAGE;
   StagePlan<Cfg::A_PER_T> pa;
   StagePlan<Cfg::B_PER_T> pb;
-  make_plan<Cfg::BM, Cfg::A_PER_T, Cfg::NT, Cfg::LDA, Cfg::A_KCONTIG>(pa, A, m0);
-  make_plan<Cfg::BN, Cfg::B_PER_T, Cfg::NT, Cfg::LDB, Cfg::B_KCONTIG>(pb, B, n0);
+  make_plan<Cfg::BM, Cfg::A_PER_T, Cfg::NT, Cfg::LDA, Cfg::A_KCONTIG, Cfg::VEC>(pa, A, m0);
+  make_plan<Cfg::BN, Cfg::B_PER_T, Cfg::NT, Cfg::LDB, Cfg::B_KCONTIG, Cfg::VEC>(pb, B, n0);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -93,21 +98,23 @@ __device__ void f64_tile_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2], const Opnd
 #pragma unroll
   for (int s = 0; s < ST - 1; ++s) {
     if (s < ntiles) {
-      issue_stage(sA + s * Cfg::A_STAGE, pa, A, kb + s * BK, ke);
-      issue_stage(sB + s * Cfg::B_STAGE, pb, B, kb + s * BK, ke);
+      issue_stage<Cfg::VEC>(sA + s * Cfg::A_STAGE, pa, A, kb + s * BK, ke);
+      issue_stage<Cfg::VEC>(sB + s * Cfg::B_STAGE, pb, B, kb + s * BK, ke);
     }
     cp_async_commit();
   }
   for (int tIdx = 0; tIdx < ntiles; ++tIdx) {
+    // One barrier a step: it shows that stage tIdx has arrived and that every warp is
+    // done with stage tIdx − 1, whose slot takes the copies issued next.
+    cp_async_wait<ST - 2>();
+    __syncthreads();
     int pre = tIdx + ST - 1;
     if (pre < ntiles) {
       int s = pre % ST;
-      issue_stage(sA + s * Cfg::A_STAGE, pa, A, kb + pre * BK, ke);
-      issue_stage(sB + s * Cfg::B_STAGE, pb, B, kb + pre * BK, ke);
+      issue_stage<Cfg::VEC>(sA + s * Cfg::A_STAGE, pa, A, kb + pre * BK, ke);
+      issue_stage<Cfg::VEC>(sB + s * Cfg::B_STAGE, pb, B, kb + pre * BK, ke);
     }
     cp_async_commit();
-    cp_async_wait<ST - 1>();
-    __syncthreads();
     const double* a_s = sA + (tIdx % ST) * Cfg::A_STAGE;
     const double* b_s = sB + (tIdx % ST) * Cfg::B_STAGE;
 #pragma unroll
@@ -129,9 +136,9 @@ __device__ void f64_tile_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2], const Opnd
 #pragma unroll
         for (int fn = 0; fn < Cfg::FN; ++fn) dmma_8x8x4(acc[fm][fn][0], acc[fm][fn][1], af[fm], bf[fn]);
     }
-    __syncthreads();
   }
   cp_async_wait<0>();
+  __syncthreads();  // the shared memory is free
 }
 
 template <class Cfg>
