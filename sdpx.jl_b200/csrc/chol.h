@@ -30,10 +30,12 @@ void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, do
 // (64×64, column-major).
 void factor_diag_inverses(const double* L, long long ld, int n, double* Dinv, cudaStream_t st);
 
-// rhs ← (L Lᵀ)^{-1} rhs by blocked forward/backward substitution (work: n).
-template <class T, int NB>
-void cholesky_solve(const T* L, long long ld, int n, const T* Dinv, T* rhs, T* work,
-                    cudaStream_t st);
+// rhs ← (L Lᵀ)⁻¹ rhs, one launch (cooperative for n > 64).  `work`
+// (cholesky_solve_work(n) doubles) and `err` must not be shared by concurrent calls;
+// *err (zero on entry, else nothing waits) becomes 1 and rhs NaN when a wait gave up.
+inline size_t cholesky_solve_work(int n) { return 2 * (size_t)ceil_div(n, 64) * 64; }
+void cholesky_solve(const double* L, long long ld, int n, const double* Dinv, double* rhs, double* work,
+                    int* err, int sms, cudaStream_t st);
 
 // Lower factors to invert together: W_b = L_b⁻¹ (n_b×n_b, column-major, ld n_b), tmp_b
 // n_b×n_b scratch.  The strict upper triangle of W must be zero on entry and is not

@@ -38,30 +38,67 @@
 namespace sdpx {
 namespace {
 
+// A cone's vectors are worked on by a group of g lanes (a power of two up to a warp,
+// chosen from the mean dimension): the elementwise parts run across the lanes, while a
+// sum adds the lanes' terms one by one in index order, so it rounds as the sequential
+// loop does.  One thread per cone had every division and load in one chain
+// (k_nt_scaling: 166 µs for 100 cones of order 64, 17 with a warp each).
+struct Lanes {
+  int g, lane;  // group size, lane in the group
+  unsigned mask;
+  __device__ explicit Lanes(int g_) : g(g_), lane(threadIdx.x & (g_ - 1)) {
+    mask = (g == 32 ? 0xffffffffu : ((1u << g) - 1)) << (threadIdx.x & 31 & ~(g - 1));
+  }
+  __device__ bool all(bool p) const { return __all_sync(mask, p); }
+  __device__ double max(double v) const {
+    for (int o = g >> 1; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(mask, v, o, g));
+    return v;
+  }
+  // acc + the terms of the first cnt lanes, in their order.
+  __device__ double fold(double acc, double term, int cnt) const {
+#pragma unroll 8
+    for (int k = 0; k < cnt; ++k) acc += __shfl_sync(mask, term, k, g);
+    return acc;
+  }
+  // acc + f(i) for i = 1 … n−1, in that order.
+  template <class F>
+  __device__ double sum(double acc, int n, F f) const {
+    for (int i0 = 1; i0 < n; i0 += g) acc = fold(acc, i0 + lane < n ? f(i0 + lane) : 0.0, min(g, n - i0));
+    return acc;
+  }
+  // max(start, f(i)) over i = 1 … n−1.
+  template <class F>
+  __device__ double maximum(double start, int n, F f) const {
+    for (int i = 1 + lane; i < n; i += g) start = fmax(start, f(i));
+    return max(start);
+  }
+  template <class F>
+  __device__ bool every(int n, F f) const {  // f(i) for i = 0 … n−1
+    bool ok = true;
+    for (int i = lane; i < n; i += g) ok = ok && f(i);
+    return all(ok);
+  }
+};
+
 // ------------------------------------------------------------ NT scaling --
 // `_soc_tail_norm` (src/soc_lorentz_kernels.jl:21-34).
-__device__ double tail_norm(const double* v, int n) {
-  double scale = 0.0;
-  for (int i = 1; i < n; ++i) scale = fmax(scale, fabs(v[i]));
+__device__ double tail_norm(const Lanes& L, const double* v, int n) {
+  const double scale = L.maximum(0.0, n, [&](int i) { return fabs(v[i]); });
   if (scale == 0.0) return scale;
-  double ss = 0.0;
-  for (int i = 1; i < n; ++i) {
+  const double ss = L.sum(0.0, n, [&](int i) {
     double y = v[i] / scale;
-    ss += y * y;
-  }
+    return y * y;
+  });
   return scale * sqrt(ss);
 }
 
 // `_soc_sqrt_determinant` (src/soc_lorentz_kernels.jl:42-62).
-__device__ bool sqrt_determinant(const double* v, int n, double* out) {
-  double scale = 0.0;
-  for (int i = 0; i < n; ++i) {
-    if (!isfinite(v[i])) return false;
-    scale = fmax(scale, fabs(v[i]));
-  }
+__device__ bool sqrt_determinant(const Lanes& L, const double* v, int n, double* out) {
+  if (!L.every(n, [&](int i) { return isfinite(v[i]); })) return false;
+  const double scale = L.maximum(fabs(v[0]), n, [&](int i) { return fabs(v[i]); });
   if (scale == 0.0) return false;
   double head = v[0];
-  double tail = tail_norm(v, n);
+  double tail = tail_norm(L, v, n);
   double margin = head - tail;
   if (!(margin > 0.0)) return false;
   double residual = (margin / scale) * (head / scale + tail / scale);
@@ -71,108 +108,117 @@ __device__ bool sqrt_determinant(const double* v, int n, double* out) {
   return isfinite(r) && r > 0.0;
 }
 
-// `_soc_nt_scaling!` (src/soc_lorentz_kernels.jl:72-185), one thread per cone.
+// `_soc_nt_scaling!` (src/soc_lorentz_kernels.jl:72-185), g lanes per cone.
 // The normalised points a = s/√det s, b = z/√det z and the midpoint raw are
 // recomputed where the reference reads its temporaries (the same division
 // gives the same value).  Outputs are written only after every check passed.
-__global__ void k_nt_scaling(int ncones, const long long* __restrict__ off,
+__global__ void k_nt_scaling(int g, int ncones, const long long* __restrict__ off,
                              const int* __restrict__ dim, const double* __restrict__ s,
                              const double* __restrict__ z, double* w, double* lam, double* eta_out,
                              double* eta2_out, int* ok_out) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const Lanes L(g);
+  int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) / g);
   if (c >= ncones) return;
   const int n = dim[c];
   const double* sc = s + off[c];
   const double* zc = z + off[c];
   double* wc = w + off[c];
   double* lc = lam + off[c];
-  ok_out[c] = 0;
-  eta_out[c] = 0.0;
-  eta2_out[c] = 0.0;
+  if (L.lane == 0) {
+    ok_out[c] = 0;
+    eta_out[c] = 0.0;
+    eta2_out[c] = 0.0;
+  }
   double ss = 0.0, zs = 0.0;
-  bool sok = sqrt_determinant(sc, n, &ss);
-  bool zok = sqrt_determinant(zc, n, &zs);
+  bool sok = sqrt_determinant(L, sc, n, &ss);
+  bool zok = sqrt_determinant(L, zc, n, &zs);
   if (!(sok && zok)) return;
   double eta = sqrt(ss) / sqrt(zs);
   double eta2 = eta * eta;
   if (!(isfinite(eta2) && eta2 > 0.0)) return;
-#define A_(i) (sc[i] / ss)
-#define B_(i) (zc[i] / zs)
-  for (int i = 0; i < n; ++i) {
-    double a = A_(i), b = B_(i);
-    double raw = (i == 0) ? a + b : a - b;
-    if (!(isfinite(a) && isfinite(b) && isfinite(raw))) return;
-  }
-  double mscale = 1.0;
-  for (int i = 0; i < n; ++i) mscale = fmax(mscale, fmax(fabs(A_(i)), fabs(B_(i))));
+  auto A = [&](int i) { return sc[i] / ss; };
+  auto B = [&](int i) { return zc[i] / zs; };
+  if (!L.every(n, [&](int i) {
+        double a = A(i), b = B(i);
+        double raw = (i == 0) ? a + b : a - b;
+        return isfinite(a) && isfinite(b) && isfinite(raw);
+      }))
+    return;
+  const double a0 = A(0), b0 = B(0);
+  const double tmax = L.maximum(0.0, n, [&](int i) { return fmax(fabs(A(i)), fabs(B(i))); });
+  const double mscale = fmax(fmax(1.0, tmax), fmax(fabs(a0), fabs(b0)));
   double inv_m = 1.0 / mscale;
-  double cross = (A_(0) * inv_m) * (B_(0) * inv_m);
-  for (int i = 1; i < n; ++i) cross += (A_(i) * inv_m) * (B_(i) * inv_m);
+  double cross = L.sum((a0 * inv_m) * (b0 * inv_m), n,
+                       [&](int i) { return (A(i) * inv_m) * (B(i) * inv_m); });
   double radicand = inv_m * inv_m + cross;
   if (!(isfinite(radicand) && radicand > 0.0)) return;
   double wscale = sqrt(2.0) * mscale * sqrt(radicand);
   if (!(isfinite(wscale) && wscale > 0.0)) return;
-  double nts = 1.0;
-  for (int i = 1; i < n; ++i) nts = fmax(nts, fabs((A_(i) - B_(i)) / wscale));
+  const double nts = L.maximum(1.0, n, [&](int i) { return fabs((A(i) - B(i)) / wscale); });
   double inv_t = 1.0 / nts;
-  double hacc = inv_t * inv_t;
-  for (int i = 1; i < n; ++i) {
-    double val = ((A_(i) - B_(i)) / wscale) / nts;
-    hacc += val * val;
-  }
+  double hacc = L.sum(inv_t * inv_t, n, [&](int i) {
+    double val = ((A(i) - B(i)) / wscale) / nts;
+    return val * val;
+  });
   double nhead = nts * sqrt(hacc);
   if (!(isfinite(nhead) && nhead > 0.0)) return;
   double gamma = wscale / 2.0;
-  double lscale = fmax(fmax(1.0, fabs(A_(0))), fmax(fabs(B_(0)), fabs(gamma)));
-  for (int i = 1; i < n; ++i) lscale = fmax(lscale, fmax(fabs(A_(i)), fabs(B_(i))));
+  double lscale = fmax(fmax(1.0, fabs(a0)), fmax(fabs(b0), fabs(gamma)));
+  lscale = fmax(lscale, tmax);
   double inv_l = 1.0 / lscale;
-  double aa_h = A_(0) * inv_l, bb_h = B_(0) * inv_l, gg = gamma * inv_l;
+  double aa_h = a0 * inv_l, bb_h = b0 * inv_l, gg = gamma * inv_l;
   double den = aa_h + bb_h + 2.0 * gg;
   if (!(isfinite(den) && den > 0.0)) return;
   double geo = sqrt(ss) * sqrt(zs);
   double lam_head = geo * gamma;
   if (!isfinite(lam_head)) return;
-  for (int pass = 0; pass < 2; ++pass) {  // pass 0 checks, pass 1 commits
-    for (int i = 1; i < n; ++i) {
-      double aa = A_(i) * inv_l, bb = B_(i) * inv_l;
-      double scaled = (gg + bb_h) * aa + (gg + aa_h) * bb;
-      double val = geo * (scaled / den) * lscale;
-      if (pass == 0) {
-        if (!isfinite(val)) return;
-      } else {
-        lc[i] = val;
-        wc[i] = (A_(i) - B_(i)) / wscale;
-      }
-    }
+  auto lambda_i = [&](int i) {
+    double aa = A(i) * inv_l, bb = B(i) * inv_l;
+    double scaled = (gg + bb_h) * aa + (gg + aa_h) * bb;
+    return geo * (scaled / den) * lscale;
+  };
+  if (!L.every(n, [&](int i) { return i == 0 || isfinite(lambda_i(i)); })) return;
+  for (int i = L.lane; i < n; i += g) {
+    lc[i] = i ? lambda_i(i) : lam_head;
+    wc[i] = i ? (A(i) - B(i)) / wscale : nhead;
   }
-#undef A_
-#undef B_
-  wc[0] = nhead;
-  lc[0] = lam_head;
-  eta_out[c] = eta;
-  eta2_out[c] = eta2;
-  ok_out[c] = 1;
+  if (L.lane == 0) {
+    eta_out[c] = eta;
+    eta2_out[c] = eta2;
+    ok_out[c] = 1;
+  }
 }
 
 // ------------------------------------------------------------- NT maps ----
-// `_soc_nt_apply_w!` / `_soc_nt_apply_winv!` / `_soc_nt_apply_hs_inverse!`
-// (src/soc_lorentz_kernels.jl:187-255) on the contiguous segment v[0..n)
-// (a cone vector, or a cone's rows of one column of B).  which = 2 may add
-// the result to `base` (out = base + Hs⁻¹v); W and W⁻¹ ignore it.
-__device__ __forceinline__ void nt_map(int which, const double* wc, double eta, double eta2,
+// `_soc_nt_apply_w!` (which = 0) / `_soc_nt_apply_winv!` (1) /
+// `_soc_nt_apply_hs_inverse!` (2) (src/soc_lorentz_kernels.jl:187-255) on a cone
+// vector v[0..n), by the lanes of a group.  which = 2 may add the result to `base`
+// (out = base + Hs⁻¹v); W and W⁻¹ ignore it.
+__device__ __forceinline__ void nt_map(const Lanes& L, int which, const double* wc, double eta, double eta2,
                                        const double* v, double* out, int n, const double* base) {
-  const double head = v[0];
+  const double head = v[0], w0 = wc[0];
   if (which == 2) {
-    double ld = wc[0] * head;
-    for (int i = 1; i < n; ++i) ld -= wc[i] * v[i];
-    double o0 = (2.0 * wc[0] * ld - head) / eta2;
-    out[0] = base ? base[0] + o0 : o0;
-    for (int i = 1; i < n; ++i) {
-      double oi = (-2.0 * wc[i] * ld + v[i]) / eta2;
-      out[i] = base ? base[i] + oi : oi;
+    const double ld = L.sum(w0 * head, n, [&](int i) { return -(wc[i] * v[i]); });
+    for (int i = L.lane; i < n; i += L.g) {
+      double o = i ? (-2.0 * wc[i] * ld + v[i]) / eta2 : (2.0 * w0 * ld - head) / eta2;
+      out[i] = base ? base[i] + o : o;
     }
     return;
   }
+  const double dt = L.sum(0.0, n, [&](int i) { return wc[i] * v[i]; });
+  if (which == 0) {
+    double corr = head + dt / (1.0 + w0);
+    for (int i = L.lane; i < n; i += L.g) out[i] = i ? eta * (v[i] + corr * wc[i]) : eta * (w0 * head + dt);
+  } else {
+    double corr = -head + dt / (1.0 + w0);
+    for (int i = L.lane; i < n; i += L.g) out[i] = i ? (v[i] + corr * wc[i]) / eta : (w0 * head - dt) / eta;
+  }
+}
+
+// The same maps (which = 0, 1) by one thread.
+__device__ __forceinline__ void nt_map(int which, const double* wc, double eta, const double* v, double* out,
+                                       int n) {
+  const double head = v[0];
   double dt = 0.0;
   for (int i = 1; i < n; ++i) dt += wc[i] * v[i];
   if (which == 0) {
@@ -186,13 +232,14 @@ __device__ __forceinline__ void nt_map(int which, const double* wc, double eta, 
   }
 }
 
-__global__ void k_nt_apply(int which, int ncones, const long long* __restrict__ off,
+__global__ void k_nt_apply(int g, int which, int ncones, const long long* __restrict__ off,
                            const int* __restrict__ dim, const double* __restrict__ w,
                            const double* __restrict__ eta, const double* __restrict__ eta2,
                            const double* __restrict__ v, double* __restrict__ out) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const Lanes L(g);
+  int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) / g);
   if (c >= ncones) return;
-  nt_map(which, w + off[c], eta[c], eta2[c], v + off[c], out + off[c], dim[c], nullptr);
+  nt_map(L, which, w + off[c], eta[c], eta2[c], v + off[c], out + off[c], dim[c], nullptr);
 }
 
 // --------------------------------------------------------------- LP pack --
@@ -209,67 +256,160 @@ __global__ void k_lp_pack(int n_lp, const double* __restrict__ weights, const in
   Dis[j] = sqrt(inv);
 }
 
-// B̂[j, e] = D^{-1/2}_j · B[j, e] for the LP rows of every column.
+// B̂[j, e] = D^{-1/2}_j · B[j, e] for the LP rows of every column: a thread keeps its
+// row's factor for eight columns, whose loads are in flight together (one element a
+// thread with a 64-bit division for its place: 230 µs at 20000 × 3000, now 142;
+// the 960 MB take 149 at the copy rate).
+constexpr int kLpCols = 8;
 __global__ void k_scale_lp(int n_lp, long long n, int m, const double* __restrict__ B,
                            const double* __restrict__ Dis, double* __restrict__ Bh) {
-  const long long tot = (long long)n_lp * m;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-       e += (long long)gridDim.x * blockDim.x) {
-    long long col = e / n_lp;
-    int j = (int)(e - col * n_lp);
-    long long idx = col * n + j;
-    Bh[idx] = Dis[j] * B[idx];
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n_lp) return;
+  const double d = Dis[j];
+  for (int c0 = blockIdx.y * kLpCols; c0 < m; c0 += gridDim.y * kLpCols) {
+    const double* src = B + c0 * n + j;
+    double* dst = Bh + c0 * n + j;
+    double v[kLpCols];
+#pragma unroll
+    for (int c = 0; c < kLpCols; ++c) v[c] = c0 + c < m ? src[c * n] : 0.0;
+#pragma unroll
+    for (int c = 0; c < kLpCols; ++c)
+      if (c0 + c < m) dst[c * n] = d * v[c];
   }
 }
 
-// B̂_k[:, e] = W_k⁻¹ B_k[:, e]: one thread per (cone, column), the cone's
-// segment of column e walked sequentially (the W⁻¹ map's order).  Adjacent
-// threads take adjacent columns of the same cone.
-__global__ void k_scale_cones(int ncones, int m, long long n, long long cone_base,
-                              const long long* __restrict__ off, const int* __restrict__ dim,
-                              const double* __restrict__ w, const double* __restrict__ eta,
-                              const double* __restrict__ B, double* __restrict__ Bh) {
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)ncones * m) return;
-  int c = (int)(t / m);
-  long long col = t - (long long)c * m;
-  long long base = col * n + cone_base + off[c];
-  nt_map(1, w + off[c], eta[c], 0.0, B + base, Bh + base, dim[c], nullptr);
+// B̂_k[:, e] = W_k⁻¹ B_k[:, e] for the cones of one tile (whole cones, at most kConeRows
+// rows, or one larger cone) and kConeCols columns.  The rows pass through shared memory,
+// so that global accesses run along the columns; a (cone, column) sum is one thread's,
+// in index order.  A thread per (cone, column) walking its rows in global memory took
+// 400 µs for 100 cones of order 64 and 3000 columns, this takes 98.
+constexpr int kConeRows = 64, kConeCols = 32, kConeLd = kConeRows + 1;
+struct ConeTile {
+  int cone, ncones, row, rows;
+};
+__global__ void __launch_bounds__(256) k_scale_cones(const ConeTile* __restrict__ tiles, int m, long long n,
+                                                     long long cone_base, const long long* __restrict__ off,
+                                                     const int* __restrict__ dim, const double* __restrict__ w,
+                                                     const double* __restrict__ eta,
+                                                     const double* __restrict__ B, double* __restrict__ Bh) {
+  __shared__ double buf[kConeCols * kConeLd], corr[kConeRows * kConeCols], ws[kConeRows], es[kConeRows];
+  __shared__ int head[kConeRows];  // per row: the cone's first row, its place in the tile
+  __shared__ int cone_of[kConeRows];
+  const ConeTile T = tiles[blockIdx.x];
+  const int tid = threadIdx.x, row = tid & (kConeRows - 1), cg = tid / kConeRows;
+  const int c0 = blockIdx.y * kConeCols, cols = min(kConeCols, m - c0);
+  const long long base = (long long)c0 * n + cone_base + T.row;
+  const int nchunk = (T.rows + kConeRows - 1) / kConeRows;
+  auto load = [&](int r0) {  // rows r0 … of the tile into buf, their w into ws
+    const int r = r0 + row;
+    double v[kConeCols / 4];
+#pragma unroll
+    for (int q = 0; q < kConeCols / 4; ++q) {
+      const int c = cg + 4 * q;
+      v[q] = r < T.rows && c < cols ? B[base + c * n + r] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kConeCols / 4; ++q) buf[(cg + 4 * q) * kConeLd + row] = v[q];
+    if (tid < kConeRows) ws[tid] = r < T.rows ? w[T.row + r] : 0.0;
+  };
+  for (int q = tid; q < T.ncones; q += blockDim.x) {
+    const int c = T.cone + q, first = (int)(off[c] - T.row), last = min(kConeRows, first + dim[c]);
+    es[q] = eta[c];
+    for (int r = first; r < last; ++r) head[r] = first, cone_of[r] = q;
+  }
+  load(0);
+  __syncthreads();
+  double hv = 0.0, dt = 0.0;  // of one larger cone: column tid
+  if (nchunk == 1) {
+    for (int p = tid; p < T.ncones * kConeCols; p += blockDim.x) {
+      const int q = p / kConeCols, c = p % kConeCols, first = (int)(off[T.cone + q] - T.row);
+      const int nq = dim[T.cone + q];
+      double* v = buf + c * kConeLd + first;
+      const double *wq = ws + first, h = v[0];
+      double t = 0.0;
+      for (int i = 1; i < nq; ++i) t += wq[i] * v[i];
+      corr[p] = -h + t / (1.0 + wq[0]);
+      v[0] = (wq[0] * h - t) / es[q];
+    }
+  } else {
+    for (int k = 0; k < nchunk; ++k) {
+      if (k) {
+        __syncthreads();
+        load(k * kConeRows);
+        __syncthreads();
+      }
+      if (tid < kConeCols) {
+        const double* v = buf + tid * kConeLd;
+        if (k == 0) hv = v[0];
+        const int e = min(kConeRows, T.rows - k * kConeRows);
+        for (int i = k == 0; i < e; ++i) dt += ws[i] * v[i];
+      }
+    }
+    __syncthreads();
+    load(0);
+    __syncthreads();
+    if (tid < kConeCols) {
+      corr[tid] = -hv + dt / (1.0 + ws[0]);
+      buf[tid * kConeLd] = (ws[0] * hv - dt) / es[0];
+    }
+  }
+  for (int k = 0; k < nchunk; ++k) {
+    if (k) {
+      __syncthreads();
+      load(k * kConeRows);
+    }
+    __syncthreads();
+    const int r = k * kConeRows + row;
+    if (r >= T.rows) continue;
+    const int first = nchunk == 1 ? head[row] : -k * kConeRows, q = nchunk == 1 ? cone_of[row] : 0;
+    const double wr = ws[row], e = es[q];
+#pragma unroll
+    for (int j = 0; j < kConeCols / 4; ++j) {
+      const int c = cg + 4 * j;
+      const double v = buf[c * kConeLd + row];
+      if (c < cols) Bh[base + c * n + r] = row == first ? v : (v + corr[q * kConeCols + c] * wr) / e;
+    }
+  }
 }
 
-// Q_ii += δ (Q holds the lower triangle from the SYRK); F = lower(Q), upper 0.
+// Q_ii += δ (Q holds the lower triangle from the SYRK); F = lower(Q).  The strict upper
+// triangle of F is left to the factorization, which zeroes it.
 __global__ void k_shift_copy_lower(int m, double* Q, double reg, double* F) {
-  const long long tot = (long long)m * m;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-       e += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(e % m), j = (int)(e / m);
-    double v = 0.0;
-    if (i > j) v = Q[e];
-    if (i == j) {
-      v = Q[e] + reg;
-      Q[e] = v;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  for (int j0 = blockIdx.y * kLpCols; j0 <= i; j0 += gridDim.y * kLpCols) {
+    double v[kLpCols];
+#pragma unroll
+    for (int c = 0; c < kLpCols; ++c) v[c] = j0 + c <= i ? Q[(size_t)(j0 + c) * m + i] : 0.0;
+#pragma unroll
+    for (int c = 0; c < kLpCols; ++c) {
+      if (j0 + c > i) continue;
+      const size_t e = (size_t)(j0 + c) * m + i;
+      if (j0 + c == i) Q[e] = v[c] = v[c] + reg;
+      F[e] = v[c];
     }
-    F[e] = v;
   }
 }
 
 // out = base + D⁻¹ v over all variables: LP entries by D⁻¹_j, cone k by Hs_k⁻¹
-// (thread per LP entry, then one thread per cone).
-__global__ void k_apply_dinv(int n_lp, const double* __restrict__ Dinv, int ncones,
+// (a thread per LP entry in the first lp_blocks blocks, then g lanes per cone).
+__global__ void k_apply_dinv(int g, int lp_blocks, int n_lp, const double* __restrict__ Dinv, int ncones,
                              long long cone_base, const long long* __restrict__ off,
                              const int* __restrict__ dim, const double* __restrict__ w,
                              const double* __restrict__ eta2, const double* __restrict__ v,
                              const double* __restrict__ base, double* __restrict__ out) {
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t < n_lp) {
+  if ((int)blockIdx.x < lp_blocks) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n_lp) return;
     double o = Dinv[t] * v[t];
     out[t] = base ? base[t] + o : o;
     return;
   }
-  long long c = t - n_lp;
+  const Lanes L(g);
+  const int c = (int)(((blockIdx.x - lp_blocks) * blockDim.x + threadIdx.x) / g);
   if (c >= ncones) return;
   long long o = cone_base + off[c];
-  nt_map(2, w + off[c], 0.0, eta2[c], v + o, out + o, dim[c], base ? base + o : nullptr);
+  nt_map(L, 2, w + off[c], 0.0, eta2[c], v + o, out + o, dim[c], base ? base + o : nullptr);
 }
 
 }  // namespace
@@ -281,11 +421,14 @@ struct NormalHandle {
   int sms = 148;
   std::string err;
   int n_lp = 0, ncones = 0, m = 0, n_weights = 0;
+  int lanes = 4, cone_tiles = 0;  // lanes per cone, tiles of k_scale_cones
   long long n = 0, nq = 0;  // variables, cone variables
   std::vector<long long> cone_off;
   std::vector<int> cone_dim;
   DBuf<long long> d_off;
-  DBuf<int> d_dim, d_row, d_ok, d_info;
+  DBuf<int> d_dim, d_row, d_ok;
+  DBuf<int> d_info;  // of the factor; [1]: a wait of the triangular solve gave up
+  DBuf<ConeTile> d_tiles;
   DBuf<unsigned> flow_flags;  // tile flags of the Cholesky launch
   DBuf<double> B, Bh, coef, weights, D, Dinv, Dis, w, lam, eta, eta2, s, z, v, out;
   DBuf<double> Q, F, Finv_diag, partial, rhs, t, red, work, u, gemv_part;
@@ -368,6 +511,18 @@ struct NormalHandle {
     if (ncones) {
       h2d(d_off.p, cone_off.data(), sizeof(long long) * ncones);
       h2d(d_dim.p, cone_dim.data(), sizeof(int) * ncones);
+      while (lanes < 32 && (long long)lanes * ncones < nq) lanes *= 2;  // about the mean order
+      std::vector<ConeTile> tiles;
+      for (int c = 0; c < ncones; ++c) {
+        const int q = cone_dim[c];
+        if (tiles.empty() || tiles.back().rows + q > kConeRows)
+          tiles.push_back({c, 1, (int)cone_off[c], q});
+        else
+          tiles.back().ncones++, tiles.back().rows += q;
+      }
+      cone_tiles = (int)tiles.size();
+      d_tiles.alloc(cone_tiles);
+      h2d(d_tiles.p, tiles.data(), sizeof(ConeTile) * cone_tiles);
     }
     d_row.alloc(n_lp);
     coef.alloc(n_lp);
@@ -387,12 +542,13 @@ struct NormalHandle {
     t.alloc(n);
     u.alloc(n);
     red.alloc(m);
-    work.alloc(m);
+    work.alloc(cholesky_solve_work(m));
     gemv_chunks = std::max(1, std::min(16, m / 64));
     gemv_part.alloc((size_t)gemv_chunks * std::max<long long>(n, m));
     plan = plan_syrk_f64(std::max(m, 1), std::max<long long>(n, 1), sms);
     partial.alloc(plan.partial_doubles);
-    d_info.alloc(1);
+    d_info.alloc(2);
+    SDPX_CUDA(cudaMemsetAsync(d_info.p, 0, 2 * sizeof(int), st));
     dmin.alloc(1);
     dmax.alloc(1);
     descs.alloc(1);
@@ -416,6 +572,21 @@ struct NormalHandle {
   }
   void sync() { SDPX_CUDA(cudaStreamSynchronize(st)); }
 
+  void launch_nt_scaling(const double* ds, const double* dz) {
+    k_nt_scaling<<<ceil_div((long long)ncones * lanes, 128), 128, 0, st>>>(
+        lanes, ncones, d_off.p, d_dim.p, ds, dz, w.p, lam.p, eta.p, eta2.p, d_ok.p);
+    SDPX_LAUNCH_CHECK();
+  }
+  // out = base + D⁻¹v (LP diag(D⁻¹), cones Hs⁻¹) on the held scaling.
+  void apply_dinv(const double* dv, const double* base, double* dout) {
+    const int lp_blocks = ceil_div(n_lp, 128);
+    const int grid = lp_blocks + ceil_div((long long)ncones * lanes, 128);
+    if (grid == 0) return;
+    k_apply_dinv<<<grid, 128, 0, st>>>(lanes, lp_blocks, n_lp, Dinv.p, ncones, n_lp, d_off.p, d_dim.p, w.p,
+                                       eta2.p, dv, base, dout);
+    SDPX_LAUNCH_CHECK();
+  }
+
   int nt_scaling(const double* hs, const double* hz, int* ok, double* hw, double* hlam,
                  double* heta, double* heta2) {
     have_scaling = false;
@@ -423,9 +594,7 @@ struct NormalHandle {
     if (!hs || !hz) throw std::invalid_argument("s and z are required");
     h2d(s.p, hs, sizeof(double) * nq);
     h2d(z.p, hz, sizeof(double) * nq);
-    k_nt_scaling<<<ceil_div(ncones, 128), 128, 0, st>>>(ncones, d_off.p, d_dim.p, s.p, z.p, w.p,
-                                                         lam.p, eta.p, eta2.p, d_ok.p);
-    SDPX_LAUNCH_CHECK();
+    launch_nt_scaling(s.p, z.p);
     std::vector<int> okv(ncones);
     d2h(okv.data(), d_ok.p, sizeof(int) * ncones);
     if (hw) d2h(hw, w.p, sizeof(double) * nq);
@@ -453,8 +622,8 @@ struct NormalHandle {
     require_scaling();
     if (ncones == 0) return;
     h2d(v.p, hv, sizeof(double) * nq);
-    k_nt_apply<<<ceil_div(ncones, 128), 128, 0, st>>>(which, ncones, d_off.p, d_dim.p, w.p, eta.p,
-                                                       eta2.p, v.p, out.p);
+    k_nt_apply<<<ceil_div((long long)ncones * lanes, 128), 128, 0, st>>>(
+        lanes, which, ncones, d_off.p, d_dim.p, w.p, eta.p, eta2.p, v.p, out.p);
     SDPX_LAUNCH_CHECK();
     d2h(hout, out.p, sizeof(double) * nq);
     sync();
@@ -472,10 +641,13 @@ struct NormalHandle {
   // B̂ rows of the cones (independent of δ) — once per scaling.
   void scale_cones() {
     if (ncones == 0 || m == 0) return;
-    long long threads = (long long)ncones * m;
-    k_scale_cones<<<ceil_div(threads, 128), 128, 0, st>>>(ncones, m, n, n_lp, d_off.p, d_dim.p,
-                                                          w.p, eta.p, B.p, Bh.p);
-    SDPX_LAUNCH_CHECK();
+    // Column tiles in slices, for the grid's y extent.
+    for (int c0 = 0; c0 < m; c0 += 65535 * kConeCols) {
+      const int cols = std::min(m - c0, 65535 * kConeCols);
+      k_scale_cones<<<dim3(cone_tiles, ceil_div(cols, kConeCols)), 256, 0, st>>>(
+          d_tiles.p, cols, n, n_lp, d_off.p, d_dim.p, w.p, eta.p, B.p + (size_t)c0 * n, Bh.p + (size_t)c0 * n);
+      SDPX_LAUNCH_CHECK();
+    }
   }
 
   // Q = B̂ᵀB̂ from three BF16 planes of B̂ on the tcgen05 split SYRK (FP32
@@ -500,9 +672,13 @@ struct NormalHandle {
     d2h(&e, serr.p, sizeof(int));
     sync();
     if (e) throw CudaError("split normal-matrix SYRK: a bounded wait gave up");
-    long long tot = (long long)m * m;
-    k_shift_copy_lower<<<(int)std::min<long long>(ceil_div(tot, 256), (long long)sms * 16), 256, 0,
-                         st>>>(m, Q.p, reg, F.p);
+    shift_copy(reg);
+  }
+
+  // +δ on the diagonal of Q, copy of lower(Q) into F.
+  void shift_copy(double reg) {
+    const dim3 grid(ceil_div(m, 256), std::min(65535, ceil_div(m, kLpCols)));
+    k_shift_copy_lower<<<grid, 256, 0, st>>>(m, Q.p, reg, F.p);
     SDPX_LAUNCH_CHECK();
     have_assembled = true;
   }
@@ -510,8 +686,7 @@ struct NormalHandle {
   // B̂ = D^{-1/2}B on the LP rows (the cone rows come from scale_cones).
   void scale_lp_rows() {
     if (n_lp > 0 && m > 0) {
-      long long tot = (long long)n_lp * m;
-      int grid = (int)std::min<long long>(ceil_div(tot, 256), (long long)sms * 16);
+      const dim3 grid(ceil_div(n_lp, 256), std::min(65535, ceil_div(m, kLpCols)));
       k_scale_lp<<<grid, 256, 0, st>>>(n_lp, n, m, B.p, Dis.p, Bh.p);
       SDPX_LAUNCH_CHECK();
     }
@@ -534,11 +709,7 @@ struct NormalHandle {
     } else {
       SDPX_CUDA(cudaMemsetAsync(Q.p, 0, sizeof(double) * (size_t)m * m, st));
     }
-    long long tot = (long long)m * m;
-    k_shift_copy_lower<<<(int)std::min<long long>(ceil_div(tot, 256), (long long)sms * 16), 256, 0,
-                         st>>>(m, Q.p, reg, F.p);
-    SDPX_LAUNCH_CHECK();
-    have_assembled = true;
+    shift_copy(reg);
   }
 
   void assemble(const double* hweights, double reg) {
@@ -577,9 +748,7 @@ struct NormalHandle {
       }
       factor_F();
       SDPX_CUDA(cudaEventRecord(ev[2], st));
-      d2h(&info, d_info.p, sizeof(int));
-      sync();
-      if (info < 0) throw CudaError("normal-matrix Cholesky: a wait for a tile gave up");
+      info = read_info();
       float a = 0.f, f = 0.f;
       SDPX_CUDA(cudaEventElapsedTime(&a, ev[0], ev[1]));
       SDPX_CUDA(cudaEventElapsedTime(&f, ev[1], ev[2]));
@@ -627,11 +796,7 @@ struct NormalHandle {
       return 0;
     }
     factor_F();
-    int info = 1;
-    d2h(&info, d_info.p, sizeof(int));
-    sync();
-    if (info < 0) throw CudaError("normal-matrix Cholesky: a wait for a tile gave up");
-    if (info != 0) return 1;
+    if (read_info() != 0) return 1;
     factor_diag_inverses(F.p, m, m, Finv_diag.p, st);
     if (split) make_inverse();
     have_factor = true;
@@ -652,14 +817,7 @@ struct NormalHandle {
 
   // Device-resident solve on rhs (n + m) already in `rhs`.
   void solve_device() {
-    const long long nthreads = n_lp + ncones;
-    const int grid = std::max(1, ceil_div(nthreads, 128));
-    // t = D⁻¹ rx
-    if (n > 0) {
-      k_apply_dinv<<<grid, 128, 0, st>>>(n_lp, Dinv.p, ncones, n_lp, d_off.p, d_dim.p, w.p, eta2.p,
-                                         rhs.p, nullptr, t.p);
-      SDPX_LAUNCH_CHECK();
-    }
+    apply_dinv(rhs.p, nullptr, t.p);  // t = D⁻¹ rx
     if (m == 0) {
       if (n > 0) SDPX_CUDA(cudaMemcpyAsync(rhs.p, t.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
       return;
@@ -667,21 +825,37 @@ struct NormalHandle {
     double* dy = rhs.p + n;
     // dy ← ry − Bᵀt, then Q⁻¹
     if (n > 0) gemv_t(B.p, n, m, t.p, -1.0, dy, 1.0, dy, st);
-    cholesky_solve<double, 64>(F.p, m, m, Finv_diag.p, dy, work.p, st);
+    cholesky_solve(F.p, m, m, Finv_diag.p, dy, work.p, d_info.p + 1, sms, st);
     if (n == 0) return;
     // dx = t + D⁻¹(B dy)
     gemv_n(B.p, n, m, dy, u.p, gemv_part.p, gemv_chunks, st);
-    k_apply_dinv<<<grid, 128, 0, st>>>(n_lp, Dinv.p, ncones, n_lp, d_off.p, d_dim.p, w.p, eta2.p,
-                                       u.p, t.p, rhs.p);
-    SDPX_LAUNCH_CHECK();
+    apply_dinv(u.p, t.p, rhs.p);
+  }
+
+  // Status of the factor and of the solves before it, read in one copy.
+  int read_info() {
+    int info[2] = {1, 0};
+    d2h(info, d_info.p, sizeof(info));
+    sync();
+    check_solve(info[1]);
+    if (info[0] < 0) throw CudaError("normal-matrix Cholesky: a wait for a tile gave up");
+    return info[0];
+  }
+  void check_solve(int err) {
+    if (!err) return;
+    SDPX_CUDA(cudaMemsetAsync(d_info.p + 1, 0, sizeof(int), st));
+    throw CudaError("normal-matrix triangular solve: a wait for a block gave up");
   }
 
   int solve(double* hrhs) {
     if (!have_factor) return 1;
     h2d(rhs.p, hrhs, sizeof(double) * (n + m));
     solve_device();
+    int err = 0;
+    d2h(&err, d_info.p + 1, sizeof(int));
     d2h(hrhs, rhs.p, sizeof(double) * (n + m));
     sync();
+    check_solve(err);
     return 0;
   }
 };
