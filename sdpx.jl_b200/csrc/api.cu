@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <initializer_list>
 #include <mutex>
 #include <map>
 #include <set>
@@ -211,9 +212,17 @@ struct Handle {
   DBuf<double> partial;
   SyrkPlan syrk;
   DBuf<double> red;                // small reduction scratch
-  double* h_red = nullptr;         // pinned mirror
+  double* h_red = nullptr;         // pinned mirror; kernels write their results here
+  struct FactorStats {             // at h_red + kFactorSlot
+    double dmin, dmax;
+    int info, err, diag_fail;
+  };
+  static constexpr int kFactorSlot = 48;
+  FactorStats* h_factor() { return reinterpret_cast<FactorStats*>(h_red + kFactorSlot); }
+  DBuf<NormWork> norm_work;
   DBuf<double> mu_user, target_user, work_L;
   DBuf<double> seg_part;           // seg_dot partials
+  DBuf<unsigned> seg_done;         // its count of finished CTAs
   int seg_parts = 8;
   double last_bpr = 0.0;
   int mixed_predicted_steps = 32;  // from the last mixed factor's condition estimate
@@ -228,9 +237,7 @@ struct Handle {
 
   // batched Cholesky workspace (dense blocks X, Y and line-search trials)
   DBuf<MatDesc<double>> d_descs;
-  DBuf<int> d_info;
-  DBuf<unsigned> flow_flags;  // tile flags of the Cholesky launches
-  DBuf<double> d_dmin, d_dmax;
+  FlowFlags flow_flags;  // tile flags of the Cholesky launches
   size_t desc_cap = 0;
   DBuf<double> trials;
   DBuf<long long> d_trial_off;
@@ -375,6 +382,28 @@ struct Handle {
     sync();
     return h_red[slot];
   }
+  // h_red[slot] = max|x| of every entry (n, x, slot) after the next sync.
+  struct Norm {
+    long long n;
+    const double* x;
+    int slot;
+  };
+  void norms(std::initializer_list<Norm> list) {
+    NormList q;
+    for (const Norm& e : list) q.add(e.n, e.x, h_red + e.slot);
+    absmax_list(q, norm_work.p, st);
+  }
+  double norm(long long n, const double* x) {
+    norms({{n, x, 0}});
+    sync();
+    return h_red[0];
+  }
+  // Σ of the user blocks' entries of (X + tx·dX)∘(Y + ty·dY) into `out`.
+  void dots(const double* Xa, const double* dXa, double tx, const double* Ya, const double* dYa, double ty,
+            double* out) {
+    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, Xa, dXa, tx, Ya, dYa, ty, seg_part.p, seg_done.p, out, st);
+  }
+  double* pinned_doubles(size_t n) { return reinterpret_cast<double*>(pinned(n * sizeof(double))); }
   void clear_red(int slot, int count = 1) {
     SDPX_CUDA(cudaMemsetAsync(red.p + slot, 0, sizeof(double) * count, st));
   }
@@ -418,12 +447,12 @@ struct Handle {
   }
 
   // The same product on every dense block, C_b = alpha·op(A_b)·op(B_b) +
-  // beta·C_b (operands from opA(b), opB(b)), as one grouped launch per eight
-  // blocks: the blocks' products are independent and each tile is computed
+  // beta·C_b (operands from opA(b), opB(b)), or + beta·Cin_b, as one grouped launch per
+  // eight blocks: the blocks' products are independent and each tile is computed
   // as gemm_f64 computes it for one block.
   template <class FA, class FB>
   void blk_gemm_all(FA opA, bool akc, FB opB, bool bkc, double* out, double alpha, double beta,
-                    int mode) {
+                    int mode, const double* cin = nullptr) {
     GemmGroups g;
     for (auto& b : dense) {
       if (g.n == kGemmGroups) {
@@ -433,6 +462,7 @@ struct Handle {
       g.A[g.n] = opA(b);
       g.B[g.n] = opB(b);
       g.C[g.n] = blk_out(out, b.off, b.k);
+      g.Cin[g.n] = cin ? cin + b.off : nullptr;
       g.alpha[g.n] = alpha;
       g.beta[g.n] = beta;
       g.mode[g.n] = mode;
@@ -456,15 +486,9 @@ struct Handle {
     if (n <= desc_cap) return;
     desc_cap = std::max<size_t>(n, 2 * desc_cap);
     d_descs.alloc(desc_cap);
-    d_info.alloc(desc_cap);
-    d_dmin.alloc(desc_cap);
-    d_dmax.alloc(desc_cap);
-    d_stats.alloc(3 * desc_cap);
   }
-  // Pinned staging for the per-round uploads (descriptor lists) and the
-  // packed read-back of the batched Cholesky results: asynchronous copies
-  // instead of staged pageable ones.  Only grown right after a sync.
-  DBuf<double> d_stats;  // one round's dmin | dmax | info, contiguous
+  // Pinned staging: descriptor lists to upload, and results that kernels write
+  // directly (no copy back).  Only grown right after a sync.
   unsigned char* h_pin = nullptr;
   size_t pin_cap = 0;
   unsigned char* pinned(size_t bytes) {
@@ -493,30 +517,28 @@ struct Handle {
     int nmax = 0;
     for (auto& q : mats) nmax = std::max(nmax, q.n);
     // Pinned layout: [descriptors | dmin (n) | dmax (n) | info (n)], the last
-    // three read back in one copy from d_stats.
+    // three written by the kernel.
     const size_t dbytes = (n * sizeof(MatDesc<double>) + 15) / 16 * 16;
-    const size_t sbytes = 2 * n * sizeof(double) + n * sizeof(int);
-    unsigned char* hp = pinned(dbytes + sbytes);
-    std::memcpy(hp, mats.data(), n * sizeof(MatDesc<double>));
-    h2d(d_descs.p, hp, n * sizeof(MatDesc<double>));
-    double* sdmin = d_stats.p;
-    double* sdmax = d_stats.p + n;
-    int* sinfo = reinterpret_cast<int*>(d_stats.p + 2 * n);
-    potrf_flow(d_descs.p, (int)n, nmax, sinfo, sdmin, sdmax, flow_flags_for((int)n, nmax), sms, st,
-               zero_upper);
-    d2h(hp + dbytes, d_stats.p, sbytes);
+    unsigned char* hp = pinned(dbytes + 2 * n * sizeof(double) + n * sizeof(int));
+    MatDesc<double>* hm = reinterpret_cast<MatDesc<double>*>(hp);
+    std::copy(mats.begin(), mats.end(), hm);
+    double* hs = reinterpret_cast<double*>(hp + dbytes);
+    int* hi = reinterpret_cast<int*>(hs + 2 * n);
+    potrf_flow(hm, d_descs.p, (int)n, nmax, hi, hs, hs + n, flow_flags, sms, st, zero_upper);
     sync();
-    const double* hs = reinterpret_cast<const double*>(hp + dbytes);
-    std::memcpy(dmin.data(), hs, n * sizeof(double));
-    std::memcpy(dmax.data(), hs + n, n * sizeof(double));
-    std::memcpy(info.data(), hs + 2 * n, n * sizeof(int));
+    std::copy(hs, hs + n, dmin.begin());
+    std::copy(hs + n, hs + 2 * n, dmax.begin());
+    std::copy(hi, hi + n, info.begin());
     for (int v : info)
       if (v < 0) throw CudaError("Cholesky: a wait for a tile gave up");
   }
-  unsigned* flow_flags_for(int nmat, int nmax) {  // potrf_flow's flag words
-    const size_t need = potrf_flow_flag_words(nmat, nmax);
-    if (flow_flags.n < need) flow_flags.alloc(2 * need);
-    return flow_flags.p;
+  // Cholesky of one matrix in place; its results are in h_factor().
+  void potrf_one(double* a, int n, const char* what) {
+    const MatDesc<double> md{a, n, n};
+    FactorStats* f = h_factor();
+    potrf_flow(&md, nullptr, 1, n, &f->info, &f->dmin, &f->dmax, flow_flags, sms, st);
+    sync();
+    if (f->info < 0) throw CudaError(std::string(what) + " Cholesky: a wait for a tile gave up");
   }
 
   // ------------------------------------------------------------ create ----
@@ -672,6 +694,10 @@ struct Handle {
     work_L.alloc(2 * std::max<size_t>((size_t)L, dense.size()) + 2);
     seg_parts = 8;
     seg_part.alloc((size_t)seg_parts * L);
+    seg_done.alloc(1);
+    seg_done.zero(st);
+    norm_work.alloc(1);
+    norm_work.zero(st);
     ensure_descs(std::max<size_t>(16, 2 * dense.size()));
     d_fail.alloc(64);
     d_tcand.alloc(64);
@@ -864,10 +890,7 @@ struct Handle {
   }
 
   void data_norms(double* maxC, double* cnorm) {
-    clear_red(0, 2);
-    absmax(K, Cst.p, red.p + 0, st);
-    absmax(m, c.p, red.p + 1, st);
-    d2h(h_red, red.p, 2 * sizeof(double));
+    norms({{K, Cst.p, 0}, {m, c.p, 1}});
     sync();
     *maxC = h_red[0];
     *cnorm = h_red[1];
@@ -887,11 +910,53 @@ struct Handle {
     }
     sync();
   }
-  void get_stacked(const double* dev_src, double* host_dst) {
-    scatter(K, d_map.p, dev_src, tmpK.p, st);
-    d2h(host_dst, tmpK.p, Ku * sizeof(double));
+  // Results of at most kStageBytes are written by the kernels into pinned memory and
+  // copied out by the host: a copy to the caller's (pageable) memory of 320 KB, the size
+  // of one k = 200 matrix, took 150 µs of driver staging, this STAGEUS.  Larger ones
+  // would spend on pinning the buffer what they save.
+  static constexpr size_t kStageBytes = 4 << 20;
+  struct VectorOut {  // n doubles as they are
+    const double* src;
+    double* dst;
+    long long n;
+  };
+  struct StackedOut {  // a stacked matrix, in the caller's block order
+    const double* src;
+    double* dst;
+  };
+  // Entries with a null destination are skipped.
+  void get_vectors(std::initializer_list<VectorOut> vecs, std::initializer_list<StackedOut> mats) {
+    size_t need = 0;
+    for (const auto& q : vecs) need += q.dst ? q.n : 0;
+    for (const auto& q : mats) need += q.dst ? Ku : 0;
+    const bool staged = need * sizeof(double) <= kStageBytes;
+    double *h = staged ? pinned_doubles(need) : nullptr, *at = h;
+    for (const auto& q : vecs)
+      if (q.dst && q.n) {
+        d2h(staged ? at : q.dst, q.src, q.n * sizeof(double));
+        at += staged ? q.n : 0;
+      }
+    for (const auto& q : mats)
+      if (q.dst) {
+        scatter(K, d_map.p, q.src, staged ? at : tmpK.p, st);
+        if (!staged) d2h(q.dst, tmpK.p, Ku * sizeof(double));
+        at += staged ? Ku : 0;
+      }
     sync();
+    if (!staged) return;
+    at = h;
+    for (const auto& q : vecs)
+      if (q.dst && q.n) {
+        std::memcpy(q.dst, at, q.n * sizeof(double));
+        at += q.n;
+      }
+    for (const auto& q : mats)
+      if (q.dst) {
+        std::memcpy(q.dst, at, Ku * sizeof(double));
+        at += Ku;
+      }
   }
+  void get_stacked(const double* dev_src, double* host_dst) { get_vectors({}, {{dev_src, host_dst}}); }
   void fixed_start(double wp, double wd) {
     iterate_changed();
     x.zero(st);
@@ -918,24 +983,17 @@ struct Handle {
     block_factors_current = false;
     // LX = chol(X), MY = chol(Y) for every dense block (batched), 1×1 by sqrt.
     std::vector<MatDesc<double>> mats;
-    if (od) {  // the dense blocks come first in the stacked layout
-      d2d(LX.p, X.p, sizeof(double) * od);
-      d2d(MY.p, Y.p, sizeof(double) * od);
-    }
+    copy_pair(od, X.p, LX.p, Y.p, MY.p, st);  // the dense blocks come first in the stacked layout
     for (auto& b : dense) mats.push_back({LX.p + b.off, b.k, b.k});
     for (auto& b : dense) mats.push_back({MY.p + b.off, b.k, b.k});
     std::vector<int> info;
     std::vector<double> dmn, dmx;
-    int fail_h = 0;
-    if (nd) {
-      SDPX_CUDA(cudaMemsetAsync(d_fail.p, 0, sizeof(int), st));
-      diag_factor(nd, od, X.p, Y.p, LX.p, MY.p, d_fail.p, st);
-    }
+    int* fail = &h_factor()->diag_fail;  // the kernel sets it; idle since the last sync
+    *fail = 0;
+    if (nd) diag_factor(nd, od, X.p, Y.p, LX.p, MY.p, fail, st);
     potrf_host_list(mats, info, dmn, dmx);
-    if (nd) {
-      d2h(&fail_h, d_fail.p, sizeof(int));
-      sync();
-    }
+    if (mats.empty()) sync();
+    const int fail_h = *fail;
     bool ok = fail_h == 0;
     size_t nb = dense.size();
     for (size_t b = 0; b < nb; ++b) {
@@ -988,35 +1046,30 @@ struct Handle {
     PhaseScope ps(this, 0);
     primal_residual(x.p, P.p);  // P = 𝒜x − X − C
     dual_residual(Y.p, d.p);    // d = c − 𝒜ᵀ vec(Y)
-    clear_red(0, 3);
     if (n_eq) {
       // d −= B·y, p = b − Bᵀx (src/step.jl:41-51)
       gemv_n(Beq.p, m, n_eq, yv.p, eq_tm.p, gemv_part.p, gemv_chunks, st);
       axpbypcz(m, 1.0, d.p, -1.0, eq_tm.p, 0.0, nullptr, d.p, st);
       gemv_t(Beq.p, m, n_eq, x.p, -1.0, beq.p, 1.0, pv.p, st);
-      absmax(n_eq, pv.p, red.p + 2, st);
     }
-    absmax(K, P.p, red.p + 0, st);
-    absmax(m, d.p, red.p + 1, st);
+    norms({{K, P.p, 0}, {m, d.p, 1}, {n_eq, pv.p, 2}});
     // R = −XY (+ μ I)
-    h2d(mu_user.p, mu, L * sizeof(double));
+    if (nd) h2d(mu_user.p, mu, L * sizeof(double));
     blk_gemm_all([&](const DenseBlk& b) { return blk_as_A(X.p, b.off, b.k); }, false,
                  [&](const DenseBlk& b) { return blk_as_B(Y.p, b.off, b.k); }, true, R.p, -1.0, 0.0,
                  KR_FULL);
     if (!use_affine && !dense.empty()) {
       std::vector<double> shifts(dense.size());
       for (size_t b = 0; b < dense.size(); ++b) shifts[b] = mu[dense[b].user];
-      h2d(work_L.p, shifts.data(), shifts.size() * sizeof(double));
-      add_diag(d_doff.p, d_dk.p, (int)dense.size(), kmax, R.p, work_L.p, 0.0, st);
+      add_diag_host(d_doff.p, d_dk.p, (int)dense.size(), kmax, R.p, shifts.data(), work_L.p, st);
     }
     diag_residual_R(nd, od, X.p, Y.p, mu_user.p, d_diag_user.p, use_affine, R.p, st);
-    d2h(h_red, red.p, 3 * sizeof(double));
-    sync();
+    *ok = 1;
+    if (factor) *ok = factor_blocks() ? 1 : 0;  // (synchronises)
+    else sync();
     *p_res = std::max(h_red[0], h_red[2]);
     *d_res = h_red[1];
     last_bpr = h_red[0];
-    *ok = 1;
-    if (factor) *ok = factor_blocks() ? 1 : 0;
   }
 
   // ------------------------------------------------------------- Schur ----
@@ -1307,10 +1360,6 @@ struct Handle {
       ozaki_syrk(panel, oz_plan, oz_digits.p, oz_exps.p, oz_partial.p, S.p, oz_err.p, st, nullptr,
                  nullptr, known ? oz_colmax.p : nullptr, od);
       kt_end(2);
-      int e = 0;
-      d2h(&e, oz_err.p, sizeof(int));
-      sync();
-      if (e) throw CudaError("int8 Gram kernel: a bounded wait gave up");
     } else {
       syrk_lower_f64(Pd, syrk, partial.p, S.p, m, m, 0.0, st);
       kt_end(2);
@@ -1319,21 +1368,21 @@ struct Handle {
   }
 
   // ------------------------------------------------------- factorisation --
+  static void throw_oz_err(int e) {
+    if (e) throw CudaError("int8 Gram kernel: a bounded wait gave up");
+  }
   // Sf ← Cholesky of S, with ≤ 6 regularised retries; returns the retries.
   int factor_S(int* ok, double* lo, double* hi) {
-    MatDesc<double> md{Sf.p, m, m};
     double reg = 0.0;
     int att = 0, info = 0;
-    ensure_descs(1);
     while (true) {
-      copy_reg(m, S.p, Sf.p, att == 0 ? 0.0 : reg, st);
-      h2d(d_descs.p, &md, sizeof(md));
-      potrf_flow(d_descs.p, 1, m, d_info.p, d_dmin.p, d_dmax.p, flow_flags_for(1, m), sms, st);
-      d2h(&info, d_info.p, sizeof(int));
-      d2h(lo, d_dmin.p, sizeof(double));
-      d2h(hi, d_dmax.p, sizeof(double));
-      sync();
-      if (info < 0) throw CudaError("Schur Cholesky: a wait for a tile gave up");
+      // The error word of the int8 products that built S comes along.
+      copy_reg(m, S.p, Sf.p, att == 0 ? 0.0 : reg, st, oz_err.p, &h_factor()->err);
+      potrf_one(Sf.p, m, "Schur");
+      throw_oz_err(h_factor()->err);
+      info = h_factor()->info;
+      *lo = h_factor()->dmin;
+      *hi = h_factor()->dmax;
       if (info == 0 || att >= 6) break;
       ++att;
       reg = (att == 1) ? kSqrtEps : reg * 10.0;
@@ -1487,14 +1536,8 @@ struct Handle {
     double cached = 0.0;
     const bool hit = allow_cache && take_rho_cache(&cached);
     if (!hit) apply_residual();
-    clear_red(0, 4);
-    if (!hit) absmax(m, rho.p, red.p + 0, st);
-    absmax(m, r.p, red.p + 1, st);
-    if (n_eq) {  // ρ_p and p enter the residual and the gate scale (src/kkt.jl:3670-3708)
-      if (!hit) absmax(n_eq, rho_p.p, red.p + 2, st);
-      absmax(n_eq, pv.p, red.p + 3, st);
-    }
-    d2h(h_red, red.p, 4 * sizeof(double));
+    // ρ_p and p enter the residual and the gate scale (src/kkt.jl:3670-3708)
+    norms({{hit ? 0 : m, rho.p, 0}, {m, r.p, 1}, {hit ? 0 : n_eq, rho_p.p, 2}, {n_eq, pv.p, 3}});
     sync();
     *res = hit ? cached : std::max(h_red[0], h_red[2]);
     *rnorm = std::max(h_red[1], h_red[3]);
@@ -1504,11 +1547,7 @@ struct Handle {
     double cached = 0.0;
     if (allow_cache && take_rho_cache(&cached)) return cached;
     apply_residual();
-    clear_red(0, 2);
-    absmax(m, rho.p, red.p, st);
-    if (!n_eq) return read_red(0);
-    absmax(n_eq, rho_p.p, red.p + 1, st);
-    d2h(h_red, red.p, 2 * sizeof(double));
+    norms({{m, rho.p, 0}, {n_eq, rho_p.p, 1}});
     sync();
     return std::max(h_red[0], h_red[1]);
   }
@@ -1528,9 +1567,7 @@ struct Handle {
     if (precision == SDPX_B200_MIXED && mixed) {
       // `_refine_mixed_direction!` (src/kernels/mixed_precision_kkt.jl:1634-1680)
       double rel = tol > 0 ? tol : 64.0 * kEps;
-      clear_red(1, 1);
-      absmax(m, r.p, red.p + 1, st);
-      double abstol = rel * std::max(read_red(1), 1.0);
+      double abstol = rel * std::max(norm(m, r.p), 1.0);
       residual = residual_norm_only(true);
       bool consistent = true;
       for (int s = 0; s < 32; ++s) {
@@ -1571,9 +1608,7 @@ struct Handle {
         return;
       }
       double rel = tol > 0 ? tol : 64.0 * kEps;
-      clear_red(1, 1);
-      absmax(m, r.p, red.p + 1, st);
-      double rn = read_red(1);
+      double rn = norm(m, r.p);
       double abstol = rel * std::max(rn, 1.0);
       residual = residual_norm_only(true);
       for (int s = 0; s < cap; ++s) {
@@ -1599,10 +1634,9 @@ struct Handle {
   // -------------------------------------------------------- right sides ---
   void rhs_from_R() {
     // Z = X⁻¹(P·Y − R); v = 𝒜ᵀ vec(Z); r = −(d + v)
-    for (auto& b : dense) d2d(T1.p + b.off, R.p + b.off, sizeof(double) * b.k * b.k);
     blk_gemm_all([&](const DenseBlk& b) { return blk_as_A(P.p, b.off, b.k); }, false,
                  [&](const DenseBlk& b) { return blk_as_B(Y.p, b.off, b.k); }, true, T1.p, 1.0,
-                 -1.0, KR_FULL);  // T1 = P·Y − R
+                 -1.0, KR_FULL, R.p);  // T1 = P·Y − R
     dense_cholsolve(T1.p, Z.p);
     diag_rhs_Z(nd, od, P.p, Y.p, R.p, LX.p, Z.p, st);
     atmul(Z.p, -1.0, d.p, -1.0, r.p);  // r = −v − d
@@ -1615,22 +1649,19 @@ struct Handle {
     PhaseScope ps(this, 4);
     std::vector<double> target(L, sigma * mu);
     if (block_local) {
-      std::vector<double> dots(L);
-      seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, nullptr, 0.0, Y.p, nullptr, 0.0, seg_part.p,
-              work_L.p, st);
-      d2h(dots.data(), work_L.p, L * sizeof(double));
+      double* xy = pinned_doubles(L);
+      dots(X.p, nullptr, 0.0, Y.p, nullptr, 0.0, xy);
       sync();
-      for (int l = 0; l < L; ++l) target[l] = sigma * dots[l] / k[l];
+      for (int l = 0; l < L; ++l) target[l] = sigma * xy[l] / k[l];
     }
     build_corrector_R(target);
     rhs_from_R();
   }
   void rhs_corrector_fixed(double beta, const double* mu) {
     PhaseScope ps(this, 4);
-    std::vector<double> aff(L), target(L);
-    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, dX.p, 1.0, Y.p, dY.p, 1.0, seg_part.p,
-            work_L.p, st);
-    d2h(aff.data(), work_L.p, L * sizeof(double));
+    std::vector<double> target(L);
+    double* aff = pinned_doubles(L);
+    dots(X.p, dX.p, 1.0, Y.p, dY.p, 1.0, aff);
     sync();
     for (int l = 0; l < L; ++l) {
       double rl = aff[l] / mu[l] / k[l];
@@ -1651,10 +1682,9 @@ struct Handle {
     if (!dense.empty()) {
       std::vector<double> sh(dense.size());
       for (size_t b = 0; b < dense.size(); ++b) sh[b] = target[dense[b].user];
-      h2d(work_L.p, sh.data(), sh.size() * sizeof(double));
-      add_diag(d_doff.p, d_dk.p, (int)dense.size(), kmax, R.p, work_L.p, 0.0, st);
+      add_diag_host(d_doff.p, d_dk.p, (int)dense.size(), kmax, R.p, sh.data(), work_L.p, st);
     }
-    h2d(target_user.p, target.data(), L * sizeof(double));
+    if (nd) h2d(target_user.p, target.data(), L * sizeof(double));
     diag_corrector_R(nd, od, X.p, Y.p, dX.p, dY.p, target_user.p, d_diag_user.p, R.p, st);
   }
   void set_rhs(int which) {
@@ -1673,10 +1703,9 @@ struct Handle {
     PhaseScope ps(this, 4);
     adx_current();
     axpbypcz(K, 1.0, adx.p, 1.0, P.p, 0.0, nullptr, dX.p, st);  // dX = 𝒜dx + P
-    for (auto& b : dense) d2d(T1.p + b.off, R.p + b.off, sizeof(double) * b.k * b.k);
     blk_gemm_all([&](const DenseBlk& b) { return blk_as_A(dX.p, b.off, b.k); }, false,
                  [&](const DenseBlk& b) { return blk_as_B(Y.p, b.off, b.k); }, true, T1.p, -1.0,
-                 1.0, KR_FULL);  // T1 = R − dX·Y
+                 1.0, KR_FULL, R.p);  // T1 = R − dX·Y
     dense_cholsolve(T1.p, dY.p);
     if (!dense.empty()) symmetrize(d_doff.p, d_dk.p, (int)dense.size(), kmax, dY.p, st);
     diag_dY(nd, od, R.p, dX.p, Y.p, LX.p, dY.p, st);
@@ -1851,26 +1880,25 @@ struct Handle {
       const DenseBlk& B = dense[reqs[q].b];
       td[q] = {reqs[q].M + B.off, reqs[q].dM + B.off, trials.p + off[q], reqs[q].t, B.k};
     }
-    if (d_trial_desc.n < n) d_trial_desc.alloc(std::max<size_t>(n, 2 * d_trial_desc.n));
+    if (n > (size_t)kTrialInline && d_trial_desc.n < n)
+      d_trial_desc.alloc(std::max<size_t>(n, 2 * d_trial_desc.n));
     // Staged at the end of the pinned area: potrf_host_list below uses its
     // start, and this copy is ordered before that call's final sync.
     const size_t tail = (n * (sizeof(MatDesc<double>) + 2 * sizeof(double) + sizeof(int)) + 64 + 15) / 16 * 16;
     unsigned char* hp = pinned(tail + n * sizeof(TrialDesc)) + tail;
     std::memcpy(hp, td.data(), n * sizeof(TrialDesc));
-    h2d(d_trial_desc.p, hp, n * sizeof(TrialDesc));
-    make_trials_list(d_trial_desc.p, (int)n, nmax, st);
+    make_trials_list(reinterpret_cast<const TrialDesc*>(hp), d_trial_desc.p, (int)n, nmax, st);
     std::vector<MatDesc<double>> mats(n);
     for (size_t q = 0; q < n; ++q) mats[q] = {trials.p + off[q], dense[reqs[q].b].k, dense[reqs[q].b].k};
     potrf_host_list(mats, info, dmn, dmx, false);
   }
 
   // The bounds of the dense blocks that step_bounds takes, from λ_min of
-  // L⁻¹·dM·L⁻ᵀ (both sides, one launch): queued into sb_out, [X blocks | Y blocks]
-  // of the block list sb_blocks.  Scratch: T1, T2, Z, tmpK2.
+  // L⁻¹·dM·L⁻ᵀ (both sides, one launch): queued into `out` (pinned), [X blocks |
+  // Y blocks] of the block list sb_blocks.  Scratch: T1, T2, Z, tmpK2.
   std::vector<int> sb_blocks;
   DBuf<StepBoundDesc> sb_desc;
-  DBuf<double> sb_out;
-  void queue_step_bounds() {
+  void queue_step_bounds(double* out) {
     const int n = (int)sb_blocks.size();
     const double *Ws[2] = {W.p, WY.p}, *dMs[2] = {dX.p, dY.p};
     double *Ts[2] = {T1.p, T2.p}, *Gs[2] = {Z.p, tmpK2.p};
@@ -1881,7 +1909,6 @@ struct Handle {
       for (int side = 0; side < 2; ++side)
         for (int b : sb_blocks) d.push_back({Gs[side] + dense[b].off, dense[b].k});
       sb_desc.alloc(d.size());
-      sb_out.alloc(d.size());
       h2d(sb_desc.p, d.data(), d.size() * sizeof(StepBoundDesc));
       sync();
     }
@@ -1905,7 +1932,7 @@ struct Handle {
         }
       flush();
     }
-    step_bounds(sb_desc.p, 2 * n, kb, sb_out.p, st);
+    step_bounds(sb_desc.p, 2 * n, kb, out, st);
   }
 
   // Fraction-to-boundary bounds of both sides (src/kernels/generic.jl:350-422):
@@ -1924,17 +1951,15 @@ struct Handle {
     const double* dMs[2] = {dX.p, dY.p};
     for (int side = 0; side < 2; ++side) {
       if (nd) {
-        diag_ftb(nd, od, Ms[side], dMs[side], red.p + 8 + side, st);
+        diag_ftb(nd, od, Ms[side], dMs[side], h_red + 8 + side, st);
       }
       for (auto& s2 : fetch_k2(Ms[side], dMs[side])) b2[side] = std::min(b2[side], ftb2(s2));
     }
     eigen = eigen && block_factors_current && !sb_blocks.empty();
-    if (nd) d2h(h_red + 8, red.p + 8, 2 * sizeof(double));
     if (eigen) {
-      queue_step_bounds();
       const size_t n = sb_blocks.size();
-      double* hb = reinterpret_cast<double*>(pinned(2 * n * sizeof(double)));
-      d2h(hb, sb_out.p, 2 * n * sizeof(double));
+      double* hb = pinned_doubles(2 * n);
+      queue_step_bounds(hb);
       sync();
       for (size_t q = 0; q < 2 * n; ++q) b2[q / n] = std::min(b2[q / n], hb[q]);
     }
@@ -2046,12 +2071,9 @@ struct Handle {
       tX = bX < 1 ? bX : 1.0;
       tY = bY < 1 ? bY : 1.0;
     }
-    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, nullptr, 0.0, Y.p, nullptr, 0.0, seg_part.p,
-            work_L.p, st);
-    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, dX.p, tX, Y.p, dY.p, tY, seg_part.p,
-            work_L.p + L, st);
-    double* c1 = reinterpret_cast<double*>(pinned(2 * (size_t)L * sizeof(double)));
-    d2h(c1, work_L.p, 2 * L * sizeof(double));  // both in one read-back
+    double* c1 = pinned_doubles(2 * (size_t)L);
+    dots(X.p, nullptr, 0.0, Y.p, nullptr, 0.0, c1);
+    dots(X.p, dX.p, tX, Y.p, dY.p, tY, c1 + L);
     sync();
     const double* c2 = c1 + L;
     double s1 = 0, s2 = 0;
@@ -2143,48 +2165,34 @@ struct Handle {
     combine(K, Y.p, tY, dY.p, st);
     combine(m, x.p, tX, dx.p, st);
     if (n_eq) combine(n_eq, yv.p, tY, dyv.p, st);  // src/solver/interior_point.jl:2228-2229
-    std::vector<double> dots(L);
-    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, nullptr, 0.0, Y.p, nullptr, 0.0, seg_part.p,
-            work_L.p, st);
-    d2h(dots.data(), work_L.p, L * sizeof(double));
-    clear_red(0, 4);
-    absmax(K, X.p, red.p + 0, st);
-    absmax(K, Y.p, red.p + 1, st);
-    absmax(m, x.p, red.p + 2, st);
-    if (n_eq) absmax(n_eq, yv.p, red.p + 3, st);
-    d2h(h_red, red.p, 4 * sizeof(double));
+    double* xy = pinned_doubles(L);
+    dots(X.p, nullptr, 0.0, Y.p, nullptr, 0.0, xy);
+    norms({{K, X.p, 0}, {K, Y.p, 1}, {m, x.p, 2}, {n_eq, yv.p, 3}});
     sync();
     double s = 0;
-    for (int l = 0; l < L; ++l) s += dots[l];
+    for (int l = 0; l < L; ++l) s += xy[l];
     *compl_total = s;
     *finite = std::isfinite(h_red[0]) && std::isfinite(h_red[1]) && std::isfinite(h_red[2]) &&
               std::isfinite(h_red[3]);
-    if (block_dots) std::memcpy(block_dots, dots.data(), L * sizeof(double));
+    if (block_dots) std::memcpy(block_dots, xy, L * sizeof(double));
   }
   void accepted_residuals(double bpr, double tX, double tY, double* pa, double* da) {
     *pa = std::fabs(1.0 - tX) * bpr;
     axpbypcz(m, 1.0 - tY, d.p, -tY, rho.p, 0.0, nullptr, d.p, st);
-    clear_red(0, 2);
-    absmax(m, d.p, red.p, st);
-    if (n_eq) {  // p+ = (1 − tX)p + tX·ρ_p (src/solver/interior_point.jl:1298-1305)
+    if (n_eq)  // p+ = (1 − tX)p + tX·ρ_p (src/solver/interior_point.jl:1298-1305)
       axpbypcz(n_eq, tX, rho_p.p, 1.0 - tX, pv.p, 0.0, nullptr, pv.p, st);
-      absmax(n_eq, pv.p, red.p + 1, st);
-    }
-    d2h(h_red, red.p, 2 * sizeof(double));
+    norms({{m, d.p, 0}, {n_eq, pv.p, 1}});
     sync();
     *da = h_red[0];
     if (n_eq) *pa = std::max(*pa, h_red[1]);
   }
   void objectives(double* po, double* dobj) {
-    std::vector<double> dots(2);
     // pObj = cᵀx ; dObj = Σ⟨C_l, Y_l⟩
-    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, Cst.p, nullptr, 0.0, Y.p, nullptr, 0.0, seg_part.p,
-            work_L.p, st);
-    std::vector<double> cy(L);
-    d2h(cy.data(), work_L.p, L * sizeof(double));
-    std::vector<double> hc(m), hx(m);
-    d2h(hc.data(), c.p, m * sizeof(double));
-    d2h(hx.data(), x.p, m * sizeof(double));
+    double* cy = pinned_doubles((size_t)L + 2 * (size_t)m);
+    double *hc = cy + L, *hx = hc + m;
+    dots(Cst.p, nullptr, 0.0, Y.p, nullptr, 0.0, cy);
+    d2h(hc, c.p, m * sizeof(double));
+    d2h(hx, x.p, m * sizeof(double));
     sync();
     double p = 0;
     for (int i = 0; i < m; ++i) p += hc[i] * hx[i];
@@ -2200,16 +2208,12 @@ struct Handle {
   void solution_residuals(double* pr, double* dr) {
     primal_residual(x.p, tmpK2.p);
     dual_residual(Y.p, work_m.p);
-    clear_red(0, 3);
     if (n_eq) {
       gemv_n(Beq.p, m, n_eq, yv.p, eq_tm.p, gemv_part.p, gemv_chunks, st);
       axpbypcz(m, 1.0, work_m.p, -1.0, eq_tm.p, 0.0, nullptr, work_m.p, st);
       gemv_t(Beq.p, m, n_eq, x.p, -1.0, beq.p, 1.0, eq_q.p, st);
-      absmax(n_eq, eq_q.p, red.p + 2, st);
     }
-    absmax(K, tmpK2.p, red.p + 0, st);
-    absmax(m, work_m.p, red.p + 1, st);
-    d2h(h_red, red.p, 3 * sizeof(double));
+    norms({{K, tmpK2.p, 0}, {m, work_m.p, 1}, {n_eq, eq_q.p, 2}});
     sync();
     *pr = std::max(h_red[0], h_red[2]);
     *dr = h_red[1];
@@ -2336,16 +2340,15 @@ struct Handle {
     apply_block_shifts(which == 0 ? X.p : Y.p, sh);
   }
   void block_dots(double* dots, double* trX, double* trY) {
-    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, X.p, nullptr, 0.0, Y.p, nullptr, 0.0, seg_part.p,
-            work_L.p, st);
-    d2h(dots, work_L.p, L * sizeof(double));
+    if (!dots || !trX || !trY) throw std::invalid_argument("dots and traces are required");
+    double* h = pinned_doubles(3 * (size_t)L);
+    this->dots(X.p, nullptr, 0.0, Y.p, nullptr, 0.0, h);
+    block_trace(d_uoff.p, d_uk.p, L, X.p, h + L, st);
+    block_trace(d_uoff.p, d_uk.p, L, Y.p, h + 2 * L, st);
     sync();
-    block_trace(d_uoff.p, d_uk.p, L, X.p, work_L.p, st);
-    d2h(trX, work_L.p, L * sizeof(double));
-    sync();
-    block_trace(d_uoff.p, d_uk.p, L, Y.p, work_L.p, st);
-    d2h(trY, work_L.p, L * sizeof(double));
-    sync();
+    std::copy(h, h + L, dots);
+    std::copy(h + L, h + 2 * L, trX);
+    std::copy(h + 2 * L, h + 3 * L, trY);
   }
 
   // -------------------------------------------------------- original data --
@@ -2708,6 +2711,7 @@ struct Handle {
   void adjoint_refined(const double* hwx, const double* hWX, const double* hWY, double* gc,
                        double* gC, int nA, const int32_t* Aidx, double* gA, int steps,
                        double* residual);
+  void adjoint_rows(int nA, const int32_t* Aidx, const double* lx, const double* xh, double* gA);
   void adjoint(const double* hwx, const double* hwy, const double* hWX, const double* hWY,
                double* gc, double* gb, double* gC, int nA, const int32_t* Aidx, double* gA);
   void equality_panel(const double* Li);
@@ -2797,22 +2801,12 @@ int sdpx_b200_set_iterate(sdpx_b200_handle* h, const double* x, const double* X,
 }
 int sdpx_b200_get_iterate(sdpx_b200_handle* h, double* x, double* X, double* Y) {
   GUARD(h, {
-    if (x) {
-      h->h.d2h(x, h->h.x.p, h->h.m * sizeof(double));
-      h->h.sync();
-    }
-    if (X) h->h.get_stacked(h->h.X.p, X);
-    if (Y) h->h.get_stacked(h->h.Y.p, Y);
+    h->h.get_vectors({{h->h.x.p, x, h->h.m}}, {{h->h.X.p, X}, {h->h.Y.p, Y}});
   });
 }
 int sdpx_b200_get_direction(sdpx_b200_handle* h, double* dx, double* dX, double* dY) {
   GUARD(h, {
-    if (dx) {
-      h->h.d2h(dx, h->h.dx.p, h->h.m * sizeof(double));
-      h->h.sync();
-    }
-    if (dX) h->h.get_stacked(h->h.dX.p, dX);
-    if (dY) h->h.get_stacked(h->h.dY.p, dY);
+    h->h.get_vectors({{h->h.dx.p, dx, h->h.m}}, {{h->h.dX.p, dX}, {h->h.dY.p, dY}});
   });
 }
 int sdpx_b200_get_rhs(sdpx_b200_handle* h, double* r) {
@@ -2847,8 +2841,11 @@ int sdpx_b200_schur_build(sdpx_b200_handle* h, int identity) {
 }
 int sdpx_b200_get_schur(sdpx_b200_handle* h, double* S) {
   GUARD(h, {
+    int e = 0;
     h->h.d2h(S, h->h.S.p, sizeof(double) * h->h.m * h->h.m);
+    h->h.d2h(&e, h->h.oz_err.p, sizeof(int));
     h->h.sync();
+    h->h.throw_oz_err(e);
   });
 }
 int sdpx_b200_factorize(sdpx_b200_handle* h, int* ok, int* att, double* q) {

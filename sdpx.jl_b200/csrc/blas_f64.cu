@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(Cfg::NT) k_gemm_grouped(const __grid_constant_
   double acc[Cfg::FM][Cfg::FN][2];
   zero_acc<Cfg>(acc);
   f64_tile_mainloop<Cfg>(acc, A, B, m0, n0, kb, ke, smem);
-  store_acc<Cfg>(acc, d.g.C[q], m0, n0, d.g.alpha[q], d.g.beta[q]);
+  store_acc<Cfg>(acc, d.g.C[q], m0, n0, d.g.alpha[q], d.g.beta[q], d.g.Cin[q]);
 }
 
 // In-place  T ← T · L  for a lower-triangular L (k×k, explicit zeros above the

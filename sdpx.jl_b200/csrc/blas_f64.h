@@ -21,6 +21,7 @@ struct GemmGroups {
   int n = 0;
   Opnd A[kGemmGroups], B[kGemmGroups];
   OutDesc C[kGemmGroups];
+  const double* Cin[kGemmGroups] = {};  // beta·Cin (C's layout); null: beta·C
   double alpha[kGemmGroups], beta[kGemmGroups];
   int mode[kGemmGroups];
 };

@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "dbuf.h"
 
 namespace sdpx {
 
@@ -13,18 +14,38 @@ struct MatDesc {
   int ld;
 };
 
-// Lower Cholesky in place of every matrix in d_mats (device array of nmat
-// descriptors, largest order nmax), one launch (potrf_flow.cu): a CTA per matrix
-// runs the pivot chain, sms/nmat − 1 others its remaining tiles, ordered by tile
-// flags.  info[b] = 0 on success, else the 1-based index of the first non-positive
-// pivot (the no-throw contract of SDPX's `kchol!`, src/kernels/generic.jl:133-155),
-// or −1 when a wait for a tile gave up (about a second).  dmin/dmax receive min/max
-// |L_ii|.  The strict upper triangle is zeroed unless zero_upper is false (positive-
-// definiteness tests that only read info/dmin/dmax).  `flags`
-// (potrf_flow_flag_words(nmat, nmax) words) must not be shared by concurrent calls.
+// Tile flags of potrf_flow, for the launches of one stream.  Each launch marks with an
+// epoch of its own, so the words are cleared only when allocated or when the count wraps.
 size_t potrf_flow_flag_words(int nmat, int nmax);
-void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, double* dmin,
-                double* dmax, unsigned* flags, int sms, cudaStream_t st, bool zero_upper = true);
+struct FlowFlags {
+  DBuf<unsigned> words;
+  unsigned epoch = 0;
+  void next(int nmat, int nmax, cudaStream_t st) {
+    const size_t need = potrf_flow_flag_words(nmat, nmax);
+    if (words.n < need) {
+      words.alloc(2 * need);
+      epoch = 0;
+    }
+    if (++epoch <= 1) {
+      words.zero(st);
+      epoch = 1;
+    }
+  }
+};
+
+// Lower Cholesky in place of nmat matrices (host array `mats`, largest order nmax), one
+// launch (potrf_flow.cu): a CTA per matrix runs the pivot chain, sms/nmat − 1 others its
+// remaining tiles, ordered by tile flags.  info[b] = 0 on success, else the 1-based index
+// of the first non-positive pivot (the no-throw contract of SDPX's `kchol!`,
+// src/kernels/generic.jl:133-155), or −1 when a wait for a tile gave up (about a second).
+// dmin/dmax receive min/max |L_ii|; the three may be pinned host memory, readable once
+// the stream is synchronised.  The strict upper triangle is zeroed unless zero_upper is
+// false (positive-definiteness tests that only read info/dmin/dmax).  d_mats takes the
+// descriptors of more than kFlowInline matrices (fewer travel with the launch).
+constexpr int kFlowInline = 16;
+void potrf_flow(const MatDesc<double>* mats, MatDesc<double>* d_mats, int nmat, int nmax, int* info,
+                double* dmin, double* dmax, FlowFlags& flags, int sms, cudaStream_t st,
+                bool zero_upper = true);
 
 // Inverses of the 64×64 diagonal tiles of a lower factor L (n×n): Dinv[s]
 // (64×64, column-major).

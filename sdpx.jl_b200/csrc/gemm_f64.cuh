@@ -172,7 +172,8 @@ __device__ __forceinline__ void for_each_acc(double (&acc)[Cfg::FM][Cfg::FN][2],
 // offset once per fragment row (instead of two index divisions per element).
 template <class Cfg>
 __device__ __forceinline__ void store_acc(double (&acc)[Cfg::FM][Cfg::FN][2], const OutDesc& C,
-                                          int m0, int n0, double alpha, double beta) {
+                                          int m0, int n0, double alpha, double beta,
+                                          const double* cin = nullptr) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int wm = warp / Cfg::WARPS_N, wn = warp % Cfg::WARPS_N;
@@ -197,7 +198,8 @@ __device__ __forceinline__ void store_acc(double (&acc)[Cfg::FM][Cfg::FN][2], co
       for (int c = 0; c < 2; ++c) {
         if (co[fn][c] < 0) continue;
         double* q = rp + co[fn][c];
-        *q = (beta == 0.0) ? alpha * acc[fm][fn][c] : alpha * acc[fm][fn][c] + beta * (*q);
+        const double* src = cin ? cin + (q - C.base) : q;
+        *q = (beta == 0.0) ? alpha * acc[fm][fn][c] : alpha * acc[fm][fn][c] + beta * (*src);
       }
   }
 }

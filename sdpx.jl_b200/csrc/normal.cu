@@ -429,11 +429,10 @@ struct NormalHandle {
   DBuf<int> d_dim, d_row, d_ok;
   DBuf<int> d_info;  // of the factor; [1]: a wait of the triangular solve gave up
   DBuf<ConeTile> d_tiles;
-  DBuf<unsigned> flow_flags;  // tile flags of the Cholesky launch
+  FlowFlags flow_flags;  // tile flags of the Cholesky launch
   DBuf<double> B, Bh, coef, weights, D, Dinv, Dis, w, lam, eta, eta2, s, z, v, out;
   DBuf<double> Q, F, Finv_diag, partial, rhs, t, red, work, u, gemv_part;
   DBuf<double> dmin, dmax;
-  DBuf<MatDesc<double>> descs;
   SyrkPlan plan;
   int gemv_chunks = 8;
   bool have_scaling = false, have_factor = false, have_assembled = false;
@@ -551,7 +550,6 @@ struct NormalHandle {
     SDPX_CUDA(cudaMemsetAsync(d_info.p, 0, 2 * sizeof(int), st));
     dmin.alloc(1);
     dmax.alloc(1);
-    descs.alloc(1);
     sync();
   }
   ~NormalHandle() {
@@ -770,11 +768,8 @@ struct NormalHandle {
 
   // Cholesky of the reduced matrix F in place.
   void factor_F() {
-    MatDesc<double> md{F.p, m, m};
-    h2d(descs.p, &md, sizeof(md));
-    const size_t need = potrf_flow_flag_words(1, m);
-    if (flow_flags.n < need) flow_flags.alloc(need);
-    potrf_flow(descs.p, 1, m, d_info.p, dmin.p, dmax.p, flow_flags.p, sms, st);
+    const MatDesc<double> md{F.p, m, m};
+    potrf_flow(&md, nullptr, 1, m, d_info.p, dmin.p, dmax.p, flow_flags, sms, st);
   }
 
   // One assembly + Cholesky attempt with LP weights already on the device

@@ -63,21 +63,25 @@ __device__ __forceinline__ void compute_sync() { bar_sync(kBarCompute, FT); }
 
 // Flag words of one matrix of nt tile rows: ready[i·nt + j] (tile final),
 // c1[j] (tile (j+1,j) updated by the panels before j), c2[j] (tile (j,j) updated
-// by the panels before j−1), then the failing pivot (1-based) and the timeout.
+// by the panels before j−1), then the failure and the timeout.
 struct Flags {
   unsigned *ready, *c1, *c2, *stop;
+  unsigned epoch;  // the value that marks
   int nt;
-  __device__ Flags(unsigned* base, int n) : ready(base), c1(base + n * n), c2(c1 + n), stop(c2 + n), nt(n) {}
+  __device__ Flags(unsigned* base, int n, unsigned ep)
+      : ready(base), c1(base + n * n), c2(c1 + n), stop(c2 + n), epoch(ep), nt(n) {}
   __device__ unsigned* tile(int i, int j) const { return ready + i * nt + j; }
+  __device__ bool set(const unsigned* f) const { return ld_acquire(f) == epoch; }
+  __device__ void mark(unsigned* f) const { st_release(f, epoch); }
 };
 
 // One thread waits for a and b; false when the matrix failed or a wait timed out.
-__device__ __forceinline__ bool poll_flags(const unsigned* a, const unsigned* b, unsigned* stop) {
+__device__ __forceinline__ bool poll_flags(const Flags& F, const unsigned* a, const unsigned* b) {
   unsigned spins = 0;
-  while (ld_acquire(a) == 0u || ld_acquire(b) == 0u) {
-    if (ld_acquire(stop) != 0u || ld_acquire(stop + 1) != 0u) return false;
+  while (!F.set(a) || !F.set(b)) {
+    if (F.set(F.stop) || F.set(F.stop + 1)) return false;
     if (++spins > kSpinLimit) {
-      atomicExch(stop + 1, 1u);
+      atomicExch(F.stop + 1, F.epoch);
       return false;
     }
   }
@@ -203,7 +207,7 @@ __device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<dou
   for (int p = 0; p < np; ++p) {
     if (!loaded) {
       int ok = 1;
-      if (threadIdx.x == 0) ok = poll_flags(F.tile(i, p), F.tile(q, p), F.stop);
+      if (threadIdx.x == 0) ok = poll_flags(F, F.tile(i, p), F.tile(q, p));
       if (!compute_and(ok)) return false;
       ra.load(M, i * FB, p * FB, h);
       if (i != q) rb.load(M, q * FB, p * FB, hq);
@@ -213,7 +217,7 @@ __device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<dou
     if (i != q) rb.store(Lb);
     int there = 1;
     if (threadIdx.x == 0)
-      there = p + 1 < np && ld_acquire(F.tile(i, p + 1)) != 0u && ld_acquire(F.tile(q, p + 1)) != 0u;
+      there = p + 1 < np && F.set(F.tile(i, p + 1)) && F.set(F.tile(q, p + 1));
     loaded = compute_and(there);
     if (loaded) {
       ra.load(M, i * FB, (p + 1) * FB, h);
@@ -245,7 +249,7 @@ __device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, in
   if (!update_tile(x, M, F, i, q, j, La, Lb)) return false;
   if (!partial) {
     int ok = 1;
-    if (threadIdx.x == 0) ok = poll_flags(F.tile(j, j), F.tile(j, j), F.stop);
+    if (threadIdx.x == 0) ok = poll_flags(F, F.tile(j, j), F.tile(j, j));
     if (!compute_and(ok)) return false;  // (also: La and Lb are free)
     load_tile<FT>(La, M, j * FB, j * FB, FB, FB, threadIdx.x);
   } else {
@@ -265,7 +269,7 @@ __device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, in
   store_tile<FT>(Lb, M, i * FB, q * FB, h, w, i == q, threadIdx.x);
   __threadfence();
   compute_sync();
-  if (threadIdx.x == 0) st_release(!partial ? F.tile(i, j) : u == 0 ? F.c2 + i : F.c1 + j, 1u);
+  if (threadIdx.x == 0) F.mark(!partial ? F.tile(i, j) : u == 0 ? F.c2 + i : F.c1 + j);
   return true;
 }
 
@@ -351,14 +355,14 @@ __device__ __forceinline__ void chain_io(const MatDesc<double> M, const Flags F,
   auto publish = [&](unsigned* f) {
     __threadfence();
     bar_sync(kBarIo, FIO);
-    if (tid == 0) st_release(f, 1u);
+    if (tid == 0) F.mark(f);
   };
   if (nt > 1 && !alone) fetch(0);
   for (int j = 0; j < nt; ++j) {
     const int w = min(FB, M.n - j * FB), h = min(FB, M.n - (j + 1) * FB);
     bar_sync(kBarFactored, FT + FIO);
     if (cs.fail != kNoFail) {
-      if (tid == 0) st_release(F.stop, (unsigned)(j * FB + cs.fail + 1));
+      if (tid == 0) F.mark(F.stop);
       return;
     }
     store_tile<FIO>(j & 1 ? T1 : T0, M, j * FB, j * FB, w, w, true, tid);
@@ -375,7 +379,7 @@ __device__ __forceinline__ void chain_io(const MatDesc<double> M, const Flags F,
     publish(F.tile(j + 1, j));
     bar_sync(kBarUpdated, FT + FIO);  // X and tile (j,j)'s buffer are free
     if (j + 2 < nt && !alone) {
-      if (tid == 0 && !poll_flags(F.c1 + j + 1, F.c2 + j + 2, F.stop)) cs.err = 1;
+      if (tid == 0 && !poll_flags(F, F.c1 + j + 1, F.c2 + j + 2)) cs.err = 1;
       bar_sync(kBarIo, FIO);
       if (cs.err) {
         bar_sync(kBarFactored, FT + FIO);
@@ -394,19 +398,24 @@ __device__ void zero_upper_part(const MatDesc<double>& M, int part, int parts, i
     for (int r = lane; r < c; r += 32) M.a[(size_t)c * M.ld + r] = 0.0;
 }
 
+struct FlowMats {
+  MatDesc<double> m[kFlowInline];
+};
+
 // gsize CTAs per matrix; CTA 0 of a group runs the chain.  Groups take the
 // matrices in turn when there are more matrices than groups.
 __global__ void __launch_bounds__(FT + FIO, 1)
-    k_potrf_flow(const MatDesc<double>* mats, int nmat, int gsize, int ngroups, unsigned* flags, int words,
-                 int* info, double* dmin, double* dmax, int zero_upper) {
+    k_potrf_flow(const __grid_constant__ FlowMats few, const MatDesc<double>* mats, int nmat, int gsize,
+                 int ngroups, unsigned* flags, int words, unsigned epoch, int* info, double* dmin,
+                 double* dmax, int zero_upper) {
   extern __shared__ __align__(16) double fsm[];
   double *T0 = fsm, *T1 = fsm + kTile, *X = fsm + 2 * kTile;
   __shared__ ChainShared cs;
   const int grp = blockIdx.x / gsize, me = blockIdx.x % gsize;
   for (int b = grp; b < nmat; b += ngroups) {
-    const MatDesc<double> M = mats[b];
+    const MatDesc<double> M = nmat <= kFlowInline ? few.m[b] : mats[b];
     const int nt = (M.n + FB - 1) / FB;
-    const Flags F(flags + (size_t)b * words, nt);
+    const Flags F(flags + (size_t)b * words, nt, epoch);
     __syncthreads();
     if (me == 0) {
       if (threadIdx.x == 0) cs.fail = kNoFail, cs.err = 0;
@@ -491,8 +500,8 @@ size_t potrf_flow_flag_words(int nmat, int nmax) {
 // A panel takes about 20 µs of it: 9 µs for the 64 pivots, 4 µs for tile (j+1,j),
 // 2 µs for tile (j+1,j+1); the rest is the way round through the other CTAs (tile
 // (j,j) out, row j+2 solved, tiles (j+2,j+1) and (j+2,j+2) updated and back).
-void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, double* dmin,
-                double* dmax, unsigned* flags, int sms, cudaStream_t st, bool zero_upper) {
+void potrf_flow(const MatDesc<double>* mats, MatDesc<double>* d_mats, int nmat, int nmax, int* info,
+                double* dmin, double* dmax, FlowFlags& flags, int sms, cudaStream_t st, bool zero_upper) {
   if (nmat <= 0 || nmax <= 0) return;
   ensure_smem(k_potrf_flow, kFlowSmem);
   const int nt = ceil_div(nmax, FB);
@@ -500,12 +509,17 @@ void potrf_flow(const MatDesc<double>* d_mats, int nmat, int nmax, int* info, do
   for (int j = 0; j < nt; ++j) tasks += flow_tasks(nt, j);
   int gsize = std::max(1, std::min(sms / nmat, 1 + tasks));
   int ngroups = std::min(nmat, sms / gsize), zu = zero_upper ? 1 : 0;
-  SDPX_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned) * words * (size_t)nmat, st));
+  FlowMats few{};
+  if (nmat <= kFlowInline) std::copy(mats, mats + nmat, few.m);
+  else SDPX_CUDA(cudaMemcpyAsync(d_mats, mats, sizeof(*mats) * nmat, cudaMemcpyHostToDevice, st));
+  flags.next(nmat, nmax, st);
+  unsigned* fw = flags.words.p;
+  unsigned ep = flags.epoch;
   if (gsize == 1) {  // no CTA waits for another
-    k_potrf_flow<<<ngroups, FT + FIO, kFlowSmem, st>>>(d_mats, nmat, gsize, ngroups, flags, words, info, dmin,
-                                                 dmax, zu);
+    k_potrf_flow<<<ngroups, FT + FIO, kFlowSmem, st>>>(few, d_mats, nmat, gsize, ngroups, fw, words, ep, info,
+                                                       dmin, dmax, zu);
   } else {
-    void* args[] = {&d_mats, &nmat, &gsize, &ngroups, &flags, &words, &info, &dmin, &dmax, &zu};
+    void* args[] = {&few, &d_mats, &nmat, &gsize, &ngroups, &fw, &words, &ep, &info, &dmin, &dmax, &zu};
     SDPX_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_potrf_flow), dim3(ngroups * gsize),
                                           dim3(FT + FIO), args, kFlowSmem, st));
   }

@@ -527,15 +527,63 @@ void absmax(long long n, const double* x, double* out, cudaStream_t st) {
   SDPX_LAUNCH_CHECK();
 }
 
+// max|x_e| of several vectors, delivered by the last block to finish (atomic ticket): a
+// launch in place of a clear, one launch per vector and a copy back, whose gaps and host
+// calls took 15-25 µs for vectors that need under 2.
+void NormList::add(long long len_, const double* x_, double* out_) {
+  if (len_ == 0) {
+    *out_ = 0.0;
+    return;
+  }
+  len[n] = len_;
+  x[n] = x_;
+  out[n] = out_;
+  first[n + 1] = first[n] + (int)std::min<long long>(512, ceil_div(len_, 1024));
+  ++n;
+}
+__global__ void __launch_bounds__(256) k_absmax_list(const __grid_constant__ NormList q, NormWork* w) {
+  __shared__ double red[32];
+  __shared__ bool last;
+  int e = 0;
+  while ((int)blockIdx.x >= q.first[e + 1]) ++e;
+  const double* x = q.x[e];
+  const long long n = q.len[e], step = (long long)(q.first[e + 1] - q.first[e]) * blockDim.x;
+  double v = 0.0;
+  for (long long i = (long long)(blockIdx.x - q.first[e]) * blockDim.x + threadIdx.x; i < n; i += step) {
+    double a = fabs(x[i]);
+    if (!(a == a)) a = 1.0 / 0.0;
+    v = fmax(v, a);
+  }
+  v = block_max(v, red);
+  if (threadIdx.x == 0) {
+    atomic_max_nonneg(&w->v[e], v);
+    __threadfence();
+    last = atomicAdd(&w->done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  if (threadIdx.x < q.n) {
+    __threadfence();
+    *q.out[threadIdx.x] = __ldcg(&w->v[threadIdx.x]);
+    w->v[threadIdx.x] = 0.0;
+  }
+  if (threadIdx.x == 0) w->done = 0;
+}
+void absmax_list(const NormList& q, NormWork* work, cudaStream_t st) {
+  if (q.n == 0) return;
+  k_absmax_list<<<q.first[q.n], 256, 0, st>>>(q, work);
+  SDPX_LAUNCH_CHECK();
+}
+
 // Segmented dot products: for segment s (rows [off[s], off[s]+len[s])),
 // out[s] = Σ (x + tx·dx)(y + ty·dy) (dx/dy may be null).  One CTA per segment
-// chunk; partials combined with a fixed-order second pass.
+// chunk; the last CTA to finish adds the partials in a fixed order.
 __global__ void k_seg_dot(const long long* off, const long long* len, int nseg, const double* x,
                           const double* dx, double tx, const double* y, const double* dy, double ty,
-                          int parts, double* part) {
+                          int parts, double* part, unsigned* done, double* out) {
   __shared__ double red[32];
+  __shared__ bool last;
   int s = blockIdx.y, p = blockIdx.x;
-  if (s >= nseg) return;
   long long o = off[s], n = len[s];
   long long per = (n + parts - 1) / parts;
   long long b = p * per, e = min(n, b + per);
@@ -548,22 +596,28 @@ __global__ void k_seg_dot(const long long* off, const long long* len, int nseg, 
     acc += a * c;
   }
   acc = block_sum(acc, red);
-  if (threadIdx.x == 0) part[(long long)s * parts + p] = acc;
-}
-__global__ void k_seg_reduce(int nseg, int parts, const double* part, double* out) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  double acc = 0.0;
-  for (int p = 0; p < parts; ++p) acc += part[(long long)s * parts + p];
-  out[s] = acc;
+  if (threadIdx.x == 0) {
+    part[(long long)s * parts + p] = acc;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x * gridDim.y - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int q = threadIdx.x; q < nseg; q += blockDim.x) {
+    double t = 0.0;
+    for (int i = 0; i < parts; ++i) t += __ldcg(part + (long long)q * parts + i);
+    out[q] = t;
+  }
+  if (threadIdx.x == 0) *done = 0;
 }
 void seg_dot(const long long* d_off, const long long* d_len, int nseg, int parts, const double* x,
              const double* dx, double tx, const double* y, const double* dy, double ty, double* part,
-             double* out, cudaStream_t st) {
+             unsigned* done, double* out, cudaStream_t st) {
   if (nseg == 0) return;
-  k_seg_dot<<<dim3(parts, nseg), 256, 0, st>>>(d_off, d_len, nseg, x, dx, tx, y, dy, ty, parts, part);
-  k_seg_reduce<<<ceil_div(nseg, 128), 128, 0, st>>>(nseg, parts, part, out);
-  SDPX_LAUNCH_CHECK_N(2);
+  k_seg_dot<<<dim3(parts, nseg), 256, 0, st>>>(d_off, d_len, nseg, x, dx, tx, y, dy, ty, parts, part, done,
+                                               out);
+  SDPX_LAUNCH_CHECK();
 }
 
 // Diagonal entries of every dense block plus the 1×1 entries: out[t] = trace.
@@ -598,6 +652,29 @@ void add_diag(const long long* d_off, const int* d_k, int nseg, int kmax, double
               const double* d_shifts, double uniform, cudaStream_t st) {
   if (nseg == 0 || kmax == 0) return;
   k_add_diag<<<dim3(ceil_div(kmax, 256), nseg), 256, 0, st>>>(d_off, d_k, nseg, M, d_shifts, uniform);
+  SDPX_LAUNCH_CHECK();
+}
+
+struct Shifts {
+  double v[kShiftInline];
+};
+__global__ void k_add_diag_inline(const long long* off, const int* kk, double* M,
+                                  const __grid_constant__ Shifts sh) {
+  const int s = blockIdx.y, k = kk[s];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x)
+    M[off[s] + i + (long long)i * k] += sh.v[s];
+}
+void add_diag_host(const long long* d_off, const int* d_k, int nseg, int kmax, double* M,
+                   const double* shifts, double* d_tmp, cudaStream_t st) {
+  if (nseg == 0 || kmax == 0) return;
+  if (nseg > kShiftInline) {
+    SDPX_CUDA(cudaMemcpyAsync(d_tmp, shifts, sizeof(double) * nseg, cudaMemcpyHostToDevice, st));
+    add_diag(d_off, d_k, nseg, kmax, M, d_tmp, 0.0, st);
+    return;
+  }
+  Shifts sh{};
+  std::copy(shifts, shifts + nseg, sh.v);
+  k_add_diag_inline<<<dim3(ceil_div(kmax, 256), nseg), 256, 0, st>>>(d_off, d_k, M, sh);
   SDPX_LAUNCH_CHECK();
 }
 
@@ -689,7 +766,7 @@ __global__ void k_diag_factor(int nd, long long od, const double* X, const doubl
   if (j >= nd) return;
   long long e = od + j;
   double x = X[e], y = Y[e];
-  if (!(x > 0) || !(y > 0)) atomicExch(fail, 1);
+  if (!(x > 0) || !(y > 0)) *fail = 1;  // (may be pinned host memory)
   LX[e] = sqrt(x);
   MY[e] = sqrt(y);
 }
@@ -837,19 +914,24 @@ void make_trials(const long long* d_off, const int* d_k, const long long* d_tria
 }
 
 // Trial matrices from a descriptor list: out_q = X_q + t_q·dX_q (k_q × k_q).
-__global__ void k_make_trials_list(const TrialDesc* d, int n) {
+struct TrialFew {
+  TrialDesc t[kTrialInline];
+};
+__global__ void k_make_trials_list(const __grid_constant__ TrialFew few, const TrialDesc* d, int n) {
   const int q = blockIdx.y;
-  if (q >= n) return;
-  const TrialDesc T = d[q];
+  const TrialDesc T = n <= kTrialInline ? few.t[q] : d[q];
   const long long tot = (long long)T.k * T.k;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
        e += (long long)gridDim.x * blockDim.x)
     T.out[e] = T.X[e] + T.t * T.dX[e];
 }
-void make_trials_list(const TrialDesc* d_list, int n, int kmax, cudaStream_t st) {
+void make_trials_list(const TrialDesc* list, TrialDesc* d_list, int n, int kmax, cudaStream_t st) {
   if (n == 0) return;
+  TrialFew few{};
+  if (n <= kTrialInline) std::copy(list, list + n, few.t);
+  else SDPX_CUDA(cudaMemcpyAsync(d_list, list, sizeof(TrialDesc) * n, cudaMemcpyHostToDevice, st));
   int g = std::max(1, std::min(64, ceil_div((long long)kmax * kmax, 256)));
-  k_make_trials_list<<<dim3(g, n), 256, 0, st>>>(d_list, n);
+  k_make_trials_list<<<dim3(g, n), 256, 0, st>>>(few, d_list, n);
   SDPX_LAUNCH_CHECK();
 }
 
@@ -875,6 +957,19 @@ void scatter(long long n, const long long* map, const double* src, double* dst, 
   SDPX_LAUNCH_CHECK();
 }
 
+__global__ void k_scatter_axpby(long long n, const long long* map, double a, const double* x, double b,
+                                const double* y, double* dst) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
+       e += (long long)gridDim.x * blockDim.x)
+    dst[map[e]] = a * x[e] + b * y[e];
+}
+void scatter_axpby(long long n, const long long* map, double a, const double* x, double b, const double* y,
+                   double* dst, cudaStream_t st) {
+  if (n == 0) return;
+  k_scatter_axpby<<<std::min(4096, ceil_div(n, 256)), 256, 0, st>>>(n, map, a, x, b, y, dst);
+  SDPX_LAUNCH_CHECK();
+}
+
 // --------------------------------------------------------- dense S helpers --
 // Full symmetric S from its lower triangle (upper ← lower).
 __global__ void k_mirror_lower(int m, double* S) {
@@ -891,7 +986,8 @@ void mirror_lower(int m, double* S, cudaStream_t st) {
 }
 
 // Sf = S (lower) with diagonal += reg·max(|S_ii|, 1)   (src/kkt.jl:1419-1445)
-__global__ void k_copy_reg(int m, const double* S, double* Sf, double reg) {
+__global__ void k_copy_reg(int m, const double* S, double* Sf, double reg, const int* err, int* err_out) {
+  if (err && blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;
   long long tot = (long long)m * m;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
        e += (long long)gridDim.x * blockDim.x) {
@@ -901,8 +997,22 @@ __global__ void k_copy_reg(int m, const double* S, double* Sf, double reg) {
     Sf[e] = v;
   }
 }
-void copy_reg(int m, const double* S, double* Sf, double reg, cudaStream_t st) {
-  k_copy_reg<<<std::min(4096, ceil_div((long long)m * m, 256)), 256, 0, st>>>(m, S, Sf, reg);
+void copy_reg(int m, const double* S, double* Sf, double reg, cudaStream_t st, const int* err, int* err_out) {
+  k_copy_reg<<<std::min(4096, ceil_div((long long)m * m, 256)), 256, 0, st>>>(m, S, Sf, reg, err, err_out);
+  SDPX_LAUNCH_CHECK();
+}
+
+__global__ void k_copy_pair(long long n, const double* s0, double* d0, const double* s1, double* d1) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
+       e += (long long)gridDim.x * blockDim.x) {
+    const double a = s0[e], b = s1[e];
+    d0[e] = a;
+    d1[e] = b;
+  }
+}
+void copy_pair(long long n, const double* s0, double* d0, const double* s1, double* d1, cudaStream_t st) {
+  if (n == 0) return;
+  k_copy_pair<<<std::min(4096, ceil_div(n, 256)), 256, 0, st>>>(n, s0, d0, s1, d1);
   SDPX_LAUNCH_CHECK();
 }
 

@@ -13,7 +13,9 @@ struct TrialDesc {
   double t;
   int k;
 };
-void make_trials_list(const TrialDesc* d_list, int n, int kmax, cudaStream_t st);
+// (`list` in host memory; d_list takes more than kTrialInline entries.)
+constexpr int kTrialInline = 16;
+void make_trials_list(const TrialDesc* list, TrialDesc* d_list, int n, int kmax, cudaStream_t st);
 
 void gemv_n(const double* A, long long K, int m, const double* x, double* out, double* part,
             int chunks, cudaStream_t st);
@@ -44,13 +46,35 @@ void axpbypcz(long long n, double a, const double* x, double b, const double* y,
 void combine(long long n, double* x, double t, const double* d, cudaStream_t st);
 void scale(long long n, double* x, double f, cudaStream_t st);
 void absmax(long long n, const double* x, double* out, cudaStream_t st);
+// out[e] = max|x_e| of every entry (NaN counts as +inf), one launch; `out` may be pinned
+// host memory.  `work` is zero between launches and belongs to one stream.
+constexpr int kNormMax = 8;
+struct NormWork {
+  double v[kNormMax];
+  unsigned done;
+};
+struct NormList {
+  int n = 0, first[kNormMax + 1] = {0};  // blocks of an entry: [first[e], first[e+1])
+  long long len[kNormMax];
+  const double* x[kNormMax];
+  double* out[kNormMax];
+  void add(long long len_, const double* x_, double* out_);  // entries of length 0 are dropped
+};
+void absmax_list(const NormList& q, NormWork* work, cudaStream_t st);
+// out[s] = Σ over segment s; `out` may be pinned host memory, `done` is zero between
+// launches.
 void seg_dot(const long long* d_off, const long long* d_len, int nseg, int parts, const double* x,
              const double* dx, double tx, const double* y, const double* dy, double ty, double* part,
-             double* out, cudaStream_t st);
+             unsigned* done, double* out, cudaStream_t st);
 void block_trace(const long long* d_off, const int* d_k, int nseg, const double* M, double* out,
                  cudaStream_t st);
 void add_diag(const long long* d_off, const int* d_k, int nseg, int kmax, double* M,
               const double* d_shifts, double uniform, cudaStream_t st);
+// The same with the shifts in host memory; d_tmp takes those of more than kShiftInline
+// segments.
+constexpr int kShiftInline = 16;
+void add_diag_host(const long long* d_off, const int* d_k, int nseg, int kmax, double* M,
+                   const double* shifts, double* d_tmp, cudaStream_t st);
 void symmetrize(const long long* d_off, const int* d_k, int nseg, int kmax, double* M,
                 cudaStream_t st);
 void gershgorin(const long long* d_off, const int* d_k, int nseg, int kmax, const double* M,
@@ -79,7 +103,14 @@ void make_trials(const long long* d_off, const int* d_k, const long long* d_tria
 void gather(long long n, const long long* map, const double* src, double* dst, cudaStream_t st);
 void scatter(long long n, const long long* map, const double* src, double* dst, cudaStream_t st);
 void mirror_lower(int m, double* S, cudaStream_t st);
-void copy_reg(int m, const double* S, double* Sf, double reg, cudaStream_t st);
+// (err_out, pinned host memory, receives *err where err is not null.)
+void copy_reg(int m, const double* S, double* Sf, double reg, cudaStream_t st, const int* err = nullptr,
+              int* err_out = nullptr);
+// (d0, d1) = (s0, s1)
+void copy_pair(long long n, const double* s0, double* d0, const double* s1, double* d1, cudaStream_t st);
+// dst[map[e]] = a·x[e] + b·y[e]
+void scatter_axpby(long long n, const long long* map, double a, const double* x, double b, const double* y,
+                   double* dst, cudaStream_t st);
 void symv_full(int m, const double* S, const double* x, double alpha, const double* b, double beta,
                double* y, cudaStream_t st);
 void ruiz_rowmax_dense(const double* A, long long K, int m, long long off, int k, double* rn,
