@@ -1352,7 +1352,7 @@ struct Handle {
         oz_plan = plan_ozaki_syrk(m, K, sms);
         oz_digits.alloc(oz_plan.digit_bytes);
         oz_exps.alloc(m);
-        oz_partial.alloc(oz_plan.partial_alloc_doubles);
+        oz_partial.alloc(oz_plan.partial_doubles);
       }
       // After the digit block products every dense row of P̂ carries its column
       // maximum already; the Gram's digit pass scans only the 1×1 rows for it.

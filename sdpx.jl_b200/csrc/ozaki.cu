@@ -196,9 +196,17 @@ __device__ __forceinline__ void oz_mma_stage(uint32_t tmem, uint32_t base, bool 
   }
 }
 
+// Lower tiles (A tile of 128 rows, B tile of 64 rows) that hold an entry with i ≥ j, one
+// A tile after the other: A tile a has 2a + 2 of them, the last one at most ⌈m/64⌉.
+__device__ __forceinline__ int2 oz_lower_tile(int p) {
+  int a = (int)((sqrt(4.0 * p + 1.0) - 1.0) * 0.5);
+  while ((a + 1) * (a + 2) <= p) ++a;
+  while (a * (a + 1) > p) --a;
+  return make_int2(a, p - a * (a + 1));
+}
+
 __global__ void __launch_bounds__(ONT, 1)
-    k_oz_syrk(const __grid_constant__ OzMaps maps, const int2* __restrict__ pairs, int npairs,
-              int kchunk, long long Kp, const int* __restrict__ exps, int m,
+    k_oz_syrk(const __grid_constant__ OzMaps maps, int npairs, int kchunk, long long Kp, const int* __restrict__ exps, int m,
               double* __restrict__ partial, int* err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -221,7 +229,7 @@ __global__ void __launch_bounds__(ONT, 1)
 
   const int u = blockIdx.x;
   const int chunk = u / npairs, pr = u % npairs;
-  const int2 tile = pairs[pr];
+  const int2 tile = oz_lower_tile(pr);
   const int ra = tile.x * OM, rb = tile.y * ON;
   const long long kb = (long long)chunk * kchunk;
   const long long ke = min(Kp, kb + kchunk);
@@ -299,40 +307,50 @@ __global__ void __launch_bounds__(ONT, 1)
   if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
-// S tile = Σ_chunks of the partial tiles, in chunk order, lower part only.
-// Four CTAs per tile, 32 rows each: coalesced reads of the row-major partials
-// (a thread's eight loads of a chunk in flight together), the 32 × 64 block
-// transposed through shared memory, each warp writing 32 consecutive rows of
-// one column of the column-major S.
-__global__ void __launch_bounds__(256) k_oz_reduce(const double* __restrict__ partial,
-                                                   const int2* __restrict__ pairs, int npairs,
+// S tile = Σ_chunks of the partial tiles, in chunk order, lower part only; the sum
+// carries its rounding errors along (TwoSum), so that it is as good with many chunks as
+// with few.
+// Sixteen CTAs per tile, 8 rows each: coalesced reads of the row-major partials (a
+// thread's loads of eight chunks in flight together: a Gram of two tiles in twenty
+// chunks took 18 µs with 32 rows a CTA and one chunk after the other, 7 now), the 8 × 64
+// block transposed through shared memory.
+__global__ void __launch_bounds__(256) k_oz_reduce(const double* __restrict__ partial, int npairs,
                                                    int nchunk, int m, double* __restrict__ S) {
-  __shared__ double blk[ON][33];
-  const int pr = blockIdx.x >> 2, r0 = (blockIdx.x & 3) * 32;
-  const int2 tile = pairs[pr];
-  constexpr int PER = 32 * ON / 256;
-  double acc[PER];
+  constexpr int ROWS = 8, BATCH = 8;
+  __shared__ double blk[ON][ROWS + 1];
+  const int pr = blockIdx.x / (OM / ROWS), r0 = (blockIdx.x % (OM / ROWS)) * ROWS;
+  const int2 tile = oz_lower_tile(pr);
+  constexpr int PER = ROWS * ON / 256;
+  double acc[PER], low[PER];
 #pragma unroll
-  for (int k = 0; k < PER; ++k) acc[k] = 0.0;
+  for (int k = 0; k < PER; ++k) acc[k] = low[k] = 0.0;
   const size_t tsz = (size_t)OM * ON;
   const double* base = partial + (size_t)pr * tsz + (size_t)r0 * ON;
-  for (int ch = 0; ch < nchunk; ++ch) {
-    const double* src = base + (size_t)ch * npairs * tsz;
-    double v[PER];
+  for (int ch = 0; ch < nchunk; ch += BATCH) {
+    double v[BATCH][PER];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) v[k] = src[threadIdx.x + k * 256];
+    for (int q = 0; q < BATCH; ++q)
 #pragma unroll
-    for (int k = 0; k < PER; ++k) acc[k] += v[k];
+      for (int k = 0; k < PER; ++k)
+        v[q][k] = ch + q < nchunk ? base[(size_t)(ch + q) * npairs * tsz + threadIdx.x + k * 256] : 0.0;
+#pragma unroll
+    for (int q = 0; q < BATCH; ++q)
+#pragma unroll
+      for (int k = 0; k < PER; ++k) {
+        const double t = acc[k] + v[q][k], z = t - acc[k];
+        low[k] += (acc[k] - (t - z)) + (v[q][k] - z);
+        acc[k] = t;
+      }
   }
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
     const int e = threadIdx.x + k * 256, r = e / ON, c = e % ON;
-    blk[c][r] = acc[k];
+    blk[c][r] = isfinite(acc[k]) ? acc[k] + low[k] : acc[k];
   }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
-    const int e = threadIdx.x + k * 256, r = e & 31, c = e >> 5;
+    const int e = threadIdx.x + k * 256, r = e % ROWS, c = e / ROWS;
     const int gi = tile.x * OM + r0 + r, gj = tile.y * ON + c;
     if (gi < m && gj < m && gi >= gj) S[gi + (size_t)gj * m] = blk[c][r];
   }
@@ -646,16 +664,6 @@ void encode_digit_map(CUtensorMap* map, const int8_t* pair_plane, int rows, long
   if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
 }
 
-// Lower tile pairs (A tile of 128 rows, B tile of 64 rows) that hold an entry
-// with i ≥ j.
-std::vector<int2> oz_pairs(int m) {
-  std::vector<int2> v;
-  const int tr = ceil_div(m, OM), tc = ceil_div(m, ON);
-  for (int a = 0; a < tr; ++a)
-    for (int b = 0; b < tc && b * ON <= a * OM + OM - 1; ++b) v.push_back(make_int2(a, b));
-  return v;
-}
-
 }  // namespace
 
 OzakiPlan plan_ozaki_syrk(int m, long long K, int sm_count) {
@@ -665,19 +673,29 @@ OzakiPlan plan_ozaki_syrk(int m, long long K, int sm_count) {
   p.Kp = std::max<long long>(64, (K + 63) / 64 * 64);
   p.ntile_r = ceil_div(m, OM);
   p.ntile_c = ceil_div(m, ON);
-  p.ntri = (int)oz_pairs(m).size();
-  // Chunks of at most 65 472 K (exact int32 levels: 65 472 · 8 · 4096 < 2^31),
-  // enough of them to give about four waves of one CTA per SM.
+  p.ntri = p.ntile_r * (p.ntile_r - 1) + std::min(2 * p.ntile_r, p.ntile_c);
+  // K chunks of at most 65 472 (exact int32 levels: 65 472 · 8 · 4096 < 2^31) and at
+  // least 128, their number by a model of the time in stages (0.77 µs of products): a
+  // CTA per SM does the units wave by wave, each at about ten stages of start-up and
+  // level sums, and a partial tile costs 0.04 to write and read.  Against chunks of 2048
+  // or more and four waves: m = 100, K = 2500
+  // 70 → 20 µs, 333 × 4010 62 → 28, 500 × 40000 201 → 157, 1000 × 50250 720 → 608.
   const long long maxc = 65472;
-  int nc = (int)std::max<long long>(1, (p.Kp + maxc - 1) / maxc);
-  while ((long long)p.ntri * nc < 4LL * sm_count && (p.Kp / (nc + 1)) >= 2048) ++nc;
-  long long kc = (p.Kp + nc - 1) / nc;
-  kc = (kc + OK - 1) / OK * OK;
-  p.kchunk = (int)kc;
-  p.nchunk = (int)((p.Kp + kc - 1) / kc);
+  const long long nmin = std::max<long long>(1, (p.Kp + maxc - 1) / maxc);
+  const long long nmax = std::max(nmin, std::min<long long>(p.Kp / 128, 16LL * sm_count / p.ntri));
+  double best = 0.0;
+  for (long long nc = nmin; nc <= nmax; ++nc) {
+    const long long kc = ((p.Kp + nc - 1) / nc + OK - 1) / OK * OK;
+    const long long units = p.ntri * ((p.Kp + kc - 1) / kc);
+    const double t = (double)((units + sm_count - 1) / sm_count) * (kc / OK + 10) + 0.04 * units;
+    if (nc == nmin || t < best) {
+      best = t;
+      p.kchunk = (int)kc;
+    }
+  }
+  p.nchunk = (int)((p.Kp + p.kchunk - 1) / p.kchunk);
   p.digit_bytes = (size_t)OZ_DIGITS * m * p.Kp;
   p.partial_doubles = (size_t)p.nchunk * p.ntri * OM * ON;
-  p.partial_alloc_doubles = p.partial_doubles + (size_t)p.ntri;  // + int2 tile pairs
   return p;
 }
 
@@ -688,13 +706,6 @@ void ozaki_syrk(const double* P, const OzakiPlan& plan, int8_t* digits, int* exp
   if (m <= 0) return;
   k_oz_digits<<<m, 256, 0, st>>>(P, plan.K, plan.Kp, m, digits, exps, dense_hi, tail_off);
   SDPX_LAUNCH_CHECK();
-  // The tile-pair table follows the partial tiles in the same buffer
-  // (plan.partial_alloc_doubles).  A copy from pageable memory returns once the
-  // host data is staged, so the local table may go out of scope afterwards.
-  const std::vector<int2> host_pairs = oz_pairs(m);
-  int2* d_pairs = reinterpret_cast<int2*>(partial + plan.partial_doubles);
-  SDPX_CUDA(cudaMemcpyAsync(d_pairs, host_pairs.data(), sizeof(int2) * host_pairs.size(),
-                            cudaMemcpyHostToDevice, st));
   OzMaps maps;
   const size_t plane = (size_t)m * plan.Kp;
   for (int d = 0; d < OPAIRS; ++d) {
@@ -704,10 +715,10 @@ void ozaki_syrk(const double* P, const OzakiPlan& plan, int8_t* digits, int* exp
   ensure_smem(k_oz_syrk, OSMEM);
   const int units = plan.ntri * plan.nchunk;
   if (ev_begin) SDPX_CUDA(cudaEventRecord(ev_begin, st));
-  k_oz_syrk<<<units, ONT, OSMEM, st>>>(maps, d_pairs, plan.ntri, plan.kchunk, plan.Kp, exps, m,
+  k_oz_syrk<<<units, ONT, OSMEM, st>>>(maps, plan.ntri, plan.kchunk, plan.Kp, exps, m,
                                        partial, err);
   if (ev_end) SDPX_CUDA(cudaEventRecord(ev_end, st));
-  k_oz_reduce<<<plan.ntri * 4, 256, 0, st>>>(partial, d_pairs, plan.ntri, plan.nchunk, m, S);
+  k_oz_reduce<<<plan.ntri * (OM / 8), 256, 0, st>>>(partial, plan.ntri, plan.nchunk, m, S);
   SDPX_LAUNCH_CHECK_N(2);
 }
 

@@ -16,14 +16,13 @@ struct OzakiPlan {
   int ntile_r = 0, ntile_c = 0, ntri = 0, nchunk = 0, kchunk = 0;
   size_t digit_bytes = 0;     // OZ_DIGITS · m · Kp
   size_t partial_doubles = 0; // nchunk · ntri · 128 · 64
-  size_t partial_alloc_doubles = 0;  // partial tiles + the tile-pair table
 };
 
 OzakiPlan plan_ozaki_syrk(int m, long long K, int sm_count);
 
 // S (m×m, column-major, lower triangle and diagonal written) = PᵀP for P
 // (K×m, column-major, ld = K).  digits: plan.digit_bytes of scratch, exps: m
-// ints, partial: plan.partial_alloc_doubles.  err: device flag set when a bounded
+// ints, partial: plan.partial_doubles.  err: device flag set when a bounded
 // wait gave up.  ev_begin/ev_end (optional) bracket the tensor-core kernel.
 // dense_hi (optional, m entries): the rows [0, tail_off) of P were written by
 // ozaki_gemm with OzGemm::colmax = dense_hi, so their per-column maxima are
