@@ -1934,6 +1934,8 @@ struct Handle {
     }
     step_bounds(sb_desc.p, 2 * n, kb, out, st);
   }
+      for (size_t q = 0; q < 2 * n; ++q)
+        if (std::isnan(hb[q])) throw CudaError("step bound: a wait in a cluster gave up");
 
   // Fraction-to-boundary bounds of both sides (src/kernels/generic.jl:350-422):
   // closed forms for 1×1 and 2×2 blocks.  Larger blocks: with `eigen` (the affine

@@ -18,17 +18,28 @@ struct LambdaScratch {
 
 // Number of eigenvalues below x of the tridiagonal (d, e2 = squared off-diagonal,
 // all scaled to norm ≤ 1): sign changes of the leading minors of T − x·I by their
-// three-term recurrence, one fma a row in the chain, rescaled every four rows.
-// e2 ≥ 1e-36 keeps two consecutive minors from vanishing together (a change of T
-// of 1e-18 of its norm).
+// three-term recurrence, one fma a row in the chain, rescaled every eight rows (within
+// which two consecutive minors grow at most 3⁸-fold and shrink to 1e-288 at worst),
+// the next eight rows' entries on their way.  e2 ≥ 1e-36 keeps two consecutive minors
+// from vanishing together (a change of T of 1e-18 of its norm).
 __device__ __forceinline__ int minors_below(const double* d, const double* e2, int k, double x) {
   double pp = 1.0, p = d[0] - x;
   int neg = __double2hiint(p) < 0;
   int i = 1;
-  for (; i + 3 < k; i += 4) {
+  constexpr int U = 8;
+  double di[U], ei[U];
+  if (i + U <= k) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const double q = fma(d[i + u] - x, p, -e2[i + u - 1] * pp);
+    for (int u = 0; u < U; ++u) di[u] = d[i + u], ei[u] = e2[i + u - 1];
+  }
+  for (; i + U <= k; i += U) {
+    double dn[U], en[U];
+    const bool more = i + 2 * U <= k;
+#pragma unroll
+    for (int u = 0; u < U; ++u) dn[u] = more ? d[i + U + u] : 0.0, en[u] = more ? e2[i + U + u - 1] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const double q = fma(di[u] - x, p, -ei[u] * pp);
       neg += (unsigned)(__double2hiint(q) ^ __double2hiint(p)) >> 31;
       pp = p;
       p = q;
@@ -37,6 +48,8 @@ __device__ __forceinline__ int minors_below(const double* d, const double* e2, i
     const double f = __hiloint2double(min(2046, max(1, 2046 - ex)) << 20, 0);  // ≈ 2^(1023−ex)
     p *= f;
     pp *= f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) di[u] = dn[u], ei[u] = en[u];
   }
   for (; i < k; ++i) {
     const double q = fma(d[i] - x, p, -e2[i - 1] * pp);

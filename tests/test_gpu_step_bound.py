@@ -85,3 +85,8 @@ def test_bounds_follow_a_changed_iterate():
         for key, M, dM in (("tX", X, dX), ("tY", Y, dY)):
             assert p1[key] == pytest.approx(_exact([4.0 * a for a in M], dM), rel=1e-10)
             assert p0[key] == pytest.approx(_exact(M, dM), rel=1e-10)
+
+
+@pytest.mark.parametrize("ks", [[31], [32], [33, 3], [63], [100], [127, 65], [224, 3], [225], [320, 17, 4], [447], [448, 15]])
+def test_affine_bounds_at_the_edges_of_the_clusters(ks):
+    test_affine_bounds_match_the_eigenvalues(ks)
