@@ -223,7 +223,8 @@ struct Handle {
   DBuf<double> mu_user, target_user, work_L;
   DBuf<double> seg_part;           // seg_dot partials
   DBuf<unsigned> seg_done;         // its count of finished CTAs
-  int seg_parts = 8;
+  DBuf<SegChunk> seg_chunks;
+  DBuf<int> seg_first;
   double last_bpr = 0.0;
   int mixed_predicted_steps = 32;  // from the last mixed factor's condition estimate
   long long mixed_guard_steps = 0;
@@ -401,7 +402,8 @@ struct Handle {
   // Σ of the user blocks' entries of (X + tx·dX)∘(Y + ty·dY) into `out`.
   void dots(const double* Xa, const double* dXa, double tx, const double* Ya, const double* dYa, double ty,
             double* out) {
-    seg_dot(d_uoff.p, d_ulen.p, L, seg_parts, Xa, dXa, tx, Ya, dYa, ty, seg_part.p, seg_done.p, out, st);
+    seg_dot(seg_chunks.p, (int)seg_chunks.n, seg_first.p, L, Xa, dXa, tx, Ya, dYa, ty, seg_part.p, seg_done.p,
+            out, st);
   }
   double* pinned_doubles(size_t n) { return reinterpret_cast<double*>(pinned(n * sizeof(double))); }
   void clear_red(int slot, int count = 1) {
@@ -692,8 +694,19 @@ struct Handle {
     mu_user.alloc(L);
     target_user.alloc(L);
     work_L.alloc(2 * std::max<size_t>((size_t)L, dense.size()) + 2);
-    seg_parts = 8;
-    seg_part.alloc((size_t)seg_parts * L);
+    std::vector<SegChunk> chunks;
+    std::vector<int> first;
+    for (int l = 0; l < L; ++l) {
+      first.push_back((int)chunks.size());
+      for (long long o = 0; o == 0 || o < seg_len[l]; o += kSegChunk)
+        chunks.push_back({seg_off[l] + o, seg_off[l] + std::min(seg_len[l], o + kSegChunk), l});
+    }
+    first.push_back((int)chunks.size());
+    seg_chunks.alloc(chunks.size());
+    seg_first.alloc(first.size());
+    h2d(seg_chunks.p, chunks.data(), chunks.size() * sizeof(SegChunk));
+    h2d(seg_first.p, first.data(), first.size() * sizeof(int));
+    seg_part.alloc(chunks.size());
     seg_done.alloc(1);
     seg_done.zero(st);
     norm_work.alloc(1);
@@ -723,116 +736,65 @@ struct Handle {
   }
 
   // ----------------------------------------------------------- scaling ----
+  DBuf<double> ruiz_work;  // row maxima | E | factors of up to eight passes
+  DBuf<double> ruiz_w;     // the factors of every entry
+  DBuf<int> ruiz_flags;    // active | pass counts | first rows
   void equilibrate(double* E_out, double* s_out, double* objscale, int32_t* passes) {
     if (mixed) mixed->a_planes_valid = false;
-    // keep the original data for final slack/residual reconstruction
-    if (!have_original) {
-      A0.alloc((size_t)K * m);
-      d2d(A0.p, A.p, sizeof(double) * K * m);
-      C0st.alloc(K);
-      d2d(C0st.p, Cst.p, sizeof(double) * K);
-      c0.alloc(m);
-      d2d(c0.p, c.p, sizeof(double) * m);
-      have_original = true;
+    const int nb = (int)dense.size(), nblk = nb + nd;
+    // Rows of the dense blocks one after the other, then the 1×1 blocks.
+    std::vector<int> row0;
+    int rows = 0;
+    for (auto& b : dense) row0.push_back(rows), rows += b.k;
+    row0.push_back(rows);
+    rows += nd;
+    if (!ruiz_work.p) {
+      ruiz_work.alloc(10 * (size_t)rows);
+      ruiz_flags.alloc(2 * (size_t)nblk + nb + 1);
     }
-    std::vector<std::vector<double>> E(L);
-    for (int l = 0; l < L; ++l) E[l].assign(k[l], 1.0);
-    std::vector<int> used(L, 0);
-    std::vector<char> active(L, 1);
-    DBuf<double> rn_d, e_d;
-    long long rows_total = 0;
-    for (auto& b : dense) rows_total += b.k;
-    rows_total += nd;
-    rn_d.alloc(rows_total);
-    e_d.alloc(rows_total);
-    std::vector<double> Chost(K);
-    for (int it = 1; it <= 8; ++it) {
-      bool any = false;
-      for (int l = 0; l < L; ++l) any = any || active[l];
-      if (!any) break;
-      // C row maxima on the host (C is small), A row maxima on the device.
-      d2h(Chost.data(), Cst.p, K * sizeof(double));
-      rn_d.zero(st);
-      long long ro = 0;
-      for (auto& b : dense) {
-        if (active[b.user]) ruiz_rowmax_dense(A.p, K, m, b.off, b.k, rn_d.p + ro, st);
-        ro += b.k;
-      }
-      if (nd) ruiz_rowmax_diag(A.p, K, m, od, nd, rn_d.p + ro, st);
-      std::vector<double> rn(rows_total);
-      d2h(rn.data(), rn_d.p, rows_total * sizeof(double));
+    double *rn = ruiz_work.p, *E_d = rn + rows, *F = E_d + rows;
+    int *active = ruiz_flags.p, *used_d = active + nblk, *row0_d = used_d + nblk;
+    // Pinned: column maxima, c, E, the blocks' pass counts, whether a block is active.
+    double* hmx = pinned_doubles(2 * (size_t)m + rows + nblk + 2);
+    double *hc = hmx + m, *hE = hc + m;
+    int *hused = reinterpret_cast<int*>(hE + rows), *any = hused + nblk;
+    std::fill(hE, hE + rows, 1.0);
+    std::fill(hused, hused + nblk, 1);
+    SDPX_CUDA(cudaMemsetAsync(rn, 0, rows * sizeof(double), st));
+    h2d(E_d, hE, rows * sizeof(double));
+    h2d(active, hused, nblk * sizeof(int));
+    h2d(row0_d, row0.data(), row0.size() * sizeof(int));
+    *any = 0;
+    int np = 0;
+    do {
+      for (int b = 0; b < nb; ++b)
+        ruiz_rowmax_dense(A.p, Cst.p, K, m, dense[b].off, dense[b].k, np, F + row0[b], rows, active + b,
+                          rn + row0[b], st);
+      ruiz_rowmax_diag(A.p, Cst.p, K, m, od, nd, np, F + row0[nb], rows, active + nb, rn + row0[nb], st);
+      ruiz_update(np + 1, nb, d_dk.p, row0_d, nd, rn, F + (size_t)np * rows, E_d, active, used_d, any, st);
       sync();
-      std::vector<double> e(rows_total, 1.0);
-      ro = 0;
-      auto handle_block = [&](int l, int kk, long long rowoff, const double* Cblk, long long cstride,
-                              bool is_diag) {
-        // rn[r] = max(rn[r], max_c |C[r,c]|)
-        for (int r0 = 0; r0 < kk; ++r0) {
-          double mx = rn[rowoff + r0];
-          for (int cc = 0; cc < kk; ++cc) {
-            double vv = std::fabs(Cblk[(is_diag ? 0 : (long long)cc * cstride) + r0]);
-            if (std::isnan(vv)) vv = INFINITY;
-            mx = std::max(mx, vv);
-          }
-          rn[rowoff + r0] = mx;
-        }
-        bool conv = false;
-        if (it >= 2) {
-          double dev = 0.0;
-          bool finite = true;
-          for (int r0 = 0; r0 < kk; ++r0) {
-            double vv = rn[rowoff + r0];
-            if (!(vv > 0)) continue;
-            if (!std::isfinite(vv)) {
-              finite = false;
-              break;
-            }
-            dev = std::max(dev, std::fabs(std::log(vv)));
-          }
-          conv = finite && dev <= 1.0 / 20.0;
-        }
-        for (int r0 = 0; r0 < kk; ++r0) {
-          double vv = rn[rowoff + r0];
-          e[rowoff + r0] = vv > 0 ? 1.0 / std::sqrt(vv) : 1.0;
-          E[l][r0] *= e[rowoff + r0];
-        }
-        used[l] = it;
-        if (conv) active[l] = 0;
-      };
-      for (auto& b : dense) {
-        if (active[b.user]) handle_block(b.user, b.k, ro, Chost.data() + b.off, b.k, false);
-        ro += b.k;
-      }
-      for (int j = 0; j < nd; ++j) {
-        int l = diag_user[j];
-        if (active[l]) handle_block(l, 1, ro + j, Chost.data() + od + j, 1, true);
-        else e[ro + j] = 1.0;
-      }
-      h2d(e_d.p, e.data(), rows_total * sizeof(double));
-      ro = 0;
-      for (auto& b : dense) {
-        if (active[b.user] || used[b.user] == it) ruiz_congruence_dense(A.p, K, m, b.off, b.k, e_d.p + ro, st);
-        ro += b.k;
-      }
-      if (nd) ruiz_congruence_diag(A.p, K, m, od, nd, e_d.p + ro, st);
-      // C ← E C E on the host copy, uploaded back
-      ro = 0;
-      for (auto& b : dense) {
-        for (int cc = 0; cc < b.k; ++cc)
-          for (int r0 = 0; r0 < b.k; ++r0)
-            Chost[b.off + (long long)cc * b.k + r0] *= e[ro + r0] * e[ro + cc];
-        ro += b.k;
-      }
-      for (int j = 0; j < nd; ++j) Chost[od + j] *= e[ro + j] * e[ro + j];
-      h2d(Cst.p, Chost.data(), K * sizeof(double));
-      sync();
-    }
+      ++np;
+    } while (*any == np && np < 8);
     // Per-variable scale s_i = max_l ‖A_i^(l)‖∞ (1 when zero), objective scale.
-    std::vector<double> mx(m), s(m), ch(m);
-    colmax(A.p, K, m, work_m.p, st);
-    d2h(mx.data(), work_m.p, m * sizeof(double));
-    d2h(ch.data(), c.p, m * sizeof(double));
+    if (ruiz_w.n < (size_t)np * K) ruiz_w.alloc((size_t)np * K);
+    ruiz_weights(nb, d_dk.p, d_doff.p, row0_d, kmax, nd, od, K, np, F, rows, ruiz_w.p, st);
+    colmax(A.p, ruiz_w.p, np, K, m, hmx, st);
+    d2h(hc, c.p, m * sizeof(double));
+    d2h(hE, E_d, rows * sizeof(double));
+    d2h(hused, used_d, nblk * sizeof(int));
     sync();
+    std::vector<double> s(m), ch(hc, hc + m);
+    const double* mx = hmx;
+    std::vector<std::vector<double>> E(L);
+    std::vector<int> used(L, 0);
+    for (int b = 0; b < nb; ++b) {
+      E[dense[b].user].assign(hE + row0[b], hE + row0[b] + dense[b].k);
+      used[dense[b].user] = hused[b];
+    }
+    for (int j = 0; j < nd; ++j) {
+      E[diag_user[j]].assign(1, hE[row0[nb] + j]);
+      used[diag_user[j]] = hused[nb + j];
+    }
     double osc = 0.0;
     for (int i = 0; i < m; ++i) {
       s[i] = mx[i] > 0 ? mx[i] : 1.0;
@@ -842,7 +804,17 @@ struct Handle {
     if (!(osc > 0 && std::isfinite(osc))) osc = 1.0;
     for (int i = 0; i < m; ++i) ch[i] /= osc;
     h2d(work_m.p, s.data(), m * sizeof(double));
-    scale_cols(A.p, K, m, work_m.p, st);
+    // The original data is kept for the final slack and residual reconstruction.
+    const bool keep = !have_original;
+    if (keep) {
+      A0.alloc((size_t)K * m);
+      C0st.alloc(K);
+      c0.alloc(m);
+      d2d(c0.p, c.p, sizeof(double) * m);
+      have_original = true;
+    }
+    scale_store(A.p, keep ? A0.p : nullptr, K, m, ruiz_w.p, np, work_m.p, st);
+    scale_store(Cst.p, keep ? C0st.p : nullptr, K, 1, ruiz_w.p, np, nullptr, st);
     if (n_eq) {  // `_scale_equality_rows!` (src/ingest.jl:1176-1184); b is unchanged
       if (!eq_have_original) {
         Beq0.alloc((size_t)m * n_eq);
@@ -912,7 +884,8 @@ struct Handle {
   }
   // Results of at most kStageBytes are written by the kernels into pinned memory and
   // copied out by the host: a copy to the caller's (pageable) memory of 320 KB, the size
-  // of one k = 200 matrix, took 150 µs of driver staging, this STAGEUS.  Larger ones
+  // of one k = 200 matrix, took 150 µs of driver staging, this 90 (most of it
+  // the first touch of new pages).  Larger ones
   // would spend on pinning the buffer what they save.
   static constexpr size_t kStageBytes = 4 << 20;
   struct VectorOut {  // n doubles as they are
@@ -1934,8 +1907,6 @@ struct Handle {
     }
     step_bounds(sb_desc.p, 2 * n, kb, out, st);
   }
-      for (size_t q = 0; q < 2 * n; ++q)
-        if (std::isnan(hb[q])) throw CudaError("step bound: a wait in a cluster gave up");
 
   // Fraction-to-boundary bounds of both sides (src/kernels/generic.jl:350-422):
   // closed forms for 1×1 and 2×2 blocks.  Larger blocks: with `eigen` (the affine
@@ -1963,6 +1934,8 @@ struct Handle {
       double* hb = pinned_doubles(2 * n);
       queue_step_bounds(hb);
       sync();
+      for (size_t q = 0; q < 2 * n; ++q)
+        if (std::isnan(hb[q])) throw CudaError("step bound: a wait in a cluster gave up");
       for (size_t q = 0; q < 2 * n; ++q) b2[q / n] = std::min(b2[q / n], hb[q]);
     }
     if (nd) {

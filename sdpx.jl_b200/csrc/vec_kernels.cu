@@ -4,6 +4,8 @@
 #include "dd.cuh"
 #include "vec_kernels.h"
 
+#include <type_traits>
+
 namespace sdpx {
 
 // ---------------------------------------------------------------- gemv ----
@@ -575,48 +577,57 @@ void absmax_list(const NormList& q, NormWork* work, cudaStream_t st) {
   SDPX_LAUNCH_CHECK();
 }
 
-// Segmented dot products: for segment s (rows [off[s], off[s]+len[s])),
-// out[s] = Σ (x + tx·dx)(y + ty·dy) (dx/dy may be null).  One CTA per segment
-// chunk; the last CTA to finish adds the partials in a fixed order.
-__global__ void k_seg_dot(const long long* off, const long long* len, int nseg, const double* x,
-                          const double* dx, double tx, const double* y, const double* dy, double ty,
-                          int parts, double* part, unsigned* done, double* out) {
+// Segmented dot products: out[s] = Σ (x + tx·dx)(y + ty·dy) over segment s (dx/dy may be
+// null).  One CTA per chunk of at most kSegChunk rows; the last CTA to finish adds the
+// chunks of a segment, a warp each, in an order of its own (the same every time).
+__global__ void __launch_bounds__(256) k_seg_dot(const SegChunk* __restrict__ chunks,
+                                                 const int* __restrict__ first, int nseg,
+                                                 const double* __restrict__ x, const double* __restrict__ dx,
+                                                 double tx, const double* __restrict__ y,
+                                                 const double* __restrict__ dy, double ty, double* part,
+                                                 unsigned* done, double* out) {
   __shared__ double red[32];
   __shared__ bool last;
-  int s = blockIdx.y, p = blockIdx.x;
-  long long o = off[s], n = len[s];
-  long long per = (n + parts - 1) / parts;
-  long long b = p * per, e = min(n, b + per);
+  const SegChunk q = chunks[blockIdx.x];
+  constexpr int PER = kSegChunk / 256;
   double acc = 0.0;
-  for (long long i = b + threadIdx.x; i < e; i += blockDim.x) {
-    double a = x[o + i];
-    if (dx) a += tx * dx[o + i];
-    double c = y[o + i];
-    if (dy) c += ty * dy[o + i];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const long long i = q.start + threadIdx.x + u * 256;
+    if (i >= q.end) break;
+    double a = x[i];
+    if (dx) a += tx * dx[i];
+    double c = y[i];
+    if (dy) c += ty * dy[i];
     acc += a * c;
   }
   acc = block_sum(acc, red);
   if (threadIdx.x == 0) {
-    part[(long long)s * parts + p] = acc;
+    part[blockIdx.x] = acc;
     __threadfence();
-    last = atomicAdd(done, 1u) == gridDim.x * gridDim.y - 1;
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int q = threadIdx.x; q < nseg; q += blockDim.x) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int s = threadIdx.x; s < nseg; s += 256)
+    if (first[s + 1] - first[s] == 1) out[s] = __ldcg(part + first[s]);
+  for (int s = warp; s < nseg; s += 8) {
+    const int b = first[s], e = first[s + 1];
+    if (e - b == 1) continue;
     double t = 0.0;
-    for (int i = 0; i < parts; ++i) t += __ldcg(part + (long long)q * parts + i);
-    out[q] = t;
+    for (int i = b + lane; i < e; i += 32) t += __ldcg(part + i);
+    t = warp_sum(t);
+    if (lane == 0) out[s] = t;
   }
   if (threadIdx.x == 0) *done = 0;
 }
-void seg_dot(const long long* d_off, const long long* d_len, int nseg, int parts, const double* x,
+void seg_dot(const SegChunk* d_chunks, int nchunk, const int* d_first, int nseg, const double* x,
              const double* dx, double tx, const double* y, const double* dy, double ty, double* part,
              unsigned* done, double* out, cudaStream_t st) {
-  if (nseg == 0) return;
-  k_seg_dot<<<dim3(parts, nseg), 256, 0, st>>>(d_off, d_len, nseg, x, dx, tx, y, dy, ty, parts, part, done,
-                                               out);
+  if (nseg == 0 || nchunk == 0) return;
+  k_seg_dot<<<nchunk, 256, 0, st>>>(d_chunks, d_first, nseg, x, dx, tx, y, dy, ty, part, done, out);
   SDPX_LAUNCH_CHECK();
 }
 
@@ -1034,134 +1045,209 @@ void symv_full(int m, const double* S, const double* x, double alpha, const doub
 }
 
 // --------------------------------------------------------- equilibration ---
-// Row maxima of |A_i| (dense block: rows r of every A_i^(l)) → rn[r].  CTA i
-// walks A_i's k×k block column by column with thread r holding row r's
-// maximum in a register (each column read coalesced, no index division, no
-// shared-memory atomics), then one atomic per row.  NaN counts as +inf.
-__global__ void k_ruiz_rowmax_dense(const double* A, long long K, int m, long long off, int k,
-                                    double* rn) {
-  const double* blk = A + (long long)blockIdx.x * K + off;
+// Ruiz passes on the unscaled data with the factors of the passes before: a pass only
+// reads 𝒜, which is written once at the end, every entry multiplied by one pass's
+// e_r·e_c after the other, as if each pass had scaled it.  (Scaling 𝒜 in every pass and C
+// on the host took 6.5 + 2.6 ms of kernels for m = 2000, k = 400 + 200, four passes, a
+// copy of 𝒜 and a round trip of C a pass.)  F holds the factors of pass p at p·rows.
+//
+// rn[r] = max(rn[r], max |A_i[r,c]·…|) over the columns i of 𝒜 and C (i = m), for a dense
+// block, after NP passes.  CTA i walks A_i's k×k block column by column with thread r
+// holding row r's maximum in a register (each column read coalesced, no index
+// division, no shared-memory atomics), then one atomic per row.  NaN counts as +inf.
+template <int NP>
+__global__ void k_ruiz_rowmax_dense(const double* __restrict__ A, const double* __restrict__ C, long long K,
+                                    int m, long long off, int k, const double* __restrict__ F, int rows,
+                                    const int* __restrict__ active, double* rn) {
+  if (!*active) return;
+  const double* blk = ((int)blockIdx.x < m ? A + (long long)blockIdx.x * K : C) + off;
   for (int r = threadIdx.x; r < k; r += blockDim.x) {
+    double er[NP + 1];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) er[p] = F[p * rows + r];
     double mx = 0.0;
 #pragma unroll 8
     for (int c = 0; c < k; ++c) {
-      double v = fabs(blk[(long long)c * k + r]);
+      double v = blk[(long long)c * k + r];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) v *= er[p] * F[p * rows + c];
+      v = fabs(v);
       if (!(v == v)) v = 1.0 / 0.0;
       mx = fmax(mx, v);
     }
     atomic_max_nonneg(rn + r, mx);
   }
 }
-void ruiz_rowmax_dense(const double* A, long long K, int m, long long off, int k, double* rn,
-                       cudaStream_t st) {
-  if (m == 0 || k == 0) return;
-  const int threads = std::min(1024, ceil_div(k, 32) * 32);
-  k_ruiz_rowmax_dense<<<m, threads, 0, st>>>(A, K, m, off, k, rn);
-  SDPX_LAUNCH_CHECK();
-}
-
-// Row maxima for the 1×1 group: rn[j] = max(rn[j], max_i |A[od+j, i]|), the
-// constraints split into chunks of 16 across blockIdx.y (an atomic per chunk)
-// so that the pass is spread over the whole GPU rather than one thread per j.
+// The same for the 1×1 group, the constraints split into chunks of 16 across blockIdx.y
+// (an atomic per chunk) so that the pass is spread over the whole GPU rather than one
+// thread per j.
 constexpr int kRuizDiagChunk = 16;
-__global__ void k_ruiz_rowmax_diag(const double* A, long long K, int m, long long od, int nd,
-                                   double* rn) {
+template <int NP>
+__global__ void k_ruiz_rowmax_diag(const double* __restrict__ A, const double* __restrict__ C, long long K,
+                                   int m, long long od, int nd, const double* __restrict__ F, int rows,
+                                   const int* __restrict__ active, double* rn) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nd) return;
-  for (int i0 = blockIdx.y * kRuizDiagChunk; i0 < m; i0 += gridDim.y * kRuizDiagChunk) {
-    const int i1 = min(m, i0 + kRuizDiagChunk);
+  if (j >= nd || !active[j]) return;
+  double e2[NP + 1];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) e2[p] = F[p * rows + j] * F[p * rows + j];
+  for (int i0 = blockIdx.y * kRuizDiagChunk; i0 <= m; i0 += gridDim.y * kRuizDiagChunk) {
+    const int i1 = min(m + 1, i0 + kRuizDiagChunk);
     double v = 0.0;
     for (int i = i0; i < i1; ++i) {
-      double a = fabs(A[od + j + (long long)i * K]);
+      double a = i < m ? A[od + j + (long long)i * K] : C[od + j];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) a *= e2[p];
+      a = fabs(a);
       if (!(a == a)) a = 1.0 / 0.0;
       v = fmax(v, a);
     }
     atomic_max_nonneg(rn + j, v);
   }
 }
-void ruiz_rowmax_diag(const double* A, long long K, int m, long long od, int nd, double* rn,
-                      cudaStream_t st) {
-  if (nd == 0 || m == 0) return;
-  dim3 grid(ceil_div(nd, 128), std::min(65535, ceil_div(m, kRuizDiagChunk)));
-  k_ruiz_rowmax_diag<<<grid, 128, 0, st>>>(A, K, m, od, nd, rn);
-  SDPX_LAUNCH_CHECK();
-}
-
-// A_i[r,c] *= e_r e_c over the rows [off, off+k²) of every column.  A flat
-// grid-stride sweep: all threads stream one contiguous window of 𝒜 (layouts
-// with one CTA walking each A_i's columns kept hundreds of separate streams
-// open and measured 0.92-0.96 ms against 0.78 ms for this one on the 400-block).
-__global__ void k_ruiz_congruence_dense(double* A, long long K, int m, long long off, int k,
-                                        const double* e) {
-  long long tot = (long long)k * k * m;
-  long long kk = (long long)k * k;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-       t += (long long)gridDim.x * blockDim.x) {
-    long long i = t / kk, q = t % kk;
-    int r = (int)(q % k), c = (int)(q / k);
-    A[i * K + off + q] *= e[r] * e[c];
+// f(integral_constant<n>) for a run-time 0 ≤ n ≤ 8.
+template <int N = 0, class F>
+static void with_passes(int n, F f) {
+  if constexpr (N <= 8) {
+    if (n == N) return f(std::integral_constant<int, N>());
+    with_passes<N + 1>(n, f);
   }
 }
-void ruiz_congruence_dense(double* A, long long K, int m, long long off, int k, const double* e,
-                           cudaStream_t st) {
-  long long tot = (long long)k * k * m;
-  if (tot == 0) return;
-  k_ruiz_congruence_dense<<<std::min(8192, ceil_div(tot, 256)), 256, 0, st>>>(A, K, m, off, k, e);
+void ruiz_rowmax_dense(const double* A, const double* C, long long K, int m, long long off, int k, int np,
+                       const double* F, int rows, const int* active, double* rn, cudaStream_t st) {
+  if (k == 0) return;
+  const int threads = std::min(512, ceil_div(k, 32) * 32);
+  with_passes(np, [&](auto n) {
+    k_ruiz_rowmax_dense<decltype(n)::value><<<m + 1, threads, 0, st>>>(A, C, K, m, off, k, F, rows, active, rn);
+  });
   SDPX_LAUNCH_CHECK();
 }
-
-// 1×1 group: A[od+j, i] *= e_j²
-__global__ void k_ruiz_congruence_diag(double* A, long long K, int m, long long od, int nd,
-                                       const double* e) {
-  long long tot = (long long)nd * m;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-       t += (long long)gridDim.x * blockDim.x) {
-    int j = (int)(t % nd);
-    long long i = t / nd;
-    A[od + j + i * K] *= e[j] * e[j];
-  }
-}
-void ruiz_congruence_diag(double* A, long long K, int m, long long od, int nd, const double* e,
-                          cudaStream_t st) {
+void ruiz_rowmax_diag(const double* A, const double* C, long long K, int m, long long od, int nd, int np,
+                      const double* F, int rows, const int* active, double* rn, cudaStream_t st) {
   if (nd == 0) return;
-  long long tot = (long long)nd * m;
-  k_ruiz_congruence_diag<<<std::min(8192, ceil_div(tot, 256)), 256, 0, st>>>(A, K, m, od, nd, e);
+  dim3 grid(ceil_div(nd, 128), std::min(65535, ceil_div(m + 1, kRuizDiagChunk)));
+  with_passes(np, [&](auto n) {
+    k_ruiz_rowmax_diag<decltype(n)::value><<<grid, 128, 0, st>>>(A, C, K, m, od, nd, F, rows, active, rn);
+  });
   SDPX_LAUNCH_CHECK();
 }
 
-// Column max |A[:, i]| → out[i]
-__global__ void k_colmax(const double* A, long long K, double* out) {
+// End of pass `it`: factors f_r = 1/√rn_r (where positive, else 1) of the active blocks
+// into F, E_r ← E_r·f_r; a block becomes inactive from the second pass on when every
+// |log rn_r| ≤ 1/20; rn ← 0.  One CTA per dense block, then 256 of the 1×1 blocks each.
+// used = last pass of a block; *any (pinned) = it while a block stays active.
+__global__ void __launch_bounds__(256) k_ruiz_update(int it, int nb, const int* __restrict__ kk,
+                                                     const int* __restrict__ row0, int nd, double* rn,
+                                                     double* F, double* E, int* active, int* used, int* any) {
+  const int b = blockIdx.x;
+  const bool dense = b < nb;
+  const int j = dense ? 0 : (b - nb) * 256 + (int)threadIdx.x;
+  const int blk = dense ? b : nb + j, r0 = dense ? row0[b] : row0[nb] + j;
+  const int n = dense ? kk[b] : j < nd ? 1 : 0;
+  const bool act = n > 0 && active[blk];
+  bool ok = true;  // every |log rn| within the limit
+  for (int r = dense ? threadIdx.x : 0; r < n; r += 256) {
+    const double v = act ? rn[r0 + r] : 0.0;
+    double f = 1.0;
+    if (v > 0) {
+      ok = ok && isfinite(v) && fabs(log(v)) <= 1.0 / 20.0;
+      f = 1.0 / sqrt(v);
+    }
+    rn[r0 + r] = 0.0;
+    F[r0 + r] = f;
+    E[r0 + r] *= f;
+  }
+  const bool conv = (dense ? __syncthreads_and(ok) : ok) && it >= 2;
+  if (!act || (dense && threadIdx.x != 0)) return;
+  used[blk] = it;
+  if (conv) active[blk] = 0;
+  else *any = it;
+}
+void ruiz_update(int it, int nb, const int* d_k, const int* d_row0, int nd, double* rn, double* F, double* E,
+                 int* active, int* used, int* any, cudaStream_t st) {
+  k_ruiz_update<<<nb + ceil_div(nd, 256), 256, 0, st>>>(it, nb, d_k, d_row0, nd, rn, F, E, active, used, any);
+  SDPX_LAUNCH_CHECK();
+}
+
+// w[p·K + q] = e_r·e_c of pass p (blockIdx.z) for every stacked entry q.
+__global__ void k_ruiz_weights(int nb, const int* __restrict__ kk, const long long* __restrict__ off,
+                               const int* __restrict__ row0, int nd, long long od, long long K,
+                               const double* __restrict__ F, int rows, double* w) {
+  const int b = blockIdx.y;
+  const double* e = F + (long long)blockIdx.z * rows + row0[b];
+  w += blockIdx.z * K;
+  if (b == nb) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += gridDim.x * blockDim.x) w[od + j] = e[j] * e[j];
+    return;
+  }
+  const int k = kk[b];
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < (long long)k * k;
+       q += (long long)gridDim.x * blockDim.x)
+    w[off[b] + q] = e[q % k] * e[q / k];
+}
+void ruiz_weights(int nb, const int* d_k, const long long* d_off, const int* d_row0, int kmax, int nd,
+                  long long od, long long K, int np, const double* F, int rows, double* w, cudaStream_t st) {
+  const long long most = std::max<long long>((long long)kmax * kmax, nd);
+  k_ruiz_weights<<<dim3(std::min(256, std::max(1, ceil_div(most, 256))), nb + 1, np), 256, 0, st>>>(
+      nb, d_k, d_off, d_row0, nd, od, K, F, rows, w);
+  SDPX_LAUNCH_CHECK();
+}
+
+// Column max of the scaled |A[:, i]| → out[i]
+template <int NP>
+__global__ void k_colmax(const double* __restrict__ A, const double* __restrict__ w, long long K, double* out) {
   __shared__ double red[32];
   int i = blockIdx.x;
   const double* col = A + (long long)i * K;
   double v = 0.0;
+#pragma unroll 4
   for (long long r = threadIdx.x; r < K; r += blockDim.x) {
-    double a = fabs(col[r]);
+    double a = col[r];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) a *= w[p * K + r];
+    a = fabs(a);
     if (!(a == a)) a = 1.0 / 0.0;
     v = fmax(v, a);
   }
   v = block_max(v, red);
   if (threadIdx.x == 0) out[i] = v;
 }
-void colmax(const double* A, long long K, int m, double* out, cudaStream_t st) {
+void colmax(const double* A, const double* w, int np, long long K, int m, double* out, cudaStream_t st) {
   if (m == 0) return;
-  k_colmax<<<m, 512, 0, st>>>(A, K, out);
+  with_passes(np, [&](auto n) { k_colmax<decltype(n)::value><<<m, 512, 0, st>>>(A, w, K, out); });
   SDPX_LAUNCH_CHECK();
 }
 
-// A[:, i] /= s_i
-__global__ void k_scale_cols(double* A, long long K, int m, const double* s) {
-  long long tot = K * m;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-       t += (long long)gridDim.x * blockDim.x) {
-    long long i = t / K;
-    A[t] /= s[i];
+// A0 ← A (unless null), A[q, i] ← A[q, i]·w_q… / s_i (s null: 1): a thread keeps its row's
+// weights for eight columns, whose loads are in flight together.
+constexpr int kScaleCols = 8;
+template <int NP>
+__global__ void k_scale_store(double* __restrict__ A, double* __restrict__ A0, long long K, int m,
+                              const double* __restrict__ w, const double* __restrict__ s) {
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (q >= K) return;
+  double wq[NP + 1];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) wq[p] = w[p * K + q];
+  for (int i0 = blockIdx.y * kScaleCols; i0 < m; i0 += gridDim.y * kScaleCols) {
+    double v[kScaleCols];
+#pragma unroll
+    for (int u = 0; u < kScaleCols; ++u) v[u] = i0 + u < m ? A[(i0 + u) * K + q] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kScaleCols; ++u) {
+      if (i0 + u >= m) break;
+      if (A0) A0[(i0 + u) * K + q] = v[u];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) v[u] *= wq[p];
+      A[(i0 + u) * K + q] = s ? v[u] / s[i0 + u] : v[u];
+    }
   }
 }
-void scale_cols(double* A, long long K, int m, const double* s, cudaStream_t st) {
-  long long tot = K * m;
-  if (tot == 0) return;
-  k_scale_cols<<<std::min(8192, ceil_div(tot, 256)), 256, 0, st>>>(A, K, m, s);
+void scale_store(double* A, double* A0, long long K, int m, const double* w, int np, const double* s,
+                 cudaStream_t st) {
+  if (K == 0 || m == 0) return;
+  const dim3 grid(ceil_div(K, 256), std::min(65535, ceil_div(m, kScaleCols)));
+  with_passes(np, [&](auto n) { k_scale_store<decltype(n)::value><<<grid, 256, 0, st>>>(A, A0, K, m, w, s); });
   SDPX_LAUNCH_CHECK();
 }
 

@@ -61,9 +61,16 @@ struct NormList {
   void add(long long len_, const double* x_, double* out_);  // entries of length 0 are dropped
 };
 void absmax_list(const NormList& q, NormWork* work, cudaStream_t st);
+// Chunks of the segments of a dot product: chunk q covers rows [start, end) of segment
+// seg; segment s owns the chunks [first[s], first[s+1]).
+struct SegChunk {
+  long long start, end;
+  int seg;
+};
+constexpr int kSegChunk = 2048;
 // out[s] = Σ over segment s; `out` may be pinned host memory, `done` is zero between
-// launches.
-void seg_dot(const long long* d_off, const long long* d_len, int nseg, int parts, const double* x,
+// launches, `part` holds a value per chunk.
+void seg_dot(const SegChunk* d_chunks, int nchunk, const int* d_first, int nseg, const double* x,
              const double* dx, double tx, const double* y, const double* dy, double ty, double* part,
              unsigned* done, double* out, cudaStream_t st);
 void block_trace(const long long* d_off, const int* d_k, int nseg, const double* M, double* out,
@@ -113,15 +120,16 @@ void scatter_axpby(long long n, const long long* map, double a, const double* x,
                    double* dst, cudaStream_t st);
 void symv_full(int m, const double* S, const double* x, double alpha, const double* b, double beta,
                double* y, cudaStream_t st);
-void ruiz_rowmax_dense(const double* A, long long K, int m, long long off, int k, double* rn,
-                       cudaStream_t st);
-void ruiz_rowmax_diag(const double* A, long long K, int m, long long od, int nd, double* rn,
-                      cudaStream_t st);
-void ruiz_congruence_dense(double* A, long long K, int m, long long off, int k, const double* e,
-                           cudaStream_t st);
-void ruiz_congruence_diag(double* A, long long K, int m, long long od, int nd, const double* e,
-                          cudaStream_t st);
-void colmax(const double* A, long long K, int m, double* out, cudaStream_t st);
-void scale_cols(double* A, long long K, int m, const double* s, cudaStream_t st);
+void ruiz_rowmax_dense(const double* A, const double* C, long long K, int m, long long off, int k, int np,
+                       const double* F, int rows, const int* active, double* rn, cudaStream_t st);
+void ruiz_rowmax_diag(const double* A, const double* C, long long K, int m, long long od, int nd, int np,
+                      const double* F, int rows, const int* active, double* rn, cudaStream_t st);
+void ruiz_update(int it, int nb, const int* d_k, const int* d_row0, int nd, double* rn, double* F, double* E,
+                 int* active, int* used, int* any, cudaStream_t st);
+void ruiz_weights(int nb, const int* d_k, const long long* d_off, const int* d_row0, int kmax, int nd,
+                  long long od, long long K, int np, const double* F, int rows, double* w, cudaStream_t st);
+void colmax(const double* A, const double* w, int np, long long K, int m, double* out, cudaStream_t st);
+void scale_store(double* A, double* A0, long long K, int m, const double* w, int np, const double* s,
+                 cudaStream_t st);
 
 }  // namespace sdpx
