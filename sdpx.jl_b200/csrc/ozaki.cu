@@ -4,8 +4,8 @@
 // Every column i of P is scaled by a power of two 2^-e_i (|P_ki| 2^-e_i < 1)
 // and written as OZ_DIGITS signed int8 digits,
 //   v = 2^-6 (d_0 + 2^-7 d_1 + 2^-14 d_2 + …),  d_0, d_t ∈ [-64, 64],
-// (d_0 = rint(64 v), then each remainder times 128 rounded), exactly, with the
-// remainder below 2^-(6+7·(OZ_DIGITS-1)) = 2^-55 of the column's largest entry.
+// the nearest multiple of 2^-(6+7·(OZ_DIGITS-1)) = 2^-55 of the column's largest entry,
+// exactly.
 // Then
 //   S_ij = 2^(e_i+e_j-12) Σ_ℓ 2^(-7ℓ) I_ℓ[i,j],   I_ℓ = Σ_{t+u=ℓ} Σ_k d_t[k,i] d_u[k,j],
 // keeping the levels ℓ ≤ OZ_DIGITS-1.  Each I_ℓ accumulates exactly in an
@@ -73,10 +73,47 @@ __device__ __forceinline__ double level_scale(int lv) {
 // Nearest integer (ties to even, as rint) of |x| < 2^51 by adding and
 // subtracting 1.5·2^52; the low word of the sum is the integer itself.
 constexpr double kRound = 6755399441055744.0;
-__device__ __forceinline__ double round_digit(double x, int& di) {
-  const double t = x + kRound;
-  di = __double2loint(t);
-  return t - kRound;
+
+// Four digits of an integer |n| ≤ 2^27, the highest in byte 3: that one in [-64, 64], the
+// others in [-64, 63] for n ≥ 0 and [-63, 64] below, so that digits of either sign are
+// equally likely and the dropped products have no bias.
+__device__ __forceinline__ unsigned digit_bytes(int n) {
+  const unsigned neg = (unsigned)(n >> 31) & 0x010101u;  // bias 63 = 64 − 1 in the lower bytes
+  const unsigned u = (unsigned)n + 135274560u - ((neg & 1u) * 16513u);
+  const unsigned b = (u & 0x7fu) | ((u << 1) & 0x7f00u) | ((u << 2) & 0x7f0000u) | ((u << 3) & 0xff000000u);
+  return (b + 0x40404040u + neg) ^ 0x80808080u;  // every byte less its bias
+}
+// The digits of four values x = 2^27·v, |v| < 1: w[t] holds digit t of x[0] … x[3].  v is
+// rounded to 2^-55 as two integers of 28 bits; their digits come from shifts and byte
+// permutes.  (With a rounding, a difference and a product in FP64 for every digit the
+// three digit passes over the rows of an m = 500, k = 200 build took 121 µs, now 104,
+// m = 1000, k = 200 + 100 326, now 264; those of the Gram's columns 67 and 161, with four
+// groups of loads in flight now 62 and 137.)
+__device__ __forceinline__ void digit_words(const double (&x)[4], unsigned (&w)[OZ_DIGITS]) {
+  unsigned z[2][4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const double t = x[q] + kRound, rest = (x[q] - (t - kRound)) * 268435456.0;
+    z[0][q] = digit_bytes(__double2loint(t));
+    z[1][q] = digit_bytes(__double2loint(rest + kRound));
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {  // 4×4 byte transpose
+    const unsigned l0 = __byte_perm(z[h][0], z[h][1], 0x5140), h0 = __byte_perm(z[h][0], z[h][1], 0x7362);
+    const unsigned l1 = __byte_perm(z[h][2], z[h][3], 0x5140), h1 = __byte_perm(z[h][2], z[h][3], 0x7362);
+    w[4 * h + 3] = __byte_perm(l0, l1, 0x5410);
+    w[4 * h + 2] = __byte_perm(l0, l1, 0x7632);
+    w[4 * h + 1] = __byte_perm(h0, h1, 0x5410);
+    w[4 * h] = __byte_perm(h0, h1, 0x7632);
+  }
+}
+// Digits of the elements k … k+3 of a row at `row` (its place in the first pair plane).
+__device__ __forceinline__ void store_digits(int8_t* row, long long plane, long long k, const double (&x)[4]) {
+  unsigned w[OZ_DIGITS];
+  digit_words(x, w);
+#pragma unroll
+  for (int t = 0; t < OZ_DIGITS; ++t)
+    *reinterpret_cast<unsigned*>(row + (t & 3) * 2 * plane + (k >> 5) * 64 + (t >> 2) * 32 + (k & 31)) = w[t];
 }
 
 // ---------------------------------------------------------------- digits --
@@ -122,27 +159,31 @@ __global__ void k_oz_digits(const double* __restrict__ P, long long K, long long
   const int e = s_exp;
   const size_t plane = (size_t)m * Kp;        // bytes per digit; a pair plane is 2·plane
   int8_t* dst = digits + (size_t)i * 2 * Kp;  // row i of every pair plane
-  // Four consecutive rows per thread: one char4 store per digit (Kp is a
+  // Four consecutive rows per thread and store, four such groups loaded at once (Kp is a
   // multiple of 64).
-  for (long long k0 = 4 * (long long)threadIdx.x; k0 < Kp; k0 += 4 * blockDim.x) {
-    double r[4];
+  constexpr int GROUPS = 4;
+  const bool pairs = (K & 1) == 0 && (reinterpret_cast<uintptr_t>(P) & 15) == 0;
+  const double sc = e != NAN_EXP && e >= -995 && e <= 1049 ? scale2(1.0, 27 - e) : 0.0;  // 2^(27−e), normal
+  for (long long kb = 4 * (long long)threadIdx.x; kb < Kp; kb += 4 * GROUPS * blockDim.x) {
+    double r[GROUPS][4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const long long k = k0 + q;
-      r[q] = (k < K && e != NAN_EXP) ? scale2(col[k], 6 - e) : 0.0;  // 64·v, |v| < 1
+    for (int g = 0; g < GROUPS; ++g) {
+      const long long k0 = kb + 4 * g * blockDim.x;
+      if (pairs && k0 + 4 <= K) {
+        const double2 u = *reinterpret_cast<const double2*>(col + k0), w = *reinterpret_cast<const double2*>(col + k0 + 2);
+        r[g][0] = u.x, r[g][1] = u.y, r[g][2] = w.x, r[g][3] = w.y;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[g][q] = k0 + q < K ? col[k0 + q] : 0.0;
+      }
     }
 #pragma unroll
-    for (int t = 0; t < OZ_DIGITS; ++t) {
-      int d0, d1, d2, d3;
-      const double a0 = round_digit(r[0], d0), a1 = round_digit(r[1], d1);
-      const double a2 = round_digit(r[2], d2), a3 = round_digit(r[3], d3);
-      *reinterpret_cast<char4*>(dst + (size_t)(t & 3) * 2 * plane + (k0 >> 5) * 64 + (t >> 2) * 32 +
-                                (k0 & 31)) =
-          make_char4((signed char)d0, (signed char)d1, (signed char)d2, (signed char)d3);
-      r[0] = (r[0] - a0) * 128.0;
-      r[1] = (r[1] - a1) * 128.0;
-      r[2] = (r[2] - a2) * 128.0;
-      r[3] = (r[3] - a3) * 128.0;
+    for (int g = 0; g < GROUPS; ++g) {
+      const long long k0 = kb + 4 * g * blockDim.x;
+      if (k0 >= Kp) break;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) r[g][q] = e == NAN_EXP ? 0.0 : sc != 0.0 ? r[g][q] * sc : scale2(r[g][q], 27 - e);
+      store_digits(dst, (long long)plane, k0, r[g]);
     }
   }
 }
@@ -358,15 +399,17 @@ __global__ void __launch_bounds__(256) k_oz_reduce(const double* __restrict__ pa
 
 // ------------------------------------------------------------ row digits --
 // One warp per row vector: largest magnitude over the kept elements, then the
-// digit planes, four consecutive elements per lane (char4 stores).
+// digit planes, four consecutive elements per lane (32-bit stores).  The first 128·HOLD
+// elements stay in registers between the two.
 struct OzRowsDev {
   const double* base;
   long long rows, is, os, es;
   int inner, len, tri;
 };
 
-__global__ void k_oz_digits_rows(const OzRowsDev r, long long Kp, long long plane,
-                                 int8_t* __restrict__ digits, int* __restrict__ exps) {
+template <int HOLD>
+__global__ void __launch_bounds__(256) k_oz_digits_rows(const OzRowsDev r, long long Kp, long long plane,
+                                                        int8_t* __restrict__ digits, int* __restrict__ exps) {
   const int lane = threadIdx.x & 31;
   const long long n = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (n >= r.rows) return;
@@ -374,9 +417,18 @@ __global__ void k_oz_digits_rows(const OzRowsDev r, long long Kp, long long plan
   int jlo = 0, jhi = r.len;
   if (r.tri == 1) jhi = (int)(n + 1 < (long long)r.len ? n + 1 : (long long)r.len);
   if (r.tri == 2) jlo = (int)(n < (long long)r.len ? n : (long long)r.len);
-  double mx = 0.0;
+  double x[HOLD][4], mx = 0.0;
   bool finite = true;
-  for (int j = jlo + lane; j < jhi; j += 32) {
+#pragma unroll
+  for (int g = 0; g < HOLD; ++g)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = 128 * g + 4 * lane + q;
+      x[g][q] = j >= jlo && j < jhi ? v[j * r.es] : 0.0;
+      finite = finite && isfinite(x[g][q]);
+      mx = fmax(mx, fabs(x[g][q]));
+    }
+  for (int j = max(jlo, 128 * HOLD) + lane; j < jhi; j += 32) {
     const double a = fabs(v[(long long)j * r.es]);
     finite = finite && isfinite(a);
     mx = fmax(mx, a);
@@ -388,25 +440,22 @@ __global__ void k_oz_digits_rows(const OzRowsDev r, long long Kp, long long plan
   if (!all_finite) e = NAN_EXP;
   if (lane == 0) exps[n] = e;
   int8_t* dst = digits + n * 2 * Kp;  // row n of every pair plane (2·plane bytes apart)
-  for (long long j0 = 4 * lane; j0 < Kp; j0 += 128) {
-    double x[4];
+#pragma unroll
+  for (int g = 0; g < HOLD; ++g) {
+    const long long j0 = 128 * g + 4 * lane;
+    if (j0 >= Kp) break;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[g][q] = e != NAN_EXP ? scale2(x[g][q], 27 - e) : 0.0;
+    store_digits(dst, plane, j0, x[g]);
+  }
+  for (long long j0 = 128 * HOLD + 4 * lane; j0 < Kp; j0 += 128) {
+    double y[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const long long j = j0 + q;
-      x[q] = (j >= jlo && j < jhi && e != NAN_EXP) ? scale2(v[j * r.es], 6 - e) : 0.0;
+      y[q] = (j >= jlo && j < jhi && e != NAN_EXP) ? scale2(v[j * r.es], 27 - e) : 0.0;
     }
-#pragma unroll
-    for (int t = 0; t < OZ_DIGITS; ++t) {
-      char4 c;
-      double d;
-      int di;
-      d = round_digit(x[0], di); c.x = (signed char)di; x[0] = (x[0] - d) * 128.0;
-      d = round_digit(x[1], di); c.y = (signed char)di; x[1] = (x[1] - d) * 128.0;
-      d = round_digit(x[2], di); c.z = (signed char)di; x[2] = (x[2] - d) * 128.0;
-      d = round_digit(x[3], di); c.w = (signed char)di; x[3] = (x[3] - d) * 128.0;
-      *reinterpret_cast<char4*>(dst + (t & 3) * 2 * plane + (j0 >> 5) * 64 + (t >> 2) * 32 +
-                                (j0 & 31)) = c;
-    }
+    store_digits(dst, plane, j0, y);
   }
 }
 
@@ -732,7 +781,12 @@ void ozaki_digits_rows(const OzRows& r, long long Kp, long long plane, int8_t* d
   OzRowsDev d{r.base, r.rows, r.is, r.os, r.es, r.inner, r.len, r.tri};
   constexpr int WARPS = 8;
   const long long blocks = (r.rows + WARPS - 1) / WARPS;
-  k_oz_digits_rows<<<(unsigned)blocks, WARPS * 32, 0, st>>>(d, Kp, plane, digits, exps);
+  if (r.len <= 128)
+    k_oz_digits_rows<1><<<(unsigned)blocks, WARPS * 32, 0, st>>>(d, Kp, plane, digits, exps);
+  else if (r.len <= 256)
+    k_oz_digits_rows<2><<<(unsigned)blocks, WARPS * 32, 0, st>>>(d, Kp, plane, digits, exps);
+  else
+    k_oz_digits_rows<4><<<(unsigned)blocks, WARPS * 32, 0, st>>>(d, Kp, plane, digits, exps);
   SDPX_LAUNCH_CHECK();
 }
 
