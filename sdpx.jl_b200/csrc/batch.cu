@@ -1164,7 +1164,7 @@ struct Engine {
   bool dd = false;  // the current optimize runs the Float64x2 Newton system
   DBuf<int> d_act;
   DBuf<int4> d_work;
-  DBuf<double> d_par, d_res;
+  DBuf<double> d_par;
   Pinned h_act, h_par, h_res, h_work;
   Pinned h_stage[2];          // upload staging (create only)
   cudaEvent_t ev_stage[2] = {nullptr, nullptr};
@@ -1276,7 +1276,6 @@ struct Engine {
     }
     d_act.alloc(N);
     d_par.alloc((size_t)N * kNIn + (N + 1) / 2);  // input rows, then the instance list
-    d_res.alloc((size_t)N * oNOut);
     h_act.ensure(N * sizeof(int));
     h_par.ensure(kStage * stage_stride());
     h_res.ensure((size_t)N * oNOut * sizeof(double));
@@ -1292,15 +1291,11 @@ struct Engine {
     pool.kq = (long long)((kmax + 7) & ~7) * FLD;  // a k×k tile64 tile (≥ kmax²)
     pool.kp = (long long)kmax * (kmax + 1) / 2;
     for (PhaseKernel kf : {k_b_residuals, k_b_rhs, k_b_dirblocks})
-      SDPX_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_bytes(3)));
-    SDPX_CUDA(cudaFuncSetAttribute(k_b_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kFactorSmem));
+      ensure_smem(kf, smem_bytes(3));
+    ensure_smem(k_b_factor, kFactorSmem);
     for (PhaseKernel kf : {k_b_affine, k_b_linesearch})
-      SDPX_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)std::max(smem_trials(), smem_bytes(3))));
-    SDPX_CUDA(cudaFuncSetAttribute(k_b_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem_bytes(4)));
+      ensure_smem(kf, std::max(smem_trials(), smem_bytes(3)));
+    ensure_smem(k_b_panel, smem_bytes(4));
     SDPX_CUDA(cudaStreamSynchronize(st));
   }
 
@@ -1317,10 +1312,8 @@ struct Engine {
     pool.dl = dl.p, pool.rl = rl.p, pool.dxl = dxl.p, pool.dxbl = dxbl.p, pool.rhol = rhol.p;
     pool.Sl = Sl.p, pool.LSl = LSl.p, pool.Gl = Gl.p;
     for (PhaseKernel kf : {k_dd_resid, k_dd_xinv, k_dd_rhs, k_dd_dirblocks})
-      SDPX_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_bytes(5)));
-    SDPX_CUDA(cudaFuncSetAttribute(k_dd_schur, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem_bytes(5)));
+      ensure_smem(kf, smem_bytes(5));
+    ensure_smem(k_dd_schur, smem_bytes(5));
     SDPX_CUDA(cudaStreamSynchronize(st));
   }
 
@@ -1350,14 +1343,19 @@ struct Engine {
       ha[q] = ids[lpt[q]];
       fill(ids[lpt[q]], hp + (size_t)q * kNIn);
     }
-    SDPX_CUDA(cudaMemcpyAsync(d_par.p, hs, bytes, cudaMemcpyHostToDevice, st));
-    kf<<<n, kThreads, smem, st>>>(pool, reinterpret_cast<const int*>(d_par.p + (size_t)n * kNIn), d_par.p,
-                                  d_res.p);
+    // A few instances read their inputs from the slot itself: a copy and its gap are 4 µs
+    // of the launch's, the reads 1 µs; with many the reads add up.  Results go
+    // straight to pinned memory.
+    const double* par = hp;
+    if (n > kDirect) {
+      SDPX_CUDA(cudaMemcpyAsync(d_par.p, hs, bytes, cudaMemcpyHostToDevice, st));
+      par = d_par.p;
+    }
+    kf<<<n, kThreads, smem, st>>>(pool, reinterpret_cast<const int*>(par + (size_t)n * kNIn), par,
+                                  static_cast<double*>(h_res.p));
     SDPX_LAUNCH_CHECK();
     ++launches;
     if (!read) return nullptr;
-    SDPX_CUDA(cudaMemcpyAsync(h_res.p, d_res.p, (size_t)n * oNOut * sizeof(double),
-                              cudaMemcpyDeviceToHost, st));
     sync_stream();
     const double* launched = static_cast<const double*>(h_res.p);
     rows.resize((size_t)n * oNOut);
@@ -1367,13 +1365,19 @@ struct Engine {
     return rows.data();
   }
   std::vector<int> lpt, work_rank;  // launch order; rank of each instance by work
-  static constexpr int kStage = 16;
+  static constexpr int kStage = 16, kDirect = 128;
   int staged = 0;  // staging slots in use
   size_t stage_stride() const { return ((size_t)N * (kNIn * sizeof(double) + sizeof(int)) + 63) & ~size_t(63); }
   void sync_stream() {
     SDPX_CUDA(cudaStreamSynchronize(st));
     staged = 0;
+    if (!schur_timed) return;
+    float ms = 0;
+    SDPX_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+    t_schur += ms * 1e-3;
+    schur_timed = false;
   }
+  bool schur_timed = false;  // ev[0], ev[1] around a Schur assembly whose time is not read yet
   std::vector<double> rows;         // output rows in the caller's order
   const double* phase(PhaseKernel kf, const std::vector<int>& ids, size_t smem, bool read) {
     return phase(kf, ids, smem, [](int, double*) {}, read);
@@ -1385,7 +1389,7 @@ struct Engine {
   void schur_dd(const std::vector<int>& ids) {
     const int n = (int)ids.size();
     if (n == 0) return;
-    SDPX_CUDA(cudaStreamSynchronize(st));
+    sync_stream();
     int* ha = static_cast<int*>(h_act.p);
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
@@ -1428,14 +1432,11 @@ struct Engine {
     const int n = (int)ids.size();
     if (n == 0) return;
     if (!dmma_attrs) {
-      SDPX_CUDA(cudaFuncSetAttribute(k_b_dmma_tp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_tp()));
-      SDPX_CUDA(cudaFuncSetAttribute(k_b_dmma_syrk<DmmaCfgKK>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)DmmaCfgKK::SMEM_BYTES));
+      ensure_smem(k_b_dmma_tp, smem_tp());
+      ensure_smem(k_b_dmma_syrk<DmmaCfgKK>, DmmaCfgKK::SMEM_BYTES);
       dmma_attrs = true;
     }
-    SDPX_CUDA(cudaStreamSynchronize(st));
+    if (schur_timed) sync_stream();  // h_act and h_work are free
     int* ha = static_cast<int*>(h_act.p);
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
@@ -1476,30 +1477,32 @@ struct Engine {
       std::copy(w->begin(), w->end(), hw + o);
       o += w->size();
     }
-    SDPX_CUDA(cudaMemcpyAsync(d_act.p, ha, n * sizeof(int), cudaMemcpyHostToDevice, st));
-    SDPX_CUDA(cudaMemcpyAsync(d_work.p, hw, nw * sizeof(int4), cudaMemcpyHostToDevice, st));
+    const int4* w = hw;  // a few instances: read in place, as in phase()
+    const int* act = ha;
+    if (n > kDirect) {
+      SDPX_CUDA(cudaMemcpyAsync(d_act.p, ha, n * sizeof(int), cudaMemcpyHostToDevice, st));
+      SDPX_CUDA(cudaMemcpyAsync(d_work.p, hw, nw * sizeof(int4), cudaMemcpyHostToDevice, st));
+      w = d_work.p;
+      act = d_act.p;
+    }
     SDPX_CUDA(cudaEventRecord(ev[0], st));
-    const int4* w = d_work.p;
-    k_b_dmma_tp<<<(int)tp.size(), kThreads, smem_tp(), st>>>(pool, d_act.p, w);
+    k_b_dmma_tp<<<(int)tp.size(), kThreads, smem_tp(), st>>>(pool, act, w);
     SDPX_LAUNCH_CHECK();
     w += tp.size();
     if (!sy64.empty()) {
       k_b_dmma_syrk<DmmaCfgKK><<<(int)sy64.size(), DmmaCfgKK::NT, DmmaCfgKK::SMEM_BYTES, st>>>(
-          pool, d_act.p, w);
+          pool, act, w);
       SDPX_LAUNCH_CHECK();
     }
     w += sy64.size();
     if (!sy32.empty()) {
       k_b_dmma_syrk<DmmaCfgKK32><<<(int)sy32.size(), DmmaCfgKK32::NT, DmmaCfgKK32::SMEM_BYTES,
-                                   st>>>(pool, d_act.p, w);
+                                   st>>>(pool, act, w);
       SDPX_LAUNCH_CHECK();
     }
     SDPX_CUDA(cudaEventRecord(ev[1], st));
     launches += 1 + (sy64.empty() ? 0 : 1) + (sy32.empty() ? 0 : 1);
-    SDPX_CUDA(cudaEventSynchronize(ev[1]));
-    float ms = 0;
-    SDPX_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-    t_schur += ms * 1e-3;
+    schur_timed = true;  // its time is read after the next wait for the stream
   }
 
   // The Schur assembly over `ids`: panel then SYRK work items, largest first
@@ -1513,7 +1516,7 @@ struct Engine {
     }
     WorkKernel syrk = syrk_kernel(threads, tile);
     if (!syrk) throw std::invalid_argument("unsupported Schur launch shape");
-    SDPX_CUDA(cudaStreamSynchronize(st));
+    sync_stream();
     int* ha = static_cast<int*>(h_act.p);
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
@@ -2138,6 +2141,7 @@ struct Engine {
       for (int rep = 0; rep < 3; ++rep) {
         const double before = t_schur;
         schur(ok, cd.threads, cd.tile, cd.grain);
+        if (schur_timed) sync_stream();
         ms_best = std::min(ms_best, (t_schur - before) * 1e3);
       }
       if (table && row < cap) {
@@ -2172,8 +2176,7 @@ struct Engine {
                                   "set every instance's solution first");
     if (d_cert.n < (size_t)N * kCertOut) d_cert.alloc((size_t)N * kCertOut);
     h_cert.ensure((size_t)N * kCertOut * sizeof(double));
-    SDPX_CUDA(cudaFuncSetAttribute(k_b_certificate, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem_bytes(1)));
+    ensure_smem(k_b_certificate, smem_bytes(1));
     k_b_certificate<<<N, kThreads, smem_bytes(1), st>>>(pool, std::max(ep, eg), std::max(ed, eg),
                                                        d_cert.p);
     SDPX_LAUNCH_CHECK();
