@@ -30,6 +30,7 @@
 #include "dbuf.h"
 #include "equality.h"
 #include "sparse_schur.h"
+#include "small_blocks.h"
 #include "step_bound.h"
 #include "dd_kernels.h"
 #include "mixed.h"
@@ -482,6 +483,19 @@ struct Handle {
     blk_gemm_all([&](const DenseBlk& b) { return blk_as_At(W.p, b.off, b.k); }, true,
                  [&](const DenseBlk& b) { return blk_as_B(T2.p, b.off, b.k); }, true, out, 1.0, 0.0,
                  KR_A_UPPER);
+  }
+
+  // out = X⁻¹·(sign·(M·Y − R)) for every dense block (R null: X⁻¹·(sign·M·Y)), sym:
+  // symmetrised.  One launch when all blocks fit a shared tile, a grouped product each
+  // otherwise.  Scratch: T1, T2.
+  void xinv_my(const double* M, const double* Rm, double sign, double* out, bool sym) {
+    if (kmax <= kSmallOrder)
+      return block_xinv_my(d_doff.p, d_dk.p, (int)dense.size(), kmax, M, Y.p, Rm, sign, W.p, out, sym, st);
+    blk_gemm_all([&](const DenseBlk& b) { return blk_as_A(M, b.off, b.k); }, false,
+                 [&](const DenseBlk& b) { return blk_as_B(Y.p, b.off, b.k); }, true, T1.p, sign,
+                 Rm ? -sign : 0.0, KR_FULL, Rm);
+    dense_cholsolve(T1.p, out);
+    if (sym) symmetrize(d_doff.p, d_dk.p, (int)dense.size(), kmax, out, st);
   }
 
   void ensure_descs(size_t n) {
@@ -1607,10 +1621,7 @@ struct Handle {
   // -------------------------------------------------------- right sides ---
   void rhs_from_R() {
     // Z = X⁻¹(P·Y − R); v = 𝒜ᵀ vec(Z); r = −(d + v)
-    blk_gemm_all([&](const DenseBlk& b) { return blk_as_A(P.p, b.off, b.k); }, false,
-                 [&](const DenseBlk& b) { return blk_as_B(Y.p, b.off, b.k); }, true, T1.p, 1.0,
-                 -1.0, KR_FULL, R.p);  // T1 = P·Y − R
-    dense_cholsolve(T1.p, Z.p);
+    xinv_my(P.p, R.p, 1.0, Z.p, false);
     diag_rhs_Z(nd, od, P.p, Y.p, R.p, LX.p, Z.p, st);
     atmul(Z.p, -1.0, d.p, -1.0, r.p);  // r = −v − d
   }
@@ -1676,11 +1687,7 @@ struct Handle {
     PhaseScope ps(this, 4);
     adx_current();
     axpbypcz(K, 1.0, adx.p, 1.0, P.p, 0.0, nullptr, dX.p, st);  // dX = 𝒜dx + P
-    blk_gemm_all([&](const DenseBlk& b) { return blk_as_A(dX.p, b.off, b.k); }, false,
-                 [&](const DenseBlk& b) { return blk_as_B(Y.p, b.off, b.k); }, true, T1.p, -1.0,
-                 1.0, KR_FULL, R.p);  // T1 = R − dX·Y
-    dense_cholsolve(T1.p, dY.p);
-    if (!dense.empty()) symmetrize(d_doff.p, d_dk.p, (int)dense.size(), kmax, dY.p, st);
+    xinv_my(dX.p, R.p, -1.0, dY.p, true);  // X⁻¹(R − dX·Y), symmetrised
     diag_dY(nd, od, R.p, dX.p, Y.p, LX.p, dY.p, st);
   }
 
@@ -1871,6 +1878,7 @@ struct Handle {
   // Y blocks] of the block list sb_blocks.  Scratch: T1, T2, Z, tmpK2.
   std::vector<int> sb_blocks;
   DBuf<StepBoundDesc> sb_desc;
+  DBuf<int> sb_list;  // sb_blocks on the device
   void queue_step_bounds(double* out) {
     const int n = (int)sb_blocks.size();
     const double *Ws[2] = {W.p, WY.p}, *dMs[2] = {dX.p, dY.p};
@@ -1885,7 +1893,14 @@ struct Handle {
       h2d(sb_desc.p, d.data(), d.size() * sizeof(StepBoundDesc));
       sync();
     }
-    for (int pass = 0; pass < 2; ++pass) {  // T = W·dM, then G = T·Wᵀ
+    if (kb <= kSmallOrder) {
+      if (sb_list.n < (size_t)n) {
+        sb_list.alloc(n);
+        h2d(sb_list.p, sb_blocks.data(), n * sizeof(int));
+      }
+      block_congruence(d_doff.p, d_dk.p, sb_list.p, n, kb, {{Ws[0], Ws[1]}, {dMs[0], dMs[1]}, {Gs[0], Gs[1]}}, st);
+    }
+    for (int pass = 0; kb > kSmallOrder && pass < 2; ++pass) {  // T = W·dM, then G = T·Wᵀ
       GemmGroups g;
       auto flush = [&]() {
         gemm_f64_grouped(g, false, pass == 0, st);

@@ -189,5 +189,62 @@ __device__ __forceinline__ void factor_tile(double* D, double* inv, int nb, int*
   if (wp < nb - 1) bar_arrive(1 + (wp & 1), 32 * (nb - wp));
 }
 
+// ---- whole k×k matrices (k ≤ 64) by FT threads: column c at c·FLD, padded with the identity
+// to 8·nb rows and columns, nb = ⌈k/8⌉, so the DMMA products need no guards and their
+// fragment reads no bank conflicts.
+
+// S ← G (k×k column-major, global); t: its transpose.  All loads are issued before the
+// first shared store (one memory round trip a matrix).
+__device__ __forceinline__ void cta_load_tile(double* S, const double* G, int k, bool t = false) {
+  const int r = threadIdx.x & 63, cb = threadIdx.x >> 6, k8 = (k + 7) & ~7;
+  double v[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int c = cb + 4 * u;
+    v[u] = (r < k && c < k) ? G[r + c * k] : (r == c ? 1.0 : 0.0);
+  }
+  if (r < k8)
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int c = cb + 4 * u;
+      if (c < k8) S[t ? r * FLD + c : c * FLD + r] = v[u];
+    }
+}
+// f(r, c, Σ_p op(A)(r, p)·B(p, c)) over the 8·nb square, for tiles A, B; ta: A
+// transposed.  first(i), last(i): the range of 8-blocks p that block row i needs (a
+// triangular A).  Each warp takes pairs of 8×8 output blocks of a block row in
+// turn, two chains to cover the pipe's latency.
+enum TileTri { kFull, kLower, kUpper };  // op(A)
+template <bool ta, TileTri tri, class F>
+__device__ __forceinline__ void cta_tile_gemm(const double* A, const double* B, int nb, F f) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int pairs = (nb + 1) / 2;
+  for (int u = warp; u < nb * pairs; u += FT / 32) {
+    const int i = u % nb, c0 = 16 * (u / nb);
+    const bool two = c0 + 8 < 8 * nb;
+    const int p0 = tri == kUpper ? 2 * i : 0, p1 = tri == kLower ? 2 * i + 2 : 2 * nb;
+    double acc[2][2] = {};
+    for (int p = p0; p < p1; ++p) {
+      const int q = 4 * p + t;
+      const double a = ta ? A[(8 * i + g) * FLD + q] : A[q * FLD + 8 * i + g];
+      mma8(acc[0][0], acc[0][1], a, B[(c0 + g) * FLD + q]);
+      if (two) mma8(acc[1][0], acc[1][1], a, B[(c0 + 8 + g) * FLD + q]);
+    }
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (v == 0 || two) f(8 * i + g, c0 + 8 * v + 2 * t + e, acc[v][e]);
+  }
+}
+
+// X⁻¹·B = Wᵀ·(W·B) for W = L_X⁻¹ in a tile: T (scratch) ← W·B, then f of the product.
+template <class F>
+__device__ __forceinline__ void cta_tile_cholsolve(const double* W, const double* B, double* T, int nb, F f) {
+  cta_tile_gemm<false, kLower>(W, B, nb, [&](int r, int c, double v) { T[c * FLD + r] = v; });
+  __syncthreads();
+  cta_tile_gemm<true, kUpper>(W, T, nb, f);
+}
+
 }  // namespace tile64
 }  // namespace sdpx
