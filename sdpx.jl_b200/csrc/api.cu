@@ -498,6 +498,28 @@ struct Handle {
     if (sym) symmetrize(d_doff.p, d_dk.p, (int)dense.size(), kmax, out, st);
   }
 
+  // Whether `bytes` of device memory fit beside `spare`.  Less than kNoQuery always
+  // does: the query costs 100 µs, a tenth of a small model's set-up.
+  static constexpr size_t kNoQuery = 32 << 20;
+  bool room_for(size_t bytes, size_t spare) {
+    if (bytes <= kNoQuery) return true;
+    size_t freeb = 0, totb = 0;
+    SDPX_CUDA(cudaMemGetInfo(&freeb, &totb));
+    return bytes + spare <= freeb + dcache::idle_bytes(dev);  // idle cached blocks are ours to reuse
+  }
+  void zero_vectors(std::initializer_list<DBuf<double>*> list) {
+    ZeroList q;
+    for (auto* b : list) {
+      q.p[q.n] = b->p;
+      q.len[q.n++] = (long long)b->n;
+      if (q.n == kZeroMax) {
+        zero_list(q, st);
+        q.n = 0;
+      }
+    }
+    zero_list(q, st);
+  }
+
   void ensure_descs(size_t n) {
     if (n <= desc_cap) return;
     desc_cap = std::max<size_t>(n, 2 * desc_cap);
@@ -659,9 +681,11 @@ struct Handle {
 
     // Workspaces.
     for (auto* b : {&x, &dx, &d, &v, &r, &rho, &work_m, &work_m2, &xbest, &keptx, &dxbest})
-      b->alloc(m), b->zero(st);
+      b->alloc(m);
     for (auto* b : {&X, &Y, &P, &R, &Z, &dX, &dY, &LX, &MY, &W, &WY, &T1, &T2, &Xbest, &Ybest, &tmpK2})
-      b->alloc(K), b->zero(st);
+      b->alloc(K);
+    zero_vectors({&x, &dx, &d, &v, &r, &rho, &work_m, &work_m2, &xbest, &keptx, &dxbest, &X, &Y, &P, &R, &Z, &dX, &dY,
+                  &LX, &MY, &W, &WY, &T1, &T2, &Xbest, &Ybest, &tmpK2});
     oz_err.alloc(1);
     oz_err.zero(st);
     gemv_chunks = std::max(1, std::min(16, m / 64));
@@ -687,11 +711,8 @@ struct Handle {
       }
       // The copy is an accelerator: it is made only when it fits beside 4 GB of
       // headroom (the solve's remaining buffers are allocated later).
-      size_t freeb = 0, totb = 0;
-      SDPX_CUDA(cudaMemGetInfo(&freeb, &totb));
-      freeb += dcache::idle_bytes(dev);
       const size_t apb = sizeof(double) * (size_t)std::max<long long>(Kt, 1) * m;
-      use_packed = apb + (4ull << 30) <= freeb;
+      use_packed = room_for(apb, 4ull << 30);
       if (use_packed) Ap.alloc((size_t)std::max<long long>(Kt, 1) * m);
       kt_fold.alloc(std::max<long long>(Kt, 1));
       adx.alloc(K);
@@ -946,10 +967,8 @@ struct Handle {
   void get_stacked(const double* dev_src, double* host_dst) { get_vectors({}, {{dev_src, host_dst}}); }
   void fixed_start(double wp, double wd) {
     iterate_changed();
-    x.zero(st);
+    zero_vectors({&x, &X, &Y});
     if (n_eq) yv.zero(st);
-    X.zero(st);
-    Y.zero(st);
     if (!dense.empty()) {
       add_diag(d_doff.p, d_dk.p, (int)dense.size(), kmax, X.p, nullptr, wp, st);
       add_diag(d_doff.p, d_dk.p, (int)dense.size(), kmax, Y.p, nullptr, wd, st);
@@ -1093,12 +1112,9 @@ struct Handle {
       }
       // Room for the cached constraint digits, the per-build scratch and the
       // Gram's digit planes (same size as the FP64 panel), with 2 GB to spare.
-      size_t freeb = 0, totb = 0;
-      SDPX_CUDA(cudaMemGetInfo(&freeb, &totb));
-      freeb += dcache::idle_bytes(dev);  // idle cached blocks are ours to reuse
       const size_t gram = oz_plan.m == m && oz_plan.K == K ? 0 : (size_t)OZ_DIGITS * m * (K + 64);
       const size_t need = adig + tdig + wdig + 4 * (size_t)(aexp + texp + wexp) + gram;
-      if (dense.empty() || !fits_int || need + (2ull << 30) > freeb) {
+      if (dense.empty() || !fits_int || !room_for(need, 2ull << 30)) {
         oz_blk_state = -1;
       } else {
         oz_adig.alloc(adig);

@@ -509,6 +509,20 @@ void scale(long long n, double* x, double f, cudaStream_t st) {
   SDPX_LAUNCH_CHECK();
 }
 
+__global__ void k_zero_list(const __grid_constant__ ZeroList q) {
+  double* p = q.p[blockIdx.y];
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < q.len[blockIdx.y];
+       e += (long long)gridDim.x * blockDim.x)
+    p[e] = 0.0;
+}
+void zero_list(const ZeroList& q, cudaStream_t st) {
+  long long most = 0;
+  for (int i = 0; i < q.n; ++i) most = std::max(most, q.len[i]);
+  if (most == 0) return;
+  k_zero_list<<<dim3(std::min(256, ceil_div(most, 256)), q.n), 256, 0, st>>>(q);
+  SDPX_LAUNCH_CHECK();
+}
+
 // ----------------------------------------------------------- reductions ----
 // out[slot] = max(out[slot], max|x|) ; finiteness folded in (NaN → +inf).
 __global__ void k_absmax(long long n, const double* x, double* out) {

@@ -45,6 +45,14 @@ void axpbypcz(long long n, double a, const double* x, double b, const double* y,
               const double* z, double* out, cudaStream_t st);
 void combine(long long n, double* x, double t, const double* d, cudaStream_t st);
 void scale(long long n, double* x, double f, cudaStream_t st);
+// Several vectors set to zero by one launch.
+constexpr int kZeroMax = 32;
+struct ZeroList {
+  int n = 0;
+  double* p[kZeroMax];
+  long long len[kZeroMax];
+};
+void zero_list(const ZeroList& q, cudaStream_t st);
 void absmax(long long n, const double* x, double* out, cudaStream_t st);
 // out[e] = max|x_e| of every entry (NaN counts as +inf), one launch; `out` may be pinned
 // host memory.  `work` is zero between launches and belongs to one stream.
