@@ -242,10 +242,7 @@ struct Handle {
   FlowFlags flow_flags;  // tile flags of the Cholesky launches
   size_t desc_cap = 0;
   DBuf<double> trials;
-  DBuf<long long> d_trial_off;
-  DBuf<double> d_tcand;
   DBuf<TrialDesc> d_trial_desc;
-  DBuf<int> d_fail;
   std::vector<double> lx_dmin, lx_dmax, my_dmin, my_dmax;
   bool diag_factor_ok = true;
 
@@ -747,8 +744,6 @@ struct Handle {
     norm_work.alloc(1);
     norm_work.zero(st);
     ensure_descs(std::max<size_t>(16, 2 * dense.size()));
-    d_fail.alloc(64);
-    d_tcand.alloc(64);
     // Gershgorin scratch
     std::vector<long long> coff(dense.size());
     long long tot = 0;
@@ -1778,71 +1773,15 @@ struct Handle {
     return lo;
   }
 
-  // PD(+margin) tests of X_b + t·dX_b for every dense block with k > 2 and
-  // every candidate t; returns pass[cand] (all blocks pass).
-  std::vector<char> dense_trials(const double* M, const double* dM, const std::vector<double>& t,
-                                 double ratio) {
-    std::vector<char> pass(t.size(), 1);
-    std::vector<int> idx;
-    for (size_t b = 0; b < dense.size(); ++b)
-      if (dense[b].k > 2) idx.push_back((int)b);
-    if (idx.empty() || t.empty()) return pass;
-    // trial buffer: per block, |t| matrices
-    std::vector<long long> toff(dense.size(), 0);
-    long long need = 0;
-    for (size_t b = 0; b < dense.size(); ++b)
-      toff[b] = need, need += (long long)t.size() * dense[b].k * dense[b].k;
-    if ((size_t)need > trials.n) trials.alloc(need);
-    if (d_trial_off.n < dense.size()) d_trial_off.alloc(dense.size());
-    h2d(d_trial_off.p, toff.data(), dense.size() * sizeof(long long));
-    if (d_tcand.n < t.size()) d_tcand.alloc(t.size());
-    h2d(d_tcand.p, t.data(), t.size() * sizeof(double));
-    make_trials(d_doff.p, d_dk.p, d_trial_off.p, (int)dense.size(), kmax, M, dM, d_tcand.p,
-                (int)t.size(), trials.p, st);
-    // (blocks with k ≤ 2 also get trial copies above; they are ignored here)
-    std::vector<MatDesc<double>> mats;
-    for (int b : idx)
-      for (size_t c2 = 0; c2 < t.size(); ++c2)
-        mats.push_back({trials.p + toff[b] + (long long)c2 * dense[b].k * dense[b].k, dense[b].k,
-                        dense[b].k});
-    std::vector<int> info;
-    std::vector<double> dmn, dmx;
-    potrf_host_list(mats, info, dmn, dmx, false);
-    size_t q = 0;
-    for (size_t bi = 0; bi < idx.size(); ++bi)
-      for (size_t c2 = 0; c2 < t.size(); ++c2, ++q) {
-        bool ok = info[q] == 0;
-        if (ok && ratio > 0)
-          ok = std::isfinite(dmn[q]) && std::isfinite(dmx[q]) && dmx[q] > 0 && dmn[q] > ratio * dmx[q];
-        if (!ok) pass[c2] = 0;
-      }
-    return pass;
-  }
-  std::vector<char> diag_trials(const double* M, const double* dM, const std::vector<double>& t,
-                                double ratio) {
-    std::vector<char> pass(t.size(), 1);
-    if (!nd || t.empty()) return pass;
-    if (d_tcand.n < t.size()) d_tcand.alloc(t.size());
-    if (d_fail.n < t.size()) d_fail.alloc(t.size());
-    h2d(d_tcand.p, t.data(), t.size() * sizeof(double));
-    SDPX_CUDA(cudaMemsetAsync(d_fail.p, 0, t.size() * sizeof(int), st));
-    diag_trial(nd, od, M, dM, d_tcand.p, (int)t.size(), ratio > 0 ? 1 : 0, d_fail.p, st);
-    std::vector<int> f(t.size());
-    d2h(f.data(), d_fail.p, t.size() * sizeof(int));
-    sync();
-    for (size_t c2 = 0; c2 < t.size(); ++c2) pass[c2] = f[c2] == 0;
-    return pass;
-  }
-  std::vector<char> all_trials(const double* M, const double* dM, const std::vector<double>& t,
-                               double ratio, const std::vector<Small2>& k2) {
-    auto p1 = dense_trials(M, dM, t, ratio);
-    auto p2 = diag_trials(M, dM, t, ratio);
-    for (size_t c2 = 0; c2 < t.size(); ++c2) {
-      bool ok = p1[c2] && p2[c2];
-      for (auto& s : k2) ok = ok && margin2(s, t[c2], ratio);
-      p1[c2] = ok;
-    }
-    return p1;
+  // Trials of the 1×1 group on one side: fail flags in h_diag_fail(side) after the next
+  // sync.
+  int* h_diag_fail(int side) { return reinterpret_cast<int*>(h_red + 16) + side * kDiagSteps; }
+  void launch_diag_trials(int side, const double* M, const double* dM, const std::vector<double>& t, double ratio) {
+    DiagSteps q;
+    q.n = (int)t.size();
+    std::copy(t.begin(), t.end(), q.t);
+    std::fill(h_diag_fail(side), h_diag_fail(side) + q.n, 0);  // (idle since the last sync)
+    diag_trial(nd, od, M, dM, q, ratio > 0 ? 1 : 0, h_diag_fail(side), st);
   }
 
   // One trial matrix  out = M_b + t·dM_b  of dense block b (side-specific M, dM).
@@ -2112,6 +2051,7 @@ struct Handle {
     double result[2] = {1.0, 1.0};
     bool done[2] = {false, false};
     constexpr int J = 8;
+    static_assert(J <= kDiagSteps, "flags of a side");
     while (!(done[0] && done[1])) {
       std::vector<double> cand[2];
       for (int side = 0; side < 2; ++side) {
@@ -2133,7 +2073,10 @@ struct Handle {
           for (double t : cand[side]) reqs.push_back({Ms[side], dMs[side], b, t});
       std::vector<int> info;
       std::vector<double> dmn, dmx;
+      for (int side = 0; side < 2; ++side)  // ahead of the dense ones, whose wait covers them
+        if (!done[side]) launch_diag_trials(side, Ms[side], dMs[side], cand[side], margin);
       run_trials(reqs, info, dmn, dmx);
+      if (reqs.empty()) sync();
       size_t q = 0;
       for (int side = 0; side < 2; ++side) {
         if (done[side]) continue;
@@ -2146,9 +2089,9 @@ struct Handle {
                    dmn[q] > margin * dmx[q];
             if (!ok) pass[c2] = 0;
           }
-        auto pd = diag_trials(Ms[side], dMs[side], cand[side], margin);
+        const int* diag_fail = h_diag_fail(side);
         for (size_t c2 = 0; c2 < cand[side].size(); ++c2) {
-          bool ok = pass[c2] && pd[c2];
+          bool ok = pass[c2] && diag_fail[c2] == 0;
           for (auto& s2 : k2[side]) ok = ok && margin2(s2, cand[side][c2], margin);
           if (ok || cand[side][c2] < min_step) {
             result[side] = cand[side][c2];

@@ -871,24 +871,24 @@ void diag_panel(long long K, int m, int nd, long long od, const double* A, const
 }
 
 // ----------------------------------------------------- line-search trials ---
-// 1×1 group: for candidate steps t[c] (c < nc), ok[c] &= (X + t dX > 0 && finite...).
-// Returns for each candidate whether all entries pass.  margin>0 additionally
-// requires a finite square root (SDPX's 1×1 `trial_has_cholesky_margin!`).
+// 1×1 group: for candidate steps t[c] (c < n), fail[c] = 1 unless X + t dX > 0 in every entry.
+// margin > 0 additionally requires a finite square root (SDPX's 1×1
+// `trial_has_cholesky_margin!`).
 __global__ void k_diag_trial(int nd, long long od, const double* X, const double* dX,
-                             const double* t, int nc, int margin, int* fail) {
+                             const __grid_constant__ DiagSteps q, int margin, int* fail) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int c = blockIdx.y;
-  if (j >= nd || c >= nc) return;
+  if (j >= nd) return;
   long long e = od + j;
-  double v = X[e] + t[c] * dX[e];
+  double v = X[e] + q.t[c] * dX[e];
   bool ok = v > 0;
   if (ok && margin) ok = isfinite(sqrt(v));
-  if (!ok) atomicExch(fail + c, 1);
+  if (!ok) fail[c] = 1;
 }
-void diag_trial(int nd, long long od, const double* X, const double* dX, const double* d_t, int nc,
-                int margin, int* d_fail, cudaStream_t st) {
-  if (nd == 0 || nc == 0) return;
-  k_diag_trial<<<dim3(ceil_div(nd, 256), nc), 256, 0, st>>>(nd, od, X, dX, d_t, nc, margin, d_fail);
+void diag_trial(int nd, long long od, const double* X, const double* dX, const DiagSteps& q, int margin, int* fail,
+                cudaStream_t st) {
+  if (nd == 0 || q.n == 0) return;
+  k_diag_trial<<<dim3(ceil_div(nd, 256), q.n), 256, 0, st>>>(nd, od, X, dX, q, margin, fail);
   SDPX_LAUNCH_CHECK();
 }
 
@@ -909,32 +909,6 @@ void diag_ftb(int nd, long long od, const double* X, const double* dX, double* d
               cudaStream_t st) {
   if (nd == 0) return;
   k_diag_ftb<<<1, 1024, 0, st>>>(nd, od, X, dX, d_out);
-  SDPX_LAUNCH_CHECK();
-}
-
-// Trial matrices  T[c] = X_block + t[c]·dX_block  for every dense block and candidate.
-__global__ void k_make_trials(const long long* off, const int* kk, const long long* trial_off,
-                              int nseg, const double* X, const double* dX, const double* t, int nc,
-                              double* trials) {
-  int s = blockIdx.y, c = blockIdx.z;
-  if (s >= nseg || c >= nc) return;
-  int k = kk[s];
-  long long tot = (long long)k * k;
-  double tc = t[c];
-  double* out = trials + trial_off[s] + (long long)c * tot;
-  const double* x = X + off[s];
-  const double* d = dX + off[s];
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-       e += (long long)gridDim.x * blockDim.x)
-    out[e] = x[e] + tc * d[e];
-}
-void make_trials(const long long* d_off, const int* d_k, const long long* d_trial_off, int nseg,
-                 int kmax, const double* X, const double* dX, const double* d_t, int nc,
-                 double* trials, cudaStream_t st) {
-  if (nseg == 0 || nc == 0) return;
-  int g = std::max(1, std::min(256, ceil_div((long long)kmax * kmax, 256)));
-  k_make_trials<<<dim3(g, nseg, nc), 256, 0, st>>>(d_off, d_k, d_trial_off, nseg, X, dX, d_t, nc,
-                                                  trials);
   SDPX_LAUNCH_CHECK();
 }
 

@@ -108,13 +108,16 @@ void diag_corrector_R(int nd, long long od, const double* X, const double* Y, co
                       cudaStream_t st);
 void diag_panel(long long K, int m, int nd, long long od, const double* A, const double* LX,
                 const double* MY, double* Pc, cudaStream_t st);
-void diag_trial(int nd, long long od, const double* X, const double* dX, const double* d_t, int nc,
-                int margin, int* d_fail, cudaStream_t st);
+constexpr int kDiagSteps = 16;
+struct DiagSteps {
+  int n = 0;
+  double t[kDiagSteps];
+};
+// (fail may be pinned host memory; zero on entry.)
+void diag_trial(int nd, long long od, const double* X, const double* dX, const DiagSteps& q, int margin, int* fail,
+                cudaStream_t st);
 void diag_ftb(int nd, long long od, const double* X, const double* dX, double* d_out,
               cudaStream_t st);
-void make_trials(const long long* d_off, const int* d_k, const long long* d_trial_off, int nseg,
-                 int kmax, const double* X, const double* dX, const double* d_t, int nc,
-                 double* trials, cudaStream_t st);
 void gather(long long n, const long long* map, const double* src, double* dst, cudaStream_t st);
 void scatter(long long n, const long long* map, const double* src, double* dst, cudaStream_t st);
 void mirror_lower(int m, double* S, cudaStream_t st);
