@@ -914,10 +914,10 @@ struct Handle {
   }
   // Results of at most kStageBytes are written by the kernels into pinned memory and
   // copied out by the host: a copy to the caller's (pageable) memory of 320 KB, the size
-  // of one k = 200 matrix, took 150 µs of driver staging, this 90 (most of it
-  // the first touch of new pages).  Larger ones
-  // would spend on pinning the buffer what they save.
-  static constexpr size_t kStageBytes = 4 << 20;
+  // of one k = 200 matrix, took 150 µs of driver staging, this 90 (most of it the first
+  // touch of new pages).  Larger ones would save 0.2 ms a call and cost the first call of a
+  // handle 4 to 20 ms for pinning 3 MB.
+  static constexpr size_t kStageBytes = 1 << 20;
   struct VectorOut {  // n doubles as they are
     const double* src;
     double* dst;
