@@ -414,7 +414,8 @@ int sdpx_b200_kernel_times(sdpx_b200_handle* h, double* ms4);
 /* Device memory (no counterpart in the reference): buffers released by
  * destroyed handles stay cached in this process for reuse by later handles
  * (allocation and release cost ≈ 1.8 and 2.9 ms per GB on the B200; a handle of
- * the m = 2000 workload holds ≈ 25 GB).  This call returns every idle cached
+ * the m = 2000 workload holds ≈ 25 GB), and so do up to 16 MB of pinned host
+ * buffers (1 to 3 ms to pin and unpin one).  This call returns every idle cached
  * block to the driver.  Always 0. */
 int sdpx_b200_trim_device_cache(void);
 

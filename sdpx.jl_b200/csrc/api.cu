@@ -296,7 +296,11 @@ struct Handle {
   ~Handle() {
     // All of the handle's device work runs on st: once st is idle its buffers
     // can return to the cache without a device-wide synchronisation.
-    if (st && cudaStreamSynchronize(st) == cudaSuccess) release_scope.begin();
+    if (st && cudaStreamSynchronize(st) == cudaSuccess) {
+      release_scope.begin();
+      red_buf.release();
+      pin_buf.release();
+    }
     for (auto& row : kt_ev)
       for (auto e : row)
         if (e) cudaEventDestroy(e);
@@ -305,8 +309,6 @@ struct Handle {
       cudaEventDestroy(p.b);
     }
     for (auto e : ev_pool) cudaEventDestroy(e);
-    if (h_red) cudaFreeHost(h_red);
-    if (h_pin) cudaFreeHost(h_pin);
     mixed.reset();
     if (st) cudaStreamDestroy(st);
   }
@@ -524,17 +526,13 @@ struct Handle {
   }
   // Pinned staging: descriptor lists to upload, and results that kernels write
   // directly (no copy back).  Only grown right after a sync.
-  unsigned char* h_pin = nullptr;
-  size_t pin_cap = 0;
+  PinnedBuf red_buf, pin_buf;  // red_buf: h_red's
   unsigned char* pinned(size_t bytes) {
-    if (bytes > pin_cap) {
+    if (bytes > pin_buf.bytes) {
       sync();
-      if (h_pin) cudaFreeHost(h_pin);
-      h_pin = nullptr;
-      pin_cap = std::max<size_t>(bytes, 2 * pin_cap);
-      SDPX_CUDA(cudaMallocHost(&h_pin, pin_cap));
+      pin_buf.alloc(std::max<size_t>(bytes, 2 * pin_buf.bytes));
     }
-    return h_pin;
+    return pin_buf.p;
   }
 
   // Batched Cholesky of host-described matrices; fills info/dmin/dmax (host).
@@ -722,7 +720,8 @@ struct Handle {
     syrk = plan_syrk_f64(m, K, sms);
     partial.alloc(syrk.partial_doubles);
     red.alloc(64);
-    SDPX_CUDA(cudaMallocHost(&h_red, 64 * sizeof(double)));
+    red_buf.alloc(64 * sizeof(double));
+    h_red = reinterpret_cast<double*>(red_buf.p);
     mu_user.alloc(L);
     target_user.alloc(L);
     work_L.alloc(2 * std::max<size_t>((size_t)L, dense.size()) + 2);
@@ -3080,6 +3079,7 @@ int sdpx_b200_counters(sdpx_b200_handle* h, int64_t* out4) {
 int sdpx_b200_get_stream(sdpx_b200_handle* h, void** stream) { GUARD(h, *stream = (void*)h->h.st); }
 int sdpx_b200_trim_device_cache(void) {
   sdpx::dcache::trim(-1);
+  sdpx::hcache::trim();
   return 0;
 }
 int sdpx_b200_launch_count(uint64_t* count) {

@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -134,6 +135,94 @@ struct ReleaseScope {
 };
 
 }  // namespace dcache
+
+// Pinned host blocks, cached the same way: pinning and unpinning a few hundred KB takes
+// 1 to 3 ms, several times what a handle's small call does.  Sizes are powers of two, so
+// that blocks of ended handles fit new ones; at most kIdleCap bytes stay idle, for any
+// device (portable memory).  A block comes back when its owner's stream is idle, and is
+// handed out zeroed.
+namespace hcache {
+
+constexpr size_t kIdleCap = 16ull << 20;
+
+struct Cache {
+  std::mutex mu;
+  std::multimap<size_t, void*> idle;
+  size_t idle_bytes = 0;
+};
+inline Cache& cache() {
+  static Cache c;
+  return c;
+}
+
+inline void trim() {
+  Cache& c = cache();
+  std::lock_guard<std::mutex> g(c.mu);
+  for (auto& b : c.idle) cudaFreeHost(b.second);
+  c.idle.clear();
+  c.idle_bytes = 0;
+}
+
+inline void* get(size_t bytes, size_t* got) {
+  size_t size = 4096;
+  while (size < bytes) size *= 2;
+  *got = size;
+  Cache& c = cache();
+  void* p = nullptr;
+  {
+    std::lock_guard<std::mutex> g(c.mu);
+    const auto it = c.idle.find(size);
+    if (it != c.idle.end()) {
+      p = it->second;
+      c.idle.erase(it);
+      c.idle_bytes -= size;
+    }
+  }
+  if (!p && cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    trim();
+    SDPX_CUDA(cudaHostAlloc(&p, size, cudaHostAllocPortable));
+  }
+  std::memset(p, 0, size);
+  return p;
+}
+
+inline void put(void* p, size_t size) {
+  Cache& c = cache();
+  {
+    std::lock_guard<std::mutex> g(c.mu);
+    if (c.idle_bytes + size <= kIdleCap) {
+      c.idle.insert({size, p});
+      c.idle_bytes += size;
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
+}  // namespace hcache
+
+// Owning pinned buffer.  release(): no queued work uses it any more; without a release the
+// destructor (a failed stream) gives the memory back to the driver.
+struct PinnedBuf {
+  unsigned char* p = nullptr;
+  size_t bytes = 0;
+  void alloc(size_t count) {
+    release();
+    p = static_cast<unsigned char*>(hcache::get(count, &bytes));
+  }
+  void release() {
+    if (p) hcache::put(p, bytes);
+    p = nullptr;
+    bytes = 0;
+  }
+  PinnedBuf() = default;
+  PinnedBuf(const PinnedBuf&) = delete;
+  PinnedBuf& operator=(const PinnedBuf&) = delete;
+  ~PinnedBuf() {
+    if (p) cudaFreeHost(p);
+  }
+};
 
 template <class T>
 struct DBuf {
