@@ -1101,18 +1101,25 @@ WorkKernel syrk_kernel(int threads, int tile) {
 // ---------------------------------------------------------------------------
 // Host side.
 
+// Blocks of at most kKeep bytes come from and go back to the pinned cache (grown and
+// released with no work of the stream in flight on them); the upload staging does not.
 struct Pinned {
+  static constexpr size_t kKeep = 4 << 20;
   void* p = nullptr;
   size_t bytes = 0;
   void ensure(size_t b) {
     if (b <= bytes) return;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
+    release();
+    if (b <= kKeep) {
+      p = hcache::get(b, &bytes);
+      return;
+    }
     SDPX_CUDA(cudaHostAlloc(&p, b, cudaHostAllocDefault));
     bytes = b;
   }
   void release() {
-    if (p) cudaFreeHost(p);
+    if (p && bytes <= kKeep) hcache::put(p, bytes);
+    else if (p) cudaFreeHost(p);
     p = nullptr;
     bytes = 0;
   }
