@@ -32,7 +32,8 @@ using CfgTnKM = F64Cfg<32, 32, 2, 2, true, false>;
 // over row tiles), so CTAs sharing a tile of the larger operand run together.
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::NT) k_gemm(Opnd A, Opnd B, OutDesc C, double alpha,
-                                                  double beta, int mode, int rows_fast) {
+                                                  double beta, int mode, int rows_fast,
+                                                  const double* cin) {
   extern __shared__ __align__(16) double smem[];
   const int n0 = (rows_fast ? blockIdx.y : blockIdx.x) * Cfg::BN;
   const int m0 = (rows_fast ? blockIdx.x : blockIdx.y) * Cfg::BM;
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(Cfg::NT) k_gemm(Opnd A, Opnd B, OutDesc C, dou
   double acc[Cfg::FM][Cfg::FN][2];
   zero_acc<Cfg>(acc);
   f64_tile_mainloop<Cfg>(acc, A, B, m0, n0, kb, ke, smem);
-  store_acc<Cfg>(acc, C, m0, n0, alpha, beta);
+  store_acc<Cfg>(acc, C, m0, n0, alpha, beta, cin);
 }
 
 // Grouped products: CTA b belongs to the group whose tile range holds it
@@ -144,14 +145,14 @@ static int gemm_sm_count() {
 
 template <class Cfg>
 static void launch_gemm_cfg(const Opnd& A, const Opnd& B, const OutDesc& C, double alpha,
-                            double beta, int mode, cudaStream_t st) {
+                            double beta, int mode, cudaStream_t st, const double* cin) {
   ensure_smem(k_gemm<Cfg>, Cfg::SMEM_BYTES);
   const int tr = ceil_div(C.rows, Cfg::BM), tc = ceil_div(C.cols, Cfg::BN);
   if (tr == 0 || tc == 0) return;
   const int rows_fast = (tr < tc && tc <= 65535) ? 1 : 0;  // grid.y is limited to 65535
   if (!rows_fast && tr > 65535) throw std::invalid_argument("gemm_f64: too many row tiles");
   dim3 grid(rows_fast ? tr : tc, rows_fast ? tc : tr);
-  k_gemm<Cfg><<<grid, Cfg::NT, Cfg::SMEM_BYTES, st>>>(A, B, C, alpha, beta, mode, rows_fast);
+  k_gemm<Cfg><<<grid, Cfg::NT, Cfg::SMEM_BYTES, st>>>(A, B, C, alpha, beta, mode, rows_fast, cin);
   SDPX_LAUNCH_CHECK();
 }
 
@@ -183,7 +184,7 @@ void gemm_f64_grouped(const GemmGroups& g, bool a_kcontig, bool b_kcontig, cudaS
   if (!tiny) {  // mixed shapes: one launch per product, as gemm_f64
     for (int q = 0; q < g.n; ++q)
       gemm_f64(g.A[q], a_kcontig, g.B[q], b_kcontig, g.C[q], g.alpha[q], g.beta[q], g.mode[q], false,
-               st);
+               st, g.Cin[q]);
     return;
   }
   if (!a_kcontig && b_kcontig) return launch_gemm_grouped<CfgTnMK>(g, st);
@@ -193,19 +194,19 @@ void gemm_f64_grouped(const GemmGroups& g, bool a_kcontig, bool b_kcontig, cudaS
 }
 
 void gemm_f64(const Opnd& A, bool a_kcontig, const Opnd& B, bool b_kcontig, const OutDesc& C,
-              double alpha, double beta, int mode, bool big, cudaStream_t st) {
-  if (big && !a_kcontig && b_kcontig) return launch_gemm_cfg<CfgBigMK>(A, B, C, alpha, beta, mode, st);
-  if (big && a_kcontig && b_kcontig) return launch_gemm_cfg<CfgBigKT>(A, B, C, alpha, beta, mode, st);
+              double alpha, double beta, int mode, bool big, cudaStream_t st, const double* cin) {
+  if (big && !a_kcontig && b_kcontig) return launch_gemm_cfg<CfgBigMK>(A, B, C, alpha, beta, mode, st, cin);
+  if (big && a_kcontig && b_kcontig) return launch_gemm_cfg<CfgBigKT>(A, B, C, alpha, beta, mode, st, cin);
   if (!big && (long long)ceil_div(C.rows, 64) * ceil_div(C.cols, 64) < gemm_sm_count()) {
-    if (!a_kcontig && b_kcontig) return launch_gemm_cfg<CfgTnMK>(A, B, C, alpha, beta, mode, st);
-    if (a_kcontig && b_kcontig) return launch_gemm_cfg<CfgTnKK>(A, B, C, alpha, beta, mode, st);
-    if (!a_kcontig && !b_kcontig) return launch_gemm_cfg<CfgTnMM>(A, B, C, alpha, beta, mode, st);
-    return launch_gemm_cfg<CfgTnKM>(A, B, C, alpha, beta, mode, st);
+    if (!a_kcontig && b_kcontig) return launch_gemm_cfg<CfgTnMK>(A, B, C, alpha, beta, mode, st, cin);
+    if (a_kcontig && b_kcontig) return launch_gemm_cfg<CfgTnKK>(A, B, C, alpha, beta, mode, st, cin);
+    if (!a_kcontig && !b_kcontig) return launch_gemm_cfg<CfgTnMM>(A, B, C, alpha, beta, mode, st, cin);
+    return launch_gemm_cfg<CfgTnKM>(A, B, C, alpha, beta, mode, st, cin);
   }
-  if (!a_kcontig && b_kcontig) return launch_gemm_cfg<CfgSmMK>(A, B, C, alpha, beta, mode, st);
-  if (a_kcontig && b_kcontig) return launch_gemm_cfg<CfgSmKK>(A, B, C, alpha, beta, mode, st);
-  if (!a_kcontig && !b_kcontig) return launch_gemm_cfg<CfgSmMM>(A, B, C, alpha, beta, mode, st);
-  return launch_gemm_cfg<CfgSmKM>(A, B, C, alpha, beta, mode, st);
+  if (!a_kcontig && b_kcontig) return launch_gemm_cfg<CfgSmMK>(A, B, C, alpha, beta, mode, st, cin);
+  if (a_kcontig && b_kcontig) return launch_gemm_cfg<CfgSmKK>(A, B, C, alpha, beta, mode, st, cin);
+  if (!a_kcontig && !b_kcontig) return launch_gemm_cfg<CfgSmMM>(A, B, C, alpha, beta, mode, st, cin);
+  return launch_gemm_cfg<CfgSmKM>(A, B, C, alpha, beta, mode, st, cin);
 }
 
 void trmm_right_lower_inplace_f64(const Opnd& T, const Opnd& L, const OutDesc& C, cudaStream_t st) {

@@ -7,10 +7,12 @@
 
 namespace sdpx {
 
-// C = alpha·A·B + beta·C over the K range selected by `mode` (KRange).
+// C = alpha·A·B + beta·C over the K range selected by `mode` (KRange), or + beta·cin (C's
+// layout) where it is given.
 // a_kcontig / b_kcontig state which index of each operand is contiguous.
 void gemm_f64(const Opnd& A, bool a_kcontig, const Opnd& B, bool b_kcontig, const OutDesc& C,
-              double alpha, double beta, int mode, bool big, cudaStream_t st);
+              double alpha, double beta, int mode, bool big, cudaStream_t st,
+              const double* cin = nullptr);
 
 // Up to kGemmGroups independent products C_g = alpha_g·A_g·B_g + beta_g·C_g
 // (K range mode_g each, the same operand contiguity for all) in one launch:
