@@ -59,7 +59,9 @@ __device__ __forceinline__ bool barrier_done(unsigned mbar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
+// (The .aligned forms take whole warps: lanes may come from loops of different lengths.)
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
@@ -270,6 +272,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_step_bound_regs(const StepBoundD
           break;
         }
       }
+      __syncwarp();
       if (lockstep) cluster_sync();
     } else {
       if (lane < N && sr < k) ex[b][sr] = make_double2(pr, cv);
@@ -397,6 +400,7 @@ __global__ void __launch_bounds__(32 * (kRowWarps + 1), 1) k_step_bound_wide(con
       }
     for (int j = 0; j + 2 < k; ++j) {
       const int b = j & 1;
+      __syncwarp();
       tile64::bar_sync(1, BT);  // the vectors of reflection j are there
       const double *u = U[b], *v = U[b ^ 1];
       double s[RPW] = {};
@@ -495,6 +499,7 @@ __global__ void __launch_bounds__(32 * (kRowWarps + 1), 1) k_step_bound_wide(con
     }
     for (int j = 0; j + 2 < k; ++j) {
       const int b = j & 1;
+      __syncwarp();
       tile64::bar_sync(1, BT);
       if (lane == 0)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar[b]), "r"(16 * k) : "memory");

@@ -1,0 +1,62 @@
+"""The eigenvalue step bounds (csrc/step_bound.cu) of lists that hold a matrix with fewer
+rows than its cluster has warps (such a cluster runs its reflections in lockstep), for
+every cluster shape (largest order up to 32, 64, 128, 224, 448), and where the whole step
+stays inside.
+
+G = L⁻¹·dM·L⁻ᵀ is formed with errors of a few k·eps·κ(M), κ = 100, relative to its norm,
+which is within 1e3 of |λ_min| for these directions."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+
+
+def _direction(ks, seed, scale_Y=1.0):
+    from sdpx_b200.cuda_backend import CudaBackend
+    from sdpx_b200.problem import ingest
+    rng = np.random.default_rng(seed)
+
+    def spd(k):
+        q, _ = np.linalg.qr(rng.standard_normal((k, k)))
+        x = (q * np.logspace(-1, 1, k)) @ q.T
+        return 0.5 * (x + x.T)
+    A = [rng.standard_normal((3, k, k)) for k in ks]
+    A = [a + a.transpose(0, 2, 1) for a in A]
+    X, Y = [spd(k) for k in ks], [scale_Y * spd(k) for k in ks]
+    be = CudaBackend(ingest(rng.standard_normal(3), A, [np.eye(k) for k in ks]))
+    be.set_iterate(np.zeros(3), X, Y)
+    assert be.compute_residuals([0.0] * len(ks), True, True)[2]
+    be.schur_build()
+    assert be.factorize()["ok"]
+    be.predictor_rhs()
+    be.solve_direction()
+    be.direction_blocks()
+    return be, X, Y
+
+
+def _exact(M, dM):
+    t = 1.0
+    for a, da in zip(M, dM):
+        W = np.linalg.inv(np.linalg.cholesky(a))
+        low = np.linalg.eigvalsh(W @ da @ W.T)[0]
+        t = min(t, -1.0 / low) if low < -1.0 else t
+    return t
+
+
+# (32: one CTA, no cluster) 4 CTAs of 4 warps beside orders below 16; 8 of 4 below 32; 16
+# of 4 below 64; 16 CTAs below 16; the smallest order beside each
+@pytest.mark.parametrize("ks", [[32, 3], [64, 15, 3], [61, 16], [128, 31, 7], [100, 3], [200, 40], [224, 63, 3],
+                                [300, 15], [448, 3, 16]])
+def test_small_orders_beside_large_ones(ks):
+    be, X, Y = _direction(ks, sum(ks))
+    with be:
+        _, dX, dY = be.get_direction()
+        p = be.affine_diagnostics(True)
+        for got, M, dM in ((p["tX"], X, dX), (p["tY"], Y, dY)):
+            want = _exact(M, dM)
+            assert abs(got - want) <= 4 * max(ks) * EPS * 1e2 * 1e3 * want
+        for _ in range(3):
+            q = be.affine_diagnostics(True)
+            assert (q["tX"], q["tY"]) == (p["tX"], p["tY"])
