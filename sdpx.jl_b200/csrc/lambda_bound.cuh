@@ -72,7 +72,10 @@ __device__ __forceinline__ double bound_from_below(double l) {
 __device__ __forceinline__ double lambda_bound_64(double* G, int k, LambdaScratch& s, int tid, int bar) {
   constexpr int LD = tile64::FLD;
   const int lane = tid & 31, r = tid >> 1, q = tid & 1;
-  auto sync = [&]() { tile64::bar_sync(bar, 128); };
+  auto sync = [&]() {
+    __syncwarp();
+    tile64::bar_sync(bar, 128);
+  };
   if (tid < k) {
     s.col[0][tid] = G[tid];
     s.v[tid] = s.w[tid] = 0.0;

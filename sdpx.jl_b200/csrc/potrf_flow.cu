@@ -49,9 +49,11 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-// Barrier of the computing threads that also returns whether ok held in all.
+// Barrier of the computing threads that also returns whether ok held in all.  (It takes
+// whole warps, and one thread may come from poll_flags.)
 __device__ __forceinline__ bool compute_and(int ok) {
   int r;
+  __syncwarp();
   asm volatile(
       "{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbar.red.and.pred q, %2, %3, p;\nselp.s32 %0, 1, 0, q;\n}"
       : "=r"(r)
@@ -297,6 +299,7 @@ __device__ __forceinline__ void chain_compute(const MatDesc<double> M, const Fla
       const int r = 8 * (nb - 1) + g;
       if (wp < 8 && r >= w)
         for (int c = 2 * t + (wp & 1) + 8 * (wp >> 1); c < FB; c += 32) D[c * FLD + r] = r == c ? 1.0 : 0.0;
+      __syncwarp();
       compute_sync();
     }
     factor_tile(D, cs.inv, nb, &cs.fail);
@@ -356,6 +359,7 @@ __device__ __forceinline__ void chain_io(const MatDesc<double> M, const Flags F,
     __threadfence();
     bar_sync(kBarIo, FIO);
     if (tid == 0) F.mark(f);
+    __syncwarp();
   };
   if (nt > 1 && !alone) fetch(0);
   for (int j = 0; j < nt; ++j) {
@@ -380,6 +384,7 @@ __device__ __forceinline__ void chain_io(const MatDesc<double> M, const Flags F,
     bar_sync(kBarUpdated, FT + FIO);  // X and tile (j,j)'s buffer are free
     if (j + 2 < nt && !alone) {
       if (tid == 0 && !poll_flags(F, F.c1 + j + 1, F.c2 + j + 2)) cs.err = 1;
+      __syncwarp();
       bar_sync(kBarIo, FIO);
       if (cs.err) {
         bar_sync(kBarFactored, FT + FIO);
