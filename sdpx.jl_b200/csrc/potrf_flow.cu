@@ -190,8 +190,9 @@ struct TileRegs {
 };
 
 // x ← the strip of tile (i, q) updated by panels 0 … np−1 (q ≤ i).  The next
-// panel's tiles are loaded while this panel's products run, when they are there.
-__device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<double>& M, const Flags& F,
+// panel's tiles are loaded while this panel's products run, when they are there.  alone:
+// they are, the CTA's own barriers order them.
+__device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<double>& M, const Flags& F, bool alone,
                                             int i, int q, int np, double* La, double* Lb) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, t = lane & 3;
   const int h = min(FB, M.n - i * FB), hq = min(FB, M.n - q * FB);
@@ -208,19 +209,26 @@ __device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<dou
   bool loaded = false;
   for (int p = 0; p < np; ++p) {
     if (!loaded) {
-      int ok = 1;
-      if (threadIdx.x == 0) ok = poll_flags(F, F.tile(i, p), F.tile(q, p));
-      if (!compute_and(ok)) return false;
+      if (!alone) {
+        int ok = 1;
+        if (threadIdx.x == 0) ok = poll_flags(F, F.tile(i, p), F.tile(q, p));
+        if (!compute_and(ok)) return false;
+      }
       ra.load(M, i * FB, p * FB, h);
       if (i != q) rb.load(M, q * FB, p * FB, hq);
     }
     compute_sync();  // the previous panel's reads of La and Lb are done
     ra.store(La);
     if (i != q) rb.store(Lb);
-    int there = 1;
-    if (threadIdx.x == 0)
-      there = p + 1 < np && F.set(F.tile(i, p + 1)) && F.set(F.tile(q, p + 1));
-    loaded = compute_and(there);
+    if (alone) {
+      loaded = p + 1 < np;
+      compute_sync();
+    } else {
+      int there = 1;
+      if (threadIdx.x == 0)
+        there = p + 1 < np && F.set(F.tile(i, p + 1)) && F.set(F.tile(q, p + 1));
+      loaded = compute_and(there);
+    }
     if (loaded) {
       ra.load(M, i * FB, (p + 1) * FB, h);
       if (i != q) rb.load(M, q * FB, (p + 1) * FB, hq);
@@ -241,17 +249,17 @@ __host__ __device__ inline int flow_tasks(int nt, int j) {
 
 // (M and F by value: by reference they would live in local memory and be read again
 // after every store.)
-__device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, int j, int u, double* La,
+__device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, bool alone, int j, int u, double* La,
                                       double* Lb, double* inv) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const bool partial = j > 0 && u < 2;
   const int i = partial ? j + 1 : j + 2 + u - (j > 0 ? 2 : 0), q = partial && u == 0 ? j + 1 : j;
   const int h = min(FB, M.n - i * FB), w = min(FB, M.n - q * FB);
   double x[8][2];
-  if (!update_tile(x, M, F, i, q, j, La, Lb)) return false;
+  if (!update_tile(x, M, F, alone, i, q, j, La, Lb)) return false;
   if (!partial) {
     int ok = 1;
-    if (threadIdx.x == 0) ok = poll_flags(F, F.tile(j, j), F.tile(j, j));
+    if (!alone && threadIdx.x == 0) ok = poll_flags(F, F.tile(j, j), F.tile(j, j));
     if (!compute_and(ok)) return false;  // (also: La and Lb are free)
     load_tile<FT>(La, M, j * FB, j * FB, FB, FB, threadIdx.x);
   } else {
@@ -269,16 +277,16 @@ __device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, in
     compute_sync();
   }
   store_tile<FT>(Lb, M, i * FB, q * FB, h, w, i == q, threadIdx.x);
-  __threadfence();
+  if (!alone) __threadfence();
   compute_sync();
-  if (threadIdx.x == 0) F.mark(!partial ? F.tile(i, j) : u == 0 ? F.c2 + i : F.c1 + j);
+  if (!alone && threadIdx.x == 0) F.mark(!partial ? F.tile(i, j) : u == 0 ? F.c2 + i : F.c1 + j);
   return true;
 }
 
 // The chain of one matrix: the computing threads' side.  Buffers: the factored
 // tile and the one that becomes the next alternate between T[0] and T[1], tile
 // (j+1,j) is in X.  alone: the matrix has no other CTA, so the tasks of each
-// panel run here too (in the buffers of the tiles not yet fetched).
+// panel run here too (in the buffers of the tiles not yet fetched), without flags.
 struct ChainShared {
   double inv[FB], tinv[FB];
   int fail, err;
@@ -319,7 +327,7 @@ __device__ __forceinline__ void chain_compute(const MatDesc<double> M, const Fla
     if (j == nt - 1) break;
     if (alone) {
       bar_sync(kBarStored, FT + FIO);  // tile (j,j) is in global memory
-      for (int u = 0; u < flow_tasks(nt, j); ++u) run_task(M, F, j, u, X, Y, cs.tinv);
+      for (int u = 0; u < flow_tasks(nt, j); ++u) run_task(M, F, true, j, u, X, Y, cs.tinv);
       bar_arrive(kBarTasks, FT + FIO);
     }
     bar_sync(kBarLoaded, FT + FIO);
@@ -434,7 +442,7 @@ __global__ void __launch_bounds__(FT + FIO, 1)
       for (int j = 0; ok && j < nt; ++j) {
         const int n = flow_tasks(nt, j);
         while (ok && first < n) {
-          ok = run_task(M, F, j, first, T0, T1, cs.tinv);
+          ok = run_task(M, F, false, j, first, T0, T1, cs.tinv);
           first += gsize - 1;
         }
         first -= n;
