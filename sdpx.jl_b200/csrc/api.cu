@@ -979,8 +979,25 @@ struct Handle {
   // Whether LX, MY, W and WY belong to the current X and Y (iterate_changed).
   bool block_factors_current = false;
   void iterate_changed() { block_factors_current = false; }
+  bool wy_current = false;  // whether WY is made, where the others are current
+  void invert_block_factors(int first_side, int last_side) {  // 0: W, 1: WY
+    TrinvList q;
+    for (int side = first_side; side <= last_side; ++side)
+      for (auto& blk : dense) {
+        if (q.count == kTrinvMax) {
+          trinv(q, st);
+          q.count = 0;
+        }
+        q.n[q.count] = blk.k;
+        q.L[q.count] = (side ? MY.p : LX.p) + blk.off;
+        q.W[q.count] = (side ? WY.p : W.p) + blk.off;
+        q.tmp[q.count] = (side ? T2.p : T1.p) + blk.off;
+        ++q.count;
+      }
+    trinv(q, st);
+  }
   bool factor_blocks() {
-    block_factors_current = false;
+    block_factors_current = wy_current = false;
     // LX = chol(X), MY = chol(Y) for every dense block (batched), 1×1 by sqrt.
     std::vector<MatDesc<double>> mats;
     copy_pair(od, X.p, LX.p, Y.p, MY.p, st);  // the dense blocks come first in the stacked layout
@@ -1006,21 +1023,12 @@ struct Handle {
     diag_factor_ok = fail_h == 0;
     if (ok && !dense.empty()) {
       // W = L_X⁻¹ for the Schur products, the block solves and the step bounds, WY =
-      // L_Y⁻¹ for the step bounds (their strict upper triangles stay zero).
-      TrinvList q;
-      for (int side = 0; side < 2; ++side)
-        for (auto& blk : dense) {
-          if (q.count == kTrinvMax) {
-            trinv(q, st);
-            q.count = 0;
-          }
-          q.n[q.count] = blk.k;
-          q.L[q.count] = (side ? MY.p : LX.p) + blk.off;
-          q.W[q.count] = (side ? WY.p : W.p) + blk.off;
-          q.tmp[q.count] = (side ? T2.p : T1.p) + blk.off;
-          ++q.count;
-        }
-      trinv(q, st);
+      // L_Y⁻¹ for the step bounds alone (their strict upper triangles stay zero).  WY comes
+      // along while both fit one list; a list more per 16 blocks costs about as much as the
+      // first, so with more blocks it waits until the bounds are asked for
+      // (residuals and factors of 100 blocks of order 200: 2.71 ms with both, 1.97 with W).
+      wy_current = 2 * nb <= (size_t)kTrinvMax;
+      invert_block_factors(0, wy_current ? 1 : 0);
     }
     block_factors_current = ok;
     return ok;
@@ -1835,6 +1843,8 @@ struct Handle {
   DBuf<int> sb_list;  // sb_blocks on the device
   void queue_step_bounds(double* out) {
     const int n = (int)sb_blocks.size();
+    if (!wy_current) invert_block_factors(1, 1);
+    wy_current = true;
     const double *Ws[2] = {W.p, WY.p}, *dMs[2] = {dX.p, dY.p};
     double *Ts[2] = {T1.p, T2.p}, *Gs[2] = {Z.p, tmpK2.p};
     int kb = 0;

@@ -60,3 +60,20 @@ def test_small_orders_beside_large_ones(ks):
         for _ in range(3):
             q = be.affine_diagnostics(True)
             assert (q["tX"], q["tY"]) == (p["tX"], p["tY"])
+
+
+# 8 blocks: the inverse factors of both sides in one list; 9 and more: those of Y are made
+# when the bounds are asked for, once for an iterate
+@pytest.mark.parametrize("ks", [[20, 70] * 4, [20, 70, 3] * 3, [9] * 40])
+def test_many_blocks(ks):
+    be, X, Y = _direction(ks, len(ks))
+    with be:
+        _, dX, dY = be.get_direction()
+        for scale in (1.0, 3.0):
+            p = [be.affine_diagnostics(True) for _ in range(2)]
+            for key, M, dM in (("tX", X, dX), ("tY", Y, dY)):
+                want = _exact([scale * a for a in M], dM)
+                assert abs(p[0][key] - want) <= 4 * max(ks) * EPS * 1e2 * 1e3 * want
+                assert p[1][key] == p[0][key]
+            be.set_iterate(np.zeros(3), [3.0 * x for x in X], [3.0 * y for y in Y])
+            assert be.compute_residuals([0.0] * len(ks), True, True)[2]
