@@ -1939,14 +1939,18 @@ struct Handle {
           probs.push_back(q);
         }
     // Each round evaluates a complete tree of the next `depth` bisection steps
-    // of every unfinished problem in one batched Cholesky; the deepest tree
-    // that keeps the batch within about one trial matrix per SM is used (a
-    // round costs about the same for any batch up to one wave).
+    // of every unfinished problem in one batched Cholesky.  Up to order 200 the
+    // deepest tree that keeps the batch within about one trial matrix per SM is
+    // used (a round costs about the same for any batch up to one wave: 30, 62, 126
+    // trials of order 130 take 0.053, 0.059, 0.076 ms, of order 200 0.076, 0.104, 0.133,
+    // to which the host adds 0.05).  Above it the products count, and fewer trials
+    // share more CTAs each: order 300 0.109, 0.178, 0.225 ms, 800 0.76, 2.15, 2.15.
     while (true) {
-      int active = 0;
-      for (auto& P : probs) active += P.finished ? 0 : 1;
+      int active = 0, order = 0;
+      for (auto& P : probs)
+        if (!P.finished) ++active, order = std::max(order, dense[P.b].k);
       int DEPTH = 4;
-      while (DEPTH < 7 && active * ((1 << (DEPTH + 1)) - 1) <= sms - 16) ++DEPTH;
+      while (DEPTH < 7 && order <= 200 && active * ((1 << (DEPTH + 1)) - 1) <= sms - 16) ++DEPTH;
       std::vector<TrialReq> reqs;
       std::vector<std::vector<double>> pts(probs.size());
       std::vector<size_t> first_req(probs.size());
