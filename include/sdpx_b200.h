@@ -335,7 +335,7 @@ int sdpx_b200_sparse_schur_info(sdpx_b200_handle* h, int64_t* active_positions,
  * call cudaMalloc — runtimes that own all device memory through their own
  * pool (e.g. a Julia or Python caching allocator) or serving loops where an
  * implicit cudaMalloc/cudaFree would synchronise the device.
- *   - m ≤ 2048 (the array holds one K chunk of every lower 64×64 tile) and
+ *   - m ≤ 2048 (the array holds one K chunk of every lower tile) and
  *     K ≤ 2^30 (the tile loop indexes K in int32); larger m or K, and NULL
  *     P or S, return -1 with a message and leave S untouched.
  *   - The first call on each device looks up the array's device address with

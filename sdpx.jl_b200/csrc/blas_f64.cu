@@ -5,6 +5,7 @@
 #include "gemm_f64.cuh"
 
 #include <atomic>
+#include <climits>
 #include <mutex>
 #include <stdexcept>
 
@@ -272,16 +273,19 @@ static SyrkPlan best_split(int m, long long K, int sms, const SyrkTile& t, long 
   return best;
 }
 
-SyrkPlan plan_syrk_f64(int m, long long K, int sm_count) {
+// The tile and split of least modelled time whose partial tiles take at most `scratch` doubles.
+static SyrkPlan best_plan(int m, long long K, int sms, long long scratch) {
   SyrkPlan best;
   double least = 0.0;
   for (const SyrkTile& t : kSyrkTiles) {
     double cycles = 0.0;
-    const SyrkPlan p = best_split(m, K, sm_count, t, kMaxChunks, &cycles);
+    const long long chunk = (long long)syrk_plan(m, K, t.bm, 1).partial_doubles;
+    const SyrkPlan p = best_split(m, K, sms, t, scratch / chunk, &cycles);
     if (&t == kSyrkTiles || cycles < least) best = p, least = cycles;
   }
   return best;
 }
+SyrkPlan plan_syrk_f64(int m, long long K, int sm_count) { return best_plan(m, K, sm_count, LLONG_MAX); }
 
 template <class Cfg>
 static void launch_syrk(const Opnd& P, const SyrkPlan& plan, double* partial, double* S, long long lds,
@@ -310,9 +314,9 @@ void syrk_lower_f64(const Opnd& P, const SyrkPlan& plan, double* partial, double
 // Allocation-free variant of the split-K lower Gram product S = PᵀP.
 //
 // The split-K partial tiles live in a fixed file-scope device array instead of
-// caller- or library-allocated memory.  One K chunk of every lower 64×64 tile
-// must fit (ntri·64·64 doubles, ntri = t(t+1)/2, t = ceil(m/64)): the stated
-// limit m ≤ 2048 (t = 32, 2.1 Mi doubles) leaves room for a second chunk.  K is
+// caller- or library-allocated memory.  One K chunk of every lower tile must fit
+// (64×64: ntri·64·64 doubles, ntri = t(t+1)/2, t = ceil(m/64); 32×32: fewer): the stated
+// limit m ≤ 2048 (t = 32, 2.1 Mi doubles) leaves room for almost a second.  K is
 // bounded by the int32 K indexing of the tile loop: chunk starts plus a chunk
 // length must stay below 2³¹, which K ≤ 2³⁰ guarantees.  Every GPU that loads
 // the library holds the array until the process exits, and all calls share it.
@@ -346,10 +350,6 @@ static double* noalloc_scratch_address() {
 size_t gram_noalloc_capacity_doubles() { return kNoAllocScratchDoubles; }
 
 void syrk_lower_f64_noalloc(const double* P, long long K, int m, double* S, cudaStream_t st) {
-  using Cfg = CfgSmKK;
-  const int nt = ceil_div(m, Cfg::BM);
-  const long long ntri = (long long)nt * (nt + 1) / 2;
-  const long long tile = (long long)Cfg::BM * Cfg::BN;
   if (m <= 0 || K <= 0) throw std::invalid_argument("gram: m and K must be positive");
   if (m > kNoAllocMaxM)
     throw std::invalid_argument("gram (allocation-free): m = " + std::to_string(m) +
@@ -357,15 +357,15 @@ void syrk_lower_f64_noalloc(const double* P, long long K, int m, double* S, cuda
   if (K > kNoAllocMaxK)
     throw std::invalid_argument("gram (allocation-free): K = " + std::to_string(K) +
                                 " exceeds the int32 K indexing (K ≤ 2^30)");
-  if (ntri * tile > (long long)kNoAllocScratchDoubles)
-    throw std::logic_error("gram (allocation-free): scratch smaller than one chunk");
   double* scratch = noalloc_scratch_address();
   int dev = 0, sms = 148;
   SDPX_CUDA(cudaGetDevice(&dev));
   SDPX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // At most as many K chunks as the scratch holds.
-  double cycles = 0.0;
-  const SyrkPlan plan = best_split(m, K, sms, kSyrkTiles[0], (long long)kNoAllocScratchDoubles / (ntri * tile), &cycles);
+  // At most as many K chunks as the scratch holds.  (By 64-tiles alone m = 2000, K = 20000,
+  // one chunk of 528 tiles for 444 places, took 4.00 ms, by 32-tiles 2.99.)
+  const SyrkPlan plan = best_plan(m, K, sms, (long long)kNoAllocScratchDoubles);
+  if (plan.partial_doubles > kNoAllocScratchDoubles)
+    throw std::logic_error("gram (allocation-free): scratch smaller than one chunk");
   Opnd Pd;
   Pd.base = P;
   Pd.kstride = 1;
