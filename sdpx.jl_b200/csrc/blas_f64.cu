@@ -87,6 +87,28 @@ __global__ void __launch_bounds__(Cfg::NT) k_trmm_right_lower_inplace(Opnd T, Op
   }
 }
 
+// Adds acc to a tile's partial sums in memory (`out`, this CTA's own; the first time they
+// are stored) and clears it, so that a running sum covers kFoldRows rows of K or a sixteenth
+// of it, whichever is more, and not a whole chunk: rms error over Σ|products| and time,
+// one sum a chunk → this, 1000×3000 4.5e-17 → 1.6e-17, 0.164 → 0.167 ms, 3000×21000 1.7e-17 →
+// 1.3e-17, 6.51 → 6.41 ms.  Reductions at the L2 need no answer (loads to add to took
+// about 2 k cycles a fold); a second set of sums in registers costs a resident CTA.
+constexpr int kFoldRows = 256;
+template <class Cfg>
+struct PartialFold {
+  static constexpr bool on = true;
+  double (&acc)[Cfg::FM][Cfg::FN][2];
+  double* out;
+  bool& first;
+  int steps;
+  __device__ __forceinline__ void operator()() const {
+    if (first) for_each_acc<Cfg>(acc, [&](int r, int c, double v) { out[c * Cfg::BM + r] = v; });
+    else for_each_acc<Cfg>(acc, [&](int r, int c, double v) { atomicAdd(out + c * Cfg::BM + r, v); });
+    zero_acc<Cfg>(acc);
+    first = false;
+  }
+};
+
 // Split-K lower SYRK.  Work unit u = chunk * ntri + tri (chunk-major, so CTAs
 // resident at the same time share one K slab of the panel in L2).  Each unit
 // writes its BM×BN partial tile to `partial` (column-major inside the tile);
@@ -105,9 +127,11 @@ __global__ void __launch_bounds__(Cfg::NT) k_syrk_splitk(Opnd P, int ntri, int k
   const int ke = min(P.k_extent, kb + kchunk);
   double acc[Cfg::FM][Cfg::FN][2];
   zero_acc<Cfg>(acc);
-  f64_tile_mainloop<Cfg>(acc, P, P, ti * Cfg::BM, tj * Cfg::BN, kb, ke, smem);
-  double* out = partial + (size_t)u * Cfg::BM * Cfg::BN;
-  for_each_acc<Cfg>(acc, [&](int r, int c, double v) { out[c * Cfg::BM + r] = v; });
+  bool first = true;
+  const PartialFold<Cfg> fold{acc, partial + (size_t)u * Cfg::BM * Cfg::BN, first,
+                              max(kFoldRows, P.k_extent / 16) / Cfg::BK};
+  f64_tile_mainloop<Cfg>(acc, P, P, ti * Cfg::BM, tj * Cfg::BN, kb, ke, smem, fold);
+  fold();
 }
 
 template <int BM, int BN>
@@ -234,8 +258,8 @@ struct SyrkTile {
 };
 constexpr SyrkTile kSyrkTiles[] = {{64, 3, 2000, 1130, 8000}, {32, 7, 800, 325, 5000}};
 // Chunks of 128 rows or more, and of 2048 or less where 16 chunks and 1 GiB of partial
-// tiles allow: a longer running sum rounds more (3000×26400: relative error of the
-// solve 6.0e-16 with chunks of 8800 rows, 4.3e-16 with 2048, no slower).
+// tiles allow (rounding does not depend on them, PartialFold; with the model alone
+// 2600×18200 took 4.50 ms instead of 4.31, 3000×21000 6.40 instead of 6.41).
 constexpr int kMaxChunks = 32, kMinChunkRows = 128, kMaxChunkRows = 2048;
 constexpr long long kPartialDoubles = 1LL << 27;
 

@@ -78,10 +78,15 @@ __device__ __forceinline__ void issue_stage(double* s, const StagePlan<PER_T>& p
   }
 }
 
-// Accumulates A[m0:m0+BM, kb:ke] · B[kb:ke, n0:n0+BN] into acc.
-template <class Cfg>
+struct NoFold {
+  static constexpr bool on = false;
+};
+
+// Accumulates A[m0:m0+BM, kb:ke] · B[kb:ke, n0:n0+BN] into acc.  fold(), where it is on,
+// takes acc away after every fold.steps steps of 16 (but the last).
+template <class Cfg, class Fold = NoFold>
 __device__ void f64_tile_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2], const Opnd& A, const Opnd& B,
-                                  int m0, int n0, int kb, int ke, double* smem) {
+                                  int m0, int n0, int kb, int ke, double* smem, Fold fold = {}) {
   constexpr int BK = Cfg::BK, ST = Cfg::STAGES;
   double* sA = smem;
   double* sB = smem + ST * Cfg::A_STAGE;
@@ -103,6 +108,8 @@ __device__ void f64_tile_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2], const Opnd
     }
     cp_async_commit();
   }
+  int left = 0;  // steps to the next fold
+  if constexpr (Fold::on) left = fold.steps;
   for (int tIdx = 0; tIdx < ntiles; ++tIdx) {
     // One barrier a step: it shows that stage tIdx has arrived and that every warp is
     // done with stage tIdx − 1, whose slot takes the copies issued next.
@@ -136,6 +143,11 @@ __device__ void f64_tile_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2], const Opnd
 #pragma unroll
         for (int fn = 0; fn < Cfg::FN; ++fn) dmma_8x8x4(acc[fm][fn][0], acc[fm][fn][1], af[fm], bf[fn]);
     }
+    if constexpr (Fold::on)
+      if (--left == 0 && tIdx + 1 < ntiles) {
+        fold();
+        left = fold.steps;
+      }
   }
   cp_async_wait<0>();
   __syncthreads();  // the shared memory is free
