@@ -181,11 +181,12 @@ enum KRange : int {
   KR_B_UPPER = 4,   // B upper triangular: k ≤ col → [0, min(K, n0+BN))
 };
 
-// Per-(kernel, device) one-time opt-in to large dynamic shared memory.
+// Per-(kernel, device) one-time opt-in to large dynamic shared memory.  The 48 KB that need
+// none hold the kernel's static arrays too (9 KB at most beside dynamic ones here).
 void smem_attr_ensure(const void* kern, size_t bytes);  // defined in api.cu
 template <class Kern>
 inline void ensure_smem(Kern kern, size_t bytes) {
-  if (bytes <= 48 * 1024) return;
+  if (bytes <= 32 * 1024) return;
   smem_attr_ensure((const void*)kern, bytes);
 }
 
