@@ -115,12 +115,13 @@ int sdpx_b200_batch_set_step_bounds(sdpx_b200_batch* b, int32_t mode);
  * the FP64 tensor-core (DMMA) products, which tile each instance by 32 or 64
  * as its k and m need) and the Schur work per CTA in
  * FLOPs (an instance's panel and SYRK are split over ceil(work / grain) CTAs;
- * grain ≤ 0: one CTA per instance). */
+ * grain ≤ 0: one CTA per instance, but grain < 0 with the DMMA products, the
+ * default: picked per call from the work of the running instances). */
 int sdpx_b200_batch_set_schur_shape(sdpx_b200_batch* b, int32_t threads, int32_t tile,
                                     double grain);
 
 /* Times every candidate Schur launch shape (24: five scalar shapes and the
- * DMMA path, each at four work grains) on the current iterate of all
+ * DMMA path, each at four work grains, the default among them) on the current iterate of all
  * instances (the fixed start when no solve ran) and keeps the fastest.
  * table (may be NULL) receives `capacity` rows of (threads, tile, grain,
  * milliseconds); *count = number of candidates timed. */

@@ -2142,8 +2142,8 @@ struct Engine {
     std::vector<Cand> cands;
     const std::pair<int, int> shapes[] = {{128, 16}, {256, 16}, {128, 32},
                                           {256, 32}, {512, 32}, {128, 64}};
-    for (double g : {0.0, 1.0e6, 4.0e6, 16.0e6})
-      for (const auto& tt : shapes) cands.push_back({tt.first, tt.second, g});
+    for (double g : {0.0, 1.0e6, 4.0e6, 16.0e6})  // (tile 64: the default in place of 0)
+      for (const auto& tt : shapes) cands.push_back({tt.first, tt.second, tt.second == 64 && g == 0.0 ? -1.0 : g});
     double best = INFINITY;
     Cand pick{schur_threads, schur_tile, grain};
     int row = 0;
