@@ -1284,7 +1284,8 @@ struct Engine {
     d_act.alloc(N);
     d_par.alloc((size_t)N * kNIn + (N + 1) / 2);  // input rows, then the instance list
     h_act.ensure(N * sizeof(int));
-    h_par.ensure(kStage * stage_stride());
+    stage_slots = (int)std::clamp<size_t>(kStageBytes / stage_stride(), 1, kStage);
+    h_par.ensure(stage_slots * stage_stride());
     h_res.ensure((size_t)N * oNOut * sizeof(double));
     pool.inst = d_inst.p;
     pool.A = A.p;
@@ -1338,10 +1339,10 @@ struct Engine {
     std::iota(lpt.begin(), lpt.end(), 0);
     std::stable_sort(lpt.begin(), lpt.end(),
                      [&](int a, int b) { return work_rank[ids[a]] < work_rank[ids[b]]; });
-    // Input rows and instance list in one copy, from the next of kStage staging slots:
+    // Input rows and instance list in one copy, from the next of the staging slots:
     // the stream is waited for only when all are in use (each read-back frees them).
     const size_t pbytes = (size_t)n * kNIn * sizeof(double), bytes = pbytes + n * sizeof(int);
-    if (staged == kStage) sync_stream();
+    if (staged == stage_slots) sync_stream();
     char* hs = static_cast<char*>(h_par.p) + (size_t)staged++ * stage_stride();
     double* hp = reinterpret_cast<double*>(hs);
     int* ha = reinterpret_cast<int*>(hs + pbytes);
@@ -1372,8 +1373,11 @@ struct Engine {
     return rows.data();
   }
   std::vector<int> lpt, work_rank;  // launch order; rank of each instance by work
+  // Up to 16 staging slots in 8 MB of pinned memory, 1.6 KB an instance: all 16 up to 5000
+  // instances, one slot from 42000 on.
   static constexpr int kStage = 16, kDirect = 128;
-  int staged = 0;  // staging slots in use
+  static constexpr size_t kStageBytes = 8 << 20;
+  int stage_slots = kStage, staged = 0;  // slots, those in use
   size_t stage_stride() const { return ((size_t)N * (kNIn * sizeof(double) + sizeof(int)) + 63) & ~size_t(63); }
   void sync_stream() {
     SDPX_CUDA(cudaStreamSynchronize(st));
