@@ -743,6 +743,7 @@ struct Handle {
     norm_work.alloc(1);
     norm_work.zero(st);
     ensure_descs(std::max<size_t>(16, 2 * dense.size()));
+    sb_max_order = step_bound_max_order();
     // Gershgorin scratch
     std::vector<long long> coff(dense.size());
     long long tot = 0;
@@ -1839,6 +1840,8 @@ struct Handle {
   // L⁻¹·dM·L⁻ᵀ (both sides, one launch): queued into `out` (pinned), [X blocks |
   // Y blocks] of the block list sb_blocks.  Scratch: T1, T2, Z, tmpK2.
   std::vector<int> sb_blocks;
+  int sb_max_order = 0;
+  bool step_bound_fits(int k) const { return k >= 3 && k <= sb_max_order; }
   DBuf<StepBoundDesc> sb_desc;
   DBuf<int> sb_list;  // sb_blocks on the device
   void queue_step_bounds(double* out) {

@@ -26,6 +26,7 @@
 #include "step_bound.h"
 #include "lambda_bound.cuh"
 
+#include <atomic>
 #include <type_traits>
 
 namespace sdpx {
@@ -567,52 +568,80 @@ void ensure_cluster16(Kern kern) {
   SDPX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
 }
 
-template <class Kern>
-void launch_cluster(Kern kern, int C, int threads, size_t smem, const StepBoundDesc* d_list, int n, double* out,
-                    cudaStream_t st) {
-  if (C > 8) ensure_cluster16(kern);
-  ensure_smem(kern, smem);
+struct ClusterConfig {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(n * C);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = C;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  SDPX_CUDA(cudaLaunchKernelEx(&cfg, kern, d_list, out));
-  SDPX_LAUNCH_CHECK();
-}
-template <int C, int NW, int Q, int R>
-void launch(const StepBoundDesc* d_list, int n, int kmax, double* out, cudaStream_t st) {
-  static_assert(32 * Q <= R * C * NW, "every row has a place");
-  const size_t smem = (6ul * (kmax + (kmax & 1)) + 1) * sizeof(double);
-  launch_cluster(k_step_bound_regs<C, NW, Q, R>, C, 32 * NW, smem, d_list, n, out, st);
-}
+  template <class Kern>
+  ClusterConfig(Kern kern, int clusters, int C, int threads, size_t smem, cudaStream_t st) {
+    if (C > 8) ensure_cluster16(kern);
+    ensure_smem(kern, smem);
+    cfg.gridDim = dim3(clusters * C);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+  }
+  ClusterConfig(const ClusterConfig&) = delete;
+};
 
-constexpr int kMaxOrder = 32 * 14;
-
-}  // namespace
-
-bool step_bound_fits(int k) { return k >= 3 && k <= kMaxOrder; }
-
+// The kernel for orders up to kmax, and f(kernel, CTAs of a cluster, threads, shared bytes).
 // Cluster and warps by the largest order: every warp repeats the vector work, so few
 // warps, and few rows in each, beat a small cluster's shorter barrier.  Cycles measured
 // (cluster × warps): k = 30  63e3 (1×8), 66e3 (4×4); 61  153e3 (1×8), 131e3 (4×4), 145e3
 // (8×4); 100  291e3 (4×8), 243e3 (8×4); 200  746e3 (8×8), 744e3 (8×4), 624e3 (16×4).
+constexpr int kOrderLimits[] = {32, 64, 128, 224, 448};
+template <int C, int NW, int Q, int R, class F>
+auto with_regs(int kmax, F f) {
+  static_assert(32 * Q <= R * C * NW, "every row has a place");
+  return f(k_step_bound_regs<C, NW, Q, R>, C, 32 * NW, (6ul * (kmax + (kmax & 1)) + 1) * sizeof(double));
+}
+template <class F>
+auto with_kernel(int kmax, F f) {
+  if (kmax <= kOrderLimits[0]) return with_regs<1, 8, 1, 4>(kmax, f);
+  if (kmax <= kOrderLimits[1]) return with_regs<4, 4, 2, 4>(kmax, f);
+  if (kmax <= kOrderLimits[2]) return with_regs<8, 4, 4, 4>(kmax, f);
+  if (kmax <= kOrderLimits[3]) return with_regs<16, 4, 7, 4>(kmax, f);
+  return f(k_step_bound_wide, kWide, 32 * (kRowWarps + 1), bound_smem_doubles(kmax) * sizeof(double));
+}
+
+}  // namespace
+
+// A part of a GPU may have no place for the larger clusters.
+int step_bound_max_order() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  SDPX_CUDA(cudaGetDevice(&dev));
+  const bool keep = dev >= 0 && dev < 64;
+  int order = keep ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (order) return order;
+  for (int limit : kOrderLimits) {
+    const bool runs = with_kernel(limit, [](auto kern, int C, int threads, size_t smem) {
+      const ClusterConfig q(kern, 1, C, threads, smem, nullptr);
+      int places = 0;
+      const bool ok = cudaOccupancyMaxActiveClusters(&places, kern, &q.cfg) == cudaSuccess && places > 0;
+      if (!ok) cudaGetLastError();
+      return ok;
+    });
+    if (!runs) break;
+    order = limit;
+  }
+  if (order == 0) order = 2;  // none (every order that needs the kernel is larger)
+  if (keep) known[dev].store(order, std::memory_order_relaxed);
+  return order;
+}
+
 void step_bounds(const StepBoundDesc* d_list, int n, int kmax, double* out, cudaStream_t st) {
   if (n <= 0) return;
-  if (kmax <= 32) return launch<1, 8, 1, 4>(d_list, n, kmax, out, st);
-  if (kmax <= 64) return launch<4, 4, 2, 4>(d_list, n, kmax, out, st);
-  if (kmax <= 128) return launch<8, 4, 4, 4>(d_list, n, kmax, out, st);
-  if (kmax <= 224) return launch<16, 4, 7, 4>(d_list, n, kmax, out, st);
-  if (kmax <= kMaxOrder)
-    return launch_cluster(k_step_bound_wide, kWide, 32 * (kRowWarps + 1), bound_smem_doubles(kmax) * sizeof(double),
-                          d_list, n, out, st);
-  throw std::invalid_argument("step_bounds: order too large");
+  if (kmax > step_bound_max_order()) throw std::invalid_argument("step_bounds: order too large");
+  with_kernel(kmax, [&](auto kern, int C, int threads, size_t smem) {
+    const ClusterConfig q(kern, n, C, threads, smem, st);
+    SDPX_CUDA(cudaLaunchKernelEx(&q.cfg, kern, d_list, out));
+    SDPX_LAUNCH_CHECK();
+  });
 }
 
 }  // namespace sdpx

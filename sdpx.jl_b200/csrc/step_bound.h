@@ -9,10 +9,11 @@ struct StepBoundDesc {
   int k;
 };
 
-// Whether an order fits the kernel (its rows in the shared memory of one cluster).
-bool step_bound_fits(int k);
+// The largest order that the current device has a kernel for (448 on a whole B200; looked
+// up once per device), orders from 3 on.
+int step_bound_max_order();
 // out[q] = min(1, −1/λ_min(G_q)) (1 when λ_min ≥ −1, 0 when G is not finite) for the
-// n matrices of the device list; kmax: the largest order, step_bound_fits(kmax).
+// n matrices of the device list; kmax: the largest order, at most that.
 void step_bounds(const StepBoundDesc* d_list, int n, int kmax, double* out, cudaStream_t st);
 
 }  // namespace sdpx

@@ -77,3 +77,12 @@ def test_many_blocks(ks):
                 assert p[1][key] == p[0][key]
             be.set_iterate(np.zeros(3), [3.0 * x for x in X], [3.0 * y for y in Y])
             assert be.compute_residuals([0.0] * len(ks), True, True)[2]
+
+
+# The clusters of every order limit have a place on a whole GPU (where one has not, larger
+# orders take the bisection).
+def test_every_cluster_shape_runs():
+    from sdpx_b200.cuda_backend import load_library
+    import torch
+    torch.cuda.init()
+    assert load_library()["_ZN4sdpx20step_bound_max_orderEv"]() == 448
