@@ -1160,7 +1160,7 @@ struct Engine {
   dcache::ReleaseScope release_scope;  // first member: destroyed last
   int dev = 0;
   cudaStream_t st = nullptr;
-  int N = 0, kmax = 0, mmax = 0;
+  int N = 0, kmax = 0, mmax = 0, sms = 148;
   std::vector<Inst> inst;
   std::vector<double> scale_p, scale_d;
   DBuf<Inst> d_inst;
@@ -1244,6 +1244,7 @@ struct Engine {
     }
     dev = device;  // sizes checked first: usage errors need no device
     SDPX_CUDA(cudaSetDevice(dev));
+    SDPX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     SDPX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     for (auto& e : ev) SDPX_CUDA(cudaEventCreate(&e));
     for (auto& e : ev_stage) SDPX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1461,7 +1462,7 @@ struct Engine {
     if (g < 0) {  // about 16 items a SM, of at least 2.5e5 flops (a launch's tail) …
       double total = 0;  // … and at most 1e6 (the finest of the timed grains, the fastest)
       for (int q = 0; q < n; ++q) total += cost(q);
-      g = std::min(1.0e6, std::max(2.5e5, total / (148.0 * 16.0)));
+      g = std::min(1.0e6, std::max(2.5e5, total / (sms * 16.0)));
     }
     auto split = [&](std::vector<int4>& w, int q, int units, double flops) {
       int parts = g > 0 ? (int)std::ceil(flops / g) : 1;
