@@ -497,11 +497,14 @@ struct Handle {
     if (sym) symmetrize(d_doff.p, d_dk.p, (int)dense.size(), kmax, out, st);
   }
 
-  // Whether `bytes` of device memory fit beside `spare`.  Less than kNoQuery always
-  // does: the query costs 100 µs, a tenth of a small model's set-up.
-  static constexpr size_t kNoQuery = 32 << 20;
-  bool room_for(size_t bytes, size_t spare) {
-    if (bytes <= kNoQuery) return true;
+  // Whether buffers of these sizes fit beside `spare`.  Idle cached blocks that serve small
+  // ones are ours already and need no look at the device's free memory: that costs
+  // 100 µs, a quarter of a small model's set-up where handles follow one another.
+  static constexpr size_t kSmallNeed = 32 << 20;
+  bool room_for(std::initializer_list<size_t> sizes, size_t spare) {
+    size_t bytes = 0;
+    for (size_t s : sizes) bytes += s;
+    if (bytes <= kSmallNeed && dcache::holds(dev, sizes)) return true;
     size_t freeb = 0, totb = 0;
     SDPX_CUDA(cudaMemGetInfo(&freeb, &totb));
     return bytes + spare <= freeb + dcache::idle_bytes(dev);  // idle cached blocks are ours to reuse
@@ -707,7 +710,7 @@ struct Handle {
       // The copy is an accelerator: it is made only when it fits beside 4 GB of
       // headroom (the solve's remaining buffers are allocated later).
       const size_t apb = sizeof(double) * (size_t)std::max<long long>(Kt, 1) * m;
-      use_packed = room_for(apb, 4ull << 30);
+      use_packed = room_for({apb}, 4ull << 30);
       if (use_packed) Ap.alloc((size_t)std::max<long long>(Kt, 1) * m);
       kt_fold.alloc(std::max<long long>(Kt, 1));
       adx.alloc(K);
@@ -1116,8 +1119,8 @@ struct Handle {
       // Room for the cached constraint digits, the per-build scratch and the
       // Gram's digit planes (same size as the FP64 panel), with 2 GB to spare.
       const size_t gram = oz_plan.m == m && oz_plan.K == K ? 0 : (size_t)OZ_DIGITS * m * (K + 64);
-      const size_t need = adig + tdig + wdig + 4 * (size_t)(aexp + texp + wexp) + gram;
-      if (dense.empty() || !fits_int || !room_for(need, 2ull << 30)) {
+      if (dense.empty() || !fits_int ||
+          !room_for({adig, tdig, wdig, 4 * (size_t)aexp, 4 * (size_t)texp, 4 * (size_t)wexp, gram}, 2ull << 30)) {
         oz_blk_state = -1;
       } else {
         oz_adig.alloc(adig);

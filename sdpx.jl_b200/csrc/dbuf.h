@@ -19,8 +19,10 @@
 
 #include <cstddef>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
+#include <set>
 #include <utility>
 
 #include "common.cuh"
@@ -75,6 +77,24 @@ inline size_t idle_bytes(int dev) {
   return (dev >= 0 && dev < kMaxDev) ? c.idle_bytes[dev] : 0;
 }
 
+// Largest idle block that a request takes.
+inline size_t take_up_to(size_t bytes) { return bytes + bytes / 4 + (1u << 20); }
+
+// Whether idle blocks of `dev` serve all these requests together.
+inline bool holds(int dev, std::initializer_list<size_t> requests) {
+  Cache& c = cache();
+  std::lock_guard<std::mutex> g(c.mu);
+  std::set<const void*> taken;
+  for (size_t bytes : requests) {
+    auto it = c.idle.lower_bound(bytes);
+    const auto end = c.idle.upper_bound(take_up_to(bytes));
+    while (it != end && (it->second.first != dev || taken.count(it->second.second))) ++it;
+    if (it == end) return false;
+    taken.insert(it->second.second);
+  }
+  return true;
+}
+
 // A block of at least `bytes` on the current device; its true size in *got.
 inline void* get(size_t bytes, int* dev_out, size_t* got) {
   int dev = 0;
@@ -83,8 +103,7 @@ inline void* get(size_t bytes, int* dev_out, size_t* got) {
   Cache& c = cache();
   {
     std::lock_guard<std::mutex> g(c.mu);
-    const size_t hi = bytes + bytes / 4 + (1u << 20);
-    for (auto it = c.idle.lower_bound(bytes); it != c.idle.end() && it->first <= hi; ++it) {
+    for (auto it = c.idle.lower_bound(bytes); it != c.idle.end() && it->first <= take_up_to(bytes); ++it) {
       if (it->second.first != dev) continue;
       void* p = it->second.second;
       *got = it->first;
