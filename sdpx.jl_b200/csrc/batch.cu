@@ -758,20 +758,31 @@ __global__ void k_b_rollback(Pool pool, const int* act, const double* par, doubl
 // B10: backtracking line search per side: the first t of 1, γ, γ², … for
 // which M + t·dM has a Cholesky factor with min|L_jj| > kRatio·max|L_jj|, or
 // the first t below kMinStep (src/kernels/threaded.jl:1751-1818).
-__global__ void __launch_bounds__(kThreads)
+// small: no instance above kSmallTrialOrder.  ctas an SM: with two the registers spill, which
+// costs an instance 10 to 25 % (order 64: 16 → 18 µs for one trial, 206 → 235 for 22, order
+// 24: 9.2 → 11.1 and 47 → 49) and pays from more instances than SMs on (512 × order 64:
+// 44 → 38, 800 → 552, order 24: 22 → 18, 170 → 118).
+template <bool small, int ctas>
+__global__ void __launch_bounds__(kThreads, ctas)
     k_b_linesearch(Pool pool, const int* act, const double* par, double* res) {
   INST_PROLOGUE
   extern __shared__ __align__(16) double sm[];
   __shared__ double inv[64], red[32];
-  __shared__ int sfail;
+  __shared__ int sfail, flags[kTrialWarps];
   const double gamma = in[kGamma], min_step = in[kMinStep], ratio = in[kRatio];
-  const double tX = cta_backtrack(pool.X + I.kk_off, pool.dX + I.kk_off, k, gamma, min_step,
-                                  ratio, sm, inv, &sfail, red);
-  const double tY = cta_backtrack(pool.Y + I.kk_off, pool.dY + I.kk_off, k, gamma, min_step,
-                                  ratio, sm, inv, &sfail, red);
+  double t[2];
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const double* M = (side ? pool.Y : pool.X) + I.kk_off;
+    const double* dM = (side ? pool.dY : pool.dX) + I.kk_off;
+    if (small || k <= kSmallTrialOrder)
+      t[side] = cta_backtrack_small(M, dM, k, gamma, min_step, ratio, sm, inv, &sfail, red, flags);
+    else
+      t[side] = cta_backtrack(M, dM, k, gamma, min_step, ratio, sm, inv, &sfail, red);
+  }
   if (threadIdx.x == 0) {
-    out[oTX] = tX;
-    out[oTY] = tY;
+    out[oTX] = t[0];
+    out[oTY] = t[1];
   }
 }
 
@@ -1205,7 +1216,11 @@ struct Engine {
 
   size_t smem_tp() const { return smem_bytes(2) + sizeof(double) * 64 * FLD; }
   size_t smem_bytes(int mats) const { return (size_t)mats * (size_t)pool.kq * sizeof(double); }
-  // Packed lower triangles of X, dX and kTrialWarps trial slots (the step-length phases).
+  size_t smem_search() const {  // a tile, or packed slots of the orders that take them
+    const size_t k = std::min(kmax, kSmallTrialOrder);
+    return std::max(smem_bytes(1), (2 + kTrialWarps) * (k * (k + 1) / 2) * sizeof(double));
+  }
+  // Packed lower triangles of X, dX and kTrialWarps trial slots (the bisection of the bounds).
   size_t smem_trials() const {
     return (size_t)(2 + kTrialWarps) * (size_t)pool.kp * sizeof(double);
   }
@@ -1302,8 +1317,10 @@ struct Engine {
     for (PhaseKernel kf : {k_b_residuals, k_b_rhs, k_b_dirblocks})
       ensure_smem(kf, smem_bytes(3));
     ensure_smem(k_b_factor, kFactorSmem);
-    for (PhaseKernel kf : {k_b_affine, k_b_linesearch})
-      ensure_smem(kf, std::max(smem_trials(), smem_bytes(3)));
+    ensure_smem(k_b_affine, std::max(smem_trials(), smem_bytes(3)));
+    for (PhaseKernel kf : {k_b_linesearch<true, 1>, k_b_linesearch<true, 2>, k_b_linesearch<false, 1>,
+                           k_b_linesearch<false, 2>})
+      ensure_smem(kf, smem_search());
     ensure_smem(k_b_panel, smem_bytes(4));
     SDPX_CUDA(cudaStreamSynchronize(st));
   }
@@ -1952,7 +1969,12 @@ struct Engine {
         R.d_res = R.sd_res;
       }
       const auto tl1 = std::chrono::steady_clock::now();
-      out = phase(k_b_linesearch, ok3, smem_bytes(1), [&](int id, double* in) {
+      bool small = true;
+      for (int id : ok3) small = small && inst[id].k <= kSmallTrialOrder;
+      const bool one_wave = (int)ok3.size() <= sms;
+      const PhaseKernel k_search = small ? (one_wave ? k_b_linesearch<true, 1> : k_b_linesearch<true, 2>)
+                                         : (one_wave ? k_b_linesearch<false, 1> : k_b_linesearch<false, 2>);
+      out = phase(k_search, ok3, smem_search(), [&](int id, double* in) {
         const Run& R = runs[id];
         in[kGamma] = R.params.backtracking;
         in[kMinStep] = R.params.minimum_step;

@@ -389,36 +389,130 @@ __device__ double cta_ftb_tree(const double* X, const double* dX, int k, double*
   }
 }
 
+// The same test for orders up to 32, without the updates of the whole triangle: lane r
+// forms row r's entry of a column from the finished columns, one product after the other
+// (per element the operations of warp_trial in their order).  L: a packed slot.
+constexpr int kSmallTrialOrder = 32;
+__device__ bool warp_trial_rows(const double* __restrict__ Xp, const double* __restrict__ dXp, double t, int k,
+                                double ratio, double* __restrict__ L) {
+  const int lane = threadIdx.x & 31;
+  double mn = INFINITY, mx = 0.0;
+  int oc = 0;  // L(i, c) at oc + i
+  for (int c = 0; c < k; ++c) {
+    const int r = max(min(lane, k - 1), c);
+    double a = Xp[oc + r] + t * dXp[oc + r];
+    int o = 0, j = 0;
+    for (; j + 4 <= c; j += 4) {
+      double u[4], v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        u[q] = L[o + r];
+        v[q] = L[o + c];
+        o += k - 1 - (j + q);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a -= u[q] * v[q];
+    }
+    for (; j < c; ++j) {
+      a -= L[o + r] * L[o + c];
+      o += k - 1 - j;
+    }
+    const double d = __shfl_sync(0xffffffffu, a, c);
+    if (!(d > 0.0)) return false;
+    double l, inv;
+    if (d > 0x1p-830 && d < 0x1p830) {
+      tile64::sqrt_rcp(d, l, inv);
+    } else {
+      l = sqrt(d);
+      inv = 1.0 / l;
+    }
+    mn = fmin(mn, l);
+    mx = fmax(mx, l);
+    if (lane >= c && lane < k) L[oc + lane] = lane == c ? l : a * inv;
+    __syncwarp();
+    oc += k - 1 - c;
+  }
+  if (!(ratio > 0.0)) return true;
+  return isfinite(mn) && isfinite(mx) && mx > 0.0 && mn > ratio * mx;
+}
+
 // Backtracking (src/kernels/threaded.jl:1751-1818): the first t of 1, γ, γ², …
 // whose trial X + t·dX passes (Cholesky and, for ratio > 0, the diagonal-ratio
-// margin), or the first t below min_step.  One trial after the other, each by the whole
-// CTA in one tile M: eight at a time, a warp each in packed slots, took 166 KB of
-// shared memory (one CTA an SM) and 5 times as long a trial.  γ ∈ (0, 1) reaches
-// min_step > 0 long before the round guard, which bounds the loop for any other
-// input.
-__device__ double cta_backtrack(const double* X, const double* dX, int k, double gamma, double min_step,
-                                double ratio, double* M, double* inv, int* sfail, double* red) {
-  const int r = threadIdx.x & 63, cb = threadIdx.x >> 6, k8 = (k + 7) & ~7;
-  double x[16], dx[16];
+// margin), or the first t below min_step.  γ ∈ (0, 1) reaches min_step > 0 long before
+// the round guard, which bounds the loop for any other input.
+//
+// Trials one after the other, each by the whole CTA in one tile M, seq of them at most;
+// true when one ended the search, else *t is the next candidate.  ROWS ≥ k: 32 or 64.
+template <int ROWS>
+__device__ __forceinline__ bool cta_trials(const double* X, const double* dX, int k, double gamma, double min_step,
+                                           double ratio, int seq, double* M, double* inv, int* sfail, double* red,
+                                           double* t) {
+  constexpr int STEP = kThreads / ROWS, U = ROWS / STEP;
+  const int r = threadIdx.x % ROWS, cb = threadIdx.x / ROWS, k8 = (k + 7) & ~7;
+  double x[U], dx[U];
 #pragma unroll
-  for (int u = 0; u < 16; ++u) {
-    const int c = cb + 4 * u;
+  for (int u = 0; u < U; ++u) {
+    const int c = cb + STEP * u;
     const bool in = r < k && c < k;
     x[u] = in ? X[r + c * k] : (r == c ? 1.0 : 0.0);
     dx[u] = in ? dX[r + c * k] : 0.0;
   }
-  double t = 1.0;
-  for (int round = 0; round < 4096; ++round) {
+  for (int round = 0; round < seq; ++round) {
     __syncthreads();
     if (r < k8)
 #pragma unroll
-      for (int u = 0; u < 16; ++u)
-        if (cb + 4 * u < k8) M[(cb + 4 * u) * FLD + r] = x[u] + t * dx[u];
+      for (int u = 0; u < U; ++u)
+        if (cb + STEP * u < k8) M[(cb + STEP * u) * FLD + r] = x[u] + *t * dx[u];
     double mn, mx;
     bool ok = cta_tile_chol(M, k, inv, sfail, &mn, &mx, red);
     if (ok && ratio > 0.0) ok = isfinite(mn) && isfinite(mx) && mx > 0 && mn > ratio * mx;
-    if (ok || t < min_step) return t;
-    t *= gamma;
+    if (ok || *t < min_step) return true;
+    *t *= gamma;
+  }
+  return false;
+}
+constexpr int kTrialRounds = 4096;
+
+// Orders above kSmallTrialOrder.  µs of a launch that takes 1, 2, 4 and 22 trials, eight at
+// a time by warp_trial / this: 1 × order 48  154 153 154 441 / 12 19 37 154, 512 × order 48
+// 344 346 344 1003 / 32 49 102 411, 512 × order 64 1199 1200 1198 3543 / 38 63 133 552.
+__device__ double cta_backtrack(const double* X, const double* dX, int k, double gamma, double min_step,
+                                double ratio, double* M, double* inv, int* sfail, double* red) {
+  double t = 1.0;
+  cta_trials<64>(X, dX, k, gamma, min_step, ratio, kTrialRounds, M, inv, sfail, red, &t);
+  return t;
+}
+
+// Smaller orders: two trials like that (none up to order 8), which is as far as most
+// searches go, then eight at a time, a warp each.  µs of a launch that takes 1, 2, 4 and
+// 22 trials, all by the CTA / eight at a time by warp_trial / this:
+//   1 × order 16     9 12 20 67      24 23 23 59      9 12 20 33
+//   512 × order 8    15 22 44 166    20 20 20 44      16 15 15 28
+//   512 × order 16   20 30 61 249    40 38 39 100     14 22 40 73
+//   512 × order 32   26 44 97 413    122 122 120 337  20 30 80 173
+// sm: a tile, or 10 packed slots of k(k+1)/2.
+__device__ double cta_backtrack_small(const double* X, const double* dX, int k, double gamma, double min_step,
+                                      double ratio, double* sm, double* inv, int* sfail, double* red, int* flags) {
+  double t = 1.0;
+  if (cta_trials<32>(X, dX, k, gamma, min_step, ratio, k <= 8 ? 0 : 2, sm, inv, sfail, red, &t)) return t;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, kp = k * (k + 1) / 2;
+  double *Xp = sm, *dXp = sm + kp, *slot = sm + (2 + w) * kp;
+  cta_load_packed(X, dX, k, Xp, dXp);
+  for (int round = 0; round < kTrialRounds / kTrialWarps; ++round) {
+    double cand[kTrialWarps], mine = 0.0;
+#pragma unroll
+    for (int j = 0; j < kTrialWarps; ++j) {
+      cand[j] = j == 0 ? t : cand[j - 1] * gamma;
+      if (j == w) mine = cand[j];
+    }
+    const bool ok = warp_trial_rows(Xp, dXp, mine, k, ratio, slot);
+    if (lane == 0) flags[w] = ok;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kTrialWarps; ++j)
+      if (flags[j] || cand[j] < min_step) return cand[j];
+    t = cand[kTrialWarps - 1] * gamma;
+    __syncthreads();  // the flags are read
   }
   return t;
 }
