@@ -86,3 +86,32 @@ def test_every_cluster_shape_runs():
     import torch
     torch.cuda.init()
     assert load_library()["_ZN4sdpx20step_bound_max_orderEv"]() == 448
+
+
+# A centring direction from a nearly central, feasible iterate: X + dX and Y + dY are inside.
+@pytest.mark.parametrize("ks", [[3], [20, 32], [64], [40, 7], [128], [200], [300, 5], [460]])
+def test_full_step_inside(ks):
+    from sdpx_b200.cuda_backend import CudaBackend
+    from sdpx_b200.problem import ingest
+    rng = np.random.default_rng(len(ks) + ks[0])
+
+    def sym(k):
+        a = rng.standard_normal((k, k))
+        return (a + a.T) / np.linalg.norm(a + a.T, 2)
+    X = [np.eye(k) + 0.1 * sym(k) for k in ks]
+    Y = [np.linalg.inv(x) + 0.05 * sym(len(x)) for x in X]
+    Y = [(y + y.T) / 2 for y in Y]
+    A = [np.array([sym(k) for _ in range(3)]) for k in ks]
+    c = sum(np.einsum("ijk,jk->i", a, y) for a, y in zip(A, Y))
+    with CudaBackend(ingest(c, A, [-x for x in X])) as be:
+        be.set_iterate(np.zeros(3), X, Y)
+        assert be.compute_residuals([1.0] * len(ks), False, True)[2]
+        be.schur_build()
+        assert be.factorize()["ok"]
+        be.predictor_rhs()
+        be.solve_direction()
+        be.direction_blocks()
+        _, dX, dY = be.get_direction()
+        assert _exact(X, dX) == 1.0 and _exact(Y, dY) == 1.0
+        p = be.affine_diagnostics(True)
+        assert p["tX"] == 1.0 and p["tY"] == 1.0
