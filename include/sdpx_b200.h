@@ -89,7 +89,9 @@ int sdpx_b200_block_margins(sdpx_b200_handle* h, double* primal, double* dual);
 
 /* Schur complement S_ij = tr(A_i X⁻¹ A_j Y) from the current block factors
  * (`schur_build!` DenseCons, src/schur.jl:511-562).  identity != 0 uses X = Y = I
- * (KKT cold start, src/solver/interior_point.jl:709-723). */
+ * (KKT cold start, src/solver/interior_point.jl:709-723).  The work is queued: a bounded
+ * wait inside it that gave up is reported by the call that next reads S, factorize or
+ * get_schur. */
 int sdpx_b200_schur_build(sdpx_b200_handle* h, int identity);
 int sdpx_b200_get_schur(sdpx_b200_handle* h, double* S /* m×m, full symmetric */);
 
