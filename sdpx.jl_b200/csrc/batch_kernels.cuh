@@ -7,8 +7,9 @@
 // the Schur panel P̂_j = L_X⁻¹A_jL_Y and S = P̂P̂ᵀ, the Schur Cholesky with
 // the reference's regularisation retries, the right-hand sides, the direction
 // blocks, the fraction-to-boundary bisection, refinement residuals, the
-// backtracking line search with its Cholesky margin and the update.  The
-// step-length trials run eight at a time, one warp each.
+// backtracking line search with its Cholesky margin and the update.  Step-length
+// trials run eight at a time, one warp each, in the bisection and in long searches of
+// orders up to 32, else one after the other by the whole CTA.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -41,7 +42,7 @@ struct Pool {
   double *X, *Y, *P, *R, *LX, *LY, *W, *dX, *dY, *Z, *Xb, *Yb;
   double *x, *dx, *d, *r, *rho, *xb, *dxb;
   double *S, *LS;
-  long long kq;  // stride of one k×k matrix slot in shared memory (kmax² of the pool)
+  long long kq;  // stride of one k×k matrix slot in shared memory (a padded tile64 tile of order kmax)
   long long kp;  // stride of one packed lower-triangle slot (kmax(kmax+1)/2)
   // Float64x2 mode: low halves of the double-double arrays (hi halves are the
   // FP64 arrays above), X⁻¹ in double-double and the low half of the panel.

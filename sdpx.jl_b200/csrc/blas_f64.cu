@@ -248,10 +248,10 @@ void trmm_right_lower_inplace_f64(const Opnd& T, const Opnd& L, const OutDesc& C
 // `rate` when the others hide it (a step of the 64-tile is 1088 cycles of DMMA issue);
 // `fixed` is a unit's prologue and store.  The partial tiles are written and read again.
 // One CTA of 128×128 an SM left nothing to hide a step's copies and barriers behind:
-// it measured no faster than one of these at any size, at most 28 TFLOP/s.  µs with the
-// reduction, 128 / 64 / 32 (K chunks from this model): 3000×26400 8677 / 7549 / 8569
-// (31.5 TFLOP/s), 1000×30150 1270 / 1085 / 1179, 1500×9000 830 / 764 / 757, 700×4000
-// 103 / 89 / 91, 317×2408 35 / 22 / 21, 61×333 39 / 23 / 13, 5×333 39 / 21 / 11.
+// it measured no faster than one of these at any size, at most 28 TFLOP/s.  µs of both
+// launches, 64 / 32 (K chunks from this model): 3000×26400 7790 / 8290 (30.5 TFLOP/s),
+// 1000×30150 1130 / 1220, 1500×9000 795 / 748, 700×4000 98 / 92, 317×2408 25 / 24, 61×333
+// 26 / 16, 5×333 25 / 14.
 struct SyrkTile {
   int bm, resident;
   double latency, rate, fixed;

@@ -506,7 +506,8 @@ size_t potrf_flow_flag_words(int nmat, int nmax) {
 // One CTA per SM fits (104 KB of shared memory, 168 registers); a group is as large
 // as the tasks of the largest matrix can use.  Measured on the B200, one matrix, ms
 // (before: panels in shared memory below 459, one cooperative launch with grid
-// barriers above; the factors are identical bit for bit):
+// barriers above; the factors are identical bit for bit, but for a column whose pivot
+// is the one exception of sqrt_rcp):
 //   n       64     128    320    512    1030   2000   3000
 //   before  0.039  0.087  0.252  0.434  0.989  1.848  3.084
 //   now     0.022  0.044  0.102  0.164  0.352  0.657  1.004
