@@ -49,11 +49,10 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-// Barrier of the computing threads that also returns whether ok held in all.  (It takes
-// whole warps, and one thread may come from poll_flags.)
+// Barrier of the computing threads that also returns whether ok held in all.  (All of them
+// execute it whatever thread 0 did before, as with __syncthreads.)
 __device__ __forceinline__ bool compute_and(int ok) {
   int r;
-  __syncwarp();
   asm volatile(
       "{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbar.red.and.pred q, %2, %3, p;\nselp.s32 %0, 1, 0, q;\n}"
       : "=r"(r)
@@ -65,13 +64,15 @@ __device__ __forceinline__ void compute_sync() { bar_sync(kBarCompute, FT); }
 
 // Flag words of one matrix of nt tile rows: ready[i·nt + j] (tile final),
 // c1[j] (tile (j+1,j) updated by the panels before j), c2[j] (tile (j,j) updated
-// by the panels before j−1), then the failure and the timeout.
+// by the panels before j−1), then the failure and the timeout.  Epoch 0, which no launch
+// has: the matrix has one CTA and no flags.
 struct Flags {
   unsigned *ready, *c1, *c2, *stop;
   unsigned epoch;  // the value that marks
   int nt;
   __device__ Flags(unsigned* base, int n, unsigned ep)
       : ready(base), c1(base + n * n), c2(c1 + n), stop(c2 + n), epoch(ep), nt(n) {}
+  __device__ bool alone() const { return epoch == 0; }
   __device__ unsigned* tile(int i, int j) const { return ready + i * nt + j; }
   __device__ bool set(const unsigned* f) const { return ld_acquire(f) == epoch; }
   __device__ void mark(unsigned* f) const { st_release(f, epoch); }
@@ -192,7 +193,7 @@ struct TileRegs {
 // x ← the strip of tile (i, q) updated by panels 0 … np−1 (q ≤ i).  The next
 // panel's tiles are loaded while this panel's products run, when they are there.  alone:
 // they are, the CTA's own barriers order them.
-__device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<double>& M, const Flags& F, bool alone,
+__device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<double>& M, const Flags& F,
                                             int i, int q, int np, double* La, double* Lb) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, t = lane & 3;
   const int h = min(FB, M.n - i * FB), hq = min(FB, M.n - q * FB);
@@ -206,6 +207,7 @@ __device__ __forceinline__ bool update_tile(double (&x)[8][2], const MatDesc<dou
       x[f][e] = (r < h && c < hq) ? __ldcg(p0 + (size_t)c * M.ld) : 0.0;
     }
   TileRegs ra, rb;
+  const bool alone = F.alone();
   bool loaded = false;
   for (int p = 0; p < np; ++p) {
     if (!loaded) {
@@ -249,17 +251,17 @@ __host__ __device__ inline int flow_tasks(int nt, int j) {
 
 // (M and F by value: by reference they would live in local memory and be read again
 // after every store.)
-__device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, bool alone, int j, int u, double* La,
+__device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, int j, int u, double* La,
                                       double* Lb, double* inv) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const bool partial = j > 0 && u < 2;
   const int i = partial ? j + 1 : j + 2 + u - (j > 0 ? 2 : 0), q = partial && u == 0 ? j + 1 : j;
   const int h = min(FB, M.n - i * FB), w = min(FB, M.n - q * FB);
   double x[8][2];
-  if (!update_tile(x, M, F, alone, i, q, j, La, Lb)) return false;
+  if (!update_tile(x, M, F, i, q, j, La, Lb)) return false;
   if (!partial) {
     int ok = 1;
-    if (!alone && threadIdx.x == 0) ok = poll_flags(F, F.tile(j, j), F.tile(j, j));
+    if (!F.alone() && threadIdx.x == 0) ok = poll_flags(F, F.tile(j, j), F.tile(j, j));
     if (!compute_and(ok)) return false;  // (also: La and Lb are free)
     load_tile<FT>(La, M, j * FB, j * FB, FB, FB, threadIdx.x);
   } else {
@@ -277,9 +279,9 @@ __device__ __noinline__ bool run_task(const MatDesc<double> M, const Flags F, bo
     compute_sync();
   }
   store_tile<FT>(Lb, M, i * FB, q * FB, h, w, i == q, threadIdx.x);
-  if (!alone) __threadfence();
+  if (!F.alone()) __threadfence();
   compute_sync();
-  if (!alone && threadIdx.x == 0) F.mark(!partial ? F.tile(i, j) : u == 0 ? F.c2 + i : F.c1 + j);
+  if (!F.alone() && threadIdx.x == 0) F.mark(!partial ? F.tile(i, j) : u == 0 ? F.c2 + i : F.c1 + j);
   return true;
 }
 
@@ -307,7 +309,6 @@ __device__ __forceinline__ void chain_compute(const MatDesc<double> M, const Fla
       const int r = 8 * (nb - 1) + g;
       if (wp < 8 && r >= w)
         for (int c = 2 * t + (wp & 1) + 8 * (wp >> 1); c < FB; c += 32) D[c * FLD + r] = r == c ? 1.0 : 0.0;
-      __syncwarp();
       compute_sync();
     }
     factor_tile(D, cs.inv, nb, &cs.fail);
@@ -327,7 +328,7 @@ __device__ __forceinline__ void chain_compute(const MatDesc<double> M, const Fla
     if (j == nt - 1) break;
     if (alone) {
       bar_sync(kBarStored, FT + FIO);  // tile (j,j) is in global memory
-      for (int u = 0; u < flow_tasks(nt, j); ++u) run_task(M, F, true, j, u, X, Y, cs.tinv);
+      for (int u = 0; u < flow_tasks(nt, j); ++u) run_task(M, F, j, u, X, Y, cs.tinv);
       bar_arrive(kBarTasks, FT + FIO);
     }
     bar_sync(kBarLoaded, FT + FIO);
@@ -367,7 +368,6 @@ __device__ __forceinline__ void chain_io(const MatDesc<double> M, const Flags F,
     __threadfence();
     bar_sync(kBarIo, FIO);
     if (tid == 0) F.mark(f);
-    __syncwarp();
   };
   if (nt > 1 && !alone) fetch(0);
   for (int j = 0; j < nt; ++j) {
@@ -392,7 +392,6 @@ __device__ __forceinline__ void chain_io(const MatDesc<double> M, const Flags F,
     bar_sync(kBarUpdated, FT + FIO);  // X and tile (j,j)'s buffer are free
     if (j + 2 < nt && !alone) {
       if (tid == 0 && !poll_flags(F, F.c1 + j + 1, F.c2 + j + 2)) cs.err = 1;
-      __syncwarp();
       bar_sync(kBarIo, FIO);
       if (cs.err) {
         bar_sync(kBarFactored, FT + FIO);
@@ -428,7 +427,7 @@ __global__ void __launch_bounds__(FT + FIO, 1)
   for (int b = grp; b < nmat; b += ngroups) {
     const MatDesc<double> M = nmat <= kFlowInline ? few.m[b] : mats[b];
     const int nt = (M.n + FB - 1) / FB;
-    const Flags F(flags + (size_t)b * words, nt, epoch);
+    const Flags F(flags + (size_t)b * words, nt, gsize == 1 ? 0u : epoch);
     __syncthreads();
     if (me == 0) {
       if (threadIdx.x == 0) cs.fail = kNoFail, cs.err = 0;
@@ -442,7 +441,7 @@ __global__ void __launch_bounds__(FT + FIO, 1)
       for (int j = 0; ok && j < nt; ++j) {
         const int n = flow_tasks(nt, j);
         while (ok && first < n) {
-          ok = run_task(M, F, false, j, first, T0, T1, cs.tinv);
+          ok = run_task(M, F, j, first, T0, T1, cs.tinv);
           first += gsize - 1;
         }
         first -= n;
