@@ -550,21 +550,54 @@ struct Handle {
     dmax.assign(n, 0.0);
     if (n == 0) return;
     ensure_descs(n);
+    constexpr int kOneTile = 64;
     int nmax = 0;
-    for (auto& q : mats) nmax = std::max(nmax, q.n);
+    size_t large = 0;
+    for (auto& q : mats) {
+      nmax = std::max(nmax, q.n);
+      large += q.n > kOneTile;
+    }
     // Pinned layout: [descriptors | dmin (n) | dmax (n) | info (n)], the last
     // three written by the kernel.
     const size_t dbytes = (n * sizeof(MatDesc<double>) + 15) / 16 * 16;
     unsigned char* hp = pinned(dbytes + 2 * n * sizeof(double) + n * sizeof(int));
     MatDesc<double>* hm = reinterpret_cast<MatDesc<double>*>(hp);
-    std::copy(mats.begin(), mats.end(), hm);
     double* hs = reinterpret_cast<double*>(hp + dbytes);
     int* hi = reinterpret_cast<int*>(hs + 2 * n);
-    potrf_flow(hm, d_descs.p, (int)n, nmax, hi, hs, hs + n, flow_flags, sms, st, zero_upper);
-    sync();
-    std::copy(hs, hs + n, dmin.begin());
-    std::copy(hs + n, hs + 2 * n, dmax.begin());
-    std::copy(hi, hi + n, info.begin());
+    // Matrices of one tile go into a launch of their own (20 µs) where they take CTAs that the
+    // larger ones can use: these have at most one for two tile rows, and would have twice
+    // as many.  Bisections of 4 × 15 trials, all in one launch → apart: blocks 460 + 10 9.0 →
+    // 3.9 ms, 200 + 10 2.1 → 1.7; where a tile row has a CTA more of them gain less than the
+    // launch (8 trials of 300 + 20, four CTAs each: 0.34 → 0.35).
+    const int group = potrf_flow_group((int)n, nmax, sms);
+    const bool apart = large > 0 && large < n && 2 * group <= ceil_div(nmax, kOneTile) &&
+                       potrf_flow_group((int)large, nmax, sms) >= 2 * group;
+    if (!apart) {
+      std::copy(mats.begin(), mats.end(), hm);
+      potrf_flow(hm, d_descs.p, (int)n, nmax, hi, hs, hs + n, flow_flags, sms, st, zero_upper);
+      sync();
+      std::copy(hs, hs + n, dmin.begin());
+      std::copy(hs + n, hs + 2 * n, dmax.begin());
+      std::copy(hi, hi + n, info.begin());
+    } else {
+      std::vector<size_t> at(n);  // a matrix's place in the pinned lists, the large ones first
+      size_t first = 0, next = large;
+      int small_max = 0;
+      for (size_t q = 0; q < n; ++q) {
+        at[q] = mats[q].n > kOneTile ? first++ : next++;
+        hm[at[q]] = mats[q];
+        if (mats[q].n <= kOneTile) small_max = std::max(small_max, mats[q].n);
+      }
+      potrf_flow(hm, d_descs.p, (int)large, nmax, hi, hs, hs + n, flow_flags, sms, st, zero_upper);
+      potrf_flow(hm + large, d_descs.p + large, (int)(n - large), small_max, hi + large, hs + large, hs + n + large,
+                 flow_flags, sms, st, zero_upper);
+      sync();
+      for (size_t q = 0; q < n; ++q) {
+        dmin[q] = hs[at[q]];
+        dmax[q] = hs[n + at[q]];
+        info[q] = hi[at[q]];
+      }
+    }
     for (int v : info)
       if (v < 0) throw CudaError("Cholesky: a wait for a tile gave up");
   }

@@ -33,6 +33,9 @@ struct FlowFlags {
   }
 };
 
+// CTAs that potrf_flow gives each of nmat matrices, the largest of order nmax.
+int potrf_flow_group(int nmat, int nmax, int sms);
+
 // Lower Cholesky in place of nmat matrices (host array `mats`, largest order nmax), one
 // launch (potrf_flow.cu): a CTA per matrix runs the pivot chain, sms/nmat − 1 others its
 // remaining tiles, ordered by tile flags.  info[b] = 0 on success, else the 1-based index

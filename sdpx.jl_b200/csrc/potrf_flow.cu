@@ -502,6 +502,13 @@ size_t potrf_flow_flag_words(int nmat, int nmax) {
   return (size_t)nmat * (nt * nt + 2 * nt + 2);
 }
 
+int potrf_flow_group(int nmat, int nmax, int sms) {
+  const int nt = ceil_div(nmax, FB);
+  int tasks = 0;
+  for (int j = 0; j < nt; ++j) tasks += flow_tasks(nt, j);
+  return std::max(1, std::min(sms / nmat, 1 + tasks));
+}
+
 // One CTA per SM fits (104 KB of shared memory, 168 registers); a group is as large
 // as the tasks of the largest matrix can use.  Measured on the B200, one matrix, ms
 // (before: panels in shared memory below 459, one cooperative launch with grid
@@ -518,9 +525,7 @@ void potrf_flow(const MatDesc<double>* mats, MatDesc<double>* d_mats, int nmat, 
   if (nmat <= 0 || nmax <= 0) return;
   ensure_smem(k_potrf_flow, kFlowSmem);
   const int nt = ceil_div(nmax, FB);
-  int words = nt * nt + 2 * nt + 2, tasks = 0;
-  for (int j = 0; j < nt; ++j) tasks += flow_tasks(nt, j);
-  int gsize = std::max(1, std::min(sms / nmat, 1 + tasks));
+  int words = nt * nt + 2 * nt + 2, gsize = potrf_flow_group(nmat, nmax, sms);
   int ngroups = std::min(nmat, sms / gsize), zu = zero_upper ? 1 : 0;
   FlowMats few{};
   if (nmat <= kFlowInline) std::copy(mats, mats + nmat, few.m);
