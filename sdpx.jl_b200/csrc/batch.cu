@@ -1112,7 +1112,8 @@ WorkKernel syrk_kernel(int threads, int tile) {
 // Host side.
 
 // Blocks of at most kKeep bytes come from and go back to the pinned cache (grown and
-// released with no work of the stream in flight on them); the upload staging does not.
+// released with no work of the stream in flight on them; drop() after a failed stream);
+// the upload staging does not.
 struct Pinned {
   static constexpr size_t kKeep = 4 << 20;
   void* p = nullptr;
@@ -1130,6 +1131,11 @@ struct Pinned {
   void release() {
     if (p && bytes <= kKeep) hcache::put(p, bytes);
     else if (p) cudaFreeHost(p);
+    p = nullptr;
+    bytes = 0;
+  }
+  void drop() {  // back to the driver
+    if (p) cudaFreeHost(p);
     p = nullptr;
     bytes = 0;
   }
@@ -1204,7 +1210,8 @@ struct Engine {
   bool solved = false;
 
   ~Engine() {
-    if (st) cudaStreamSynchronize(st);
+    if (st && cudaStreamSynchronize(st) != cudaSuccess)
+      for (Pinned* b : {&h_act, &h_par, &h_res, &h_work, &h_cert, &h_stage[0], &h_stage[1]}) b->drop();
     release_scope.begin();
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
