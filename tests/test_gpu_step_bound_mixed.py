@@ -115,3 +115,35 @@ def test_full_step_inside(ks):
         assert _exact(X, dX) == 1.0 and _exact(Y, dY) == 1.0
         p = be.affine_diagnostics(True)
         assert p["tX"] == 1.0 and p["tY"] == 1.0
+
+
+# Late iterates: κ(X) = κ(Y) far above the 100 of the other tests.  A Cholesky test decides on
+# M + t·dM up to k·eps·‖M‖, that is up to k·eps·κ(M) of the smallest eigenvalue, and the
+# eigenvalue bound is formed with errors of the same size (κ enters once: W and Wᵀ bring its
+# square root each); the direction's own scale adds the 1e3 of the tests above.
+@pytest.mark.parametrize("ks", [[12], [61, 17], [130], [300, 40]])
+@pytest.mark.parametrize("kappa", [1e6, 1e9])
+def test_ill_conditioned_iterates_match_the_bisection(ks, kappa):
+    from sdpx_b200.cuda_backend import CudaBackend
+    from sdpx_b200.problem import ingest
+    rng = np.random.default_rng(sum(ks))
+    half = np.log10(kappa) / 2
+
+    def spd(k, sign):
+        q, _ = np.linalg.qr(rng.standard_normal((k, k)))
+        x = (q * np.logspace(-sign * half, sign * half, k)) @ q.T
+        return 0.5 * (x + x.T)
+    A = [rng.standard_normal((3, k, k)) for k in ks]
+    A = [a + a.transpose(0, 2, 1) for a in A]
+    X, Y = [spd(k, 1) for k in ks], [spd(k, -1) for k in ks]
+    with CudaBackend(ingest(rng.standard_normal(3), A, [np.eye(k) for k in ks])) as be:
+        be.set_iterate(np.zeros(3), X, Y)
+        assert be.compute_residuals([0.0] * len(ks), True, True)[2]
+        be.schur_build()
+        assert be.factorize()["ok"]
+        be.predictor_rhs()
+        be.solve_direction()
+        be.direction_blocks()
+        p = be.affine_diagnostics(True)
+        for key, t in zip(("tX", "tY"), be.line_search("fraction_to_boundary", 1.0, 1.0, 0.9, 1e-300, 0.0)):
+            assert abs(p[key] - t) <= 8 * max(ks) * EPS * kappa * 1e3 * t
